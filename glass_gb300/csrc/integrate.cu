@@ -32,22 +32,15 @@
 #include "autotune.cuh"
 #include "sampling.cuh"
 #include "stack.cuh"
+#include "warp_band.cuh"
 
 namespace gg {
-
-// Fused warp (integrate_matrix_warped_*): a frame's samples come from its
-// source pixels through the inverse of its matrix instead of from the stack.
-struct FusedFrame {
-  float m[9][2];  // inverse, float-float
-  int affine;
-  unsigned src_nonfinite;  // non-finite source pixels of the frame
-  int pad[2];
-};
 
 struct IntegrateArgs {
   const float* slots;
   const int* slot_of_frame;
   int64_t stride;
+  const float* const* base;  // optional first sample of every frame (else its slot's)
   int64_t pixels;
   int frames;
   const float* weights;  // device [frames], raw values
@@ -458,7 +451,7 @@ __device__ __forceinline__ void load_frame_table(const IntegrateArgs& a, FrameTa
   for (int f = threadIdx.x; f < a.frames; f += blockDim.x) {
     const float w = a.weights ? a.weights[f] : 1.0f;
     t.w[f] = (isfinite(w) && w > 0.0f) ? w : 0.0f;
-    t.base[f] = a.slots + static_cast<int64_t>(a.slot_of_frame[f]) * a.stride;
+    t.base[f] = a.base ? a.base[f] : a.slots + static_cast<int64_t>(a.slot_of_frame[f]) * a.stride;
   }
   if (threadIdx.x < 32) {
     unsigned bad = 0, invalid_w = 0, non_unit = 0, active = 0;
@@ -1535,45 +1528,48 @@ static void validate_integrate(const gg_integrate_params_t& p) {
 
 static IntegrateArgs integrate_args(gg_stack* s, const float* d_weights, const gg_integrate_params_t& p);
 
-void launch_integrate(gg_stack* s, const float* d_weights, const gg_integrate_params_t& p) {
-  const IntegrateArgs a = integrate_args(s, d_weights, p);
+static void launch_integrate_args(const IntegrateArgs& a, cudaStream_t stream) {
   const int n = a.frames;
   if (n <= 32) {
-    switch (p.rejection) {
+    switch (a.rejection) {
       case GG_REJECT_NONE:
-        n <= 8 ? launch_col<8, GG_REJECT_NONE>(a, s->stream)
-               : n <= 16 ? launch_col<16, GG_REJECT_NONE>(a, s->stream) : launch_col<32, GG_REJECT_NONE>(a, s->stream);
+        n <= 8 ? launch_col<8, GG_REJECT_NONE>(a, stream)
+               : n <= 16 ? launch_col<16, GG_REJECT_NONE>(a, stream) : launch_col<32, GG_REJECT_NONE>(a, stream);
         break;
       case GG_REJECT_SIGMA_CLIP:
-        n <= 8 ? launch_col<8, GG_REJECT_SIGMA_CLIP>(a, s->stream)
-               : n <= 16 ? launch_col<16, GG_REJECT_SIGMA_CLIP>(a, s->stream)
-                         : launch_col<32, GG_REJECT_SIGMA_CLIP>(a, s->stream);
+        n <= 8 ? launch_col<8, GG_REJECT_SIGMA_CLIP>(a, stream)
+               : n <= 16 ? launch_col<16, GG_REJECT_SIGMA_CLIP>(a, stream)
+                         : launch_col<32, GG_REJECT_SIGMA_CLIP>(a, stream);
         break;
       case GG_REJECT_WINSORIZED:
-        n <= 8 ? launch_col<8, GG_REJECT_WINSORIZED>(a, s->stream)
-               : n <= 16 ? launch_col<16, GG_REJECT_WINSORIZED>(a, s->stream)
-                         : launch_col<32, GG_REJECT_WINSORIZED>(a, s->stream);
+        n <= 8 ? launch_col<8, GG_REJECT_WINSORIZED>(a, stream)
+               : n <= 16 ? launch_col<16, GG_REJECT_WINSORIZED>(a, stream)
+                         : launch_col<32, GG_REJECT_WINSORIZED>(a, stream);
         break;
       default:
-        n <= 8 ? launch_col<8, GG_REJECT_LINEAR_FIT>(a, s->stream)
-               : n <= 16 ? launch_col<16, GG_REJECT_LINEAR_FIT>(a, s->stream)
-                         : launch_col<32, GG_REJECT_LINEAR_FIT>(a, s->stream);
+        n <= 8 ? launch_col<8, GG_REJECT_LINEAR_FIT>(a, stream)
+               : n <= 16 ? launch_col<16, GG_REJECT_LINEAR_FIT>(a, stream)
+                         : launch_col<32, GG_REJECT_LINEAR_FIT>(a, stream);
         break;
     }
   }
-  else if (p.rejection != GG_REJECT_LINEAR_FIT && n <= 512) {
+  else if (a.rejection != GG_REJECT_LINEAR_FIT && n <= 512) {
     // one warp per pixel (the linear fit's serial rank walks stay below)
     // two pixels per warp up to 256 frames (16 lanes x NPL values each)
-    if (n <= 64) launch_warp<4, 0, 16>(a, s->stream);
-    else if (n <= 128) launch_warp<8, 0, 16>(a, s->stream);
-    else if (n <= 256) launch_warp<16, 0, 16>(a, s->stream);
-    else launch_warp<16>(a, s->stream);
+    if (n <= 64) launch_warp<4, 0, 16>(a, stream);
+    else if (n <= 128) launch_warp<8, 0, 16>(a, stream);
+    else if (n <= 256) launch_warp<16, 0, 16>(a, stream);
+    else launch_warp<16>(a, stream);
   }
-  else if (n <= 64) launch_reg<64>(a, s->stream);
-  else if (n <= 128) launch_smem<4>(a, s->stream);
-  else if (n <= 256) launch_smem<8>(a, s->stream);
-  else if (n <= 512) launch_smem<16>(a, s->stream);
+  else if (n <= 64) launch_reg<64>(a, stream);
+  else if (n <= 128) launch_smem<4>(a, stream);
+  else if (n <= 256) launch_smem<8>(a, stream);
+  else if (n <= 512) launch_smem<16>(a, stream);
   else fail(GG_ERR_INVALID_ARGUMENT, "frame_count above 512 is not supported by the resident integrator");
+}
+
+void launch_integrate(gg_stack* s, const float* d_weights, const gg_integrate_params_t& p) {
+  launch_integrate_args(integrate_args(s, d_weights, p), s->stream);
   s->last_count_dtype = p.count_dtype;
 }
 
@@ -1768,9 +1764,70 @@ static void ensure_fused_buffers(gg_stack* s) {
     check_cuda(cudaMalloc(&s->d_fused_frames, sizeof(FusedFrame) * n), "cudaMalloc(fused frames)");
     check_cuda(cudaMalloc(&s->d_fused_counts, sizeof(unsigned) * n), "cudaMalloc(fused counts)");
     check_cuda(cudaMalloc(&s->d_fused_geometric, sizeof(float) * s->pixels), "cudaMalloc(fused coverage)");
-    s->bytes_allocated += static_cast<int64_t>(sizeof(FusedFrame) + sizeof(unsigned)) * n + 4 * s->pixels;
+    // descriptors of the band warp, then the frames' band base pointers
+    const size_t items = warp_item_bytes() * n;
+    check_cuda(cudaMalloc(&s->d_band_items, items + sizeof(float*) * n), "cudaMalloc(fused band items)");
+    s->bytes_allocated += static_cast<int64_t>(sizeof(FusedFrame) + sizeof(unsigned)) * n + 4 * s->pixels +
+                          static_cast<int64_t>(items + sizeof(float*) * n);
+  }
+  if (warp_band_layout(s).rows == 0 && !s->d_band_own) {
+    // frames so wide that the spare slots hold less than a row of each
+    const int64_t row = (s->width + 63) / 64 * 64;
+    check_cuda(cudaMalloc(reinterpret_cast<void**>(&s->d_band_own), sizeof(float) * row * n),
+               "cudaMalloc(fused band rows)");
+    s->bytes_allocated += 4 * row * n;
   }
 }
+
+// Fused warp + integration in bands of rows: every frame is warped into its
+// band buffer (the tiled warp of warp.cu), then the resident integrator runs
+// over the band.  The tiled warp samples from shared memory and plans whole
+// tiles, which the column kernel's per-pixel sampling through L1 cannot: for
+// 32 x 2048 x 2048, Lanczos3, winsorized, 2.0 ms (warp 1.25, integration 0.77)
+// against 6.5 ms (a 1.0 ms pass that counted the invalid samples, 5.5 ms).
+static void launch_band_sequence(gg_stack* s, const FusedFrame* d_frames, int interp, float clamp,
+                                 const float* d_weights, const gg_integrate_params_t& p) {
+  BandLayout band = warp_band_layout(s);
+  float* own = nullptr;
+  if (band.rows == 0) {
+    own = s->d_band_own;
+    band.capacity = (s->width + 63) / 64 * 64;
+    band.rows = 1;
+  }
+  auto** base = reinterpret_cast<const float**>(static_cast<char*>(s->d_band_items) +
+                                                warp_item_bytes() * static_cast<size_t>(s->frames));
+  launch_warp_band_prepare(s, s->d_band_items, d_frames, interp, clamp, band, own, base, s->d_fused_counts);
+  IntegrateArgs a = integrate_args(s, d_weights, p);
+  a.nonfinite = s->d_fused_counts;
+  a.base = base;
+  const size_t count_bytes = a.count_u16 ? 2 : 4;
+  for (int row0 = 0; row0 < s->height; row0 += band.rows) {
+    const int row1 = static_cast<int>(std::min<int64_t>(s->height, row0 + band.rows));
+    const int64_t p0 = static_cast<int64_t>(row0) * s->width;
+    launch_warp_band(s, s->d_band_items, interp, clamp, row0, row1, s->d_fused_counts, s->d_fused_geometric);
+    IntegrateArgs b = a;
+    b.pixels = static_cast<int64_t>(row1 - row0) * s->width;
+    b.master += p0;
+    b.weight += p0;
+    b.coverage = static_cast<char*>(b.coverage) + p0 * count_bytes;
+    b.low = static_cast<char*>(b.low) + p0 * count_bytes;
+    b.high = static_cast<char*>(b.high) + p0 * count_bytes;
+    if (b.dq) b.dq += p0;
+    b.geometric = s->d_fused_geometric + p0;
+    launch_integrate_args(b, s->stream);
+  }
+  s->last_count_dtype = p.count_dtype;
+  s->has_fused_geometric = true;
+}
+
+// Up to 32 frames and this many samples the column kernel samples the frames
+// itself: three launches, where a band takes four or five.  Measured, column
+// against band, microseconds per call: Lanczos3 8 x 128^2 37 / 59, 8 x 256^2
+// 56 / 58, 16 x 256^2 81 / 83, 32 x 256^2 130 / 130, 8 x 512^2 124 / 87,
+// 32 x 512^2 371 / 250; bilinear 8 x 256^2 38 / 52, 8 x 512^2 75 / 69,
+// 16 x 512^2 107 / 107, 32 x 512^2 169 / 198, 32 x 1024^2 699 / 511.
+constexpr int64_t kFusedColumnSamplesLanczos = int64_t(1) << 20;
+constexpr int64_t kFusedColumnSamplesBilinear = int64_t(1) << 22;
 
 // The device part of the fused warp-integration: every argument already on
 // the device, nothing but kernel launches on the stack's stream (so it can
@@ -1778,6 +1835,11 @@ static void ensure_fused_buffers(gg_stack* s) {
 static void launch_fused_sequence(gg_stack* s, FusedFrame* d_frames, int interp, float clamp, const float* d_weights,
                                   const gg_integrate_params_t& p) {
   const int n = static_cast<int>(s->frames);
+  if (n > 32 || s->pixels * n > (interp == GG_INTERP_LANCZOS3 ? kFusedColumnSamplesLanczos
+                                                                 : kFusedColumnSamplesBilinear)) {
+    launch_band_sequence(s, d_frames, interp, clamp, d_weights, p);
+    return;
+  }
   note_launch();
   fused_prepare_kernel<<<(n + 127) / 128, 128, 0, s->stream>>>(d_frames, s->d_frame_nonfinite, s->d_fused_counts, n);
   check_cuda(cudaGetLastError(), "fused_prepare launch");
@@ -1817,17 +1879,7 @@ static void launch_fused_sequence(gg_stack* s, FusedFrame* d_frames, int interp,
   else
     fused_nonfinite_kernel<GG_INTERP_LANCZOS3><<<count_grid, 256, 0, s->stream>>>(a, s->d_fused_counts);
   check_cuda(cudaGetLastError(), "fused_nonfinite launch");
-  if (n > 32) {  // one warp per pixel over a sampled [frame][32 px] tile
-    auto run = [&](auto tag) {
-      constexpr int I = decltype(tag)::value;
-      if (n <= 64) launch_warp<2, I>(a, s->stream);
-      else if (n <= 128) launch_warp<4, I>(a, s->stream);
-      else if (n <= 256) launch_warp<8, I>(a, s->stream);
-      else launch_warp<16, I>(a, s->stream);
-    };
-    if (interp == GG_INTERP_BILINEAR) run(std::integral_constant<int, GG_INTERP_BILINEAR>{});
-    else run(std::integral_constant<int, GG_INTERP_LANCZOS3>{});
-  } else if (interp == GG_INTERP_BILINEAR) {
+  if (interp == GG_INTERP_BILINEAR) {
     if (p.rejection == GG_REJECT_NONE) launch_fused<GG_REJECT_NONE, GG_INTERP_BILINEAR>(a, s->stream);
     else if (p.rejection == GG_REJECT_SIGMA_CLIP) launch_fused<GG_REJECT_SIGMA_CLIP, GG_INTERP_BILINEAR>(a, s->stream);
     else launch_fused<GG_REJECT_WINSORIZED, GG_INTERP_BILINEAR>(a, s->stream);

@@ -206,7 +206,7 @@ static void stack_free(gg_stack* s) {
                       s->d_dq,       s->d_warp_coverage, s->d_weights,    s->d_partials,
                       s->d_raw_lane[0], s->d_raw_lane[1], s->d_warp_items, s->d_error,
                       s->d_cat_xy,   s->d_cat_n,         s->d_fused_frames, s->d_fused_counts,
-                      s->d_fused_geometric};
+                      s->d_fused_geometric, s->d_band_items, s->d_band_own};
   for (void* p : dev_ptrs) {
     if (p) cudaFree(p);
   }

@@ -116,6 +116,8 @@ struct gg_stack {
   unsigned* d_fused_counts = nullptr;
   float* d_fused_geometric = nullptr;
   bool has_fused_geometric = false;
+  void* d_band_items = nullptr;  // band warp descriptors and base pointers
+  float* d_band_own = nullptr;   // band rows, where the spare slots hold none
 
   // Per-frame registration catalogs: the brightest kCatalogPoints star
   // centroids of each frame's last detection (x, y float64) and their count.

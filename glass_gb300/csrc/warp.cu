@@ -27,6 +27,7 @@
 //   - Lanczos3 weights are paired even/odd polynomials in (t - 1/2)^2
 //     (sampling.cuh); interior tiles of finite frames run a straight-line
 //     form without per-pixel tests.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -35,6 +36,7 @@
 
 #include "sampling.cuh"
 #include "stack.cuh"
+#include "warp_band.cuh"
 
 namespace gg {
 
@@ -51,29 +53,28 @@ constexpr int kFreshRows = 4;
 struct WarpItem {
   int frame;
   int src_slot;     // filled on the device
-  int dst_slot;     // filled on the device
+  int dst_slot;     // filled on the device (-1: not a slot)
   unsigned src_nonfinite;
   int affine;
   int int_shift;  // inverse is an exact integer translation
-  int pad[2];
+  float* dst;     // first row of the output rows (filled on the device)
   float m[9][2];  // inverse matrix, float-float (hi, lo), row-major
 };
 
 struct WarpArgs {
   float* slots;
-  int* slot_of_frame;
-  int* spare_slot;
-  unsigned* nonfinite;
+  unsigned* nonfinite;  // per frame: non-finite output samples are added
   WarpItem* items;
   int item_count;
   int64_t stride;
   int width;
   int height;
+  int row0, row1;  // output rows [row0, row1); row0 is the first row at WarpItem::dst
   int tiles_x;
-  int tiles_y;
-  int interp;
+  int tiles_y;     // of those rows
   float fill;
   float clamp;
+  int every_row;  // coordinates of tiles that are not interior afresh for every row
   float* coverage;  // optional accumulator (+1 per covered pixel)
   int* error;
 };
@@ -134,7 +135,8 @@ __device__ __forceinline__ Coef load_coef(const WarpItem* p) {
   return c;
 }
 
-// Tile plan: box origin for the source footprint of output tile (tx, ty).
+// Tile plan: box origin for the source footprint of the output tile whose
+// first pixel is (tile_x0, tile_y0).
 struct TilePlan {
   int bx, by, fits, interior;
 };
@@ -142,9 +144,9 @@ struct TilePlan {
 // interior: an affine map sends the whole tile at least one pixel inside the
 // valid source range (valid_lo <= s <= valid_hi on both axes), so no pixel
 // of the tile needs its own validity test.
-__device__ __forceinline__ TilePlan plan_tile(const Coef& it, int tile_x, int tile_y, int radius, float valid_lo,
+__device__ __forceinline__ TilePlan plan_tile(const Coef& it, int tile_x0, int tile_y0, int radius, float valid_lo,
                                               float valid_hi_x, float valid_hi_y) {
-  const float x0 = static_cast<float>(tile_x * kTileW), y0 = static_cast<float>(tile_y * kTileH);
+  const float x0 = static_cast<float>(tile_x0), y0 = static_cast<float>(tile_y0);
   const float cx[4] = {x0, x0 + kTileW - 1, x0, x0 + kTileW - 1};
   const float cy[4] = {y0, y0, y0 + kTileH - 1, y0 + kTileH - 1};
   float minx = kInfF, maxx = -kInfF, miny = kInfF, maxy = -kInfF;
@@ -174,15 +176,14 @@ __device__ __forceinline__ TilePlan plan_tile(const Coef& it, int tile_x, int ti
   return p;
 }
 
-// The output rows of one thread in a 64 x 48 tile (rows ly, ly + 4, ...).
+// The output pixels of one thread in a 64 x 48 tile: column ox, rows oy0,
+// oy0 + 4, ...; dst is the frame's output row 0.
 // FINITE: the source frame holds no non-finite sample (every Lanczos3 window
 // takes the plain normalised sum); returns the count of non-finite outputs.
 template <int INTERP, bool FINITE>
 __device__ __forceinline__ unsigned warp_tile_rows(const WarpArgs& a, const Coef& co, const TapSource& ts, float* dst,
-                                                   int tile_x, int tile_y, int lx, int ly, bool interior,
-                                                   bool int_shift) {
+                                                   int ox, int oy0, bool interior, bool int_shift) {
   constexpr int radius = (INTERP == GG_INTERP_LANCZOS3) ? 3 : 1;
-  const int ox = tile_x * kTileW + lx;
   unsigned bad = 0;
   // Affine source coordinates step by 4 output rows: (sx, sy) += 4 (b, e)
   // in float-float (exact scaling by 4, one TwoSum per axis), with a fresh
@@ -193,12 +194,12 @@ __device__ __forceinline__ unsigned warp_tile_rows(const WarpArgs& a, const Coef
   const float step_y_hi = 4.0f * co.m[4][0], step_y_lo = 4.0f * co.m[4][1];
 #pragma unroll 1
   for (int r = 0; r < kRowsPerThread; ++r) {
-    const int oy = tile_y * kTileH + ly + 4 * r;
-    const bool inside = ox < a.width && oy < a.height;
+    const int oy = oy0 + 4 * r;
+    const bool inside = ox < a.width && oy < a.row1;
     bool valid = false;
     float value = a.fill;
     if (co.affine) {
-      if (r % kFreshRows == 0) {
+      if (r % kFreshRows == 0 || a.every_row) {
         row_ok = source_coord(co, static_cast<float>(ox), static_cast<float>(oy), sx_row, sy_row);
       } else {
         sx_row = ff_add_ff(sx_row, step_x_hi, step_x_lo);
@@ -339,7 +340,8 @@ __global__ void __launch_bounds__(kWarpThreads, 3) warp_tiles_kernel(const __gri
     const float vlo = INTERP == GG_INTERP_LANCZOS3 ? 2.0f : 0.0f;
     const float vhx = static_cast<float>(a.width) - (INTERP == GG_INTERP_LANCZOS3 ? 3.0f : 1.0f);
     const float vhy = static_cast<float>(a.height) - (INTERP == GG_INTERP_LANCZOS3 ? 3.0f : 1.0f);
-    TilePlan p = plan_tile(load_coef(ip), t % a.tiles_x, t / a.tiles_x, radius, vlo, vhx, vhy);
+    TilePlan p = plan_tile(load_coef(ip), t % a.tiles_x * kTileW, a.row0 + t / a.tiles_x * kTileH, radius, vlo, vhx,
+                           vhy);
     if (!USE_TMA) p.fits = 0;
     s_interior[buf] = p.interior;
     s_bx[buf] = p.bx;
@@ -365,11 +367,11 @@ __global__ void __launch_bounds__(kWarpThreads, 3) warp_tiles_kernel(const __gri
     const Coef co = load_coef(ip);
     const int it_frame = __ldg(&ip->frame);
     const int it_src = __ldg(&ip->src_slot);
-    const int it_dst = __ldg(&ip->dst_slot);
+    float* const it_dst = ip->dst;
     const unsigned it_nonfinite = __ldg(&ip->src_nonfinite);
     const bool int_shift = __ldg(&ip->int_shift) != 0;
     const int t = item - item_index * tiles;
-    const int tile_x = t % a.tiles_x, tile_y = t / a.tiles_x;
+    const int tile_x0 = t % a.tiles_x * kTileW, tile_y0 = a.row0 + t / a.tiles_x * kTileH;
     const bool fit = s_fit[buf] != 0;
     const bool interior = s_interior[buf] != 0;
     if (fit) {
@@ -390,19 +392,19 @@ __global__ void __launch_bounds__(kWarpThreads, 3) warp_tiles_kernel(const __gri
       ts.bx = s_bx[buf];
       ts.by = s_by[buf];
       ts.width = a.width;
-      float* dst = a.slots + static_cast<int64_t>(it_dst) * a.stride;
+      float* dst = it_dst - static_cast<int64_t>(a.row0) * a.width;
       // the renormalising path (and its out-of-line call) only for frames
       // that hold non-finite samples; the straight-line form for the common
       // interior tile
-      const bool full_tile = (tile_x + 1) * kTileW <= a.width && (tile_y + 1) * kTileH <= a.height;
+      const bool full_tile = tile_x0 + kTileW <= a.width && tile_y0 + kTileH <= a.row1;
       unsigned bad;
       if (INTERP == GG_INTERP_LANCZOS3 && fit && interior && co.affine && it_nonfinite == 0u && !int_shift &&
           a.clamp < 0.0f && a.coverage == nullptr && full_tile)
-        bad = warp_tile_rows_fast(a, co, ts.tile, ts.bx, ts.by, dst, tile_x * kTileW + lx, tile_y * kTileH + ly);
+        bad = warp_tile_rows_fast(a, co, ts.tile, ts.bx, ts.by, dst, tile_x0 + lx, tile_y0 + ly);
       else if (INTERP == GG_INTERP_LANCZOS3 && it_nonfinite == 0u)
-        bad = warp_tile_rows<INTERP, true>(a, co, ts, dst, tile_x, tile_y, lx, ly, interior, int_shift);
+        bad = warp_tile_rows<INTERP, true>(a, co, ts, dst, tile_x0 + lx, tile_y0 + ly, interior, int_shift);
       else
-        bad = warp_tile_rows<INTERP, false>(a, co, ts, dst, tile_x, tile_y, lx, ly, interior, int_shift);
+        bad = warp_tile_rows<INTERP, false>(a, co, ts, dst, tile_x0 + lx, tile_y0 + ly, interior, int_shift);
       const unsigned warp_bad = __reduce_add_sync(0xffffffffu, bad);
       if ((tid & 31) == 0 && warp_bad) atomicAdd(a.nonfinite + it_frame, warp_bad);
     }
@@ -417,12 +419,13 @@ __global__ void __launch_bounds__(kWarpThreads, 3) warp_tiles_kernel(const __gri
 
 // Resolve slots for the batch and move the source non-finite counts aside.
 __global__ void warp_prepare_kernel(WarpItem* items, int count, const int* slot_of_frame, const int* spare,
-                                    unsigned* nonfinite) {
+                                    unsigned* nonfinite, float* slots, int64_t stride) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= count) return;
   const int f = items[k].frame;
   items[k].src_slot = slot_of_frame[f];
   items[k].dst_slot = spare[k];
+  items[k].dst = slots + spare[k] * stride;
   items[k].src_nonfinite = nonfinite[f];
   nonfinite[f] = 0u;
 }
@@ -514,6 +517,33 @@ static void launch_warp_tiles(gg_stack* s, const WarpArgs& args, bool use_tma) {
   check_cuda(cudaGetLastError(), "warp kernel launch");
 }
 
+// Arguments of a launch over output rows [row0, row1) of `count` frames.
+static WarpArgs warp_args(gg_stack* s, WarpItem* d_items, int count, int row0, int row1) {
+  WarpArgs a{};
+  a.slots = s->d_slots;
+  a.items = d_items;
+  a.item_count = count;
+  a.stride = s->stride;
+  a.width = static_cast<int>(s->width);
+  a.height = static_cast<int>(s->height);
+  a.row0 = row0;
+  a.row1 = row1;
+  a.tiles_x = (a.width + kTileW - 1) / kTileW;
+  a.tiles_y = (row1 - row0 + kTileH - 1) / kTileH;
+  a.error = s->d_error;
+  return a;
+}
+
+static void launch_warp_rows(gg_stack* s, const WarpArgs& a, int interp) {
+  const bool use_tma = s->has_slot_tmap;
+  if (interp == GG_INTERP_NEAREST)
+    launch_warp_tiles<GG_INTERP_NEAREST>(s, a, use_tma);
+  else if (interp == GG_INTERP_BILINEAR)
+    launch_warp_tiles<GG_INTERP_BILINEAR>(s, a, use_tma);
+  else
+    launch_warp_tiles<GG_INTERP_LANCZOS3>(s, a, use_tma);
+}
+
 // Host descriptors of a warp batch (validated; inverse coefficients).
 static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd) {
   std::vector<WarpItem> items(static_cast<size_t>(count));
@@ -545,36 +575,19 @@ static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices
 // launches on the stack's stream (safe inside a stream capture).
 static void launch_warp_items(gg_stack* s, WarpItem* d_items, int64_t count, int interp, float fill, float clamp,
                               bool track_coverage) {
-  const bool use_tma = s->has_slot_tmap;
   for (int64_t k0 = 0; k0 < count; k0 += s->spares) {
     const int nb = static_cast<int>(std::min<int64_t>(s->spares, count - k0));
     note_launch();
     warp_prepare_kernel<<<(nb + 127) / 128, 128, 0, s->stream>>>(d_items + k0, nb, s->d_slot_of_frame,
-                                                                 s->d_spare_slot, s->d_frame_nonfinite);
+                                                                 s->d_spare_slot, s->d_frame_nonfinite, s->d_slots,
+                                                                 s->stride);
     check_cuda(cudaGetLastError(), "warp_prepare launch");
-    WarpArgs a{};
-    a.slots = s->d_slots;
-    a.slot_of_frame = s->d_slot_of_frame;
-    a.spare_slot = s->d_spare_slot;
+    WarpArgs a = warp_args(s, d_items + k0, nb, 0, static_cast<int>(s->height));
     a.nonfinite = s->d_frame_nonfinite;
-    a.items = d_items + k0;
-    a.item_count = nb;
-    a.stride = s->stride;
-    a.width = static_cast<int>(s->width);
-    a.height = static_cast<int>(s->height);
-    a.tiles_x = static_cast<int>((s->width + kTileW - 1) / kTileW);
-    a.tiles_y = static_cast<int>((s->height + kTileH - 1) / kTileH);
-    a.interp = interp;
     a.fill = fill;
     a.clamp = clamp;
     a.coverage = track_coverage ? s->d_warp_coverage : nullptr;
-    a.error = s->d_error;
-    if (interp == GG_INTERP_NEAREST)
-      launch_warp_tiles<GG_INTERP_NEAREST>(s, a, use_tma);
-    else if (interp == GG_INTERP_BILINEAR)
-      launch_warp_tiles<GG_INTERP_BILINEAR>(s, a, use_tma);
-    else
-      launch_warp_tiles<GG_INTERP_LANCZOS3>(s, a, use_tma);
+    launch_warp_rows(s, a, interp);
     note_launch();
     warp_finish_kernel<<<(nb + 127) / 128, 128, 0, s->stream>>>(d_items + k0, nb, s->d_slot_of_frame,
                                                                 s->d_spare_slot);
@@ -610,6 +623,190 @@ void* warp_items_device(gg_stack* s, const int64_t* indices, int64_t count, cons
     check_cuda(err, "cudaMemcpy(graph warp items)");
   }
   return d;
+}
+
+// ---- warp of every frame into a band of rows (fused warp + integration) --------
+BandLayout warp_band_layout(const gg_stack* s) {
+  BandLayout b;
+  b.per_slot = static_cast<int>((s->frames + s->spares - 1) / s->spares);
+  b.capacity = b.per_slot == 1 ? s->stride : s->stride / b.per_slot / 64 * 64;
+  b.rows = static_cast<int>(std::min<int64_t>(s->height, b.capacity / s->width));
+  // whole tile rows, so that only the last band has partial tiles
+  if (b.rows < s->height && b.rows > kTileH) b.rows -= b.rows % kTileH;
+  return b;
+}
+
+size_t warp_item_bytes() { return sizeof(WarpItem); }
+
+// Descriptors and band buffers of every frame from its inverse coefficients.
+// `own` (capacity samples per frame) takes the place of the spare slots when
+// they hold less than a row per frame.
+__global__ void warp_band_prepare_kernel(WarpItem* items, const FusedFrame* frames, int count,
+                                         const int* slot_of_frame, const int* spare, const unsigned* nonfinite,
+                                         float* slots, int64_t stride, int per_slot, int64_t capacity, float* own,
+                                         const float** base, unsigned* counts) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= count) return;
+  WarpItem it{};
+  it.frame = k;
+  it.src_slot = slot_of_frame[k];
+  it.dst_slot = -1;
+  it.src_nonfinite = nonfinite[k];
+  it.affine = frames[k].affine;
+  it.dst = own ? own + k * capacity : slots + spare[k / per_slot] * stride + (k % per_slot) * capacity;
+  for (int q = 0; q < 9; ++q) {
+    it.m[q][0] = frames[k].m[q][0];
+    it.m[q][1] = frames[k].m[q][1];
+  }
+  items[k] = it;
+  base[k] = it.dst;
+  counts[k] = 0u;
+}
+
+template <int INTERP>
+__device__ __forceinline__ bool sample_valid(const Coef& co, int x, int y, int width, int height, FFv& sx, FFv& sy) {
+  if (!source_coord(co, static_cast<float>(x), static_cast<float>(y), sx, sy)) return false;
+  const float W = static_cast<float>(width), H = static_cast<float>(height);
+  if (INTERP == GG_INTERP_LANCZOS3) return ff_ge(sx, 2.0f) && ff_lt(sx, W - 3.0f) && ff_ge(sy, 2.0f) && ff_lt(sy, H - 3.0f);
+  return ff_ge(sx, 0.0f) && ff_le(sx, W - 1.0f) && ff_ge(sy, 0.0f) && ff_le(sy, H - 1.0f);
+}
+
+// Whether any sample of a frame's warp is non-finite, known before the first
+// of several bands is integrated (one count is enough: it selects the
+// integrator's all-valid formulas).  The valid source range is convex, so an
+// affine map whose four corners are valid has only valid samples; the other
+// frames have an invalid one.  What is left is scanned: projective maps, and
+// frames that hold non-finite samples themselves.
+template <int INTERP>
+__global__ void __launch_bounds__(256) warp_nonfinite_kernel(WarpArgs a, unsigned* counts) {
+  const WarpItem* ip = a.items + blockIdx.y;
+  const Coef co = load_coef(ip);
+  const unsigned src_nonfinite = ip->src_nonfinite;
+  bool corners = true;
+  FFv cx, cy;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    corners = corners && sample_valid<INTERP>(co, (c & 1) ? a.width - 1 : 0, (c & 2) ? a.height - 1 : 0, a.width,
+                                              a.height, cx, cy);
+  if (!corners) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) counts[blockIdx.y] = 1u;
+    return;
+  }
+  if (co.affine && src_nonfinite == 0u) return;
+  TapSource ts;
+  ts.tile = nullptr;
+  ts.src = a.slots + static_cast<int64_t>(ip->src_slot) * a.stride;
+  ts.bx = ts.by = 0;
+  ts.width = a.width;
+  const int64_t pixels = static_cast<int64_t>(a.width) * a.height;
+  bool bad = false;
+  for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < pixels && !bad;
+       p += int64_t(gridDim.x) * blockDim.x) {
+    const int y = static_cast<int>(p / a.width), x = static_cast<int>(p - static_cast<int64_t>(y) * a.width);
+    FFv sx, sy;
+    if (!sample_valid<INTERP>(co, x, y, a.width, a.height, sx, sy)) {
+      bad = true;
+      break;
+    }
+    int x0, y0;
+    float tx, ty, v;
+    ff_floor_frac(sx, x0, tx);
+    ff_floor_frac(sy, y0, ty);
+    if (INTERP == GG_INTERP_BILINEAR) v = sample_bilinear(ts, x0, y0, tx, ty, a.width, a.height);
+    else if (!sample_lanczos3(ts, x0, y0, tx, ty, src_nonfinite == 0u, a.clamp, v)) v = __int_as_float(0x7fc00000);
+    bad = !isfinite(v);
+  }
+  if (bad) counts[blockIdx.y] = 1u;
+}
+
+// Frames with a geometrically valid sample, per pixel of a band.  One CTA per
+// 64 x 48 tile: a frame that maps the whole tile inside its valid range counts
+// for every pixel without a test (all but the tiles along the border), the
+// others are evaluated pixel by pixel.  Where a Lanczos3 frame holds
+// non-finite samples, a window may have no weight left: its warped sample
+// tells (NaN).
+template <int INTERP>
+__global__ void __launch_bounds__(kWarpThreads) warp_geometry_kernel(WarpArgs a, float* geometric) {
+  __shared__ int s_inside, s_mixed;
+  __shared__ int s_list[512];
+  const int tile_x0 = blockIdx.x % a.tiles_x * kTileW, tile_y0 = a.row0 + blockIdx.x / a.tiles_x * kTileH;
+  if (threadIdx.x == 0) s_inside = s_mixed = 0;
+  __syncthreads();
+  constexpr bool kLanczos = INTERP == GG_INTERP_LANCZOS3;
+  const float vlo = kLanczos ? 2.0f : 0.0f, off = kLanczos ? 3.0f : 1.0f;
+  for (int f = threadIdx.x; f < a.item_count; f += kWarpThreads) {
+    const WarpItem* ip = a.items + f;
+    const bool by_value = kLanczos && ip->src_nonfinite != 0u;
+    const TilePlan p = plan_tile(load_coef(ip), tile_x0, tile_y0, kLanczos ? 3 : 1, vlo,
+                                 static_cast<float>(a.width) - off, static_cast<float>(a.height) - off);
+    if (p.interior && !by_value) atomicAdd(&s_inside, 1);
+    else s_list[atomicAdd(&s_mixed, 1)] = f;
+  }
+  __syncthreads();
+  const int ox = tile_x0 + (threadIdx.x & 63);
+  if (ox >= a.width) return;
+  int n[kRowsPerThread];
+#pragma unroll
+  for (int r = 0; r < kRowsPerThread; ++r) n[r] = s_inside;
+  for (int i = 0; i < s_mixed; ++i) {
+    const WarpItem* ip = a.items + s_list[i];
+    const Coef co = load_coef(ip);
+    const bool by_value = kLanczos && ip->src_nonfinite != 0u;
+    const float* dst = ip->dst - static_cast<int64_t>(a.row0) * a.width;
+    FFv sx, sy;
+#pragma unroll
+    for (int r = 0; r < kRowsPerThread; ++r) {
+      const int oy = tile_y0 + (threadIdx.x >> 6) + 4 * r;
+      if (oy >= a.row1) continue;
+      if (by_value) n[r] += !isnan(dst[static_cast<int64_t>(oy) * a.width + ox]);
+      else n[r] += sample_valid<INTERP>(co, ox, oy, a.width, a.height, sx, sy);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < kRowsPerThread; ++r) {
+    const int oy = tile_y0 + (threadIdx.x >> 6) + 4 * r;
+    if (oy < a.row1) geometric[static_cast<int64_t>(oy) * a.width + ox] = static_cast<float>(n[r]);
+  }
+}
+
+void launch_warp_band(gg_stack* s, void* d_items, int interp, float clamp, int row0, int row1, unsigned* counts,
+                      float* geometric) {
+  WarpArgs a = warp_args(s, static_cast<WarpItem*>(d_items), static_cast<int>(s->frames), row0, row1);
+  a.nonfinite = counts;
+  a.fill = NAN;
+  a.clamp = clamp;
+  a.every_row = 1;  // the same validity as the geometric coverage below
+  launch_warp_rows(s, a, interp);
+  const unsigned tiles = static_cast<unsigned>(a.tiles_x) * static_cast<unsigned>(a.tiles_y);
+  note_launch();
+  if (interp == GG_INTERP_BILINEAR)
+    warp_geometry_kernel<GG_INTERP_BILINEAR><<<tiles, kWarpThreads, 0, s->stream>>>(a, geometric);
+  else
+    warp_geometry_kernel<GG_INTERP_LANCZOS3><<<tiles, kWarpThreads, 0, s->stream>>>(a, geometric);
+  check_cuda(cudaGetLastError(), "warp_geometry launch");
+}
+
+void launch_warp_band_prepare(gg_stack* s, void* d_items, const FusedFrame* d_frames, int interp, float clamp,
+                              const BandLayout& band, float* own, const float** base, unsigned* counts) {
+  const int n = static_cast<int>(s->frames);
+  auto* items = static_cast<WarpItem*>(d_items);
+  note_launch();
+  warp_band_prepare_kernel<<<(n + 127) / 128, 128, 0, s->stream>>>(
+      items, d_frames, n, s->d_slot_of_frame, s->d_spare_slot, s->d_frame_nonfinite, s->d_slots, s->stride,
+      band.per_slot, band.capacity, own, base, counts);
+  check_cuda(cudaGetLastError(), "warp_band_prepare launch");
+  if (band.rows >= s->height) return;
+  WarpArgs a = warp_args(s, items, n, 0, static_cast<int>(s->height));
+  a.clamp = clamp;
+  const dim3 grid(static_cast<unsigned>(std::max<int64_t>(
+                      1, std::min<int64_t>((s->pixels + 255) / 256, sm_count() * 8 / n + 1))),
+                  static_cast<unsigned>(n));
+  note_launch();
+  if (interp == GG_INTERP_BILINEAR)
+    warp_nonfinite_kernel<GG_INTERP_BILINEAR><<<grid, 256, 0, s->stream>>>(a, counts);
+  else
+    warp_nonfinite_kernel<GG_INTERP_LANCZOS3><<<grid, 256, 0, s->stream>>>(a, counts);
+  check_cuda(cudaGetLastError(), "warp_nonfinite launch");
 }
 
 void launch_warp_items_device(gg_stack* s, void* d_items, int64_t count, int interp, float fill, float clamp) {
