@@ -29,52 +29,21 @@
 #include <type_traits>
 #include <vector>
 
+#include "async.cuh"
 #include "autotune.cuh"
+#include "integrate.cuh"
 #include "sampling.cuh"
-#include "stack.cuh"
-#include "warp_band.cuh"
 
 namespace gg {
-
-struct IntegrateArgs {
-  const float* slots;
-  const int* slot_of_frame;
-  int64_t stride;
-  const float* const* base;  // optional first sample of every frame (else its slot's)
-  int64_t pixels;
-  int frames;
-  const float* weights;  // device [frames], raw values
-  const unsigned* nonfinite;
-  int rejection;
-  float low_sigma;
-  float high_sigma;
-  int min_samples;
-  float max_frac;
-  int lfc_iterations;
-  float* master;
-  float* weight;
-  void* coverage;
-  void* low;
-  void* high;
-  int16_t* dq;
-  int count_u16;
-  const float* geometric;  // optional warp coverage (float32 per pixel)
-  // fused warp only
-  const FusedFrame* fused;
-  int width, height;
-  float clamp;
-  float* geometric_out;  // frames with a geometrically valid sample, per pixel
-  int tile_w, tile_h;    // fused path: 2-D pixel tiles (tile_w * tile_h == threads), 0 = rows
-  int64_t tiles_x;       // tiles per image row
-  int64_t tile_slots;    // tiles * threads
-};
 
 // One fused sample of frame f at output pixel (x, y): the value the warp
 // kernel would have written (NaN fill when invalid); `geo` counts the
 // samples the warp would have marked covered.
+// Out of line: the column kernel keeps the sampler out of its unrolled register
+// code.
 template <int INTERP>
-__device__ __forceinline__ float fused_sample_inline(const IntegrateArgs& a, const float* src, const FusedFrame& fz,
-                                                     int x, int y, int& geo) {
+__device__ __noinline__ float fused_sample(const IntegrateArgs& a, const float* src, const FusedFrame& fz, int x,
+                                           int y, int& geo) {
   const float nan = __int_as_float(0x7fc00000);
   FFv sx, sy;
   if (!source_coord(fz, static_cast<float>(x), static_cast<float>(y), sx, sy)) return nan;
@@ -100,42 +69,6 @@ __device__ __forceinline__ float fused_sample_inline(const IntegrateArgs& a, con
   }
   ++geo;
   return v;
-}
-
-// Out-of-line copy for the column kernel, which keeps the sampler out of its
-// unrolled register code; the warp-per-pixel tile fill inlines it.
-template <int INTERP>
-__device__ __noinline__ float fused_sample(const IntegrateArgs& a, const float* src, const FusedFrame& fz, int x,
-                                           int y, int& geo) {
-  return fused_sample_inline<INTERP>(a, src, fz, x, y, geo);
-}
-
-constexpr float kInf = __builtin_huge_valf();
-
-// ---- sorting network (Batcher odd-even merge sort, fully unrolled) --------
-// Loop counters are kept additive (log2 of p and k) so that nvcc unrolls the
-// whole network and v[] stays in registers.
-template <int N>
-__device__ __forceinline__ void sort_network(float (&v)[N]) {
-  constexpr int LOG2N = (N <= 1) ? 0 : (N <= 2) ? 1 : (N <= 4) ? 2 : (N <= 8) ? 3 : (N <= 16) ? 4 : (N <= 32) ? 5 : 6;
-  static_assert((1 << LOG2N) == N, "sort_network needs a power-of-two size up to 64");
-#pragma unroll
-  for (int lp = 0; lp < LOG2N; ++lp) {
-#pragma unroll
-    for (int lk = lp; lk >= 0; --lk) {
-#pragma unroll
-      for (int a = 0; a < N; ++a) {
-        // Comparator (a, a+k) of stage (p, k); all conditions fold at compile time.
-        const int p = 1 << lp, k = 1 << lk, j0 = k % p;
-        if (a >= j0 && a + k < N && ((a - j0) % (2 * k)) < k && (a / (2 * p)) == ((a + k) / (2 * p))) {
-          const float lo = fminf(v[a], v[a + k]);
-          const float hi = fmaxf(v[a], v[a + k]);
-          v[a] = lo;
-          v[a + k] = hi;
-        }
-      }
-    }
-  }
 }
 
 // ---- percentiles ------------------------------------------------------------
@@ -166,55 +99,10 @@ __device__ __forceinline__ float percentile_all(const float* S, int T, int n, fl
   return __fadd_rn(lv, __fmul_rn(__fsub_rn(uv, lv), f));
 }
 
-__device__ __forceinline__ float clipf(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
-
-// ---- output ---------------------------------------------------------------
-// DQ bits: contracts.py:77-88; rules: resident_cuda.py:3110-3297.
-__device__ __forceinline__ void write_outputs(const IntegrateArgs& a, int64_t p, float master, float weight, int cov,
-                                              int nlow, int nhigh, int active_frames) {
-  a.master[p] = master;
-  a.weight[p] = weight;
-  if (a.count_u16) {
-    static_cast<uint16_t*>(a.coverage)[p] = static_cast<uint16_t>(min(cov, 65535));
-    static_cast<uint16_t*>(a.low)[p] = static_cast<uint16_t>(min(nlow, 65535));
-    static_cast<uint16_t*>(a.high)[p] = static_cast<uint16_t>(min(nhigh, 65535));
-  } else {
-    static_cast<float*>(a.coverage)[p] = static_cast<float>(cov);
-    static_cast<float*>(a.low)[p] = static_cast<float>(nlow);
-    static_cast<float*>(a.high)[p] = static_cast<float>(nhigh);
-  }
-  if (a.dq) {
-    int bits = 0;
-    bool invalid = !isfinite(master) || !isfinite(weight) || !(weight > 0.0f);
-    if (cov <= 0) {
-      bits |= 64;
-      invalid = true;
-    }
-    if (a.geometric) {
-      const float g = a.geometric[p];
-      if (!isfinite(g) || g <= 0.5f) {
-        bits |= 64;
-        invalid = true;
-      } else if (active_frames > 0 && g < static_cast<float>(active_frames) - 0.5f) {
-        bits |= 64;
-      }
-    }
-    if (invalid) bits |= 1;
-    if (nlow > 0) bits |= 256;
-    if (nhigh > 0) bits |= 512;
-    a.dq[p] = static_cast<int16_t>(bits);
-  }
-}
-
 // ---- per-pixel statistics over a column ------------------------------------
 // The column is reachable two ways: `sorted` holds the valid samples in
 // ascending order at ranks [0, cnt) with stride T (+inf beyond), and the
 // frame-order view is provided by the caller's RawView.
-struct CenterScale {
-  float center;
-  float scale;
-};
-
 // Fallback scale: std of the valid samples (rejection.py:231 all-valid,
 // rejection.py:323-349 otherwise).
 template <class Sorted>
@@ -486,38 +374,12 @@ __device__ __forceinline__ void load_frame_table(const IntegrateArgs& a, FrameTa
 // error-free, and squared deviations are summed from both ends of the sorted
 // column inwards for the same reason.  Rejection counts are binary searches.
 
-__device__ __forceinline__ void ff_merge2(FF& a, const FF& b) {
-  float s, e;
-  two_sum(a.hi, b.hi, s, e);
-  a.hi = s;
-  a.lo = __fadd_rn(__fadd_rn(a.lo, b.lo), e);
-}
-
 // Fast2Sum: error-free when |a.hi| >= |x| (or a.hi == 0).
 __device__ __forceinline__ void ff_add_fast(FF& a, float x) {
   const float s = __fadd_rn(a.hi, x);
   const float e = __fsub_rn(x, __fsub_rn(s, a.hi));
   a.hi = s;
   a.lo = __fadd_rn(a.lo, e);
-}
-
-// True when every value in [lo, hi] lies within a factor of two of c (same
-// sign), so x - c is exact in float32 (Sterbenz).
-__device__ __forceinline__ bool sterbenz_interval(float lo, float hi, float c) {
-  if (c > 0.0f) return lo >= 0.5f * c && hi <= 2.0f * c;
-  if (c < 0.0f) return hi <= 0.5f * c && lo >= 2.0f * c;
-  return false;
-}
-
-// Number of sorted valid values < t (strict) or <= t.
-__device__ __forceinline__ int count_below(const float* S, int T, int cnt, float t, bool inclusive) {
-  int lo = 0, hi = cnt;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    const float v = S[mid * T];
-    if (inclusive ? (v <= t) : (v < t)) lo = mid + 1; else hi = mid;
-  }
-  return lo;
 }
 
 // Sum of S[i0..i1) (clipped to [lo, hi]) without rounding error loss.
@@ -942,7 +804,8 @@ __global__ void __launch_bounds__(T) integrate_smem_kernel(IntegrateArgs a) {
   }
 }
 
-// ---- kernel W: 32 < N <= 32 * NPL, one warp per pixel ------------------------
+// ---- kernel W: 256 < N <= 512, one warp per pixel ------------------------------
+// (integrate_px.cu has 33 to 256 frames.)
 // A CTA stages a tile of kWarpTilePx consecutive pixels of every frame in
 // shared memory ([frame][pixel], rows padded to kWarpTilePx + 1 floats so a
 // warp reading one pixel's column is bank-conflict free; every frame row is
@@ -951,40 +814,22 @@ __global__ void __launch_bounds__(T) integrate_smem_kernel(IntegrateArgs a) {
 // warp-wide bitonic network (in-register steps within a lane, shuffles
 // across lanes), and every sum of the statistics and of the integration is a
 // per-lane float-float sum combined across the warp.  The shared-memory cost
-// is 4 * 33 B per frame instead of a sorted column per thread, so an SM keeps
-// tens of warps in flight at N = 200.  WARP = GG_INTERP_* fills the tile by
-// sampling every frame through its inverse matrix (fused warp + integration
-// of more than 32 frames) and counts each pixel's geometrically valid
-// samples in shared memory.
+// is 4 * 33 B per frame instead of a sorted column per thread.
 constexpr int kWarpTilePx = 32;
 constexpr int kWarpTileRow = kWarpTilePx + 1;
 constexpr int kWarpThreads = 256;
 
-// (hi, lo) float-float sum over each segment of LANES lanes (the whole warp
-// by default), in every lane of the segment.  TwoSum is exact and
+// (hi, lo) float-float sum over the warp, in every lane.  TwoSum is exact and
 // symmetric, so both partners of each butterfly step hold the same pair.
-template <int LANES = 32>
 __device__ __forceinline__ void ff_warp_reduce(FF& s) {
 #pragma unroll
-  for (int off = LANES / 2; off > 0; off >>= 1) {
+  for (int off = 16; off > 0; off >>= 1) {
     const float oh = __shfl_xor_sync(0xffffffffu, s.hi, off);
     const float ol = __shfl_xor_sync(0xffffffffu, s.lo, off);
     float h, e;
     two_sum(s.hi, oh, h, e);
     s.hi = h;
     s.lo = __fadd_rn(__fadd_rn(s.lo, ol), e);
-  }
-}
-
-// Integer sum over each segment of LANES lanes, in every lane of it.
-template <int LANES>
-__device__ __forceinline__ int seg_sum(int x) {
-  if constexpr (LANES == 32) {
-    return __reduce_add_sync(0xffffffffu, x);
-  } else {
-#pragma unroll
-    for (int off = LANES / 2; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-    return x;
   }
 }
 
@@ -996,14 +841,11 @@ __device__ __forceinline__ int seg_sum(int x) {
 // and a max per pair) and a lane whose block sorts descending reverses its
 // registers afterwards; below NPL the direction of a pair is a compile-time
 // function of its register index.
-// With LANES = 16 the two half-warps sort two columns of 16 * NPL values
-// independently (every partner distance stays below 16); `lane` is then the
-// lane within the half.
-template <int NPL, int LANES = 32>
+template <int NPL>
 __device__ __forceinline__ void warp_bitonic_sort(float (&v)[NPL], int lane) {
-  constexpr int M = LANES * NPL;
+  constexpr int M = 32 * NPL;
   constexpr int LOGM = (M == 64) ? 6 : (M == 128) ? 7 : (M == 256) ? 8 : 9;
-  static_assert(M == (1 << LOGM) && NPL >= 2 && NPL <= 16, "LANES * NPL must be 64 .. 512");
+  static_assert(M == (1 << LOGM) && NPL >= 2 && NPL <= 16, "32 * NPL must be 64 .. 512");
 #pragma unroll
   for (int ls = 1; ls <= LOGM; ++ls) {
     const int size = 1 << ls;
@@ -1058,8 +900,8 @@ __device__ __forceinline__ void warp_bitonic_sort(float (&v)[NPL], int lane) {
 
 // Value of warp-uniform rank i; the register index i % NPL is warp-uniform,
 // so a switch on it (uniform branch) replaces a per-lane select chain.
-template <int NPL, int LANES = 32>
-__device__ __forceinline__ float warp_rank(const float (&v)[NPL], int i, int seg = 0) {
+template <int NPL>
+__device__ __forceinline__ float warp_rank(const float (&v)[NPL], int i) {
   float t = v[0];
   switch (i & (NPL - 1)) {
     case 0: if constexpr (0 < NPL) t = v[0]; break;
@@ -1079,49 +921,48 @@ __device__ __forceinline__ float warp_rank(const float (&v)[NPL], int i, int seg
     case 14: if constexpr (14 < NPL) t = v[14]; break;
     case 15: if constexpr (15 < NPL) t = v[15]; break;
   }
-  return __shfl_sync(0xffffffffu, t, seg * LANES + i / NPL);
+  return __shfl_sync(0xffffffffu, t, i / NPL);
 }
 
-// percentile_valid / percentile_all on the warp's sorted column.  With
-// LANES = 16 the two halves rank their own columns; the shuffles run in
-// every lane whatever the counts (a half with no samples gets 0).
-template <int NPL, int LANES = 32>
-__device__ __forceinline__ float warp_percentile_valid(const float (&v)[NPL], int cnt, float fraction, int seg = 0) {
+// percentile_valid / percentile_all on the warp's sorted column (0 for a column
+// without samples).
+template <int NPL>
+__device__ __forceinline__ float warp_percentile_valid(const float (&v)[NPL], int cnt, float fraction) {
   const int c = cnt > 0 ? cnt : 1;
   const float pos = __fmul_rn(static_cast<float>(c - 1), fraction);
   const int lower = static_cast<int>(floorf(pos));
   const int upper = min(lower + 1, c - 1);
   const float t = __fsub_rn(pos, static_cast<float>(lower));
-  const float lv = warp_rank<NPL, LANES>(v, lower, seg);
-  const float uv = warp_rank<NPL, LANES>(v, upper, seg);
+  const float lv = warp_rank<NPL>(v, lower);
+  const float uv = warp_rank<NPL>(v, upper);
   if (cnt <= 0) return 0.0f;
   return __fadd_rn(__fmul_rn(lv, __fsub_rn(1.0f, t)), __fmul_rn(uv, t));
 }
 
-template <int NPL, int LANES = 32>
-__device__ __forceinline__ float warp_percentile_all(const float (&v)[NPL], int n, float fraction, int seg = 0) {
-  if (n == 1) return warp_rank<NPL, LANES>(v, 0, seg);
+template <int NPL>
+__device__ __forceinline__ float warp_percentile_all(const float (&v)[NPL], int n, float fraction) {
+  if (n == 1) return warp_rank<NPL>(v, 0);
   const float pos = __fmul_rn(fraction, static_cast<float>(n - 1));
   const int lower = static_cast<int>(floorf(pos));
   const int upper = static_cast<int>(ceilf(pos));
   const float f = __fsub_rn(pos, static_cast<float>(lower));
-  const float lv = warp_rank<NPL, LANES>(v, lower, seg);
+  const float lv = warp_rank<NPL>(v, lower);
   if (upper == lower) return lv;
-  const float uv = warp_rank<NPL, LANES>(v, upper, seg);
+  const float uv = warp_rank<NPL>(v, upper);
   return __fadd_rn(lv, __fmul_rn(__fsub_rn(uv, lv), f));
 }
 
 // Mean (hi, lo) and float-float squared deviations of the valid ranks after
 // clipping to [lo, hi] (+-inf: no clipping); the two passes of std_of_valid
 // and winsorized_stats.
-template <int NPL, int LANES = 32>
+template <int NPL>
 __device__ __forceinline__ float warp_clipped_std(const float (&v)[NPL], int lane, int cnt, bool allvalid, float lo,
                                                   float hi, float& mean_out) {
   FF s1;
 #pragma unroll
   for (int k = 0; k < NPL; ++k)
     if (lane * NPL + k < cnt) s1.add(clipf(v[k], lo, hi));
-  ff_warp_reduce<LANES>(s1);
+  ff_warp_reduce(s1);
   float mh, ml;
   if (allvalid) {
     ff_div_pair(s1.hi, s1.lo, static_cast<float>(cnt), mh, ml);
@@ -1135,44 +976,23 @@ __device__ __forceinline__ float warp_clipped_std(const float (&v)[NPL], int lan
 #pragma unroll
   for (int k = 0; k < NPL; ++k)
     if (lane * NPL + k < cnt) ff_add_sqdev(sv, clipf(v[k], lo, hi), mh, ml);
-  ff_warp_reduce<LANES>(sv);
+  ff_warp_reduce(sv);
   float q, ql;
   ff_div_pair(sv.hi, sv.lo, static_cast<float>(cnt), q, ql);
   return ff_sqrt_f32(q, ql);
 }
 
-__device__ __forceinline__ void cp_async4(float* dst, const float* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory");
-}
-
-// PIPE (resident frames only): two tile buffers; the copies of the next tile
+// PIPE: two tile buffers; the copies of the next tile
 // (cp.async, one 4-byte sample per thread and step) are in flight while the
 // warps integrate the current one.
-// LANES = 16: two pixels per warp, one per half (columns of at most
-// 16 * NPL frames): the per-pixel scalar work and the butterfly reductions
-// are shared by two pixels.
-template <int NPL, int WARP, bool PIPE = false, int LANES = 32>
-__global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4) : 1)
-    integrate_warp_kernel(IntegrateArgs a) {
-  extern __shared__ float smem_tiles[];  // [frames][kWarpTileRow] (x2 with PIPE), then (fused) [frames] FusedFrame
+template <int NPL, bool PIPE>
+__global__ void __launch_bounds__(kWarpThreads) integrate_warp_kernel(IntegrateArgs a) {
+  extern __shared__ float smem_tiles[];  // [frames][kWarpTileRow] (x2 with PIPE)
   __shared__ FrameTable<32 * NPL> tab;
-  __shared__ int s_geo[kWarpTilePx];
-  static_assert(!(PIPE && WARP != 0), "the pipelined tile copy serves resident frames only");
-  FusedFrame* fz = reinterpret_cast<FusedFrame*>(smem_tiles + a.frames * kWarpTileRow);
-  if constexpr (WARP != 0)
-    for (int f = threadIdx.x; f < a.frames; f += blockDim.x) fz[f] = a.fused[f];
   load_frame_table<32 * NPL>(a, tab);
   const bool allvalid = tab.allvalid != 0;
   const bool unit = tab.unit != 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int hl = lane & (LANES - 1), seg = lane / LANES;
   const int N = a.frames;
   const int64_t P = a.pixels;
   const int64_t tiles = (P + kWarpTilePx - 1) / kWarpTilePx;
@@ -1203,78 +1023,56 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
       }
     } else {
       __syncthreads();  // the previous tile's columns are consumed
-      if constexpr (WARP != 0) {
-        if (threadIdx.x < kWarpTilePx) s_geo[threadIdx.x] = 0;
-        __syncthreads();
-      }
       for (int i = threadIdx.x; i < N * kWarpTilePx; i += kWarpThreads) {
         const int f = i / kWarpTilePx, px = i - f * kWarpTilePx;
         const int64_t p = p0 + px;
-        float v = 0.0f;
-        if constexpr (WARP == 0) {
-          if (p < P) v = __ldcs(tab.base[f] + p);
-        } else if (p < P) {
-          const int py = static_cast<int>(p / a.width),
-                    pxx = static_cast<int>(p - static_cast<int64_t>(py) * a.width);
-          int geo = 0;
-          v = fused_sample_inline<WARP>(a, tab.base[f], fz[f], pxx, py, geo);
-          if (geo) atomicAdd(&s_geo[px], 1);
-        }
-        tile[f * kWarpTileRow + px] = v;
+        tile[f * kWarpTileRow + px] = p < P ? __ldcs(tab.base[f] + p) : 0.0f;
       }
     }
     __syncthreads();
-    // LANES = 32: one warp per pixel; LANES = 16: each half-warp takes a
-    // pixel, the halves 16 tile columns apart (their column loads fall in
-    // disjoint shared-memory banks).  Every shuffle below runs in all 32
-    // lanes; a half whose pixel lies past the frame works on the tile's zero
-    // padding and writes nothing.
-    constexpr int kPixelsPerPass = 32 / LANES;
-    for (int pb = warp; pb < kWarpTilePx / kPixelsPerPass; pb += kWarpThreads / 32) {
-      const int px = pb + seg * (kWarpTilePx / kPixelsPerPass);
+    for (int px = warp; px < kWarpTilePx; px += kWarpThreads / 32) {
       const int64_t p = p0 + px;
-      const bool in_frame = p < P;
-      if (!__any_sync(0xffffffffu, in_frame)) break;
+      if (p >= P) break;
       const float* col = tile + px;
-      // column: lane l of the segment holds frames l, l + LANES, ... (+inf when invalid)
+      // column: lane l holds frames l, l + 32, ... (+inf when invalid)
       float v[NPL];
       int c = 0;
 #pragma unroll
       for (int k = 0; k < NPL; ++k) {
-        const int f = k * LANES + hl;
+        const int f = k * 32 + lane;
         const float x = f < N ? col[f * kWarpTileRow] : kInf;
-        const bool ok = in_frame && f < N && tab.w[f] > 0.0f && isfinite(x);
+        const bool ok = f < N && tab.w[f] > 0.0f && isfinite(x);
         v[k] = ok ? x : kInf;
         c += ok ? 1 : 0;
       }
-      const int cnt = seg_sum<LANES>(c);
+      const int cnt = __reduce_add_sync(0xffffffffu, c);
       int nl = 0, nh = 0;
       float lt = -kInf, ht = kInf;
       bool use_thresholds = false;
       if (a.rejection != GG_REJECT_NONE) {
-        warp_bitonic_sort<NPL, LANES>(v, hl);
+        warp_bitonic_sort<NPL>(v, lane);
         CenterScale cs{0.0f, 0.0f};
         if (a.rejection == GG_REJECT_WINSORIZED) {
           float med, q25, q75;
           if (allvalid) {
-            med = warp_percentile_all<NPL, LANES>(v, N, 0.5f, seg);
-            q25 = warp_percentile_all<NPL, LANES>(v, N, 0.25f, seg);
-            q75 = warp_percentile_all<NPL, LANES>(v, N, 0.75f, seg);
+            med = warp_percentile_all<NPL>(v, N, 0.5f);
+            q25 = warp_percentile_all<NPL>(v, N, 0.25f);
+            q75 = warp_percentile_all<NPL>(v, N, 0.75f);
           } else {
-            med = warp_percentile_valid<NPL, LANES>(v, cnt, 0.5f, seg);
-            q25 = warp_percentile_valid<NPL, LANES>(v, cnt, 0.25f, seg);
-            q75 = warp_percentile_valid<NPL, LANES>(v, cnt, 0.75f, seg);
+            med = warp_percentile_valid<NPL>(v, cnt, 0.5f);
+            q25 = warp_percentile_valid<NPL>(v, cnt, 0.25f);
+            q75 = warp_percentile_valid<NPL>(v, cnt, 0.75f);
           }
           float scale1 = __fdiv_rn(__fsub_rn(q75, q25), 1.349f);
           const bool ok1 = allvalid ? (scale1 > 0.0f) : (scale1 > 0.0f && isfinite(scale1));
           if (__any_sync(0xffffffffu, !ok1)) {
             float unused;
-            const float sd = warp_clipped_std<NPL, LANES>(v, hl, cnt, allvalid, -kInf, kInf, unused);
+            const float sd = warp_clipped_std<NPL>(v, lane, cnt, allvalid, -kInf, kInf, unused);
             if (!ok1) scale1 = sd;
           }
           const float lo1 = __fsub_rn(med, __fmul_rn(ls, scale1));
           const float hi1 = __fadd_rn(med, __fmul_rn(hs, scale1));
-          const float scale = warp_clipped_std<NPL, LANES>(v, hl, cnt, allvalid, lo1, hi1, cs.center);
+          const float scale = warp_clipped_std<NPL>(v, lane, cnt, allvalid, lo1, hi1, cs.center);
           const bool ok2 = allvalid ? (scale > 0.0f) : (scale > 0.0f && isfinite(scale));
           cs.scale = ok2 ? scale : scale1;
           if (cnt <= 0) cs = CenterScale{0.0f, 0.0f};
@@ -1284,9 +1082,9 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
           const int cc = cnt > 0 ? cnt : 1;
           const int h = cc / 2;
           const int l = (cc & 1) ? h : h - 1;
-          const float ml = warp_rank<NPL, LANES>(v, l, seg), mh = warp_rank<NPL, LANES>(v, h, seg);
+          const float ml = warp_rank<NPL>(v, l), mh = warp_rank<NPL>(v, h);
           float scale = 0.0f;
-          if (hl == 0 && cnt > 0) {
+          if (lane == 0 && cnt > 0) {
             float sum = 0.0f;
             for (int f = 0; f < N; ++f) {
               const float x = col[f * kWarpTileRow];
@@ -1303,7 +1101,7 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
             }
             scale = __fsqrt_rn(__fdiv_rn(var, static_cast<float>(cnt)));
           }
-          scale = __shfl_sync(0xffffffffu, scale, seg * LANES);
+          scale = __shfl_sync(0xffffffffu, scale, 0);
           if (cnt > 0) {
             cs.center = __fmul_rn(__fadd_rn(ml, mh), 0.5f);
             cs.scale = scale;
@@ -1314,13 +1112,13 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
         int cl = 0, ch = 0;
 #pragma unroll
         for (int k = 0; k < NPL; ++k) {
-          if (hl * NPL + k < cnt) {
+          if (lane * NPL + k < cnt) {
             cl += v[k] < lt;
             ch += v[k] > ht;
           }
         }
-        nl = seg_sum<LANES>(cl);
-        nh = seg_sum<LANES>(ch);
+        nl = __reduce_add_sync(0xffffffffu, cl);
+        nh = __reduce_add_sync(0xffffffffu, ch);
         use_thresholds = true;
         if (nl + nh > 0) {
           // cpu/integration.py:85-99
@@ -1339,13 +1137,13 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
 #pragma unroll
         for (int k = 0; k < NPL; ++k) {
           const float x = v[k];
-          if (hl * NPL + k < cnt && !(use_thresholds && (x < lt || x > ht))) {
+          if (lane * NPL + k < cnt && !(use_thresholds && (x < lt || x > ht))) {
             ws.add(x);
             ++kept;
           }
         }
-        ff_warp_reduce<LANES>(ws);
-        kept = seg_sum<LANES>(kept);
+        ff_warp_reduce(ws);
+        kept = __reduce_add_sync(0xffffffffu, kept);
         if (kept > 0) {
           master = ff_div_f32(ws.hi, ws.lo, static_cast<float>(kept));
           weight = static_cast<float>(kept);
@@ -1354,8 +1152,8 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
         FF ws, wsum;
 #pragma unroll
         for (int k = 0; k < NPL; ++k) {
-          const int f = k * LANES + hl;
-          if (in_frame && f < N) {
+          const int f = k * 32 + lane;
+          if (f < N) {
             const float x = col[f * kWarpTileRow];
             const float w = tab.w[f];
             if (w > 0.0f && isfinite(x) && !(use_thresholds && (x < lt || x > ht))) {
@@ -1365,16 +1163,15 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
             }
           }
         }
-        ff_warp_reduce<LANES>(ws);
-        ff_warp_reduce<LANES>(wsum);
-        kept = seg_sum<LANES>(kept);
+        ff_warp_reduce(ws);
+        ff_warp_reduce(wsum);
+        kept = __reduce_add_sync(0xffffffffu, kept);
         if (kept > 0 && wsum.hi > 0.0f) {
           master = ff_div_ff(ws.hi, ws.lo, wsum.hi, wsum.lo);
           weight = wsum.value_f32();
         }
       }
-      if (hl == 0 && in_frame) {
-        if constexpr (WARP != 0) a.geometric_out[p] = static_cast<float>(s_geo[px]);
+      if (lane == 0) {
         write_outputs(a, p, master, weight, kept, nl, nh, tab.active);
       }
     }
@@ -1382,15 +1179,12 @@ __global__ void __launch_bounds__(kWarpThreads, LANES == 16 ? (NPL >= 16 ? 3 : 4
   }
 }
 
-template <int NPL, int WARP = 0, int LANES = 32>
 static void launch_warp(const IntegrateArgs& args, cudaStream_t stream) {
   const size_t tile_bytes = static_cast<size_t>(args.frames) * kWarpTileRow * sizeof(float);
-  // resident frames: double-buffered tiles while two of them stay under 100 KB
-  constexpr bool kCanPipe = WARP == 0;
-  const bool pipe = kCanPipe && 2 * tile_bytes <= 100 * 1024;
-  const size_t smem = tile_bytes * (pipe ? 2 : 1) +
-                      (WARP != 0 ? static_cast<size_t>(args.frames) * sizeof(FusedFrame) : 0);
-  auto kern = pipe ? integrate_warp_kernel<NPL, WARP, kCanPipe, LANES> : integrate_warp_kernel<NPL, WARP, false, LANES>;
+  // double-buffered tiles while two of them stay under 100 KB
+  const bool pipe = 2 * tile_bytes <= 100 * 1024;
+  const size_t smem = tile_bytes * (pipe ? 2 : 1);
+  auto kern = pipe ? integrate_warp_kernel<16, true> : integrate_warp_kernel<16, false>;
   check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
              "cudaFuncSetAttribute(integrate_warp)");
   int per_sm = 0;
@@ -1554,12 +1348,11 @@ static void launch_integrate_args(const IntegrateArgs& a, cudaStream_t stream) {
     }
   }
   else if (a.rejection != GG_REJECT_LINEAR_FIT && n <= 512) {
-    // one warp per pixel (the linear fit's serial rank walks stay below)
-    // two pixels per warp up to 256 frames (16 lanes x NPL values each)
-    if (n <= 64) launch_warp<4, 0, 16>(a, stream);
-    else if (n <= 128) launch_warp<8, 0, 16>(a, stream);
-    else if (n <= 256) launch_warp<16, 0, 16>(a, stream);
-    else launch_warp<16>(a, stream);
+    // one thread per pixel while a warp's columns fit its share of shared
+    // memory, one warp per pixel above (the linear fit's serial rank walks
+    // stay below)
+    if (n <= 256) launch_integrate_px(a, stream);
+    else launch_warp(a, stream);
   }
   else if (n <= 64) launch_reg<64>(a, stream);
   else if (n <= 128) launch_smem<4>(a, stream);
