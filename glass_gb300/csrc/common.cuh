@@ -55,8 +55,18 @@ long long launch_count();
 // that needs a few hundred bytes of parameters would otherwise wait for
 // gigabytes of unrelated upload.  The host block may be reused as soon as the
 // call returns.
-constexpr std::size_t kParamUploadMax = 64 * 1024;
+constexpr std::size_t kParamUploadMax = 96 * 1024;
 void upload_params(cudaStream_t stream, void* dst, const void* src, std::size_t bytes, const char* what);
+
+// Resident CTAs per SM of a kernel with `smem` bytes of dynamic shared memory;
+// raises the kernel's dynamic shared memory limit to that size where it is
+// lower.  Asked of the runtime once per device, kernel and launch shape: the
+// attribute and occupancy calls cost microseconds of every launch otherwise.
+int kernel_ctas_per_sm(const void* kernel, int threads, std::size_t smem, const char* what);
+template <class... A>
+int kernel_ctas_per_sm(void (*kernel)(A...), int threads, std::size_t smem, const char* what) {
+  return kernel_ctas_per_sm(reinterpret_cast<const void*>(kernel), threads, smem, what);
+}
 
 // Grid sizing for streaming kernels: a whole number of waves over the SMs.
 int sm_count();

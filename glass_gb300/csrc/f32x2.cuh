@@ -1,6 +1,11 @@
 // Two float32 lanes in one register pair (add, subtract, multiply and FMA of
 // sm_100 and later: one instruction for both lanes, each rounded as the scalar
-// instruction rounds it).
+// instruction rounds it).  Measured on this card: 64 lane pairs per clock and SM,
+// the same lanes as the scalar forms for half the issue slots.
+//
+// An f2_add of two f2_mul results is contracted to an FMA by the assembler in
+// spite of its .rn (seen on 25 % of random operands with CUDA 13.0; an f2_add of
+// one product and something else is not): add such products lane by lane.
 #pragma once
 
 #include "common.cuh"

@@ -139,9 +139,8 @@ inline bool invert3(const double* m, double* inv) {
 }
 
 // Float-float coefficients (and the affine flag) of the inverse of a forward
-// matrix; false when the matrix is singular.
-inline bool inverse_coefficients(const double* fwd, float (*m)[2], int& affine) {
-  double inv[9];
+// matrix, and the inverse itself; false when the matrix is singular.
+inline bool inverse_coefficients(const double* fwd, float (*m)[2], int& affine, double* inv) {
   if (!invert3(fwd, inv)) return false;
   // An affine matrix has an affine inverse; the cofactor formula leaves
   // inv[8] = det * (1 / det), which may round to 1 - 2^-53 and would send
@@ -158,6 +157,11 @@ inline bool inverse_coefficients(const double* fwd, float (*m)[2], int& affine) 
     m[q][1] = static_cast<float>(inv[q] - static_cast<double>(hi));
   }
   return true;
+}
+
+inline bool inverse_coefficients(const double* fwd, float (*m)[2], int& affine) {
+  double inv[9];
+  return inverse_coefficients(fwd, m, affine, inv);
 }
 
 }  // namespace gg

@@ -3,6 +3,7 @@
 // memory (engine/warp.py:99-152; warp_kernels.cu:371-777).
 #pragma once
 
+#include "f32x2.cuh"
 #include "geometry.cuh"
 
 namespace gg {
@@ -10,7 +11,7 @@ namespace gg {
 constexpr float kInfF = __builtin_huge_valf();
 // Shared-memory source box of the tiled warp (columns x rows).
 constexpr int kBoxW = 80;
-constexpr int kBoxH = 64;
+constexpr int kBoxH = 80;
 
 // sin(pi u) for |u| <= 1/2 and sin / cos of |x| <= pi/3 by their Taylor
 // series (truncation below 1e-9 on these ranges), evaluated by Horner.
@@ -46,7 +47,7 @@ constexpr float kPiF = 3.14159265358979323846f;
 // E_c even and O_c odd, evaluated as degree-5 polynomials in u^2 (fit error
 // below 3e-10, coefficients from glass_gb300/lanczos_poly.py), so the six
 // weights cost 36 FMAs and no transcendental or division.  Each weight is
-// within 1.3e-7 of the exact value (float32 rounding included); callers
+// within 1.3e-7 of the exact value (float24 rounding included); callers
 // that need the exact weights 0, 0, 1, 0, 0, 0 of an integer coordinate
 // (exact integer translations) take the source sample directly.
 // pair A (c = 0.5): max fit error 7.3e-11
@@ -113,6 +114,53 @@ __device__ __forceinline__ void lanczos3_weights(float t, float (&w)[6]) {
   w[3] = __fsub_rn(ea, oa);
   w[4] = __fsub_rn(eb, ob);
   w[5] = __fsub_rn(ec, oc);
+}
+
+// The coefficients of the six polynomials above (even a, odd a, even b, ...),
+// highest power first, twice each: a packed FMA takes no immediate operand, and
+// a pair of moves per coefficient would cost as much as the FMA saves.
+static __device__ __constant__ float2 kLanczos3Pairs[6][6] = {
+    {{1.680220594e-03f, 1.680220594e-03f}, {-9.777043946e-03f, -9.777043946e-03f}, {2.186747268e-02f, 2.186747268e-02f},
+     {6.364143640e-02f, 6.364143640e-02f}, {-4.488392770e-01f, -4.488392770e-01f}, {6.079270840e-01f, 6.079270840e-01f}},
+    {{2.676349832e-03f, 2.676349832e-03f}, {-2.544626780e-02f, -2.544626780e-02f}, {1.599001437e-01f, 1.599001437e-01f},
+     {-6.481293440e-01f, -6.481293440e-01f}, {1.468628168e+00f, 1.468628168e+00f}, {-1.329050660e+00f, -1.329050660e+00f}},
+    {{-4.255278502e-03f, -4.255278502e-03f}, {2.526676841e-02f, 2.526676841e-02f}, {-6.422392279e-02f, -6.422392279e-02f},
+     {-6.639494002e-02f, -6.639494002e-02f}, {5.606142282e-01f, 5.606142282e-01f}, {-1.350949109e-01f, -1.350949109e-01f}},
+    {{-1.830645255e-03f, -1.830645255e-03f}, {1.821853220e-02f, 1.821853220e-02f}, {-1.171571687e-01f, -1.171571687e-01f},
+     {4.563217461e-01f, 4.563217461e-01f}, {-8.275418282e-01f, -8.275418282e-01f}, {1.801265478e-01f, 1.801265478e-01f}},
+    {{4.921542015e-03f, 4.921542015e-03f}, {-3.034376726e-02f, -3.034376726e-02f}, {9.083209187e-02f, 9.083209187e-02f},
+     {-6.445738673e-02f, -6.445738673e-02f}, {-8.637610078e-02f, -8.637610078e-02f}, {2.431708388e-02f, 2.431708388e-02f}},
+    {{5.886373110e-04f, 5.886373110e-04f}, {-7.546908688e-03f, -7.546908688e-03f}, {5.576262996e-02f, 5.576262996e-02f},
+     {-2.164693773e-01f, -2.164693773e-01f}, {3.049877286e-01f, 3.049877286e-01f}, {-6.355997920e-02f, -6.355997920e-02f}}};
+
+// lanczos3_weights of four offsets, each of two samples, with the same roundings;
+// the offsets are given times 2^24.
+__device__ __forceinline__ void lanczos3_weights2(const F2 (&t24)[4], F2 (&w)[4][6]) {
+  F2 u[4], x[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    u[k] = f2_fma(t24[k], f2(5.9604644775390625e-08f), f2(-0.5f));
+    x[k] = f2_mul(u[k], u[k]);
+  }
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {  // taps at distance 1/2, 3/2, 5/2
+    F2 e[4], o[4];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const float2 ce = kLanczos3Pairs[2 * c][i], co = kLanczos3Pairs[2 * c + 1][i];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        e[k] = i == 0 ? f2(ce.x, ce.y) : f2_fma(e[k], x[k], f2(ce.x, ce.y));
+        o[k] = i == 0 ? f2(co.x, co.y) : f2_fma(o[k], x[k], f2(co.x, co.y));
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      o[k] = f2_mul(u[k], o[k]);
+      w[k][2 - c] = f2_add(e[k], o[k]);
+      w[k][3 + c] = f2_sub(e[k], o[k]);
+    }
+  }
 }
 
 // Lanczos3 weights with relative (not only absolute) accuracy, for the

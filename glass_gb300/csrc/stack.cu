@@ -6,6 +6,9 @@
 // index/loaded checks, 5979-8865 calibration entry points) and the module
 // functions cuda_available / get_device_info / host_pinned_empty_*.
 #include <algorithm>
+#include <map>
+#include <mutex>
+#include <utility>
 #include <atomic>
 #include <cmath>
 #include <mutex>
@@ -78,6 +81,34 @@ void upload_params(cudaStream_t stream, void* dst, const void* src, std::size_t 
     if (n <= kSmall) launch_param_block<kSmall>(stream, d + off, h + off, n, what);
     else launch_param_block<kLarge>(stream, d + off, h + off, n, what);
   }
+}
+
+int kernel_ctas_per_sm(const void* kernel, int threads, std::size_t smem, const char* what) {
+  struct Shape {
+    int threads;
+    std::size_t smem;
+    int per_sm;
+  };
+  struct Known {
+    std::size_t limit = 0;  // dynamic shared memory allowed so far
+    std::vector<Shape> shapes;
+  };
+  static std::mutex mutex;
+  static std::map<std::pair<int, const void*>, Known> known;
+  int device = 0;
+  check_cuda(cudaGetDevice(&device), "cudaGetDevice");
+  std::lock_guard<std::mutex> lock(mutex);
+  Known& k = known[{device, kernel}];
+  for (const Shape& s : k.shapes)
+    if (s.threads == threads && s.smem == smem) return s.per_sm;
+  if (smem > k.limit) {
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), what);
+    k.limit = smem;
+  }
+  int per_sm = 0;
+  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem), what);
+  k.shapes.push_back({threads, smem, std::max(per_sm, 1)});
+  return std::max(per_sm, 1);
 }
 
 int sm_count() {

@@ -16,20 +16,29 @@
 //   - source coordinates are evaluated in float-float (TwoProd/TwoSum) from
 //     the float64 inverse, so floor/validity decisions agree with the float64
 //     reference without float64 arithmetic on the device;
-//   - each CTA owns a 64x48 output tile; its source footprint (an 80x64 box
-//     for the small rotations registration produces) is copied to shared
-//     memory by one cp.async.bulk.tensor (TMA) load, double-buffered against
-//     the previous tile's compute.  Footprints that do not fit the box (large
-//     rotation/scale) and image widths that TMA cannot describe (W % 4 != 0)
-//     read the taps straight from global memory instead;
+//   - each CTA takes 64x64 output tiles; a tile's source footprint (an 80x80
+//     box for the small rotations registration produces) is copied to shared
+//     memory by one cp.async.bulk.tensor (TMA) load while the SM's other CTAs
+//     compute.  Footprints that do not fit the box (large rotation/scale) and
+//     image widths that TMA cannot describe (W % 4 != 0) read the taps straight
+//     from global memory instead;
 //   - output goes to a spare slot; a follow-up kernel swaps the frame->slot
 //     table, so nothing is copied back (8 B/pixel instead of 16 B);
 //   - Lanczos3 weights are paired even/odd polynomials in (t - 1/2)^2
-//     (sampling.cuh); interior tiles of finite frames run a straight-line
-//     form without per-pixel tests.
+//     (sampling.cuh); tiles of affine maps run straight-line rows: two columns
+//     per thread in packed float32, coordinates in fixed point, two output rows
+//     from seven source rows.  Projective maps, the overshoot clamp, nearest
+//     and very large footprints take the general path (warp_tile_rows).
+//
+// Bound: the FMA pipe (of 143 instructions per Lanczos3 pixel, the weights are
+// 41 packed, the taps 21; 57 % of the pipe, 56 % of the issue slots at 16 warps
+// per SM).  15 moving frames of 2048^2: Lanczos3 642 -> 438 us, bilinear 417 ->
+// 159 us; frames with non-finite samples (23 of 512^2, Lanczos3) 275 -> 227 us.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
+#include <type_traits>
 #include <vector>
 
 #include <cudaTypedefs.h>
@@ -42,13 +51,15 @@
 namespace gg {
 
 constexpr int kTileW = 64;
-constexpr int kTileH = 48;
-constexpr int kWarpThreads = 256;  // 64 x 4; each thread covers kTileH / 4 rows
-constexpr int kRowsPerThread = kTileH / 4;
+constexpr int kTileH = 64;       // rows of a tile
+constexpr int kSmallTileH = 16;  // where a launch has few tiles
+constexpr int kWarpThreads = 128;
+constexpr int kRowClasses = 4;  // rows y, y + 4, y + 8, ... of a tile share a chain of coordinates
 // Affine source coordinates are stepped by 4 output rows in float-float and
 // evaluated afresh every kFreshRows rows: at most three steps of rounding
 // separate a coordinate from the float64-faithful evaluation, so floor and
-// fraction decisions stay those of a direct evaluation.
+// fraction decisions stay those of a direct evaluation.  Tile heights are
+// multiples of 16 rows, so a row's chain does not depend on its tile.
 constexpr int kFreshRows = 4;
 
 struct WarpItem {
@@ -60,6 +71,7 @@ struct WarpItem {
   int int_shift;  // inverse is an exact integer translation
   float* dst;     // first row of the output rows (filled on the device)
   float m[9][2];  // inverse matrix, float-float (hi, lo), row-major
+  double inv[6];  // its first two rows
 };
 
 struct WarpArgs {
@@ -72,10 +84,9 @@ struct WarpArgs {
   int height;
   int row0, row1;  // output rows [row0, row1); row0 is the first row at WarpItem::dst
   int tiles_x;
-  int tiles_y;     // of those rows
+  int tiles_y;     // of those rows (set by the launch)
   float fill;
   float clamp;
-  int every_row;  // coordinates of tiles that are not interior afresh for every row
   float* coverage;  // optional accumulator (+1 per covered pixel)
   int* error;
 };
@@ -102,48 +113,82 @@ __device__ __forceinline__ Coef load_coef(const WarpItem* p) {
 // first pixel is (tile_x0, tile_y0).
 struct TilePlan {
   int bx, by, fits, interior;
+  int grid;  // affine, and small enough for the fixed-point coordinates
 };
 
 // interior: an affine map sends the whole tile at least one pixel inside the
 // valid source range (valid_lo <= s <= valid_hi on both axes), so no pixel
 // of the tile needs its own validity test.
-__device__ __forceinline__ TilePlan plan_tile(const Coef& it, int tile_x0, int tile_y0, int radius, float valid_lo,
-                                              float valid_hi_x, float valid_hi_y) {
-  const float x0 = static_cast<float>(tile_x0), y0 = static_cast<float>(tile_y0);
-  const float cx[4] = {x0, x0 + kTileW - 1, x0, x0 + kTileW - 1};
-  const float cy[4] = {y0, y0, y0 + kTileH - 1, y0 + kTileH - 1};
-  float minx = kInfF, maxx = -kInfF, miny = kInfF, maxy = -kInfF;
-  bool ok = true;
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    FFv sx, sy;
-    ok &= source_coord(it, cx[c], cy[c], sx, sy);
-    minx = fminf(minx, sx.hi);
-    maxx = fmaxf(maxx, sx.hi);
-    miny = fminf(miny, sy.hi);
-    maxy = fmaxf(maxy, sy.hi);
-  }
-  TilePlan p{0, 0, 0, 0};
-  if (!ok || !(maxx - minx < 1.0e6f) || !(maxy - miny < 1.0e6f) || fabsf(minx) > 1.0e8f || fabsf(miny) > 1.0e8f)
+// Source range of a tile: bounding box of its corners' source points; !ok: a
+// corner has none.
+struct TileRange {
+  float minx, maxx, miny, maxy;
+  bool ok;
+};
+
+__device__ __forceinline__ TilePlan plan_of_range(const TileRange& s, bool affine, int radius, float valid_lo,
+                                                  float valid_hi_x, float valid_hi_y) {
+  TilePlan p{0, 0, 0, 0, 0};
+  if (!s.ok || !(s.maxx - s.minx < 1.0e6f) || !(s.maxy - s.miny < 1.0e6f) || fabsf(s.minx) > 1.0e8f ||
+      fabsf(s.miny) > 1.0e8f)
     return p;
   // taps span [floor(s) - (radius-1), floor(s) + radius]; one pixel of margin.
-  const int lo_x = static_cast<int>(floorf(minx)) - radius;
-  const int hi_x = static_cast<int>(floorf(maxx)) + radius + 1;  // inclusive
-  const int lo_y = static_cast<int>(floorf(miny)) - radius;
-  const int hi_y = static_cast<int>(floorf(maxy)) + radius + 1;
+  const int lo_x = static_cast<int>(floorf(s.minx)) - radius;
+  const int hi_x = static_cast<int>(floorf(s.maxx)) + radius + 1;  // inclusive
+  const int lo_y = static_cast<int>(floorf(s.miny)) - radius;
+  const int hi_y = static_cast<int>(floorf(s.maxy)) + radius + 1;
   p.bx = lo_x >= 0 ? (lo_x & ~3) : -((-lo_x + 3) & ~3);  // 16-byte aligned x (TMA rule)
   p.by = lo_y;
   p.fits = (hi_x - p.bx < kBoxW) && (hi_y - p.by < kBoxH);
-  p.interior = it.affine && minx >= valid_lo + 1.0f && maxx <= valid_hi_x - 1.0f && miny >= valid_lo + 1.0f &&
-               maxy <= valid_hi_y - 1.0f;
+  p.grid = affine && s.maxx - s.minx < 256.0f && s.maxy - s.miny < 256.0f;
+  p.interior = affine && s.minx >= valid_lo + 1.0f && s.maxx <= valid_hi_x - 1.0f && s.miny >= valid_lo + 1.0f &&
+               s.maxy <= valid_hi_y - 1.0f;
   return p;
 }
 
-// The output pixels of one thread in a 64 x 48 tile: column ox, rows oy0,
+template <int TH>
+__device__ __forceinline__ TilePlan plan_tile(const Coef& it, int tile_x0, int tile_y0, int radius, float valid_lo,
+                                              float valid_hi_x, float valid_hi_y) {
+  TileRange s{kInfF, -kInfF, kInfF, -kInfF, true};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    FFv sx, sy;
+    s.ok &= source_coord(it, static_cast<float>(tile_x0 + (c & 1) * (kTileW - 1)),
+                         static_cast<float>(tile_y0 + (c >> 1) * (TH - 1)), sx, sy);
+    s.minx = fminf(s.minx, sx.hi);
+    s.maxx = fmaxf(s.maxx, sx.hi);
+    s.miny = fminf(s.miny, sy.hi);
+    s.maxy = fmaxf(s.maxy, sy.hi);
+  }
+  return plan_of_range(s, it.affine != 0, radius, valid_lo, valid_hi_x, valid_hi_y);
+}
+
+// plan_tile by a whole warp, a corner per lane (the plan in every lane).
+template <int TH>
+__device__ __forceinline__ TilePlan plan_tile_warp(const Coef& it, int tile_x0, int tile_y0, int radius,
+                                                   float valid_lo, float valid_hi_x, float valid_hi_y) {
+  const int c = threadIdx.x & 3;
+  FFv sx, sy;
+  TileRange s;
+  s.ok = __all_sync(0xffffffffu, source_coord(it, static_cast<float>(tile_x0 + (c & 1) * (kTileW - 1)),
+                                              static_cast<float>(tile_y0 + (c >> 1) * (TH - 1)), sx, sy));
+  s.minx = s.maxx = sx.hi;
+  s.miny = s.maxy = sy.hi;
+#pragma unroll
+  for (int off = 1; off < 4; off <<= 1) {
+    s.minx = fminf(s.minx, __shfl_xor_sync(0xffffffffu, s.minx, off));
+    s.maxx = fmaxf(s.maxx, __shfl_xor_sync(0xffffffffu, s.maxx, off));
+    s.miny = fminf(s.miny, __shfl_xor_sync(0xffffffffu, s.miny, off));
+    s.maxy = fmaxf(s.maxy, __shfl_xor_sync(0xffffffffu, s.maxy, off));
+  }
+  return plan_of_range(s, it.affine != 0, radius, valid_lo, valid_hi_x, valid_hi_y);
+}
+
+// The output pixels of one column and row class of a tile: column ox, rows oy0,
 // oy0 + 4, ...; dst is the frame's output row 0.
 // FINITE: the source frame holds no non-finite sample (every Lanczos3 window
 // takes the plain normalised sum); returns the count of non-finite outputs.
-template <int INTERP, bool FINITE>
+template <int INTERP, bool FINITE, int TH>
 __device__ __forceinline__ unsigned warp_tile_rows(const WarpArgs& a, const Coef& co, const TapSource& ts, float* dst,
                                                    int ox, int oy0, bool interior, bool int_shift) {
   constexpr int radius = (INTERP == GG_INTERP_LANCZOS3) ? 3 : 1;
@@ -156,13 +201,13 @@ __device__ __forceinline__ unsigned warp_tile_rows(const WarpArgs& a, const Coef
   const float step_x_hi = 4.0f * co.m[1][0], step_x_lo = 4.0f * co.m[1][1];
   const float step_y_hi = 4.0f * co.m[4][0], step_y_lo = 4.0f * co.m[4][1];
 #pragma unroll 1
-  for (int r = 0; r < kRowsPerThread; ++r) {
+  for (int r = 0; r < TH / kRowClasses; ++r) {
     const int oy = oy0 + 4 * r;
     const bool inside = ox < a.width && oy < a.row1;
     bool valid = false;
     float value = a.fill;
     if (co.affine) {
-      if (r % kFreshRows == 0 || a.every_row) {
+      if (r % kFreshRows == 0) {
         row_ok = source_coord(co, static_cast<float>(ox), static_cast<float>(oy), sx_row, sy_row);
       } else {
         sx_row = ff_add_ff(sx_row, step_x_hi, step_x_lo);
@@ -223,68 +268,394 @@ __device__ __forceinline__ unsigned warp_tile_rows(const WarpArgs& a, const Coef
   return bad;
 }
 
-// The common Lanczos3 tile in straight-line form: an affine map, the whole
-// 64 x 48 tile inside the output and mapped at least one pixel inside the
-// valid source range, its footprint staged in the shared-memory box, a source
-// frame without non-finite samples, no clamp and no coverage map.  Every
-// pixel is then valid and takes the plain normalised 6 x 6 sum, so the rows
-// need no per-pixel tests (same arithmetic as the general path).
-__device__ __forceinline__ unsigned warp_tile_rows_fast(const WarpArgs& a, const Coef& co, const float* box, int bx,
-                                                        int by, float* dst, int ox, int oy0) {
-  FFv sx, sy;
-  const float step_x_hi = 4.0f * co.m[1][0], step_x_lo = 4.0f * co.m[1][1];
-  const float step_y_hi = 4.0f * co.m[4][0], step_y_lo = 4.0f * co.m[4][1];
-  float* out = dst + static_cast<int64_t>(oy0) * a.width + ox;
-  const int64_t out_step = 4 * static_cast<int64_t>(a.width);
+// ---- straight-line rows ---------------------------------------------------------
+// Tiles of an affine map (Lanczos3: without clamp), with the arithmetic of
+// the general path but for the coordinates' last bits.  A thread takes 16 (4 in
+// small tiles) consecutive rows of two columns, x and x + 32, as the two lanes of
+// packed float32.  Interior tiles (mapped at least one pixel inside the valid
+// source range, whole inside the output) need no test per pixel; the others are
+// masked.
+
+// Source coordinates within a tile, in fixed point with 54 fraction bits
+// relative to a whole origin (the staged box, or the tile's first source pixel):
+// a step along a row or column is an exact integer add on the otherwise idle
+// integer pipe, where the float-float step took 11 of the FMA pipe's operations
+// per axis.  The tile's first coordinate is evaluated in float64, the steps'
+// rounding moves a coordinate by at most 128 x 2^-55 pixels within a tile: as
+// close to the float64 reference as its own rounding.
+constexpr int kGridBits = 54;
+
+struct TileGrid {
+  long long x0, y0;  // source of the tile's first pixel, relative to (ox, oy)
+  long long a, d, b, e;  // steps of x and y along a row, down a column
+  int ox, oy;
+};
+
+// By a whole warp: lanes 0 to 5 make one value each.
+__device__ __forceinline__ void tile_grid_warp(const double* inv, int tile_x0, int tile_y0, bool staged, int bx,
+                                               int by, TileGrid& out) {
+  const int lane = threadIdx.x & 31, axis = lane & 1;
+  const double* row = inv + 3 * axis;
+  constexpr double kOne = static_cast<double>(1ll << kGridBits);
+  double v;
+  int origin = 0;
+  if (lane < 2) {
+    v = fma(row[0], static_cast<double>(tile_x0), fma(row[1], static_cast<double>(tile_y0), row[2]));
+    origin = staged ? (axis ? by : bx) : static_cast<int>(floor(v));
+    v -= origin;
+  } else {
+    v = lane < 4 ? row[0] : row[1];
+  }
+  if (lane < 6) (&out.x0)[lane] = __double2ll_rn(v * kOne);
+  if (lane < 2) (&out.ox)[lane] = origin;
+}
+
+constexpr float kTwoToMinus24 = 5.9604644775390625e-08f;
+
+// The coordinates of a thread's two columns, x and x + 32, down its rows.
+struct RowWalk {
+  long long xa, xb, ya, yb;
+  __device__ __forceinline__ RowWalk(const TileGrid& g, int lx, int ly) {
+    xa = g.x0 + lx * g.a + ly * g.b;
+    ya = g.y0 + lx * g.d + ly * g.e;
+    xb = xa + 32 * g.a;
+    yb = ya + 32 * g.d;
+  }
+  __device__ __forceinline__ void next(const TileGrid& g) {
+    xa += g.b;
+    xb += g.b;
+    ya += g.e;
+    yb += g.e;
+  }
+  static __device__ __forceinline__ int whole(long long v) { return static_cast<int>(v >> kGridBits); }
+  // 2^24 times the fractions of both columns, rounded once to float32: two exact
+  // halves of 24 bits and an FMA.
+  static __device__ __forceinline__ F2 fraction24(long long p, long long q) {
+    auto high = [](long long v) { return __uint2float_rn(static_cast<unsigned>(v >> (kGridBits - 24)) & 0xffffffu); };
+    auto low = [](long long v) { return __uint2float_rn(static_cast<unsigned>(v >> (kGridBits - 48)) & 0xffffffu); };
+    return f2_fma(f2(low(p), low(q)), f2(kTwoToMinus24), f2(high(p), high(q)));
+  }
+  __device__ __forceinline__ F2 x24() const { return fraction24(xa, xb); }
+  __device__ __forceinline__ F2 y24() const { return fraction24(ya, yb); }
+};
+
+// Pixels of a masked tile: those inside the output (columns left of ncols, rows
+// above nrows of the tile) are written, and valid where the source coordinate
+// lies in [lo, hi) on both axes.
+struct TileMask {
+  long long lox, hix, loy, hiy;
+  int ncols, nrows;
+  float* coverage;  // optional: +1 per valid pixel, laid out like the output
+};
+
+__device__ __forceinline__ TileMask tile_mask(const TileGrid& g, bool lanczos, int width, int height, int tile_x0,
+                                              int tile_y0, int row1, float* coverage) {
+  auto fixed = [](int v) { return static_cast<long long>(min(max(v, -511), 511)) << kGridBits; };
+  const int lo = lanczos ? 2 : 0, off = lanczos ? 3 : 1;
+  TileMask m;
+  m.lox = fixed(lo - g.ox);
+  m.loy = fixed(lo - g.oy);
+  // bilinear takes the last sample itself too
+  m.hix = fixed(width - off - g.ox) + (lanczos ? 0 : 1);
+  m.hiy = fixed(height - off - g.oy) + (lanczos ? 0 : 1);
+  m.ncols = width - tile_x0;
+  m.nrows = row1 - tile_y0;
+  m.coverage = coverage;
+  return m;
+}
+
+// Samples of the staged box (kBoxW columns) or of the frame itself, at positions
+// relative to the grid's origin; (x0, y0) to (x1, y1) are the first and last that
+// a window may start at.  CLAMP keeps the windows of invalid pixels inside the
+// frame (the staged box holds them all).
+template <bool STAGED>
+struct Window {
+  static constexpr bool kStaged = STAGED;
+  using Index = std::conditional_t<STAGED, int, int64_t>;
+  const float* data;
+  int width;
+  int x0, x1, y0, y1;
+  __device__ __forceinline__ int pitch() const { return STAGED ? kBoxW : width; }
+  template <bool CLAMP>
+  __device__ __forceinline__ Index at(int x, int y) const {
+    if constexpr (CLAMP && !STAGED) {
+      x = min(max(x, x0), x1);
+      y = min(max(y, y0), y1);
+    }
+    return static_cast<Index>(y) * pitch() + x;
+  }
+  __device__ __forceinline__ float load(Index i) const { return STAGED ? data[i] : __ldg(data + i); }
+};
+
+// Writes one pixel of a masked tile (`sampled`: its window has a value); returns
+// whether it is non-finite.
+__device__ __forceinline__ unsigned write_masked(const TileMask& m, float* out, int64_t at, int lx, int ly,
+                                                 long long x, long long y, float value, float fill,
+                                                 bool sampled = true) {
+  const bool valid = sampled && x >= m.lox && x < m.hix && y >= m.loy && y < m.hiy;
+  if (lx >= m.ncols || ly >= m.nrows) return 0u;
+  const float v = valid ? value : fill;
+  out[at] = v;
+  if (m.coverage && valid) atomicAdd(m.coverage + at, 1.0f);
+  return isfinite(v) ? 0u : 1u;
+}
+
+// Non-finite samples among those that a thread wrote (all finite but for
+// overflow: counted only when their product with zero is not zero).
+__device__ __forceinline__ unsigned count_nonfinite(F2 probe, const float* out, int64_t pitch, int rows) {
+  if (f2_sum(probe) == 0.0f) return 0u;
   unsigned bad = 0;
-#pragma unroll 1
-  for (int r = 0; r < kRowsPerThread; ++r) {
-    if (r % kFreshRows == 0) {
-      source_coord(co, static_cast<float>(ox), static_cast<float>(oy0 + 4 * r), sx, sy);
-    } else {
-      sx = ff_add_ff(sx, step_x_hi, step_x_lo);
-      sy = ff_add_ff(sy, step_y_hi, step_y_lo);
-    }
-    int x0, y0;
-    float tx, ty;
-    ff_floor_frac(sx, x0, tx);
-    ff_floor_frac(sy, y0, ty);
-    float wx[6], wy[6];
-    lanczos3_weights(tx, wx);
-    lanczos3_weights(ty, wy);
-    float swx = 0.0f, swy = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      swx += wx[i];
-      swy += wy[i];
-    }
-    const float* r0 = box + (y0 - 2 - by) * kBoxW + (x0 - 2 - bx);
-    float acc = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 6; ++j) {
-      float row = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 6; ++i) row = __fmaf_rn(wx[i], r0[j * kBoxW + i], row);
-      acc = __fmaf_rn(wy[j], row, acc);
-    }
-    const float wsum = swx * swy;
-    const float value = fabsf(wsum) > 1.0e-12f ? __fdividef(acc, wsum) : a.fill;
-    out[r * out_step] = value;
-    bad += isfinite(value) ? 0u : 1u;
+  for (int r = 0; r < rows; ++r) {
+    bad += isfinite(out[r * pitch]) ? 0u : 1u;
+    bad += isfinite(out[r * pitch + 32]) ? 0u : 1u;
   }
   return bad;
 }
 
-template <int INTERP, bool USE_TMA>
-__global__ void __launch_bounds__(kWarpThreads, 3) warp_tiles_kernel(const __grid_constant__ CUtensorMap tmap,
+// __fdividef for a divisor that needs no scaling (near 1).
+__device__ __forceinline__ float quotient_near_one(float a, float b) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+  return __fmul_rn(a, r);
+}
+
+// Sums of both columns' 6 x 6 windows at na, nb.
+template <bool STAGED>
+__device__ __forceinline__ F2 window_sum(const Window<STAGED>& win, typename Window<STAGED>::Index na,
+                                         typename Window<STAGED>::Index nb, const F2 (&wx)[6], const F2 (&wy)[6]) {
+  F2 acc;
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    F2 row;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const F2 v = f2(win.load(na + j * win.pitch() + i), win.load(nb + j * win.pitch() + i));
+      row = i == 0 ? f2_mul(wx[0], v) : f2_fma(wx[i], v, row);
+    }
+    acc = j == 0 ? f2_mul(wy[0], row) : f2_fma(wy[j], row, acc);
+  }
+  return acc;
+}
+
+// Lanczos3, two rows at a time: where the second row's windows lie one source
+// row below the first's (nearly always: scale and rotation move them by
+// hundredths of a pixel per row), the seven source rows are loaded once for
+// both, 21 loads per sample instead of 36.  (Windows kept in registers over all
+// 16 rows need 6 loads, but a loop unrolled by 6 rows, and 30 KB of it starved
+// the instruction cache: 843 us for five 4096^2 frames.)
+template <int ROWS, bool STAGED, bool MASK>
+__device__ __forceinline__ unsigned lanczos3_rows(const TileGrid& grid, const Window<STAGED> win,
+                                                  const TileMask& mask, float fill, float* out, int64_t out_pitch,
+                                                  int lx, int ly) {
+  RowWalk at(grid, lx, ly);
+  const int pitch = win.pitch();
+  F2 probe;
+  unsigned bad = 0;
+#pragma unroll 1
+  for (int r = 0; r < ROWS; r += 2) {
+    typename Window<STAGED>::Index na[2], nb[2];
+    F2 t[4], w[4][6], wsum[2];  // x and y of the first row, x and y of the second
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      t[2 * q] = at.x24();
+      t[2 * q + 1] = at.y24();
+      na[q] = win.template at<MASK>(RowWalk::whole(at.xa) - 2, RowWalk::whole(at.ya) - 2);
+      nb[q] = win.template at<MASK>(RowWalk::whole(at.xb) - 2, RowWalk::whole(at.yb) - 2);
+      at.next(grid);
+    }
+    lanczos3_weights2(t, w);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      F2 swx = w[2 * q][0], swy = w[2 * q + 1][0];
+#pragma unroll
+      for (int i = 1; i < 6; ++i) {
+        swx = f2_add(swx, w[2 * q][i]);
+        swy = f2_add(swy, w[2 * q + 1][i]);
+      }
+      wsum[q] = f2_mul(swx, swy);
+    }
+    F2 acc[2];
+    if (__builtin_expect(__all_sync(0xffffffffu, na[1] == na[0] + pitch && nb[1] == nb[0] + pitch), 1)) {
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+        F2 v[6];
+#pragma unroll
+        for (int i = 0; i < 6; ++i) v[i] = f2(win.load(na[0] + j * pitch + i), win.load(nb[0] + j * pitch + i));
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const int k = j - q;  // row of this window
+          if (k < 0 || k > 5) continue;
+          F2 row = f2_mul(w[2 * q][0], v[0]);
+#pragma unroll
+          for (int i = 1; i < 6; ++i) row = f2_fma(w[2 * q][i], v[i], row);
+          acc[q] = k == 0 ? f2_mul(w[2 * q + 1][0], row) : f2_fma(w[2 * q + 1][k], row, acc[q]);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 2; ++q) acc[q] = window_sum(win, na[q], nb[q], w[2 * q], w[2 * q + 1]);
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      float sa, sb, da, db;
+      f2_split(acc[q], sa, sb);
+      f2_split(wsum[q], da, db);
+      // all taps count: the weights sum to 1 within a few per cent
+      const float va = quotient_near_one(sa, da), vb = quotient_near_one(sb, db);
+      if constexpr (MASK) {
+        // the walk has moved on by two rows
+        const long long k = 2 - q;
+        bad += write_masked(mask, out, (r + q) * out_pitch, lx, ly + r + q, at.xa - k * grid.b, at.ya - k * grid.e,
+                            va, fill);
+        bad += write_masked(mask, out, (r + q) * out_pitch + 32, lx + 32, ly + r + q, at.xb - k * grid.b,
+                            at.yb - k * grid.e, vb, fill);
+      } else {
+        out[(r + q) * out_pitch] = va;
+        out[(r + q) * out_pitch + 32] = vb;
+        probe = f2_fma(f2(va, vb), F2(), probe);
+      }
+    }
+  }
+  return MASK ? bad : count_nonfinite(probe, out, out_pitch, ROWS);
+}
+
+// Lanczos3 from a frame with non-finite samples: the float-float sums over the
+// finite taps and their weights (lanczos3_nonfinite), where a tap that does not
+// count adds an exact zero.
+template <int ROWS, bool STAGED>
+__device__ __forceinline__ unsigned lanczos3_renorm_rows(const TileGrid& grid, const Window<STAGED> win,
+                                                         const TileMask& mask, float fill, float* out,
+                                                         int64_t out_pitch, int lx, int ly) {
+  RowWalk at(grid, lx, ly);
+  const int pitch = win.pitch();
+  unsigned bad = 0;
+#pragma unroll 1
+  for (int r = 0; r < ROWS; ++r) {
+    float wxa[6], wxb[6], wya[6], wyb[6], ta, tb;
+    f2_split(f2_mul(at.x24(), f2(kTwoToMinus24)), ta, tb);
+    lanczos3_weights_trig(ta, wxa);
+    lanczos3_weights_trig(tb, wxb);
+    f2_split(f2_mul(at.y24(), f2(kTwoToMinus24)), ta, tb);
+    lanczos3_weights_trig(ta, wya);
+    lanczos3_weights_trig(tb, wyb);
+    auto na = win.template at<true>(RowWalk::whole(at.xa) - 2, RowWalk::whole(at.ya) - 2);
+    auto nb = win.template at<true>(RowWalk::whole(at.xb) - 2, RowWalk::whole(at.yb) - 2);
+    FF2 sum, weight;
+#pragma unroll 1
+    for (int j = 0; j < 6; ++j, na += pitch, nb += pitch) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) {
+        const float a = win.load(na + i), b = win.load(nb + i);
+        const bool fa = isfinite(a), fb = isfinite(b);
+        const F2 v = f2(fa ? a : 0.0f, fb ? b : 0.0f);
+        const F2 w = f2(fa ? wya[j] * wxa[i] : 0.0f, fb ? wyb[j] * wxb[i] : 0.0f);
+        const F2 p = f2_mul(w, v);
+        const F2 pe = f2_fma(w, v, f2_sub(F2(), p));
+        sum.add(p);
+        sum.lo = f2_add(sum.lo, pe);
+        weight.add(w);
+      }
+    }
+    float sh[2], sl[2], wh[2], wl[2];
+    f2_split(sum.hi, sh[0], sh[1]);
+    f2_split(sum.lo, sl[0], sl[1]);
+    f2_split(weight.hi, wh[0], wh[1]);
+    f2_split(weight.lo, wl[0], wl[1]);
+    float value[2];
+    bool sampled[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      sampled[k] = fabsf(__fadd_rn(wh[k], wl[k])) > 1.0e-12f;
+      value[k] = ff_div_ff(sh[k], sl[k], wh[k], wl[k]);
+    }
+    bad += write_masked(mask, out, r * out_pitch, lx, ly + r, at.xa, at.ya, value[0], fill, sampled[0]);
+    bad += write_masked(mask, out, r * out_pitch + 32, lx + 32, ly + r, at.xb, at.yb, value[1], fill, sampled[1]);
+    at.next(grid);
+  }
+  return bad;
+}
+
+// Lanczos3 by a whole shift: the weights are exactly 0, 0, 1, 0, 0, 0, so each
+// sample is the source's own, or none where that is not finite.
+template <int ROWS, bool STAGED>
+__device__ __forceinline__ unsigned shifted_rows(const TileGrid& grid, const Window<STAGED> win, const TileMask& mask,
+                                                 float fill, float* out, int64_t out_pitch, int lx, int ly) {
+  RowWalk at(grid, lx, ly);
+  unsigned bad = 0;
+#pragma unroll 4
+  for (int r = 0; r < ROWS; ++r) {
+    const auto na = win.template at<true>(RowWalk::whole(at.xa) - 2, RowWalk::whole(at.ya) - 2);
+    const auto nb = win.template at<true>(RowWalk::whole(at.xb) - 2, RowWalk::whole(at.yb) - 2);
+    const float a = win.load(na + 2 * win.pitch() + 2), b = win.load(nb + 2 * win.pitch() + 2);
+    bad += write_masked(mask, out, r * out_pitch, lx, ly + r, at.xa, at.ya, a, fill, isfinite(a));
+    bad += write_masked(mask, out, r * out_pitch + 32, lx + 32, ly + r, at.xb, at.yb, b, fill, isfinite(b));
+    at.next(grid);
+  }
+  return bad;
+}
+
+// Sum of two packed products, lane by lane (each product rounded).
+__device__ __forceinline__ F2 add_products(F2 a, F2 b) {
+  float ax, ay, bx, by;
+  f2_split(a, ax, ay);
+  f2_split(b, bx, by);
+  return f2(__fadd_rn(ax, bx), __fadd_rn(ay, by));
+}
+
+// Bilinear.
+template <int ROWS, bool STAGED, bool MASK>
+__device__ __forceinline__ unsigned bilinear_rows(const TileGrid& grid, const Window<STAGED> win,
+                                                  const TileMask& mask, float fill, float* out, int64_t out_pitch,
+                                                  int lx, int ly) {
+  RowWalk at(grid, lx, ly);
+  const int pitch = win.pitch();
+  F2 probe;
+  unsigned bad = 0;
+#pragma unroll 4
+  for (int r = 0; r < ROWS; ++r) {
+    const F2 tx = f2_mul(at.x24(), f2(kTwoToMinus24)), ty = f2_mul(at.y24(), f2(kTwoToMinus24));
+    const int xa = RowWalk::whole(at.xa), xb = RowWalk::whole(at.xb);
+    const int ya = RowWalk::whole(at.ya), yb = RowWalk::whole(at.yb);
+    const auto na = win.template at<MASK>(xa, ya), nb = win.template at<MASK>(xb, yb);
+    // the last column's and row's right and lower neighbours are themselves
+    const int ra = !MASK || xa < win.x1 ? 1 : 0, rb = !MASK || xb < win.x1 ? 1 : 0;
+    const int da = !MASK || ya < win.y1 ? pitch : 0, db = !MASK || yb < win.y1 ? pitch : 0;
+    const F2 v00 = f2(win.load(na), win.load(nb)), v01 = f2(win.load(na + ra), win.load(nb + rb));
+    const F2 v10 = f2(win.load(na + da), win.load(nb + db));
+    const F2 v11 = f2(win.load(na + da + ra), win.load(nb + db + rb));
+    const F2 one = f2(1.0f), ox_ = f2_sub(one, tx), oy_ = f2_sub(one, ty);
+    const F2 top = add_products(f2_mul(v00, ox_), f2_mul(v01, tx));
+    const F2 bottom = add_products(f2_mul(v10, ox_), f2_mul(v11, tx));
+    const F2 v = add_products(f2_mul(top, oy_), f2_mul(bottom, ty));
+    float va, vb;
+    f2_split(v, va, vb);
+    if constexpr (MASK) {
+      bad += write_masked(mask, out, r * out_pitch, lx, ly + r, at.xa, at.ya, va, fill);
+      bad += write_masked(mask, out, r * out_pitch + 32, lx + 32, ly + r, at.xb, at.yb, vb, fill);
+    } else {
+      out[r * out_pitch] = va;
+      out[r * out_pitch + 32] = vb;
+      probe = f2_fma(v, F2(), probe);
+    }
+    at.next(grid);
+  }
+  return MASK ? bad : count_nonfinite(probe, out, out_pitch, ROWS);
+}
+
+// Two box buffers: the next tile's copy is in flight while this one's rows are
+// computed.
+constexpr size_t kWarpTileBytes = size_t(2) * kBoxH * kBoxW * sizeof(float);
+
+template <int INTERP, bool USE_TMA, int TH>
+__global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __grid_constant__ CUtensorMap tmap,
                                                                   WarpArgs a) {
-  __shared__ alignas(128) float tile[2][kBoxH * kBoxW];
+  extern __shared__ __align__(128) float warp_boxes[];  // USE_TMA: [2][kBoxH * kBoxW]
   __shared__ alignas(8) uint64_t bar[2];
-  __shared__ int s_bx[2], s_by[2], s_fit[2], s_interior[2];
+  __shared__ TilePlan s_plan[2];
+  __shared__ TileGrid s_grid[2];
   __shared__ int s_abort;
-  constexpr int radius = (INTERP == GG_INTERP_LANCZOS3) ? 3 : 1;
+  constexpr bool kLanczos = INTERP == GG_INTERP_LANCZOS3;
   const int tid = threadIdx.x;
-  const int lx = tid & 63, ly = tid >> 6;
   const int tiles = a.tiles_x * a.tiles_y;
   const int items = a.item_count * tiles;
   if (tid == 0) {
@@ -295,49 +666,47 @@ __global__ void __launch_bounds__(kWarpThreads, 3) warp_tiles_kernel(const __gri
   }
   __syncthreads();
 
+  // Warp 0 plans a tile and starts its copy.
   auto issue = [&](int item, int buf) {
-    // thread 0 only
     const WarpItem* ip = a.items + item / tiles;
-    const int t = item % tiles;
+    const Coef co = load_coef(ip);
+    const int t = item % tiles, tile_x0 = t % a.tiles_x * kTileW, tile_y0 = a.row0 + t / a.tiles_x * TH;
     // validity ranges: bilinear 0 <= s <= W - 1; Lanczos3 2 <= s < W - 3
-    const float vlo = INTERP == GG_INTERP_LANCZOS3 ? 2.0f : 0.0f;
-    const float vhx = static_cast<float>(a.width) - (INTERP == GG_INTERP_LANCZOS3 ? 3.0f : 1.0f);
-    const float vhy = static_cast<float>(a.height) - (INTERP == GG_INTERP_LANCZOS3 ? 3.0f : 1.0f);
-    TilePlan p = plan_tile(load_coef(ip), t % a.tiles_x * kTileW, a.row0 + t / a.tiles_x * kTileH, radius, vlo, vhx,
-                           vhy);
+    const float vlo = kLanczos ? 2.0f : 0.0f, off = kLanczos ? 3.0f : 1.0f;
+    TilePlan p = plan_tile_warp<TH>(co, tile_x0, tile_y0, kLanczos ? 3 : 1, vlo, static_cast<float>(a.width) - off,
+                                static_cast<float>(a.height) - off);
     if (!USE_TMA) p.fits = 0;
-    s_interior[buf] = p.interior;
-    s_bx[buf] = p.bx;
-    s_by[buf] = p.by;
-    s_fit[buf] = p.fits;
+    if (INTERP != GG_INTERP_NEAREST && p.grid)
+      tile_grid_warp(ip->inv, tile_x0, tile_y0, p.fits != 0, p.bx, p.by, s_grid[buf]);
+    if (tid != 0) return;
+    s_plan[buf] = p;
     if (p.fits) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       mbar_expect_tx(&bar[buf], kBoxW * kBoxH * 4);
-      tma_load_3d(tile[buf], &tmap, p.bx, p.by, __ldg(&ip->src_slot), &bar[buf]);
+      tma_load_3d(warp_boxes + buf * (kBoxH * kBoxW), &tmap, p.bx, p.by, __ldg(&ip->src_slot), &bar[buf]);
     }
   };
 
   unsigned phase[2] = {0u, 0u};
   int item = blockIdx.x;
-  if (tid == 0 && item < items) issue(item, 0);
+  if (tid < 32 && item < items) issue(item, 0);
   __syncthreads();
   for (int i = 0; item < items; ++i, item += gridDim.x) {
     const int buf = i & 1;
     const int next = item + gridDim.x;
-    if (tid == 0 && next < items) issue(next, buf ^ 1);
+    if (tid < 32 && next < items) issue(next, buf ^ 1);
+    const TilePlan p = s_plan[buf];
+    const float* tile = warp_boxes + buf * (kBoxH * kBoxW);
     const int item_index = item / tiles;
     const WarpItem* ip = a.items + item_index;
-    const Coef co = load_coef(ip);
     const int it_frame = __ldg(&ip->frame);
-    const int it_src = __ldg(&ip->src_slot);
-    float* const it_dst = ip->dst;
-    const unsigned it_nonfinite = __ldg(&ip->src_nonfinite);
+    const float* src = a.slots + static_cast<int64_t>(__ldg(&ip->src_slot)) * a.stride;
+    float* const dst = ip->dst - static_cast<int64_t>(a.row0) * a.width;
+    const bool finite = __ldg(&ip->src_nonfinite) == 0u;
     const bool int_shift = __ldg(&ip->int_shift) != 0;
     const int t = item - item_index * tiles;
-    const int tile_x0 = t % a.tiles_x * kTileW, tile_y0 = a.row0 + t / a.tiles_x * kTileH;
-    const bool fit = s_fit[buf] != 0;
-    const bool interior = s_interior[buf] != 0;
-    if (fit) {
+    const int tile_x0 = t % a.tiles_x * kTileW, tile_y0 = a.row0 + t / a.tiles_x * TH;
+    if (p.fits) {
       // Bounded wait: on expiry flag the error, give the copy one more
       // bounded wait to land, finish this item (its output is discarded by
       // the host) and leave the loop with the whole CTA.
@@ -348,33 +717,61 @@ __global__ void __launch_bounds__(kWarpThreads, 3) warp_tiles_kernel(const __gri
       }
       phase[buf] ^= 1u;
     }
-    {
-      TapSource ts;
-      ts.tile = fit ? tile[buf] : nullptr;
-      ts.src = a.slots + static_cast<int64_t>(it_src) * a.stride;
-      ts.bx = s_bx[buf];
-      ts.by = s_by[buf];
-      ts.width = a.width;
-      float* dst = it_dst - static_cast<int64_t>(a.row0) * a.width;
-      // the renormalising path (and its out-of-line call) only for frames
-      // that hold non-finite samples; the straight-line form for the common
-      // interior tile
-      const bool full_tile = tile_x0 + kTileW <= a.width && tile_y0 + kTileH <= a.row1;
-      unsigned bad;
-      if (INTERP == GG_INTERP_LANCZOS3 && fit && interior && co.affine && it_nonfinite == 0u && !int_shift &&
-          a.clamp < 0.0f && a.coverage == nullptr && full_tile)
-        bad = warp_tile_rows_fast(a, co, ts.tile, ts.bx, ts.by, dst, tile_x0 + lx, tile_y0 + ly);
-      else if (INTERP == GG_INTERP_LANCZOS3 && it_nonfinite == 0u)
-        bad = warp_tile_rows<INTERP, true>(a, co, ts, dst, tile_x0 + lx, tile_y0 + ly, interior, int_shift);
+    const bool full_tile = tile_x0 + kTileW <= a.width && tile_y0 + TH <= a.row1;
+    unsigned bad = 0;
+    if (INTERP != GG_INTERP_NEAREST && p.grid && (!kLanczos || a.clamp < 0.0f) &&
+        (p.fits || !kLanczos || (a.width >= 6 && a.height >= 6))) {
+      const int lx = tid & 31, ly = (tid >> 5) * (TH / 4);
+      const TileGrid& grid = s_grid[buf];
+      const int64_t first = static_cast<int64_t>(tile_y0 + ly) * a.width + tile_x0 + lx;
+      const TileMask mask = tile_mask(grid, kLanczos, a.width, a.height, tile_x0, tile_y0, a.row1,
+                                      a.coverage ? a.coverage + first : nullptr);
+      float* out = dst + first;
+      auto rows = [&](auto win, auto masked) {
+        constexpr bool kMask = decltype(masked)::value;
+        if constexpr (kLanczos)
+          return lanczos3_rows<TH / 4, decltype(win)::kStaged, kMask>(grid, win, mask, a.fill, out, a.width, lx, ly);
+        else
+          return bilinear_rows<TH / 4, decltype(win)::kStaged, kMask>(grid, win, mask, a.fill, out, a.width, lx, ly);
+      };
+      auto tile_rows = [&](auto win) {
+        if constexpr (kLanczos) {
+          constexpr bool kStaged = decltype(win)::kStaged;
+          if (int_shift) return shifted_rows<TH / 4, kStaged>(grid, win, mask, a.fill, out, a.width, lx, ly);
+          if (!finite) return lanczos3_renorm_rows<TH / 4, kStaged>(grid, win, mask, a.fill, out, a.width, lx, ly);
+        }
+        return p.interior && full_tile && a.coverage == nullptr ? rows(win, std::false_type{})
+                                                                : rows(win, std::true_type{});
+      };
+      constexpr int kSpan = kLanczos ? 6 : 1;  // of a window's possible places
+      const int x0 = -grid.ox, y0 = -grid.oy, x1 = a.width - kSpan + x0, y1 = a.height - kSpan + y0;
+      if (USE_TMA && p.fits)
+        bad = tile_rows(Window<true>{tile, kBoxW, x0, x1, y0, y1});
       else
-        bad = warp_tile_rows<INTERP, false>(a, co, ts, dst, tile_x0 + lx, tile_y0 + ly, interior, int_shift);
-      const unsigned warp_bad = __reduce_add_sync(0xffffffffu, bad);
-      if ((tid & 31) == 0 && warp_bad) atomicAdd(a.nonfinite + it_frame, warp_bad);
+        bad = tile_rows(Window<false>{src + static_cast<int64_t>(grid.oy) * a.width + grid.ox, a.width, x0, x1, y0, y1});
+    } else {
+      const Coef co = load_coef(ip);
+      TapSource ts;
+      ts.tile = p.fits ? tile : nullptr;
+      ts.src = src;
+      ts.bx = p.bx;
+      ts.by = p.by;
+      ts.width = a.width;
+#pragma unroll 1
+      for (int c = tid / kTileW; c < kRowClasses; c += kWarpThreads / kTileW) {
+        const int ox = tile_x0 + tid % kTileW, oy0 = tile_y0 + c;
+        if (kLanczos && finite)
+          bad += warp_tile_rows<INTERP, true, TH>(a, co, ts, dst, ox, oy0, p.interior != 0, int_shift);
+        else
+          bad += warp_tile_rows<INTERP, false, TH>(a, co, ts, dst, ox, oy0, p.interior != 0, int_shift);
+      }
     }
+    const unsigned warp_bad = __reduce_add_sync(0xffffffffu, bad);
+    if ((tid & 31) == 0 && warp_bad) atomicAdd(a.nonfinite + it_frame, warp_bad);
     __syncthreads();
     if (s_abort) {
-      // Let the prefetch already issued for the next item land before exit.
-      if (next < items && s_fit[buf ^ 1]) mbar_wait_bounded(&bar[buf ^ 1], phase[buf ^ 1], 1 << 24);
+      // Let the copy already issued for the next item land before exit.
+      if (next < items && s_plan[buf ^ 1].fits) mbar_wait_bounded(&bar[buf ^ 1], phase[buf ^ 1], 1 << 24);
       break;
     }
   }
@@ -467,16 +864,23 @@ static void ensure_warp_coverage(gg_stack* s) {
   check_cuda(cudaMemsetAsync(s->d_warp_coverage, 0, sizeof(float) * s->pixels, s->stream), "cudaMemsetAsync");
 }
 
-template <int INTERP>
-static void launch_warp_tiles(gg_stack* s, const WarpArgs& args, bool use_tma) {
-  int per_sm = 0;
-  auto kern = use_tma ? warp_tiles_kernel<INTERP, true> : warp_tiles_kernel<INTERP, false>;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarpThreads, 0), "occupancy(warp)");
+template <int INTERP, int TH>
+static void launch_warp_tiles(gg_stack* s, WarpArgs args) {
+  const bool use_tma = s->has_slot_tmap;
+  args.tiles_y = (args.row1 - args.row0 + TH - 1) / TH;
+  auto kern = use_tma ? warp_tiles_kernel<INTERP, true, TH> : warp_tiles_kernel<INTERP, false, TH>;
+  const size_t smem = use_tma ? kWarpTileBytes : 0;
+  const int per_sm = kernel_ctas_per_sm(kern, kWarpThreads, smem, "warp launch shape");
   const int64_t items = static_cast<int64_t>(args.item_count) * args.tiles_x * args.tiles_y;
-  const unsigned grid =
-      static_cast<unsigned>(std::min<int64_t>(items, static_cast<int64_t>(sm_count()) * std::max(per_sm, 1)));
+  unsigned grid =
+      static_cast<unsigned>(std::min<int64_t>(items, static_cast<int64_t>(sm_count()) * per_sm));
+  // A stride that shares no factor with the tiles of a row takes every CTA
+  // through all tile columns: the slow border tiles of the first and last
+  // column would fall to few CTAs otherwise.
+  if (items > grid)
+    while (std::gcd(grid, static_cast<unsigned>(args.tiles_x)) != 1) --grid;
   note_launch();
-  kern<<<grid, kWarpThreads, 0, s->stream>>>(s->slot_tmap, args);
+  kern<<<grid, kWarpThreads, smem, s->stream>>>(s->slot_tmap, args);
   check_cuda(cudaGetLastError(), "warp kernel launch");
 }
 
@@ -492,19 +896,23 @@ static WarpArgs warp_args(gg_stack* s, WarpItem* d_items, int count, int row0, i
   a.row0 = row0;
   a.row1 = row1;
   a.tiles_x = (a.width + kTileW - 1) / kTileW;
-  a.tiles_y = (row1 - row0 + kTileH - 1) / kTileH;
   a.error = s->d_error;
   return a;
 }
 
 static void launch_warp_rows(gg_stack* s, const WarpArgs& a, int interp) {
-  const bool use_tma = s->has_slot_tmap;
+  // With less than two 64-row tiles per SM the launch takes as long as a tile
+  // does: 16-row tiles spread it over four times as many CTAs.
+  const int64_t tiles = static_cast<int64_t>(a.item_count) * a.tiles_x * ((a.row1 - a.row0 + kTileH - 1) / kTileH);
+  const bool small = tiles < 2 * sm_count();
   if (interp == GG_INTERP_NEAREST)
-    launch_warp_tiles<GG_INTERP_NEAREST>(s, a, use_tma);
+    launch_warp_tiles<GG_INTERP_NEAREST, kTileH>(s, a);
   else if (interp == GG_INTERP_BILINEAR)
-    launch_warp_tiles<GG_INTERP_BILINEAR>(s, a, use_tma);
+    small ? launch_warp_tiles<GG_INTERP_BILINEAR, kSmallTileH>(s, a)
+          : launch_warp_tiles<GG_INTERP_BILINEAR, kTileH>(s, a);
   else
-    launch_warp_tiles<GG_INTERP_LANCZOS3>(s, a, use_tma);
+    small ? launch_warp_tiles<GG_INTERP_LANCZOS3, kSmallTileH>(s, a)
+          : launch_warp_tiles<GG_INTERP_LANCZOS3, kTileH>(s, a);
 }
 
 // Host descriptors of a warp batch (validated; inverse coefficients).
@@ -520,7 +928,9 @@ static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices
     WarpItem& it = items[static_cast<size_t>(k)];
     std::memset(&it, 0, sizeof(it));
     it.frame = static_cast<int>(indices[k]);
-    if (!inverse_coefficients(m, it.m, it.affine)) fail(GG_ERR_INVALID_ARGUMENT, "warp matrix is singular");
+    double inv[9];
+    if (!inverse_coefficients(m, it.m, it.affine, inv)) fail(GG_ERR_INVALID_ARGUMENT, "warp matrix is singular");
+    std::copy(inv, inv + 6, it.inv);
     // an exact integer translation (identity linear part, integer shifts):
     // its inverse is one too and every source coordinate is an integer
     it.int_shift = (m[0] == 1.0 && m[1] == 0.0 && m[3] == 0.0 && m[4] == 1.0 && m[6] == 0.0 && m[7] == 0.0 &&
@@ -620,6 +1030,7 @@ __global__ void warp_band_prepare_kernel(WarpItem* items, const FusedFrame* fram
   for (int q = 0; q < 9; ++q) {
     it.m[q][0] = frames[k].m[q][0];
     it.m[q][1] = frames[k].m[q][1];
+    if (q < 6) it.inv[q] = static_cast<double>(it.m[q][0]) + static_cast<double>(it.m[q][1]);
   }
   items[k] = it;
   base[k] = it.dst;
@@ -683,7 +1094,7 @@ __global__ void __launch_bounds__(256) warp_nonfinite_kernel(WarpArgs a, unsigne
 }
 
 // Frames with a geometrically valid sample, per pixel of a band.  One CTA per
-// 64 x 48 tile: a frame that maps the whole tile inside its valid range counts
+// tile: a frame that maps the whole tile inside its valid range counts
 // for every pixel without a test (all but the tiles along the border), the
 // others are evaluated pixel by pixel.  Where a Lanczos3 frame holds
 // non-finite samples, a window may have no weight left: its warped sample
@@ -700,7 +1111,7 @@ __global__ void __launch_bounds__(kWarpThreads) warp_geometry_kernel(WarpArgs a,
   for (int f = threadIdx.x; f < a.item_count; f += kWarpThreads) {
     const WarpItem* ip = a.items + f;
     const bool by_value = kLanczos && ip->src_nonfinite != 0u;
-    const TilePlan p = plan_tile(load_coef(ip), tile_x0, tile_y0, kLanczos ? 3 : 1, vlo,
+    const TilePlan p = plan_tile<kTileH>(load_coef(ip), tile_x0, tile_y0, kLanczos ? 3 : 1, vlo,
                                  static_cast<float>(a.width) - off, static_cast<float>(a.height) - off);
     if (p.interior && !by_value) atomicAdd(&s_inside, 1);
     else s_list[atomicAdd(&s_mixed, 1)] = f;
@@ -708,9 +1119,10 @@ __global__ void __launch_bounds__(kWarpThreads) warp_geometry_kernel(WarpArgs a,
   __syncthreads();
   const int ox = tile_x0 + (threadIdx.x & 63);
   if (ox >= a.width) return;
-  int n[kRowsPerThread];
+  constexpr int kRows = kTileH * kTileW / kWarpThreads, kStep = kWarpThreads / kTileW;
+  int n[kRows];
 #pragma unroll
-  for (int r = 0; r < kRowsPerThread; ++r) n[r] = s_inside;
+  for (int r = 0; r < kRows; ++r) n[r] = s_inside;
   for (int i = 0; i < s_mixed; ++i) {
     const WarpItem* ip = a.items + s_list[i];
     const Coef co = load_coef(ip);
@@ -718,16 +1130,16 @@ __global__ void __launch_bounds__(kWarpThreads) warp_geometry_kernel(WarpArgs a,
     const float* dst = ip->dst - static_cast<int64_t>(a.row0) * a.width;
     FFv sx, sy;
 #pragma unroll
-    for (int r = 0; r < kRowsPerThread; ++r) {
-      const int oy = tile_y0 + (threadIdx.x >> 6) + 4 * r;
+    for (int r = 0; r < kRows; ++r) {
+      const int oy = tile_y0 + (threadIdx.x >> 6) + kStep * r;
       if (oy >= a.row1) continue;
       if (by_value) n[r] += !isnan(dst[static_cast<int64_t>(oy) * a.width + ox]);
       else n[r] += sample_valid<INTERP>(co, ox, oy, a.width, a.height, sx, sy);
     }
   }
 #pragma unroll
-  for (int r = 0; r < kRowsPerThread; ++r) {
-    const int oy = tile_y0 + (threadIdx.x >> 6) + 4 * r;
+  for (int r = 0; r < kRows; ++r) {
+    const int oy = tile_y0 + (threadIdx.x >> 6) + kStep * r;
     if (oy < a.row1) geometric[static_cast<int64_t>(oy) * a.width + ox] = static_cast<float>(n[r]);
   }
 }
@@ -738,8 +1150,8 @@ void launch_warp_band(gg_stack* s, void* d_items, int interp, float clamp, int r
   a.nonfinite = counts;
   a.fill = NAN;
   a.clamp = clamp;
-  a.every_row = 1;  // the same validity as the geometric coverage below
   launch_warp_rows(s, a, interp);
+  a.tiles_y = (row1 - row0 + kTileH - 1) / kTileH;
   const unsigned tiles = static_cast<unsigned>(a.tiles_x) * static_cast<unsigned>(a.tiles_y);
   note_launch();
   if (interp == GG_INTERP_BILINEAR)
