@@ -9,13 +9,19 @@
 //   if pedestal != 0: v = v + pedestal
 // Every operation is rounded separately (no FMA), as NumPy does.
 //
-// GB300 design: one launch calibrates a batch of up to GG_MAX_BATCH_FRAMES
-// frames.  Each thread owns 8 consecutive pixels, loads the masters for them
-// once (16-byte vector loads) and then streams the batch's frames through
-// registers: 16 B of uint16 in and 32 B of float32 out per frame, so the
-// masters cost 12 B per pixel per batch instead of per frame.  Raw frames
-// arrive over PCIe/C2C on a copy stream into one of two lane buffers while the
-// previous lane is being decoded (cudaEvent handshakes).
+// GB300 design: one launch calibrates a batch of frames.  Each thread owns 8
+// consecutive pixels, loads the masters for them once (16-byte vector loads) and
+// then streams the batch's frames through registers, four frames' loads in
+// flight: 16 B of uint16 in and 32 B of float32 out per frame, so the masters
+// cost 12 B per pixel per batch instead of per frame.  Frames of a pixel count
+// that is no multiple of 8 start at any 2-byte offset: their 16 bytes come out of
+// two aligned loads.  The last CTA publishes the frames' non-finite counts.
+// Raw frames arrive over PCIe/C2C on a copy stream into one of two lane buffers
+// while the previous lane is being decoded (cudaEvent handshakes).
+//
+// Bound: HBM.  16 frames of 4096^2 in one launch 335 us, 5.4 TB/s of the
+// algorithmic bytes (357 us in launches of 8 frames, which read the masters
+// twice); 20 frames of 1537 x 2047 120 us (192 us one sample at a time).
 #include <algorithm>
 #include <vector>
 
@@ -32,6 +38,8 @@ struct CalibArgs {
   float* slots;
   const int* slot_of_frame;
   unsigned* nonfinite;
+  unsigned* counts;  // of this launch, zero before and after
+  unsigned* ticket;
   int64_t stride;
   int64_t pixels;
   int nframes;
@@ -64,74 +72,120 @@ __device__ __forceinline__ float decode_u16(uint16_t raw, int big_endian_bzero) 
   return static_cast<float>(raw);
 }
 
-// Vector path: P % 8 == 0.  Thread t owns pixels [8t, 8t+8).
-__global__ void __launch_bounds__(256) calibrate_u16_vec8_kernel(CalibArgs a) {
+// 8 raw samples from any 2-byte aligned address.
+struct Raw8 {
+  unsigned w[4];
+};
+
+__device__ __forceinline__ Raw8 load_raw8(const uint16_t* p, const uint16_t* first, const uint16_t* last) {
+  const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+  const unsigned shift = static_cast<unsigned>(at) & 15u;  // the same in every thread of a frame
+  Raw8 r;
+  if (shift == 0) {
+    const uint4 v = __ldcs(reinterpret_cast<const uint4*>(p));
+    r.w[0] = v.x;
+    r.w[1] = v.y;
+    r.w[2] = v.z;
+    r.w[3] = v.w;
+    return r;
+  }
+  const auto* lo = reinterpret_cast<const uint4*>(at - shift);
+  if (reinterpret_cast<const uint16_t*>(lo) < first || reinterpret_cast<const uint16_t*>(lo + 2) > last) {
+    // the buffer's first and last samples
+#pragma unroll
+    for (int k = 0; k < 4; ++k) r.w[k] = p[2 * k] | static_cast<unsigned>(p[2 * k + 1]) << 16;
+    return r;
+  }
+  const uint4 a = __ldg(lo), b = __ldg(lo + 1);
+  const unsigned v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  unsigned s[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const unsigned q = shift >> 2;
+    s[k] = q == 0 ? v[k] : q == 1 ? v[k + 1] : q == 2 ? v[k + 2] : v[min(k + 3, 7)];
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) r.w[k] = __funnelshift_r(s[k], s[k + 1], (shift & 2u) * 8u);
+  return r;
+}
+
+// uint16 frames.  Thread t owns pixels [8t, 8t + 8); the last P % 8 pixels of
+// every frame go one by one.
+__global__ void __launch_bounds__(256) calibrate_u16_kernel(CalibArgs a) {
   const int64_t groups = a.pixels / 8;
+  const uint16_t* last = a.raw + static_cast<int64_t>(a.nframes) * a.pixels;
   for (int64_t g = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; g < groups;
        g += int64_t(gridDim.x) * blockDim.x) {
     const int64_t p0 = g * 8;
     float b[8], d[8], f[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) b[k] = d[k] = f[k] = 0.0f;
-    if (a.has_bias) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(a.bias + p0));
-      const float4 v = __ldg(reinterpret_cast<const float4*>(a.bias + p0) + 1);
-      b[0] = u.x; b[1] = u.y; b[2] = u.z; b[3] = u.w; b[4] = v.x; b[5] = v.y; b[6] = v.z; b[7] = v.w;
-    }
-    if (a.has_dark) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(a.dark + p0));
-      const float4 v = __ldg(reinterpret_cast<const float4*>(a.dark + p0) + 1);
-      d[0] = u.x; d[1] = u.y; d[2] = u.z; d[3] = u.w; d[4] = v.x; d[5] = v.y; d[6] = v.z; d[7] = v.w;
-    }
-    if (a.has_flat) {
-      const float4 u = __ldg(reinterpret_cast<const float4*>(a.flat + p0));
-      const float4 v = __ldg(reinterpret_cast<const float4*>(a.flat + p0) + 1);
-      f[0] = u.x; f[1] = u.y; f[2] = u.z; f[3] = u.w; f[4] = v.x; f[5] = v.y; f[6] = v.z; f[7] = v.w;
-    }
-    for (int fi = 0; fi < a.nframes; ++fi) {
-      const uint4 r = __ldcs(reinterpret_cast<const uint4*>(a.raw + fi * a.pixels + p0));
-      const uint16_t raw[8] = {static_cast<uint16_t>(r.x & 0xffffu), static_cast<uint16_t>(r.x >> 16),
-                               static_cast<uint16_t>(r.y & 0xffffu), static_cast<uint16_t>(r.y >> 16),
-                               static_cast<uint16_t>(r.z & 0xffffu), static_cast<uint16_t>(r.z >> 16),
-                               static_cast<uint16_t>(r.w & 0xffffu), static_cast<uint16_t>(r.w >> 16)};
-      float out[8];
-      bool bad = false;
+    auto master = [&](const float* m, float (&v)[8]) {
+      const float4 u = __ldg(reinterpret_cast<const float4*>(m + p0));
+      const float4 w = __ldg(reinterpret_cast<const float4*>(m + p0) + 1);
+      v[0] = u.x; v[1] = u.y; v[2] = u.z; v[3] = u.w; v[4] = w.x; v[5] = w.y; v[6] = w.z; v[7] = w.w;
+    };
+    if (a.has_bias) master(a.bias, b);
+    if (a.has_dark) master(a.dark, d);
+    if (a.has_flat) master(a.flat, f);
+    constexpr int kAhead = 4;
+    for (int f0 = 0; f0 < a.nframes; f0 += kAhead) {
+      Raw8 r[kAhead];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        out[k] = calibrate_one(decode_u16(raw[k], a.big_endian_bzero), b[k], d[k], f[k], a);
-        bad |= !isfinite(out[k]);
-      }
-      float* dst = a.slots + static_cast<int64_t>(a.slot_of_frame[a.frame[fi]]) * a.stride + p0;
-      __stcs(reinterpret_cast<float4*>(dst), make_float4(out[0], out[1], out[2], out[3]));
-      __stcs(reinterpret_cast<float4*>(dst) + 1, make_float4(out[4], out[5], out[6], out[7]));
-      if (__any_sync(__activemask(), bad)) {
-        int nbad = 0;
+      for (int q = 0; q < kAhead; ++q)
+        if (f0 + q < a.nframes) r[q] = load_raw8(a.raw + (f0 + q) * a.pixels + p0, a.raw, last);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) nbad += !isfinite(out[k]);
-        if (nbad) atomicAdd(a.nonfinite + a.frame[fi], static_cast<unsigned>(nbad));
+      for (int q = 0; q < kAhead; ++q) {
+        if (f0 + q >= a.nframes) break;
+        const int frame = a.frame[f0 + q];
+        float out[8];
+        bool bad = false;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const auto raw = static_cast<uint16_t>(r[q].w[k / 2] >> (16 * (k & 1)));
+          out[k] = calibrate_one(decode_u16(raw, a.big_endian_bzero), b[k], d[k], f[k], a);
+          bad |= !isfinite(out[k]);
+        }
+        float* dst = a.slots + static_cast<int64_t>(a.slot_of_frame[frame]) * a.stride + p0;
+        __stcs(reinterpret_cast<float4*>(dst), make_float4(out[0], out[1], out[2], out[3]));
+        __stcs(reinterpret_cast<float4*>(dst) + 1, make_float4(out[4], out[5], out[6], out[7]));
+        if (bad) {
+          unsigned nbad = 0;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) nbad += !isfinite(out[k]);
+          atomicAdd(a.counts + frame, nbad);
+        }
       }
     }
   }
+  const int tail = static_cast<int>(a.pixels - groups * 8);
+  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < int64_t(tail) * a.nframes;
+       i += int64_t(gridDim.x) * blockDim.x) {
+    const int fi = static_cast<int>(i / tail), frame = a.frame[fi];
+    const int64_t p = groups * 8 + (i - static_cast<int64_t>(fi) * tail);
+    const float out = calibrate_one(decode_u16(a.raw[fi * a.pixels + p], a.big_endian_bzero), a.has_bias ? a.bias[p] : 0.0f,
+                                    a.has_dark ? a.dark[p] : 0.0f, a.has_flat ? a.flat[p] : 0.0f, a);
+    a.slots[static_cast<int64_t>(a.slot_of_frame[frame]) * a.stride + p] = out;
+    if (!isfinite(out)) atomicAdd(a.counts + frame, 1u);
+  }
+  if (last_cta(a.ticket, gridDim.x))
+    for (int i = threadIdx.x; i < a.nframes; i += blockDim.x)
+      a.nonfinite[a.frame[i]] = atomicExch(a.counts + a.frame[i], 0u);
 }
 
-// Scalar path for any P (odd shapes, float32 lights).
-__global__ void __launch_bounds__(256) calibrate_scalar_kernel(CalibArgs a) {
+// One float32 light.
+__global__ void __launch_bounds__(256) calibrate_f32_kernel(CalibArgs a) {
+  const int frame = a.frame[0];
+  float* dst = a.slots + static_cast<int64_t>(a.slot_of_frame[frame]) * a.stride;
   for (int64_t p = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; p < a.pixels;
        p += int64_t(gridDim.x) * blockDim.x) {
-    const float b = a.has_bias ? a.bias[p] : 0.0f;
-    const float d = a.has_dark ? a.dark[p] : 0.0f;
-    const float f = a.has_flat ? a.flat[p] : 0.0f;
-    for (int fi = 0; fi < a.nframes; ++fi) {
-      const float light = a.raw ? decode_u16(a.raw[fi * a.pixels + p], a.big_endian_bzero) : a.light_f32[p];
-      const float out = calibrate_one(light, b, d, f, a);
-      a.slots[static_cast<int64_t>(a.slot_of_frame[a.frame[fi]]) * a.stride + p] = out;
-      warp_count_add(a.nonfinite + a.frame[fi], !isfinite(out));
-    }
+    const float out = calibrate_one(a.light_f32[p], a.has_bias ? a.bias[p] : 0.0f, a.has_dark ? a.dark[p] : 0.0f,
+                                    a.has_flat ? a.flat[p] : 0.0f, a);
+    dst[p] = out;
+    warp_count_add(a.counts + frame, !isfinite(out));
   }
-}
-
-__global__ void zero_counters_kernel(unsigned* counters, CalibArgs a) {
-  if (threadIdx.x < a.nframes) counters[a.frame[threadIdx.x]] = 0u;
+  if (last_cta(a.ticket, gridDim.x) && threadIdx.x == 0)
+    a.nonfinite[frame] = atomicExch(a.counts + frame, 0u);
 }
 
 __global__ void __launch_bounds__(256) count_nonfinite_kernel(const float* frame, int64_t n, unsigned* counter) {
@@ -157,6 +211,8 @@ static CalibArgs make_args(gg_stack* s, const gg_calib_params_t& p) {
   a.slots = s->d_slots;
   a.slot_of_frame = s->d_slot_of_frame;
   a.nonfinite = s->d_frame_nonfinite;
+  a.counts = s->d_count_acc;
+  a.ticket = s->d_tickets + s->frames + 1;
   a.stride = s->stride;
   a.pixels = s->pixels;
   a.has_bias = s->has_bias;
@@ -177,18 +233,10 @@ void launch_calibrate(gg_stack* s, const CalibLaunch& job, const gg_calib_params
   a.nframes = job.nframes;
   for (int i = 0; i < job.nframes; ++i) a.frame[i] = job.frame[i];
   note_launch();
-  zero_counters_kernel<<<1, 32, 0, s->stream>>>(s->d_frame_nonfinite, a);
-  const bool aligned = (s->pixels % 8 == 0) && job.raw != nullptr &&
-                       (reinterpret_cast<uintptr_t>(job.raw) % 16 == 0);
-  if (aligned) {
-    const unsigned grid = grid_for(static_cast<size_t>(s->pixels / 8), 256, 8);
-    note_launch();
-    calibrate_u16_vec8_kernel<<<grid, 256, 0, s->stream>>>(a);
-  } else {
-    const unsigned grid = grid_for(static_cast<size_t>(s->pixels), 256, 8);
-    note_launch();
-    calibrate_scalar_kernel<<<grid, 256, 0, s->stream>>>(a);
-  }
+  if (job.raw != nullptr)
+    calibrate_u16_kernel<<<grid_for(static_cast<size_t>((s->pixels + 7) / 8), 256, 8), 256, 0, s->stream>>>(a);
+  else
+    calibrate_f32_kernel<<<grid_for(static_cast<size_t>(s->pixels), 256, 8), 256, 0, s->stream>>>(a);
   check_cuda(cudaGetLastError(), "calibrate kernel launch");
 }
 
@@ -327,13 +375,16 @@ int gg_stack_calibrate_u16_device(gg_stack* s, const int64_t* indices, int64_t c
   for (int64_t k = 0; k < count; ++k) stack_require_index(s, indices[k]);
   stack_activate(s);
   const auto* raw = static_cast<const uint16_t*>(dev_raw);
-  for (int64_t k0 = 0; k0 < count; k0 += GG_MAX_BATCH_FRAMES) {
-    const int nb = static_cast<int>(std::min<int64_t>(GG_MAX_BATCH_FRAMES, count - k0));
+  for (int64_t k0 = 0; k0 < count;) {
     CalibLaunch job{};
     job.raw = raw + static_cast<size_t>(k0) * static_cast<size_t>(s->pixels);
     job.big_endian_bzero = big_endian_bzero;
-    job.nframes = nb;
-    for (int i = 0; i < nb; ++i) job.frame[i] = static_cast<int>(indices[k0 + i]);
+    // a frame that comes again starts another launch
+    auto repeated = [&](int64_t k) {
+      return std::find(job.frame, job.frame + job.nframes, static_cast<int>(indices[k])) != job.frame + job.nframes;
+    };
+    while (k0 < count && job.nframes < GG_MAX_BATCH_FRAMES && !repeated(k0))
+      job.frame[job.nframes++] = static_cast<int>(indices[k0++]);
     launch_calibrate(s, job, *params);
   }
   for (int64_t k = 0; k < count; ++k) stack_mark_loaded(s, indices[k]);
@@ -375,11 +426,13 @@ int gg_stack_calibrate_u16_staged(gg_stack* s, const int64_t* indices, int64_t c
   RawStage& r = raw_stage(s);
   for (int64_t k = 0; k < count; ++k) require(r.uploaded[indices[k]] != 0, "frame has no staged raw samples");
   stack_activate(s);
-  // runs of consecutive frame indices share one launch (their staged copies are contiguous)
+  // runs of consecutive frame indices share one launch (their staged copies are
+  // contiguous); short runs, as a launch waits for the uploads of all its frames
+  constexpr int64_t kStagedBatch = 8;
   int64_t k0 = 0;
   while (k0 < count) {
     int64_t k1 = k0 + 1;
-    while (k1 < count && k1 - k0 < GG_MAX_BATCH_FRAMES && indices[k1] == indices[k1 - 1] + 1) ++k1;
+    while (k1 < count && k1 - k0 < kStagedBatch && indices[k1] == indices[k1 - 1] + 1) ++k1;
     for (int64_t k = k0; k < k1; ++k)
       check_cuda(cudaStreamWaitEvent(s->stream, r.ready[indices[k]], 0), "cudaStreamWaitEvent(raw ready)");
     CalibLaunch job{};
@@ -450,9 +503,9 @@ int gg_calibrate_tile_f32(const float* host_light, const float* host_bias, const
       check_cuda(cudaMemcpy(d[i], srcs[i], bytes, cudaMemcpyHostToDevice), "cudaMemcpy(calibrate tile)");
     }
     check_cuda(cudaMalloc(&d[4], bytes), "cudaMalloc(calibrate out)");
-    check_cuda(cudaMalloc(&d_counter, sizeof(unsigned)), "cudaMalloc(counter)");
+    check_cuda(cudaMalloc(&d_counter, 3 * sizeof(unsigned)), "cudaMalloc(counter)");
     check_cuda(cudaMalloc(&d_slot, sizeof(int)), "cudaMalloc(slot)");
-    check_cuda(cudaMemset(d_counter, 0, sizeof(unsigned)), "cudaMemset");
+    check_cuda(cudaMemset(d_counter, 0, 3 * sizeof(unsigned)), "cudaMemset");
     check_cuda(cudaMemset(d_slot, 0, sizeof(int)), "cudaMemset");
     CalibArgs a{};
     a.light_f32 = d[0];
@@ -462,6 +515,8 @@ int gg_calibrate_tile_f32(const float* host_light, const float* host_bias, const
     a.slots = d[4];
     a.slot_of_frame = d_slot;
     a.nonfinite = d_counter;
+    a.counts = d_counter + 1;
+    a.ticket = d_counter + 2;
     a.stride = n;
     a.pixels = n;
     a.nframes = 1;
@@ -474,7 +529,7 @@ int gg_calibrate_tile_f32(const float* host_light, const float* host_bias, const
     a.flat_floor = params->flat_floor;
     a.pedestal = params->pedestal;
     note_launch();
-    calibrate_scalar_kernel<<<grid_for(static_cast<size_t>(n), 256, 4), 256>>>(a);
+    calibrate_f32_kernel<<<grid_for(static_cast<size_t>(n), 256, 4), 256>>>(a);
     check_cuda(cudaGetLastError(), "calibrate kernel launch");
     check_cuda(cudaMemcpy(host_out, d[4], bytes, cudaMemcpyDeviceToHost), "cudaMemcpy(calibrate out)");
   } catch (...) {

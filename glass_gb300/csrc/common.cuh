@@ -18,7 +18,7 @@
 #include "../../include/glass_gb300.h"
 
 // Frames handled by one calibration launch (frame indices travel by value).
-#define GG_MAX_BATCH_FRAMES 8
+#define GG_MAX_BATCH_FRAMES 32
 
 namespace gg {
 
@@ -183,6 +183,21 @@ __device__ __forceinline__ void ff_add_sqdev(FF& acc, float x, float mh, float m
   const float pe = __fmaf_rn(d, d, -p);
   acc.add(p);
   acc.lo = __fadd_rn(acc.lo, __fmaf_rn(__fmul_rn(2.0f, d), de, pe));
+}
+
+// True in every thread of the grid's last CTA to get here (all the others'
+// global writes are visible to it then); `ticket` is 0 before and after.
+__device__ __forceinline__ bool last_cta(unsigned* ticket, unsigned ctas) {
+  __shared__ int s_last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    s_last = atomicAdd(ticket, 1u) == ctas - 1u;
+    if (s_last) *ticket = 0u;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last != 0;
 }
 
 // Warp-aggregated counter increment (one atomic per warp).

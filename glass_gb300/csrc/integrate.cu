@@ -1185,10 +1185,7 @@ static void launch_warp(const IntegrateArgs& args, cudaStream_t stream) {
   const bool pipe = 2 * tile_bytes <= 100 * 1024;
   const size_t smem = tile_bytes * (pipe ? 2 : 1);
   auto kern = pipe ? integrate_warp_kernel<16, true> : integrate_warp_kernel<16, false>;
-  check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-             "cudaFuncSetAttribute(integrate_warp)");
-  int per_sm = 0;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kWarpThreads, smem), "occupancy");
+  const int per_sm = kernel_ctas_per_sm(kern, kWarpThreads, smem, "launch shape (integrate_warp)");
   const int64_t tiles = (args.pixels + kWarpTilePx - 1) / kWarpTilePx;
   const int64_t resident = static_cast<int64_t>(std::max(per_sm, 1)) * sm_count();
   const unsigned grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(tiles, resident)));
@@ -1202,10 +1199,7 @@ static void launch_reg(const IntegrateArgs& args, cudaStream_t stream) {
   constexpr int T = 128;
   const size_t smem = size_t(2) * NB * T * sizeof(float);
   auto kern = integrate_reg_kernel<NB, T>;
-  check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-             "cudaFuncSetAttribute(integrate)");
-  int per_sm = 0;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem), "occupancy");
+  const int per_sm = kernel_ctas_per_sm(kern, T, smem, "launch shape (integrate)");
   const unsigned grid = grid_for(static_cast<size_t>(args.pixels), T, std::max(per_sm, 1));
   note_launch();
   kern<<<grid, T, smem, stream>>>(args);
@@ -1217,10 +1211,7 @@ static void launch_col(const IntegrateArgs& args, cudaStream_t stream) {
   constexpr int T = 128;
   const size_t smem = size_t(NB) * T * sizeof(float);
   auto run_kernel = [&](auto kern) {
-    check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-               "cudaFuncSetAttribute(integrate)");
-    int per_sm = 0;
-    check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem), "occupancy");
+    const int per_sm = kernel_ctas_per_sm(kern, T, smem, "launch shape (integrate)");
     const unsigned grid = grid_for(static_cast<size_t>(args.pixels), T, std::max(per_sm, 1));
     note_launch();
     kern<<<grid, T, smem, stream>>>(args);
@@ -1299,10 +1290,7 @@ static void launch_smem(const IntegrateArgs& args, cudaStream_t stream) {
   constexpr int T = 32;
   const size_t smem = size_t(2) * MR * 32 * T * sizeof(float);
   auto kern = integrate_smem_kernel<MR, T>;
-  check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-             "cudaFuncSetAttribute(integrate)");
-  int per_sm = 0;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem), "occupancy");
+  const int per_sm = kernel_ctas_per_sm(kern, T, smem, "launch shape (integrate)");
   const unsigned grid = grid_for(static_cast<size_t>(args.pixels), T, std::max(per_sm, 1));
   note_launch();
   kern<<<grid, T, smem, stream>>>(args);
@@ -1378,10 +1366,7 @@ static void launch_batch(std::vector<gg_stack*>& stacks, const std::vector<Integ
   bt.stacks = static_cast<int>(stacks.size());
   auto launch = [&](auto kern, int NBv) {
     const size_t smem = size_t(NBv) * T * sizeof(float);
-    check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-               "cudaFuncSetAttribute(integrate batch)");
-    int per_sm = 0;
-    check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem), "occupancy");
+    const int per_sm = kernel_ctas_per_sm(kern, T, smem, "launch shape (integrate batch)");
     const double budget = static_cast<double>(sm_count()) * std::max(per_sm, 1);
     double work = 0.0;
     for (const IntegrateArgs& a : args) work += static_cast<double>(a.pixels) * a.frames;
@@ -1501,10 +1486,7 @@ static void launch_fused(const IntegrateArgs& a, cudaStream_t stream) {
   constexpr int T = 128;
   const size_t smem = size_t(32) * T * sizeof(float);
   auto kern = integrate_col_kernel<32, T, MODE, INTERP>;
-  check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-             "cudaFuncSetAttribute(fused integrate)");
-  int per_sm = 0;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, T, smem), "occupancy");
+  const int per_sm = kernel_ctas_per_sm(kern, T, smem, "launch shape (fused integrate)");
   // pixel tile shape (tile_w x tile_h = T): wider tiles coalesce the map
   // writes, taller ones share the Lanczos / bilinear source rows in L1
   static const int kTiles[3][2] = {{128, 1}, {64, 2}, {32, 4}};

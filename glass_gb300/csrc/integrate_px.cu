@@ -567,11 +567,7 @@ static int px_best_warps() {
   int most = 0, pick = 1;
   for (int w = kPxMaxWarps; w >= 2; --w) {
     if (kWarpBytes * w + sizeof(PxTable<NB, L>) > 227 * 1024) continue;
-    int per_sm = 0;
-    check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(kWarpBytes * w)),
-               "cudaFuncSetAttribute(integrate_px)");
-    check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * w, kWarpBytes * w), "occupancy");
+    const int per_sm = kernel_ctas_per_sm(kern, 32 * w, kWarpBytes * w, "launch shape (integrate_px)");
     if (per_sm * w > most) {
       most = per_sm * w;
       pick = w;
@@ -589,10 +585,7 @@ static void launch_px(const IntegrateArgs& args, cudaStream_t stream) {
   // small frames: fewer warps per CTA, so that every SM has one
   const int warps = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(best, tiles / sm_count())));
   const size_t smem = kWarpBytes * warps;
-  check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-             "cudaFuncSetAttribute(integrate_px)");
-  int per_sm = 0;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem), "occupancy");
+  const int per_sm = kernel_ctas_per_sm(kern, 32 * warps, smem, "launch shape (integrate_px)");
   const int64_t ctas = std::min<int64_t>((tiles + warps - 1) / warps, int64_t(std::max(per_sm, 1)) * sm_count());
   note_launch();
   kern<<<static_cast<unsigned>(ctas), 32 * warps, smem, stream>>>(args);

@@ -151,11 +151,25 @@ void stack_mark_loaded(gg_stack* s, int64_t index) {
 
 void stack_read_slots(gg_stack* s, std::vector<int>& out) {
   out.resize(static_cast<size_t>(s->frames));
+  if (s->host_slots_valid && !s->slots_captured) {
+    check_cuda(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize(slot table)");
+    out = s->host_slots;
+    return;
+  }
   check_cuda(cudaMemcpyAsync(s->h_slot_table_pinned, s->d_slot_of_frame, sizeof(int) * s->frames,
                              cudaMemcpyDeviceToHost, s->stream),
              "cudaMemcpyAsync(slot table)");
   check_cuda(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize(slot table)");
   std::copy(s->h_slot_table_pinned, s->h_slot_table_pinned + s->frames, out.begin());
+  s->host_slots = out;
+  s->host_slots_valid = true;
+}
+
+void stack_slots_moved(gg_stack* s) {
+  s->host_slots_valid = false;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  check_cuda(cudaStreamIsCapturing(s->stream, &capture), "cudaStreamIsCapturing");
+  if (capture != cudaStreamCaptureStatusNone) s->slots_captured = true;
 }
 
 static void* device_alloc(gg_stack* s, size_t bytes, const char* what) {
@@ -232,6 +246,7 @@ static void stack_free(gg_stack* s) {
   if (s->ln_scratch && s->ln_scratch_free) s->ln_scratch_free(s->ln_scratch);
   if (s->raw_stage && s->raw_stage_free) s->raw_stage_free(s->raw_stage);
   void* dev_ptrs[] = {s->d_slots,    s->d_slot_of_frame, s->d_spare_slot, s->d_frame_nonfinite,
+                      s->d_tickets,  s->d_count_acc,
                       s->d_bias,     s->d_dark,          s->d_flat,       s->d_master,
                       s->d_weight,   s->d_coverage,      s->d_low,        s->d_high,
                       s->d_dq,       s->d_warp_coverage, s->d_weights,    s->d_partials,
@@ -401,6 +416,12 @@ int gg_stack_create(int64_t frame_count, int64_t height, int64_t width, gg_stack
     s->has_slot_tmap = (s->width % 4 == 0) && make_slot_tensor_map(s, kBoxW, kBoxH);
 
     check_cuda(cudaMemsetAsync(s->d_slots, 0, slot_bytes, s->stream), "cudaMemsetAsync(stack)");
+    s->d_tickets = static_cast<unsigned*>(device_alloc(s, sizeof(unsigned) * (frame_count + 2), "tickets"));
+    s->d_count_acc = static_cast<unsigned*>(device_alloc(s, sizeof(unsigned) * frame_count, "sample counts"));
+    check_cuda(cudaMemsetAsync(s->d_tickets, 0, sizeof(unsigned) * (frame_count + 2), s->stream),
+               "cudaMemsetAsync(tickets)");
+    check_cuda(cudaMemsetAsync(s->d_count_acc, 0, sizeof(unsigned) * frame_count, s->stream),
+               "cudaMemsetAsync(sample counts)");
     check_cuda(cudaMemsetAsync(s->d_frame_nonfinite, 0, sizeof(unsigned) * frame_count, s->stream),
                "cudaMemsetAsync(nonfinite)");
     const int64_t m = std::max(frame_count, s->spares);

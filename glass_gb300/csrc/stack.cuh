@@ -41,6 +41,19 @@ struct gg_stack {
   // statistics formulas (engine/rejection.py:39-44) without another pass.
   unsigned* d_frame_nonfinite = nullptr;
 
+  // Kernels whose last CTA finishes the launch's work (last_cta): tickets per
+  // frame, then one for the warp and one for the calibration; counts of a
+  // calibration in progress.  All zero between launches.
+  unsigned* d_tickets = nullptr;     // [frames + 2]
+  unsigned* d_count_acc = nullptr;   // [frames]
+
+  // Host copy of the frame->slot table, while no warp has moved a frame since
+  // it was read.  A stack whose warps have been captured into a graph moves
+  // frames at replays that the library does not see: it is read each time.
+  std::vector<int> host_slots;
+  bool host_slots_valid = false;
+  bool slots_captured = false;
+
   // Calibration masters (float32, P each).
   float* d_bias = nullptr;
   float* d_dark = nullptr;
@@ -161,6 +174,8 @@ struct CalibLaunch {
   int nframes;
   int frame[GG_MAX_BATCH_FRAMES];
 };
+// The warp of `s` has been (or will be) enqueued: its host slot table is stale.
+void stack_slots_moved(gg_stack* s);
 void launch_calibrate(gg_stack* s, const CalibLaunch& job, const gg_calib_params_t& p);
 void launch_count_nonfinite(gg_stack* s, int64_t frame);
 void launch_frame_stats(gg_stack* s, const int64_t* indices, int64_t count, int blocks_per_frame);

@@ -6,8 +6,9 @@
 // weight |mean|/std (resident_cuda.py:1948-1956).  Here every thread keeps
 // float-float sums of v and v^2 (TwoSum/TwoProd), a warp folds them with
 // shuffles, and each CTA writes one (sum, sum2, count) triple of doubles; the
-// host adds the partials.  One launch covers all requested frames
-// (grid.y = frame).
+// host adds the partials, or, for the frame weights, each frame's last CTA.  One
+// launch covers all requested frames (grid.y = frame).
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -22,9 +23,66 @@ __device__ __forceinline__ void ff_merge(FF& a, const FF& b) {
   a.lo = __fadd_rn(__fadd_rn(a.lo, b.lo), e);
 }
 
-__global__ void __launch_bounds__(256) frame_stats_kernel(const float* slots, const int* slot_of_frame, int64_t stride,
-                                                          int64_t pixels, const int* frames, double* partials) {
-  const int frame = frames[blockIdx.y];
+// simple_snr weights from the per-CTA partials (resident_cuda.py:1948-1956):
+//   valid == 0 -> 0;  std <= eps -> 1/eps;  else max(|mean|/std, eps)
+// A frame whose prior weight is not finite and positive keeps weight 0
+// (zero-weight frames are skipped, resident_cuda.py:12766-12770); otherwise
+// the prior multiplies the SNR weight in float64 (the registration-agreement
+// multiplier, resident_cuda.py:12800-12804).
+// One warp: lanes fold the CTA partials, then a shuffle reduction.
+struct SnrArgs {
+  const double* partials;  // [frames][blocks][3]
+  int blocks;
+  float eps;
+  int mode;
+  float* weights;      // by frame
+  unsigned* tickets;   // by frame (last_cta)
+};
+
+__device__ __forceinline__ void snr_weight(const SnrArgs& a, int f, float pw) {
+  const int lane = threadIdx.x & 31;
+  if (!(isfinite(pw) && pw > 0.0f) || a.mode == 0) {
+    if (lane == 0) a.weights[f] = (isfinite(pw) && pw > 0.0f) ? pw : 0.0f;
+    return;
+  }
+  double sum = 0.0, sum2 = 0.0, n = 0.0;
+  for (int b = lane; b < a.blocks; b += 32) {
+    const double* q = a.partials + (static_cast<int64_t>(f) * a.blocks + b) * 3;
+    sum += __ldcg(q);
+    sum2 += __ldcg(q + 1);
+    n += __ldcg(q + 2);
+  }
+  for (int off = 16; off > 0; off >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    sum2 += __shfl_xor_sync(0xffffffffu, sum2, off);
+    n += __shfl_xor_sync(0xffffffffu, n, off);
+  }
+  if (lane != 0) return;
+  if (n <= 0.0) {
+    a.weights[f] = 0.0f;
+    return;
+  }
+  const double mean = sum / n;
+  double var = sum2 / n - mean * mean;
+  if (var < 0.0) var = 0.0;
+  const double sd = sqrt(var);
+  const double e = static_cast<double>(a.eps);
+  const double w = sd <= e ? 1.0 / e : fmax(fabs(mean) / sd, e);
+  a.weights[f] = static_cast<float>(w * static_cast<double>(pw));
+}
+
+// Prior weights of the frames: in the launch parameters, in device memory
+// (`more`), or none.
+template <int CAP>
+struct PriorBlock {
+  int given;
+  const float* more;
+  float w[CAP];
+  __device__ __forceinline__ float at(int f) const { return !given ? 1.0f : (more ? more[f] : w[f]); }
+};
+
+__device__ __forceinline__ void frame_stats_partial(const float* slots, const int* slot_of_frame, int64_t stride,
+                                                    int64_t pixels, int frame, double* partials) {
   const float* src = slots + static_cast<int64_t>(slot_of_frame[frame]) * stride;
   // Two independent accumulator pairs over float4 loads (slots are 256 B
   // aligned), then the scalar tail.
@@ -71,48 +129,43 @@ __global__ void __launch_bounds__(256) frame_stats_kernel(const float* slots, co
   }
 }
 
-// simple_snr weights from the per-CTA partials (resident_cuda.py:1948-1956):
-//   valid == 0 -> 0;  std <= eps -> 1/eps;  else max(|mean|/std, eps)
-// A frame whose prior weight is not finite and positive keeps weight 0
-// (zero-weight frames are skipped, resident_cuda.py:12766-12770); otherwise
-// the prior multiplies the SNR weight in float64 (the registration-agreement
-// multiplier, resident_cuda.py:12800-12804).
-// One warp per frame: lanes fold the CTA partials, then a shuffle reduction.
-__global__ void snr_weights_kernel(const double* partials, int blocks, const int* frames, int count,
-                                   const float* prior, float eps, int mode, float* weights) {
-  const int k = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (k >= count) return;
-  const int f = frames[k];
-  const float pw = prior ? prior[k] : 1.0f;
-  if (!(isfinite(pw) && pw > 0.0f) || mode == 0) {
-    if (lane == 0) weights[f] = (isfinite(pw) && pw > 0.0f) ? pw : 0.0f;
-    return;
-  }
-  double sum = 0.0, sum2 = 0.0, n = 0.0;
-  for (int b = lane; b < blocks; b += 32) {
-    const double* q = partials + (static_cast<int64_t>(k) * blocks + b) * 3;
-    sum += q[0];
-    sum2 += q[1];
-    n += q[2];
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    sum += __shfl_xor_sync(0xffffffffu, sum, off);
-    sum2 += __shfl_xor_sync(0xffffffffu, sum2, off);
-    n += __shfl_xor_sync(0xffffffffu, n, off);
-  }
-  if (lane != 0) return;
-  if (n <= 0.0) {
-    weights[f] = 0.0f;
-    return;
-  }
-  const double mean = sum / n;
-  double var = sum2 / n - mean * mean;
-  if (var < 0.0) var = 0.0;
-  const double sd = sqrt(var);
-  const double e = static_cast<double>(eps);
-  const double w = sd <= e ? 1.0 / e : fmax(fabs(mean) / sd, e);
-  weights[f] = static_cast<float>(w * static_cast<double>(pw));
+__global__ void __launch_bounds__(256) frame_stats_kernel(const float* slots, const int* slot_of_frame, int64_t stride,
+                                                          int64_t pixels, const int* frames, double* partials) {
+  frame_stats_partial(slots, slot_of_frame, stride, pixels, frames[blockIdx.y], partials);
+}
+
+// Statistics of every frame (grid.y) and, in each frame's last CTA, its weight.
+template <int CAP>
+__global__ void __launch_bounds__(256) frame_weights_kernel(const float* slots, const int* slot_of_frame,
+                                                            int64_t stride, int64_t pixels, SnrArgs a,
+                                                            double* partials,
+                                                            const __grid_constant__ PriorBlock<CAP> prior) {
+  const int f = blockIdx.y;
+  frame_stats_partial(slots, slot_of_frame, stride, pixels, f, partials);
+  if (last_cta(a.tickets + f, gridDim.x) && threadIdx.x < 32) snr_weight(a, f, prior.at(f));
+}
+
+// mode 0: the prior alone.
+template <int CAP>
+__global__ void prior_weights_kernel(int frames, SnrArgs a, const __grid_constant__ PriorBlock<CAP> prior) {
+  const int f = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+  if (f < frames) snr_weight(a, f, prior.at(f));
+}
+
+template <int CAP>
+static void launch_weights(gg_stack* s, const SnrArgs& a, const float* host_prior, const float* more) {
+  PriorBlock<CAP> prior;
+  prior.given = host_prior != nullptr;
+  prior.more = more;
+  if (host_prior && !more) std::copy(host_prior, host_prior + s->frames, prior.w);
+  const auto frames = static_cast<unsigned>(s->frames);
+  note_launch();
+  if (a.mode == GG_WEIGHTS_SIMPLE_SNR)
+    frame_weights_kernel<CAP><<<dim3(a.blocks, frames), 256, 0, s->stream>>>(
+        s->d_slots, s->d_slot_of_frame, s->stride, s->pixels, a, s->d_partials, prior);
+  else
+    prior_weights_kernel<CAP><<<(frames + 3) / 4, 128, 0, s->stream>>>(static_cast<int>(frames), a, prior);
+  check_cuda(cudaGetLastError(), "frame weights launch");
 }
 
 // Per-CTA (sum, sum2, count) partials of the given frames (device frame list).
@@ -139,27 +192,29 @@ int gg_stack_compute_weights(gg_stack* s, int mode, const float* host_prior, flo
   const int64_t count = s->frames;
   const int blocks = static_cast<int>(std::min<int64_t>(sm_count() * 2, (s->pixels + 255) / 256));
   const size_t partial_doubles = static_cast<size_t>(count) * blocks * 3;
-  // partials | frame list (ints) | prior weights (floats)
+  // partials, then (above 1024 frames) the prior weights
   stack_ensure_partials(s, partial_doubles + static_cast<size_t>(count));
-  int* d_frames = reinterpret_cast<int*>(s->d_partials + partial_doubles);
-  float* d_prior = reinterpret_cast<float*>(d_frames + count);
-  int* h_frames = reinterpret_cast<int*>(s->h_partials_pinned + partial_doubles);
-  float* h_prior = reinterpret_cast<float*>(h_frames + count);
-  for (int64_t k = 0; k < count; ++k) {
-    h_frames[k] = static_cast<int>(k);
-    h_prior[k] = host_prior ? host_prior[k] : 1.0f;
+  SnrArgs a{};
+  a.partials = s->d_partials;
+  a.blocks = blocks;
+  a.eps = eps;
+  a.mode = mode;
+  a.weights = s->d_weights;
+  a.tickets = s->d_tickets;
+  if (count <= 64) {
+    launch_weights<64>(s, a, host_prior, nullptr);
+  } else if (count <= 1024) {
+    launch_weights<1024>(s, a, host_prior, nullptr);
+  } else {
+    float* d_prior = nullptr;
+    if (host_prior) {
+      d_prior = reinterpret_cast<float*>(s->d_partials + partial_doubles);
+      float* h_prior = reinterpret_cast<float*>(s->h_partials_pinned + partial_doubles);
+      std::copy(host_prior, host_prior + count, h_prior);
+      upload_params(s->stream, d_prior, h_prior, sizeof(float) * count, "cudaMemcpyAsync(prior weights)");
+    }
+    launch_weights<64>(s, a, host_prior, d_prior);
   }
-  upload_params(s->stream, d_frames, h_frames, sizeof(int) * count * 2, "cudaMemcpyAsync(weights frames)");
-  if (mode == GG_WEIGHTS_SIMPLE_SNR) {
-    note_launch();
-    frame_stats_kernel<<<dim3(blocks, static_cast<unsigned>(count)), 256, 0, s->stream>>>(
-        s->d_slots, s->d_slot_of_frame, s->stride, s->pixels, d_frames, s->d_partials);
-    check_cuda(cudaGetLastError(), "frame_stats kernel launch");
-  }
-  note_launch();
-  snr_weights_kernel<<<static_cast<unsigned>((count + 3) / 4), 128, 0, s->stream>>>(
-      s->d_partials, blocks, d_frames, static_cast<int>(count), d_prior, eps, mode, s->d_weights);
-  check_cuda(cudaGetLastError(), "snr_weights kernel launch");
   if (host_weights_out) {
     check_cuda(cudaMemcpyAsync(s->h_weights_pinned, s->d_weights, sizeof(float) * count, cudaMemcpyDeviceToHost,
                                s->stream),

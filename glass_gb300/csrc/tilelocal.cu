@@ -236,12 +236,7 @@ int gg_stack_integrate_tile_local(gg_stack* s, int mode, const float* host_weigh
   a.low = static_cast<float*>(s->d_low);
   a.high = static_cast<float*>(s->d_high);
   const size_t smem = sizeof(float) * n * kTlThreads;
-  check_cuda(cudaFuncSetAttribute(tile_local_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  static_cast<int>(smem)),
-             "cudaFuncSetAttribute(tile-local)");
-  int per_sm = 0;
-  check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tile_local_kernel, kTlThreads, smem),
-             "occupancy");
+  const int per_sm = kernel_ctas_per_sm(tile_local_kernel, kTlThreads, smem, "launch shape (tile-local)");
   note_launch();
   tile_local_kernel<<<grid_for(static_cast<size_t>(s->pixels), kTlThreads, std::max(per_sm, 1)), kTlThreads, smem,
                       s->stream>>>(a);

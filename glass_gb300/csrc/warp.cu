@@ -22,7 +22,7 @@
 //     compute.  Footprints that do not fit the box (large rotation/scale) and
 //     image widths that TMA cannot describe (W % 4 != 0) read the taps straight
 //     from global memory instead;
-//   - output goes to a spare slot; a follow-up kernel swaps the frame->slot
+//   - output goes to a spare slot; the launch's last CTA swaps the frame->slot
 //     table, so nothing is copied back (8 B/pixel instead of 16 B);
 //   - Lanczos3 weights are paired even/odd polynomials in (t - 1/2)^2
 //     (sampling.cuh); tiles of affine maps run straight-line rows: two columns
@@ -77,6 +77,10 @@ struct WarpItem {
 struct WarpArgs {
   float* slots;
   unsigned* nonfinite;  // per frame: non-finite output samples are added
+  // in-place warp: the last CTA makes the output slots the frames' own
+  int* slot_of_frame;  // nullptr: not an in-place warp
+  int* spare;
+  unsigned* ticket;
   WarpItem* items;
   int item_count;
   int64_t stride;
@@ -775,27 +779,58 @@ __global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __gri
       break;
     }
   }
+  if (a.slot_of_frame != nullptr && last_cta(a.ticket, gridDim.x)) {
+    // the warped frame lives in the spare slot, and its old slot is spare
+    for (int k = tid; k < a.item_count; k += kWarpThreads) {
+      a.slot_of_frame[a.items[k].frame] = a.items[k].dst_slot;
+      a.spare[k] = a.items[k].src_slot;
+    }
+  }
 }
 
 // Resolve slots for the batch and move the source non-finite counts aside.
+__device__ __forceinline__ void warp_prepare_item(WarpItem& it, int k, const int* slot_of_frame, const int* spare,
+                                                  unsigned* nonfinite, float* slots, int64_t stride) {
+  it.src_slot = slot_of_frame[it.frame];
+  it.dst_slot = spare[k];
+  it.dst = slots + spare[k] * stride;
+  it.src_nonfinite = nonfinite[it.frame];
+  nonfinite[it.frame] = 0u;
+}
+
 __global__ void warp_prepare_kernel(WarpItem* items, int count, const int* slot_of_frame, const int* spare,
                                     unsigned* nonfinite, float* slots, int64_t stride) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= count) return;
-  const int f = items[k].frame;
-  items[k].src_slot = slot_of_frame[f];
-  items[k].dst_slot = spare[k];
-  items[k].dst = slots + spare[k] * stride;
-  items[k].src_nonfinite = nonfinite[f];
-  nonfinite[f] = 0u;
+  if (k < count) warp_prepare_item(items[k], k, slot_of_frame, spare, nonfinite, slots, stride);
 }
 
-// The warped frame now lives in the spare slot; the old slot becomes spare.
-__global__ void warp_finish_kernel(const WarpItem* items, int count, int* slot_of_frame, int* spare) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// The same with the descriptors in the launch parameters.
+template <int CAP>
+struct WarpItemBlock {
+  WarpItem items[CAP];
+};
+
+template <int CAP>
+__global__ void __launch_bounds__(128) warp_prepare_block_kernel(const __grid_constant__ WarpItemBlock<CAP> block,
+                                                                 WarpItem* items, int count, const int* slot_of_frame,
+                                                                 const int* spare, unsigned* nonfinite, float* slots,
+                                                                 int64_t stride) {
+  const int k = threadIdx.x;
   if (k >= count) return;
-  slot_of_frame[items[k].frame] = items[k].dst_slot;
-  spare[k] = items[k].src_slot;
+  WarpItem it = block.items[k];
+  warp_prepare_item(it, k, slot_of_frame, spare, nonfinite, slots, stride);
+  items[k] = it;
+}
+
+template <int CAP>
+static void launch_prepare_block(gg_stack* s, WarpItem* d_items, const std::vector<WarpItem>& items) {
+  WarpItemBlock<CAP> block;
+  std::copy(items.begin(), items.end(), block.items);
+  note_launch();
+  warp_prepare_block_kernel<CAP><<<1, 128, 0, s->stream>>>(block, d_items, static_cast<int>(items.size()),
+                                                          s->d_slot_of_frame, s->d_spare_slot, s->d_frame_nonfinite,
+                                                          s->d_slots, s->stride);
+  check_cuda(cudaGetLastError(), "warp_prepare launch");
 }
 
 __global__ void fill_kernel(float* p, int64_t n, float v) {
@@ -944,27 +979,30 @@ static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices
 
 // The kernels of a warp batch whose descriptors are already in device
 // memory (d_items, `count` of them): per group of at most `spares` frames,
-// resolve slots, warp into the spare slots, swap the slot table.  Only
-// launches on the stack's stream (safe inside a stream capture).
+// resolve slots (unless that is done: `prepared`), warp into the spare slots,
+// swap the slot table.  Only launches on the stack's stream (safe inside a stream
+// capture).
 static void launch_warp_items(gg_stack* s, WarpItem* d_items, int64_t count, int interp, float fill, float clamp,
-                              bool track_coverage) {
+                              bool track_coverage, bool prepared = false) {
+  stack_slots_moved(s);
   for (int64_t k0 = 0; k0 < count; k0 += s->spares) {
     const int nb = static_cast<int>(std::min<int64_t>(s->spares, count - k0));
-    note_launch();
-    warp_prepare_kernel<<<(nb + 127) / 128, 128, 0, s->stream>>>(d_items + k0, nb, s->d_slot_of_frame,
-                                                                 s->d_spare_slot, s->d_frame_nonfinite, s->d_slots,
-                                                                 s->stride);
-    check_cuda(cudaGetLastError(), "warp_prepare launch");
+    if (!prepared) {
+      note_launch();
+      warp_prepare_kernel<<<(nb + 127) / 128, 128, 0, s->stream>>>(d_items + k0, nb, s->d_slot_of_frame,
+                                                                   s->d_spare_slot, s->d_frame_nonfinite, s->d_slots,
+                                                                   s->stride);
+      check_cuda(cudaGetLastError(), "warp_prepare launch");
+    }
     WarpArgs a = warp_args(s, d_items + k0, nb, 0, static_cast<int>(s->height));
     a.nonfinite = s->d_frame_nonfinite;
     a.fill = fill;
     a.clamp = clamp;
     a.coverage = track_coverage ? s->d_warp_coverage : nullptr;
+    a.slot_of_frame = s->d_slot_of_frame;
+    a.spare = s->d_spare_slot;
+    a.ticket = s->d_tickets + s->frames;
     launch_warp_rows(s, a, interp);
-    note_launch();
-    warp_finish_kernel<<<(nb + 127) / 128, 128, 0, s->stream>>>(d_items + k0, nb, s->d_slot_of_frame,
-                                                                s->d_spare_slot);
-    check_cuda(cudaGetLastError(), "warp_finish launch");
   }
 }
 
@@ -973,13 +1011,24 @@ void warp_frames(gg_stack* s, const int64_t* indices, int64_t count, const doubl
   const std::vector<WarpItem> items = warp_items_host(s, indices, count, fwd);
   ensure_warp_items(s, std::max<int64_t>(count, s->spares));
   if (track_coverage) ensure_warp_coverage(s);
+  auto* d_items = static_cast<WarpItem*>(s->d_warp_items);
+  // a batch that fits the launch parameters and the spare slots at once
+  constexpr int kSmallBlock = 16, kLargeBlock = 96;
+  static_assert(sizeof(WarpItemBlock<kLargeBlock>) <= 16384, "launch parameters");
+  if (count <= std::min<int64_t>(s->spares, kLargeBlock)) {
+    if (count <= kSmallBlock) launch_prepare_block<kSmallBlock>(s, d_items, items);
+    else launch_prepare_block<kLargeBlock>(s, d_items, items);
+    launch_warp_items(s, d_items, count, interp, fill, clamp, track_coverage, true);
+    if (track_coverage) s->warp_coverage_frames += count;
+    return;
+  }
   // The staging buffer may still feed the previous call's copy.
   check_cuda(cudaEventSynchronize(s->warp_items_free), "cudaEventSynchronize(warp items)");
   std::memcpy(s->h_warp_items, items.data(), sizeof(WarpItem) * items.size());
   upload_params(s->stream, s->d_warp_items, s->h_warp_items, sizeof(WarpItem) * items.size(),
                 "cudaMemcpyAsync(warp items)");
   check_cuda(cudaEventRecord(s->warp_items_free, s->stream), "cudaEventRecord(warp items)");
-  launch_warp_items(s, static_cast<WarpItem*>(s->d_warp_items), count, interp, fill, clamp, track_coverage);
+  launch_warp_items(s, d_items, count, interp, fill, clamp, track_coverage);
   if (track_coverage) s->warp_coverage_frames += count;
 }
 
