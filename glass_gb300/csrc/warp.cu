@@ -92,6 +92,7 @@ struct WarpArgs {
   float fill;
   float clamp;
   float* coverage;  // optional accumulator (+1 per covered pixel)
+  int counted;      // whole tiles (counts_whole) are in it already
   int* error;
 };
 
@@ -646,6 +647,15 @@ __device__ __forceinline__ unsigned bilinear_rows(const TileGrid& grid, const Wi
   return MASK ? bad : count_nonfinite(probe, out, out_pitch, ROWS);
 }
 
+// Whether every pixel of a tile is known to be valid: such tiles take the
+// unmasked rows.
+template <int INTERP, int TH>
+__device__ __forceinline__ bool counts_whole(const WarpArgs& a, const TilePlan& p, bool finite, int tile_x0,
+                                             int tile_y0) {
+  const bool full_tile = tile_x0 + kTileW <= a.width && tile_y0 + TH <= a.row1;
+  return p.interior && p.grid && full_tile && (INTERP != GG_INTERP_LANCZOS3 || (finite && a.clamp < 0.0f));
+}
+
 // Two box buffers: the next tile's copy is in flight while this one's rows are
 // computed.
 constexpr size_t kWarpTileBytes = size_t(2) * kBoxH * kBoxW * sizeof(float);
@@ -721,7 +731,7 @@ __global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __gri
       }
       phase[buf] ^= 1u;
     }
-    const bool full_tile = tile_x0 + kTileW <= a.width && tile_y0 + TH <= a.row1;
+    const bool whole = counts_whole<INTERP, TH>(a, p, finite, tile_x0, tile_y0);
     unsigned bad = 0;
     if (INTERP != GG_INTERP_NEAREST && p.grid && (!kLanczos || a.clamp < 0.0f) &&
         (p.fits || !kLanczos || (a.width >= 6 && a.height >= 6))) {
@@ -744,8 +754,8 @@ __global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __gri
           if (int_shift) return shifted_rows<TH / 4, kStaged>(grid, win, mask, a.fill, out, a.width, lx, ly);
           if (!finite) return lanczos3_renorm_rows<TH / 4, kStaged>(grid, win, mask, a.fill, out, a.width, lx, ly);
         }
-        return p.interior && full_tile && a.coverage == nullptr ? rows(win, std::false_type{})
-                                                                : rows(win, std::true_type{});
+        return whole && (a.coverage == nullptr || a.counted) ? rows(win, std::false_type{})
+                                                            : rows(win, std::true_type{});
       };
       constexpr int kSpan = kLanczos ? 6 : 1;  // of a window's possible places
       const int x0 = -grid.ox, y0 = -grid.oy, x1 = a.width - kSpan + x0, y1 = a.height - kSpan + y0;
@@ -786,6 +796,31 @@ __global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __gri
       a.spare[k] = a.items[k].src_slot;
     }
   }
+}
+
+// Frames with a geometrically valid sample, per pixel of a band: this kernel
+// writes each tile's frames that count for the whole tile (all but those whose
+// border crosses it), the warp then adds the others' valid pixels.
+template <int INTERP, int TH>
+__global__ void __launch_bounds__(kWarpThreads) warp_geometry_kernel(WarpArgs a) {
+  __shared__ int s_inside;
+  const int tile_x0 = blockIdx.x % a.tiles_x * kTileW, tile_y0 = a.row0 + blockIdx.x / a.tiles_x * TH;
+  if (threadIdx.x == 0) s_inside = 0;
+  __syncthreads();
+  constexpr bool kLanczos = INTERP == GG_INTERP_LANCZOS3;
+  const float vlo = kLanczos ? 2.0f : 0.0f, off = kLanczos ? 3.0f : 1.0f;
+  for (int f = threadIdx.x; f < a.item_count; f += kWarpThreads) {
+    const WarpItem* ip = a.items + f;
+    const TilePlan p = plan_tile<TH>(load_coef(ip), tile_x0, tile_y0, kLanczos ? 3 : 1, vlo,
+                                     static_cast<float>(a.width) - off, static_cast<float>(a.height) - off);
+    if (counts_whole<INTERP, TH>(a, p, ip->src_nonfinite == 0u, tile_x0, tile_y0)) atomicAdd(&s_inside, 1);
+  }
+  __syncthreads();
+  const float n = static_cast<float>(s_inside);
+  const int ox = tile_x0 + (threadIdx.x & 63);
+  if (ox >= a.width) return;
+  for (int oy = tile_y0 + (threadIdx.x >> 6); oy < min(tile_y0 + TH, a.row1); oy += kWarpThreads / kTileW)
+    a.coverage[static_cast<int64_t>(oy) * a.width + ox] = n;
 }
 
 // Resolve slots for the batch and move the source non-finite counts aside.
@@ -900,9 +935,17 @@ static void ensure_warp_coverage(gg_stack* s) {
 }
 
 template <int INTERP, int TH>
+static void launch_warp_geometry(gg_stack* s, const WarpArgs& a) {
+  note_launch();
+  warp_geometry_kernel<INTERP, TH><<<static_cast<unsigned>(a.tiles_x * a.tiles_y), kWarpThreads, 0, s->stream>>>(a);
+  check_cuda(cudaGetLastError(), "warp_geometry launch");
+}
+
+template <int INTERP, int TH>
 static void launch_warp_tiles(gg_stack* s, WarpArgs args) {
   const bool use_tma = s->has_slot_tmap;
   args.tiles_y = (args.row1 - args.row0 + TH - 1) / TH;
+  if (args.counted) launch_warp_geometry<INTERP, TH>(s, args);
   auto kern = use_tma ? warp_tiles_kernel<INTERP, true, TH> : warp_tiles_kernel<INTERP, false, TH>;
   const size_t smem = use_tma ? kWarpTileBytes : 0;
   const int per_sm = kernel_ctas_per_sm(kern, kWarpThreads, smem, "warp launch shape");
@@ -1142,72 +1185,15 @@ __global__ void __launch_bounds__(256) warp_nonfinite_kernel(WarpArgs a, unsigne
   if (bad) counts[blockIdx.y] = 1u;
 }
 
-// Frames with a geometrically valid sample, per pixel of a band.  One CTA per
-// tile: a frame that maps the whole tile inside its valid range counts
-// for every pixel without a test (all but the tiles along the border), the
-// others are evaluated pixel by pixel.  Where a Lanczos3 frame holds
-// non-finite samples, a window may have no weight left: its warped sample
-// tells (NaN).
-template <int INTERP>
-__global__ void __launch_bounds__(kWarpThreads) warp_geometry_kernel(WarpArgs a, float* geometric) {
-  __shared__ int s_inside, s_mixed;
-  __shared__ int s_list[512];
-  const int tile_x0 = blockIdx.x % a.tiles_x * kTileW, tile_y0 = a.row0 + blockIdx.x / a.tiles_x * kTileH;
-  if (threadIdx.x == 0) s_inside = s_mixed = 0;
-  __syncthreads();
-  constexpr bool kLanczos = INTERP == GG_INTERP_LANCZOS3;
-  const float vlo = kLanczos ? 2.0f : 0.0f, off = kLanczos ? 3.0f : 1.0f;
-  for (int f = threadIdx.x; f < a.item_count; f += kWarpThreads) {
-    const WarpItem* ip = a.items + f;
-    const bool by_value = kLanczos && ip->src_nonfinite != 0u;
-    const TilePlan p = plan_tile<kTileH>(load_coef(ip), tile_x0, tile_y0, kLanczos ? 3 : 1, vlo,
-                                 static_cast<float>(a.width) - off, static_cast<float>(a.height) - off);
-    if (p.interior && !by_value) atomicAdd(&s_inside, 1);
-    else s_list[atomicAdd(&s_mixed, 1)] = f;
-  }
-  __syncthreads();
-  const int ox = tile_x0 + (threadIdx.x & 63);
-  if (ox >= a.width) return;
-  constexpr int kRows = kTileH * kTileW / kWarpThreads, kStep = kWarpThreads / kTileW;
-  int n[kRows];
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) n[r] = s_inside;
-  for (int i = 0; i < s_mixed; ++i) {
-    const WarpItem* ip = a.items + s_list[i];
-    const Coef co = load_coef(ip);
-    const bool by_value = kLanczos && ip->src_nonfinite != 0u;
-    const float* dst = ip->dst - static_cast<int64_t>(a.row0) * a.width;
-    FFv sx, sy;
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      const int oy = tile_y0 + (threadIdx.x >> 6) + kStep * r;
-      if (oy >= a.row1) continue;
-      if (by_value) n[r] += !isnan(dst[static_cast<int64_t>(oy) * a.width + ox]);
-      else n[r] += sample_valid<INTERP>(co, ox, oy, a.width, a.height, sx, sy);
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const int oy = tile_y0 + (threadIdx.x >> 6) + kStep * r;
-    if (oy < a.row1) geometric[static_cast<int64_t>(oy) * a.width + ox] = static_cast<float>(n[r]);
-  }
-}
-
 void launch_warp_band(gg_stack* s, void* d_items, int interp, float clamp, int row0, int row1, unsigned* counts,
                       float* geometric) {
   WarpArgs a = warp_args(s, static_cast<WarpItem*>(d_items), static_cast<int>(s->frames), row0, row1);
   a.nonfinite = counts;
   a.fill = NAN;
   a.clamp = clamp;
+  a.coverage = geometric;
+  a.counted = 1;
   launch_warp_rows(s, a, interp);
-  a.tiles_y = (row1 - row0 + kTileH - 1) / kTileH;
-  const unsigned tiles = static_cast<unsigned>(a.tiles_x) * static_cast<unsigned>(a.tiles_y);
-  note_launch();
-  if (interp == GG_INTERP_BILINEAR)
-    warp_geometry_kernel<GG_INTERP_BILINEAR><<<tiles, kWarpThreads, 0, s->stream>>>(a, geometric);
-  else
-    warp_geometry_kernel<GG_INTERP_LANCZOS3><<<tiles, kWarpThreads, 0, s->stream>>>(a, geometric);
-  check_cuda(cudaGetLastError(), "warp_geometry launch");
 }
 
 void launch_warp_band_prepare(gg_stack* s, void* d_items, const FusedFrame* d_frames, int interp, float clamp,
