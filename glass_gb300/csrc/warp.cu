@@ -823,6 +823,96 @@ __global__ void __launch_bounds__(kWarpThreads) warp_geometry_kernel(WarpArgs a)
     a.coverage[static_cast<int64_t>(oy) * a.width + ox] = n;
 }
 
+// One tile per CTA of an image's affine warp, windows from global memory.
+template <int INTERP, int TH>
+__global__ void __launch_bounds__(kWarpThreads, 4) affine_tiles_kernel(const __grid_constant__ WarpItem item,
+                                                                    const float* src, float* dst, int finite,
+                                                                    WarpArgs a) {
+  __shared__ TilePlan s_plan;
+  __shared__ TileGrid s_grid;
+  constexpr bool kLanczos = INTERP == GG_INTERP_LANCZOS3;
+  const int tid = threadIdx.x;
+  const int tile_x0 = blockIdx.x % a.tiles_x * kTileW, tile_y0 = blockIdx.x / a.tiles_x * TH;
+  Coef co;
+#pragma unroll
+  for (int q = 0; q < 9; ++q) {
+    co.m[q][0] = item.m[q][0];
+    co.m[q][1] = item.m[q][1];
+  }
+  co.affine = item.affine;
+  if (tid < 32) {
+    const float off = kLanczos ? 3.0f : 1.0f;
+    const TilePlan p = plan_tile_warp<TH>(co, tile_x0, tile_y0, kLanczos ? 3 : 1, kLanczos ? 2.0f : 0.0f,
+                                          static_cast<float>(a.width) - off, static_cast<float>(a.height) - off);
+    if (p.grid) tile_grid_warp(item.inv, tile_x0, tile_y0, false, 0, 0, s_grid);
+    if (tid == 0) s_plan = p;
+  }
+  __syncthreads();
+  const TilePlan p = s_plan;
+  if (p.grid && (!kLanczos || (a.width >= 6 && a.height >= 6))) {
+    const TileGrid& grid = s_grid;
+    const int lx = tid & 31, ly = (tid >> 5) * (TH / 4);
+    float* out = dst + static_cast<int64_t>(tile_y0 + ly) * a.width + tile_x0 + lx;
+    const TileMask mask = tile_mask(grid, kLanczos, a.width, a.height, tile_x0, tile_y0, a.row1, nullptr);
+    constexpr int kSpan = kLanczos ? 6 : 1;
+    const int x0 = -grid.ox, y0 = -grid.oy;
+    const Window<false> win{src + static_cast<int64_t>(grid.oy) * a.width + grid.ox, a.width, x0,
+                            a.width - kSpan + x0, y0, a.height - kSpan + y0};
+    const bool whole = counts_whole<INTERP, TH>(a, p, finite != 0, tile_x0, tile_y0);
+    if constexpr (kLanczos) {
+      if (!finite) lanczos3_renorm_rows<TH / 4, false>(grid, win, mask, a.fill, out, a.width, lx, ly);
+      else if (whole) lanczos3_rows<TH / 4, false, false>(grid, win, mask, a.fill, out, a.width, lx, ly);
+      else lanczos3_rows<TH / 4, false, true>(grid, win, mask, a.fill, out, a.width, lx, ly);
+    } else {
+      if (whole) bilinear_rows<TH / 4, false, false>(grid, win, mask, a.fill, out, a.width, lx, ly);
+      else bilinear_rows<TH / 4, false, true>(grid, win, mask, a.fill, out, a.width, lx, ly);
+    }
+    return;
+  }
+  TapSource ts;
+  ts.tile = nullptr;
+  ts.src = src;
+  ts.bx = ts.by = 0;
+  ts.width = a.width;
+#pragma unroll 1
+  for (int c = tid / kTileW; c < kRowClasses; c += kWarpThreads / kTileW) {
+    const int ox = tile_x0 + tid % kTileW, oy0 = tile_y0 + c;
+    if (kLanczos && finite) warp_tile_rows<INTERP, true, TH>(a, co, ts, dst, ox, oy0, p.interior != 0, false);
+    else warp_tile_rows<INTERP, false, TH>(a, co, ts, dst, ox, oy0, p.interior != 0, false);
+  }
+}
+
+void launch_affine_warp(const float* src, int height, int width, const double* theta, int interp, float fill,
+                        bool finite, float* dst, cudaStream_t stream) {
+  WarpItem item{};
+  item.affine = 1;
+  for (int q = 0; q < 6; ++q) {
+    item.inv[q] = theta[q];
+    item.m[q][0] = static_cast<float>(theta[q]);
+    item.m[q][1] = static_cast<float>(theta[q] - static_cast<double>(item.m[q][0]));
+  }
+  item.m[8][0] = 1.0f;
+  WarpArgs a{};
+  a.width = width;
+  a.height = a.row1 = height;
+  a.tiles_x = (width + kTileW - 1) / kTileW;
+  a.fill = fill;
+  a.clamp = -1.0f;
+  auto launch = [&](auto kern, int th) {
+    const int64_t tiles = static_cast<int64_t>(a.tiles_x) * ((height + th - 1) / th);
+    note_launch();
+    kern<<<static_cast<unsigned>(tiles), kWarpThreads, 0, stream>>>(item, src, dst, finite ? 1 : 0, a);
+    check_cuda(cudaGetLastError(), "affine warp launch");
+  };
+  const bool small = static_cast<int64_t>(a.tiles_x) * ((height + kTileH - 1) / kTileH) < 2 * sm_count();
+  if (interp == GG_INTERP_BILINEAR)
+    small ? launch(affine_tiles_kernel<GG_INTERP_BILINEAR, kSmallTileH>, kSmallTileH)
+          : launch(affine_tiles_kernel<GG_INTERP_BILINEAR, kTileH>, kTileH);
+  else
+    small ? launch(affine_tiles_kernel<GG_INTERP_LANCZOS3, kSmallTileH>, kSmallTileH)
+          : launch(affine_tiles_kernel<GG_INTERP_LANCZOS3, kTileH>, kTileH);
+}
+
 // Resolve slots for the batch and move the source non-finite counts aside.
 __device__ __forceinline__ void warp_prepare_item(WarpItem& it, int k, const int* slot_of_frame, const int* spare,
                                                   unsigned* nonfinite, float* slots, int64_t stride) {

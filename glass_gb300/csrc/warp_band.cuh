@@ -1,5 +1,5 @@
-// Interface between the warp (warp.cu) and the fused warp + integration
-// (integrate.cu).
+// Interface of the warp (warp.cu) to the fused warp + integration (integrate.cu)
+// and to the differentiable warp (adjoint.cu).
 #pragma once
 
 #include "stack.cuh"
@@ -38,5 +38,10 @@ void launch_warp_band_prepare(gg_stack* s, void* d_items, const FusedFrame* d_fr
 // stack's stream (safe inside a stream capture).
 void launch_warp_band(gg_stack* s, void* d_items, int interp, float clamp, int row0, int row1, unsigned* counts,
                       float* geometric);
+
+// Warp of one device image by inverse affine parameters; finite: the image is
+// known to hold no non-finite sample.
+void launch_affine_warp(const float* src, int height, int width, const double* theta, int interp, float fill,
+                        bool finite, float* dst, cudaStream_t stream);
 
 }  // namespace gg
