@@ -14,10 +14,11 @@
 //   star_detect.py:103-118), then the brightest `max_stars`.
 //
 // GB300 layout:
-//   - order statistics by a 3-pass radix select over the frame (11+11+10 key
-//     bits, per-CTA shared-memory histograms fed by per-thread run-length
-//     counters and folded with global atomics); the MAD reuses it with key
-//     |v - median|;
+//   - order statistics in one pass over the frame: a sample gives a key band
+//     around the wanted ranks, the pass keeps the band's keys and a cluster per
+//     frame selects among them; the MAD does the same with key |v - median|.
+//     Frames whose band misses (heavily tied data) take a 3-pass radix select
+//     (11+11+10 key bits, per-CTA histograms folded with global atomics);
 //   - candidates are appended with one atomic per warp, then one CTA per
 //     frame sorts them into raster order in shared memory, measures flux and
 //     centroid one warp per candidate, resolves the flux-ordered
@@ -31,6 +32,7 @@
 #include <cstring>
 #include <vector>
 
+#include <cooperative_groups.h>
 #include <math_constants.h>
 
 #include "stack.cuh"
@@ -45,7 +47,7 @@ struct StarFrameState {
   unsigned count;        // valid (finite) pixels
   unsigned candidates;   // appended candidates (may exceed capacity)
   unsigned overflow;
-  unsigned pad;
+  unsigned ticket;       // CTAs that have finished (zero between launches)
   unsigned prefix[2];    // radix-select prefix per requested rank
   unsigned residual[2];  // rank remaining inside the prefix bucket
   float median;
@@ -62,9 +64,6 @@ struct StarFrameState {
   unsigned below;             // finite keys under band_lo
   unsigned inside;            // keys in the band (appended, may exceed capacity)
   int resolved[2];            // 1: the order statistic came from the band
-  // radix select inside the band (bracket_band_* kernels)
-  unsigned band_prefix[2], band_rank[2];
-  int band_ok, band_shift;
 };
 
 __device__ __forceinline__ unsigned float_key(float v) {
@@ -83,9 +82,66 @@ struct SelectArgs {
   const int* frames;   // [count]
   StarFrameState* state;
   unsigned* hist;      // [count][2][kSelBins]
-  int pass;            // 0, 1, 2
   int mode;            // 0: v, 1: |v - median|
 };
+
+// Locate each rank's bucket in the frame's complete histogram (a warp prefix
+// scan over 32 runs of bins).  Pass 0 sets the ranks from the valid count
+// (median of n: n//2 and n//2 - 1 when n is even, both n//2 when odd).
+template <int PASS>
+__device__ void select_digit(const SelectArgs& a, StarFrameState& st, const unsigned (*hs)[kSelBins]) {
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  const unsigned count = __ldcg(&st.count);
+  constexpr int kBins = PASS == 2 ? 1024 : kSelBins;
+  constexpr int kPer = kBins / 32;
+  constexpr int kBits = PASS == 2 ? 10 : 11;
+  unsigned prefix[2];
+  for (int r = 0; r < 2; ++r) {
+    const unsigned* hr = hs[PASS == 0 ? 0 : r];
+    unsigned rem;
+    if constexpr (PASS == 0) {
+      const unsigned hi = count / 2;
+      rem = r == 1 || (count & 1u) ? hi : (hi > 0 ? hi - 1 : 0);
+    } else {
+      rem = st.residual[r];
+    }
+    unsigned loc = 0;
+    for (int b = 0; b < kPer; ++b) loc += hr[lane * kPer + b];
+    unsigned incl = loc;
+    for (int off = 1; off < 32; off <<= 1) {
+      const unsigned v = __shfl_up_sync(0xffffffffu, incl, off);
+      if (lane >= off) incl += v;
+    }
+    const unsigned excl = incl - loc;
+    const bool here = excl <= rem && rem < incl;
+    unsigned bucket = static_cast<unsigned>(kBins - 1), left = 0u;  // empty frame (rank past the end)
+    if (here) {
+      left = rem - excl;
+      int b = lane * kPer;
+      while (left >= hr[b]) {
+        left -= hr[b];
+        ++b;
+      }
+      bucket = static_cast<unsigned>(b);
+    }
+    const unsigned owner = __ballot_sync(0xffffffffu, here);
+    const int from = owner ? __ffs(owner) - 1 : 0;
+    bucket = __shfl_sync(0xffffffffu, bucket, from);
+    left = __shfl_sync(0xffffffffu, left, from);
+    prefix[r] = ((PASS == 0 ? 0u : st.prefix[r]) << kBits) | bucket;
+    __syncwarp();
+    if (lane == 0) {
+      st.prefix[r] = prefix[r];
+      st.residual[r] = left;
+    }
+  }
+  if (PASS == 2 && lane == 0) {
+    // Both keys are complete: value = mean of the two middle values.
+    const float med = count ? __fmul_rn(__fadd_rn(key_float(prefix[0]), key_float(prefix[1])), 0.5f) : 0.0f;
+    if (a.mode == 0) st.median = med; else st.mad = med;
+  }
+}
 
 // Histogram pass: digit of `pass` for keys matching each rank's prefix.
 // Sky pixels share their leading digits, so each thread keeps a run-length
@@ -169,92 +225,29 @@ __global__ void __launch_bounds__(256) select_hist_kernel(SelectArgs a) {
     if (v) atomicAdd(g + i, v);
   }
   if (PASS == 0 && a.mode == 0 && threadIdx.x == 0 && s_valid) atomicAdd(&a.state[k].count, s_valid);
-}
-
-// One block per frame: locate each rank's bucket in the histogram (copied to
-// shared memory, then a warp prefix scan over 32 runs of bins).
-// ranks: pass 0 sets them from the valid count (median of n: n//2 and
-// n//2 - 1 when n is even, both n//2 when odd).
-__global__ void __launch_bounds__(256) select_scan_kernel(SelectArgs a, int frames) {
-  __shared__ unsigned hs[2][kSelBins];
-  __shared__ unsigned s_bucket[2], s_rem[2];
-  const int k = blockIdx.x;
-  if (k >= frames) return;
-  StarFrameState& st = a.state[k];
-  if (st.resolved[a.mode]) return;  // the sample bracket found it
-  const unsigned* g = a.hist + static_cast<int64_t>(k) * 2 * kSelBins;
-  const int nbins = a.pass == 2 ? 1024 : kSelBins;
-  const int nh = a.pass == 0 ? 1 : 2;
-  for (int i = threadIdx.x; i < nh * kSelBins; i += blockDim.x) (&hs[0][0])[i] = g[i];
-  if (threadIdx.x == 0 && a.pass == 0) {
-    const unsigned n = st.count;
-    const unsigned hi = n / 2;
-    const unsigned lo = (n & 1u) ? hi : (hi > 0 ? hi - 1 : 0);
-    st.residual[0] = lo;
-    st.residual[1] = hi;
+  // the frame's last CTA finds the digit and leaves the histogram zeroed
+  if (!last_cta(&a.state[k].ticket, gridDim.x)) return;
+  for (int i = threadIdx.x; i < nh * kSelBins; i += blockDim.x) {
+    (&h[0][0])[i] = __ldcg(g + i);
+    g[i] = 0u;
   }
   __syncthreads();
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    const int per = nbins / 32;
-    for (int r = 0; r < 2; ++r) {
-      const unsigned* hr = hs[a.pass == 0 ? 0 : r];
-      const unsigned rem = st.residual[r];
-      unsigned loc = 0;
-      for (int b = 0; b < per; ++b) loc += hr[lane * per + b];
-      unsigned incl = loc;
-      for (int off = 1; off < 32; off <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, incl, off);
-        if (lane >= off) incl += v;
-      }
-      const unsigned excl = incl - loc;
-      if (lane == 0) {  // empty frame (rank past the end): keeps the state defined
-        s_bucket[r] = static_cast<unsigned>(nbins - 1);
-        s_rem[r] = 0u;
-      }
-      __syncwarp();
-      if (excl <= rem && rem < incl) {
-        unsigned left = rem - excl;
-        int b = lane * per;
-        while (left >= hr[b]) {
-          left -= hr[b];
-          ++b;
-        }
-        s_bucket[r] = static_cast<unsigned>(b);
-        s_rem[r] = left;
-      }
-      __syncwarp();
-    }
-    if (lane == 0) {
-      const int bits = a.pass == 2 ? 10 : 11;
-      for (int r = 0; r < 2; ++r) {
-        const unsigned prev = a.pass == 0 ? 0u : st.prefix[r];
-        st.prefix[r] = (prev << bits) | s_bucket[r];
-        st.residual[r] = s_rem[r];
-      }
-    }
-  }
-  if (threadIdx.x == 0) {
-    if (a.pass == 2) {
-      // Both keys are complete: value = mean of the two middle values.
-      const float lo = key_float(st.prefix[0]);
-      const float hi = key_float(st.prefix[1]);
-      const float med = st.count ? __fmul_rn(__fadd_rn(lo, hi), 0.5f) : 0.0f;
-      if (a.mode == 0) st.median = med; else st.mad = med;
-    }
-  }
+  select_digit<PASS>(a, a.state[k], h);
 }
 
 // ---- order statistics by a sample bracket ------------------------------------
-// One pass over the frame instead of three: a sample of kBracketSamples
-// evenly spaced pixels is sorted in shared memory and gives a key band that
-// holds the wanted ranks (the middle ranks of the finite pixels) with a
-// seven-sigma margin; the pass counts the finite keys below the band and
-// copies the keys inside it to a per-frame buffer, where a radix select over
-// the band's key range finds the exact order statistics.  A frame whose band
-// misses the ranks or overflows the buffer (heavily tied data) keeps
-// resolved = 0 and goes through the three-pass radix select above.
+// One pass over the frame instead of three: the middle ranks of
+// kBracketSamples evenly spaced pixels give a key band that holds the wanted
+// ranks (the middle ranks of the finite pixels) with a seven-sigma margin; the
+// pass counts the finite keys below the band and copies the keys inside it to
+// a per-frame buffer, where a radix select over the band's key range finds the
+// exact order statistics.  A frame whose band misses the ranks or overflows
+// the buffer (heavily tied data) keeps resolved = 0 and goes through the
+// three-pass radix select above.
 constexpr int kBracketSamples = 32768;
+constexpr int kSampleThreads = 1024;
+constexpr int kSampleCtas = 8;  // per frame: the scattered reads of the sample
+constexpr unsigned kNoKey = 0xffffffffu;  // above every finite key
 
 struct BracketArgs {
   const float* slots;
@@ -263,12 +256,9 @@ struct BracketArgs {
   int64_t pixels;
   const int* frames;
   StarFrameState* state;
-  unsigned* band;      // [count][band_cap]
-  int64_t band_cap;
+  unsigned* band;      // [count][band_cap]; holds the sample's keys first (band_cap >= its size)
+  int64_t band_cap;    // a multiple of 4
   int mode;            // 0: v, 1: |v - median|
-  unsigned* ghist;     // [count][2][256] band histograms (zero between passes)
-  int pass;            // radix pass of the band select (0..3)
-  int count_frames;
 };
 
 __device__ __forceinline__ bool bracket_key(float v, int mode, float median, unsigned& key) {
@@ -277,53 +267,87 @@ __device__ __forceinline__ bool bracket_key(float v, int mode, float median, uns
   return true;
 }
 
-__global__ void __launch_bounds__(1024) bracket_sample_kernel(BracketArgs a) {
-  extern __shared__ unsigned keys[];  // kBracketSamples (or pixels, if fewer)
-  __shared__ unsigned s_valid;
-  const int k = blockIdx.x;
+// The sample's two band edges.  Several CTAs per frame read the scattered
+// pixels; the last one holds the 32768 keys in registers and finds the two
+// ranks bit by bit from the top, counting the keys below a trial prefix: 32
+// rounds of register compares and one block sum each, whatever the values.
+// The rounds bound it: 338 us as a bitonic sort of the sample in shared memory
+// by one CTA per frame, 43 us here (8 frames of 4096^2).
+__global__ void __launch_bounds__(kSampleThreads) bracket_sample_kernel(BracketArgs a) {
+  const int k = blockIdx.y;
   StarFrameState& st = a.state[k];
-  const float* src = a.slots + static_cast<int64_t>(a.slot_of_frame[a.frames[k]]) * a.stride;
+  unsigned* keys = a.band + static_cast<int64_t>(k) * a.band_cap;
   const int n = static_cast<int>(a.pixels < kBracketSamples ? a.pixels : static_cast<int64_t>(kBracketSamples));
-  int m = 1;
-  while (m < n) m <<= 1;
-  if (threadIdx.x == 0) s_valid = 0u;
-  __syncthreads();
-  unsigned valid = 0;
-  const float median = st.median;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    unsigned key = 0xffffffffu;
-    if (i < n) {
-      const int64_t pos = ((2 * static_cast<int64_t>(i) + 1) * a.pixels) / (2 * static_cast<int64_t>(n));
-      if (bracket_key(__ldg(src + pos), a.mode, median, key)) ++valid;
-      else key = 0xffffffffu;
+  {
+    const float* src = a.slots + static_cast<int64_t>(a.slot_of_frame[a.frames[k]]) * a.stride;
+    const float median = st.median;
+    constexpr int kPer = kBracketSamples / (kSampleThreads * kSampleCtas);
+    const int first = static_cast<int>(blockIdx.x) * kSampleThreads * kPer + static_cast<int>(threadIdx.x);
+    float v[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = first + u * kSampleThreads;
+      if (i < n) v[u] = __ldg(src + ((2 * static_cast<int64_t>(i) + 1) * a.pixels) / (2 * static_cast<int64_t>(n)));
     }
-    keys[i] = key;
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+      const int i = first + u * kSampleThreads;
+      unsigned key = kNoKey;
+      if (i < n) {
+        bracket_key(v[u], a.mode, median, key);
+        keys[i] = key;
+      }
+    }
   }
+  if (!last_cta(&st.ticket, gridDim.x)) return;
+  constexpr int kKeys = kBracketSamples / kSampleThreads;
+  unsigned key[kKeys];
+  int valid = 0;
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u) {
+    const int i = u * kSampleThreads + static_cast<int>(threadIdx.x);
+    key[u] = i < n ? __ldcg(keys + i) : kNoKey;
+  }
+#pragma unroll
+  for (int u = 0; u < kKeys; ++u) valid += key[u] != kNoKey ? 1 : 0;
+  // sums of a round: both counts in one word (at most 32768 each); a slot is
+  // cleared two rounds before it is added to
+  __shared__ unsigned s_sum[4];
+  __shared__ int s_valid;
+  if (threadIdx.x < 4) s_sum[threadIdx.x] = 0u;
+  if (threadIdx.x == 0) s_valid = 0;
+  __syncthreads();
   valid = __reduce_add_sync(0xffffffffu, valid);
   if ((threadIdx.x & 31) == 0 && valid) atomicAdd(&s_valid, valid);
   __syncthreads();
-  for (int size = 2; size <= m; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int i = threadIdx.x; i < m; i += blockDim.x) {
-        const int j = i ^ stride;
-        if (j > i) {
-          const unsigned x = keys[i], y = keys[j];
-          if (((i & size) == 0) == (x > y)) {
-            keys[i] = y;
-            keys[j] = x;
-          }
-        }
-      }
-      __syncthreads();
+  const int sv = s_valid;
+  // middle of the finite samples +- 7 binomial sigma (+8 for small samples)
+  const int margin = static_cast<int>(ceilf(3.5f * sqrtf(static_cast<float>(sv)))) + 8;
+  const unsigned rank_lo = static_cast<unsigned>(max(0, sv / 2 - margin));
+  const unsigned rank_hi = static_cast<unsigned>(max(0, min(sv - 1, sv / 2 + margin)));
+  unsigned p_lo = 0u, p_hi = 0u;
+  for (int bit = 31; bit >= 0; --bit) {
+    const unsigned t_lo = p_lo | (1u << bit), t_hi = p_hi | (1u << bit);
+    unsigned c_lo = 0u, c_hi = 0u;
+#pragma unroll
+    for (int u = 0; u < kKeys; ++u) c_lo += key[u] < t_lo ? 1u : 0u;
+    if (t_hi != t_lo) {
+#pragma unroll
+      for (int u = 0; u < kKeys; ++u) c_hi += key[u] < t_hi ? 1u : 0u;
+    } else {
+      c_hi = c_lo;
     }
+    const unsigned both = __reduce_add_sync(0xffffffffu, c_lo | (c_hi << 16));
+    if ((threadIdx.x & 31) == 0) atomicAdd(&s_sum[bit & 3], both);
+    if (threadIdx.x == 0) s_sum[(bit - 2) & 3] = 0u;
+    __syncthreads();
+    const unsigned sum = s_sum[bit & 3];
+    if ((sum & 0xffffu) <= rank_lo) p_lo = t_lo;
+    if ((sum >> 16) <= rank_hi) p_hi = t_hi;
   }
   if (threadIdx.x == 0) {
-    const int sv = static_cast<int>(s_valid);
-    // middle of the finite samples +- 7 binomial sigma (+8 for small samples)
-    const int margin = static_cast<int>(ceilf(3.5f * sqrtf(static_cast<float>(sv)))) + 8;
-    const int c = sv / 2;
-    st.band_lo = sv > 0 ? keys[max(0, c - margin)] : 0u;
-    st.band_hi = sv > 0 ? keys[min(sv - 1, c + margin)] : 0u;
+    st.band_lo = sv > 0 ? p_lo : 0u;
+    st.band_hi = sv > 0 ? p_hi : 0u;
     st.below = 0u;
     st.inside = 0u;
     if (a.mode == 0) st.count = 0u;
@@ -331,20 +355,23 @@ __global__ void __launch_bounds__(1024) bracket_sample_kernel(BracketArgs a) {
 }
 
 // One pass over a frame: the finite samples below the band and the band's
-// keys (appended to the frame's band buffer in no particular order).  Each
-// block iteration covers 16 samples per thread (four float4 loads issued
-// first) and reserves the band slots of all its in-band samples with one
-// atomic, so the per-frame counter sees one atomic per 4096 samples.  The
-// per-sample tests are unsigned range checks on the order-preserving keys:
-// a finite float32 has a key in [0x00800000, 0xff7fffff] (float_key), so
-// mode 0 needs no separate isfinite; mode 1 (|v - median|) tests the sample
-// itself.
+// keys (appended to the frame's band buffer in no particular order).  A warp
+// takes 16 samples per lane at a time (four float4 loads issued first),
+// collects its in-band keys in shared memory and hands them over in runs of
+// kBandStage, coalesced and with one atomic each; no barrier in the loop.  The
+// per-sample tests are unsigned range checks on the order-preserving keys: a
+// finite float32 has a key in [0x00800000, 0xff7fffff] (float_key), so mode 0
+// needs no separate isfinite; mode 1 (|v - median|) tests the sample itself.
+// Bound by memory: 8 frames of 4096^2 in 107 us, 129 us with three barriers
+// and one atomic per 4096 samples.
 constexpr int kBracketThreads = 256;
+constexpr int kBandStage = 256;
 
 template <int MODE>
 __global__ void __launch_bounds__(kBracketThreads) bracket_pass_kernel(BracketArgs a) {
-  __shared__ unsigned s_warp[kBracketThreads / 32];
-  __shared__ unsigned s_base;
+  constexpr int kLoads = 4;
+  constexpr int kSamples = 32 * 4 * kLoads;  // per warp and iteration
+  __shared__ unsigned s_keys[kBracketThreads / 32][kBandStage + kSamples];
   const int k = blockIdx.y;
   StarFrameState& st = a.state[k];
   const unsigned lo = st.band_lo, hi = st.band_hi;
@@ -357,17 +384,28 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_pass_kernel(BracketAr
   const float* src = a.slots + static_cast<int64_t>(a.slot_of_frame[a.frames[k]]) * a.stride;
   unsigned* band = a.band + static_cast<int64_t>(k) * a.band_cap;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned* stage = s_keys[warp];
+  unsigned staged = 0;  // the same in every lane
   unsigned below = 0, valid = 0;
-  constexpr int kLoads = 4;
+  auto flush = [&]() {
+    __syncwarp();
+    unsigned base = 0u;
+    if (lane == 0) base = atomicAdd(&st.inside, staged);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    for (unsigned i = lane; i < staged; i += 32)
+      if (static_cast<int64_t>(base) + i < a.band_cap) band[static_cast<int64_t>(base) + i] = stage[i];
+    __syncwarp();
+    staged = 0u;
+  };
   const int64_t n4 = a.pixels / 4;
   const float4* src4 = reinterpret_cast<const float4*>(src);
-  const int64_t gstride = int64_t(gridDim.x) * blockDim.x * kLoads;
-  // every thread of the block runs the same trip count (the barriers need them all)
-  for (int64_t base = blockIdx.x * int64_t(blockDim.x) * kLoads; base < n4; base += gstride) {
+  const int64_t gstride = int64_t(gridDim.x) * (blockDim.x * kLoads);
+  for (int64_t base = (int64_t(blockIdx.x) * (kBracketThreads / 32) + warp) * (32 * kLoads); base < n4;
+       base += gstride) {
     float4 q[kLoads];
 #pragma unroll
     for (int u = 0; u < kLoads; ++u) {
-      const int64_t i = base + u * int64_t(blockDim.x) + threadIdx.x;
+      const int64_t i = base + u * 32 + lane;
       q[u] = i < n4 ? __ldg(src4 + i) : make_float4(CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, CUDART_INF_F);
     }
     unsigned key[4 * kLoads];
@@ -394,7 +432,7 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_pass_kernel(BracketAr
         in_mask |= (fin && key[j] - lo <= span) ? (1u << j) : 0u;
       }
     }
-    // block-wide exclusive prefix of the in-band counts, one reservation
+    if (!__any_sync(0xffffffffu, in_mask != 0u)) continue;
     const unsigned mine = __popc(in_mask);
     unsigned incl = mine;
 #pragma unroll
@@ -402,28 +440,14 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_pass_kernel(BracketAr
       const unsigned n = __shfl_up_sync(0xffffffffu, incl, off);
       if (lane >= off) incl += n;
     }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned total = 0;
+    unsigned pos = staged + incl - mine;
 #pragma unroll
-      for (int w = 0; w < kBracketThreads / 32; ++w) {
-        const unsigned c = s_warp[w];
-        s_warp[w] = total;
-        total += c;
-      }
-      s_base = total ? atomicAdd(&st.inside, total) : 0u;
-    }
-    __syncthreads();
-    int64_t pos = static_cast<int64_t>(s_base) + s_warp[warp] + (incl - mine);
-    while (in_mask) {
-      const int j = __ffs(in_mask) - 1;
-      in_mask &= in_mask - 1u;
-      if (pos < a.band_cap) band[pos] = key[j];
-      ++pos;
-    }
-    __syncthreads();  // s_warp and s_base are rewritten by the next iteration
+    for (int j = 0; j < 4 * kLoads; ++j)
+      if ((in_mask >> j) & 1u) stage[pos++] = key[j];
+    staged += __shfl_sync(0xffffffffu, incl, 31);
+    if (staged >= kBandStage) flush();
   }
+  if (staged) flush();
   // the last pixels % 4 samples: one warp, one atomic per in-band sample
   if (blockIdx.x == 0 && threadIdx.x < 32) {
     for (int64_t p = n4 * 4 + threadIdx.x; p < a.pixels; p += 32) {
@@ -447,99 +471,105 @@ __global__ void __launch_bounds__(kBracketThreads) bracket_pass_kernel(BracketAr
 
 // The two middle ranks' keys inside the band by an MSB-first radix select
 // over key - band_lo (8 bits per pass), then the median / MAD as the float32
-// mean of the two middle values (np.median).  The band of a 9600 x 6422
-// frame holds ~1.6 M keys, so each pass spreads it over several CTAs per
-// frame (shared histograms merged into a per-frame global histogram) and one
-// warp per frame picks the digit:
-//   bracket_band_init   the ranks inside the band (or no band select when
-//                       the order statistics lie outside it: the radix
-//                       fallback then takes the frame), passes from the
-//                       bits of the band's key range
-//   bracket_band_hist   per pass, CTAs x frames
-//   bracket_band_digit  per pass, one warp per frame
-//   bracket_band_finish the value of the two ranks
-__global__ void bracket_band_init_kernel(BracketArgs a) {
-  const int k = blockIdx.x;
+// mean of the two middle values (np.median); no band select when the order
+// statistics lie outside it: the radix fallback then takes the frame.  The
+// band of a 9600 x 6422 frame holds ~1.6 M keys, so a cluster of CTAs shares
+// it, one cluster barrier per pass: every CTA sums the cluster's histograms
+// over distributed shared memory and finds the digits for itself.  Bound by
+// the passes' latency: 36 us for 8 frames of 4096^2 (0.4 M keys each), 94 us
+// as ten launches.
+constexpr int kBandCtas = 8;
+constexpr int kBandThreads = 512;
+
+__global__ void __cluster_dims__(kBandCtas, 1, 1) __launch_bounds__(kBandThreads) bracket_band_kernel(BracketArgs a) {
+  namespace cg = cooperative_groups;
+  __shared__ unsigned hist[2][512];  // [pass parity][rank * 256 + digit]
+  __shared__ unsigned total[512];
+  __shared__ unsigned s_digit[2], s_rank[2];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int k = blockIdx.y;
   StarFrameState& st = a.state[k];
-  unsigned* g = a.ghist + static_cast<int64_t>(k) * 512;
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) g[i] = 0u;
-  if (threadIdx.x != 0) return;
   const unsigned n = st.count;
   const unsigned rhi = n / 2, rlo = (n & 1u) ? rhi : (rhi > 0 ? rhi - 1 : 0);
-  const bool ok = n > 0 && static_cast<int64_t>(st.inside) <= a.band_cap && st.below <= rlo &&
-                  rhi < st.below + st.inside;
-  st.band_ok = ok ? 1 : 0;
-  st.band_rank[0] = ok ? rlo - st.below : 0u;
-  st.band_rank[1] = ok ? rhi - st.below : 0u;
-  st.band_prefix[0] = st.band_prefix[1] = 0u;
-  st.resolved[a.mode] = 0;
-  if (!ok && a.mode == 0) st.count = 0u;  // the radix passes count the finite pixels again
-  const unsigned range = st.band_hi - st.band_lo;
-  int top = 0;  // bits of the key range
-  while (top < 32 && (range >> top) != 0u) ++top;
-  st.band_shift = ((top + 7) / 8) * 8 - 8;  // first pass's digit shift (< 0: a one-value band)
-}
-
-__global__ void __launch_bounds__(256) bracket_band_hist_kernel(BracketArgs a) {
-  __shared__ unsigned hist[2][256];
-  const int k = blockIdx.y;
-  const StarFrameState& st = a.state[k];
-  const int shift = st.band_shift - 8 * a.pass;
-  if (!st.band_ok || shift < 0) return;
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) (&hist[0][0])[i] = 0u;
-  __syncthreads();
-  const unsigned lo = st.band_lo, pre0 = st.band_prefix[0], pre1 = st.band_prefix[1];
-  const int hi_shift = shift + 8;
+  const unsigned inside = st.inside, below = st.below;
+  const unsigned lo = st.band_lo, range = st.band_hi - lo;
+  const bool ok = n > 0 && static_cast<int64_t>(inside) <= a.band_cap && below <= rlo && rhi < below + inside;
+  unsigned rank[2] = {rlo - below, rhi - below};
+  unsigned prefix[2] = {0u, 0u};
+  const int top = 32 - __clz(range);  // bits of the key range
   const unsigned* band = a.band + static_cast<int64_t>(k) * a.band_cap;
-  const int64_t m = st.inside;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < m; i += int64_t(gridDim.x) * blockDim.x) {
-    const unsigned d = band[i] - lo;
-    const unsigned hp = hi_shift >= 32 ? 0u : (d >> hi_shift);
-    const unsigned digit = (d >> shift) & 255u;
-    if (hp == pre0) atomicAdd(&hist[0][digit], 1u);
-    if (hp == pre1 && pre1 != pre0) atomicAdd(&hist[1][digit], 1u);
-  }
-  __syncthreads();
-  unsigned* g = a.ghist + static_cast<int64_t>(k) * 512;
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) {
-    const unsigned c = (&hist[0][0])[i];
-    if (c) atomicAdd(g + i, c);
-  }
-}
-
-__global__ void bracket_band_digit_kernel(BracketArgs a) {
-  const int k = blockIdx.x;
-  StarFrameState& st = a.state[k];
-  const int shift = st.band_shift - 8 * a.pass;
-  if (!st.band_ok || shift < 0) return;
-  unsigned* g = a.ghist + static_cast<int64_t>(k) * 512;
-  if (threadIdx.x < 2) {
-    const int r = threadIdx.x;
-    const unsigned* h = (r == 1 && st.band_prefix[1] == st.band_prefix[0]) ? g : g + 256 * r;
-    unsigned rank = st.band_rank[r];
-    int b = 0;
-    while (b < 255 && rank >= h[b]) {
-      rank -= h[b];
-      ++b;
+  const unsigned step = kBandCtas * kBandThreads;
+  const unsigned first = cluster.block_rank() * kBandThreads + threadIdx.x;
+  int parity = 0;
+  if (ok) {  // the same in every CTA of the cluster
+    for (int shift = ((top + 7) / 8) * 8 - 8; shift >= 0; shift -= 8, parity ^= 1) {
+      unsigned* h = hist[parity];
+      h[threadIdx.x] = 0u;
+      __syncthreads();
+      const bool split = prefix[0] != prefix[1];
+      auto add = [&](unsigned key) {
+        const unsigned d = key - lo;
+        const unsigned hp = shift >= 24 ? 0u : (d >> (shift + 8));
+        const unsigned digit = (d >> shift) & 255u;
+        if (hp == prefix[0]) atomicAdd(&h[digit], 1u);
+        if (split && hp == prefix[1]) atomicAdd(&h[256 + digit], 1u);
+      };
+      const uint4* band4 = reinterpret_cast<const uint4*>(band);
+#pragma unroll 4
+      for (unsigned i = first; i < inside / 4; i += step) {
+        const uint4 q = band4[i];
+        add(q.x);
+        add(q.y);
+        add(q.z);
+        add(q.w);
+      }
+      if (first < (inside & 3u)) add(band[(inside & ~3u) + first]);
+      cluster.sync();
+      unsigned sum = 0u;
+#pragma unroll
+      for (int c = 0; c < kBandCtas; ++c) sum += cluster.map_shared_rank(h, c)[threadIdx.x];
+      total[threadIdx.x] = sum;
+      __syncthreads();
+      if (threadIdx.x < 64) {
+        const int r = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const unsigned* t = total + (split ? 256 * r : 0);
+        unsigned loc = 0;
+        for (int b = 0; b < 8; ++b) loc += t[lane * 8 + b];
+        unsigned incl = loc;
+        for (int off = 1; off < 32; off <<= 1) {
+          const unsigned v = __shfl_up_sync(0xffffffffu, incl, off);
+          if (lane >= off) incl += v;
+        }
+        const unsigned excl = incl - loc;
+        if (excl <= rank[r] && rank[r] < incl) {
+          unsigned left = rank[r] - excl;
+          int b = lane * 8;
+          while (left >= t[b]) {
+            left -= t[b];
+            ++b;
+          }
+          s_digit[r] = static_cast<unsigned>(b);
+          s_rank[r] = left;
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        prefix[r] = (prefix[r] << 8) | s_digit[r];
+        rank[r] = s_rank[r];
+      }
     }
-    __syncwarp(0x3u);
-    st.band_rank[r] = rank;
-    st.band_prefix[r] = (st.band_prefix[r] << 8) | static_cast<unsigned>(b);
   }
-  __syncwarp();
-  for (int i = threadIdx.x; i < 512; i += blockDim.x) g[i] = 0u;  // ready for the next pass
-}
-
-__global__ void bracket_band_finish_kernel(BracketArgs a) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= a.count_frames) return;
-  StarFrameState& st = a.state[k];
-  if (!st.band_ok) return;
-  const float vlo = key_float(st.band_lo + st.band_prefix[0]);
-  const float vhi = key_float(st.band_lo + st.band_prefix[1]);
-  const float med = __fmul_rn(__fadd_rn(vlo, vhi), 0.5f);
-  if (a.mode == 0) st.median = med; else st.mad = med;
-  st.resolved[a.mode] = 1;
+  // no CTA leaves while another may read its histogram, or before all have read the state
+  cluster.sync();
+  if (first != 0) return;
+  st.resolved[a.mode] = ok ? 1 : 0;
+  if (ok) {
+    const float med = __fmul_rn(__fadd_rn(key_float(lo + prefix[0]), key_float(lo + prefix[1])), 0.5f);
+    if (a.mode == 0) st.median = med; else st.mad = med;
+  } else if (a.mode == 0) {
+    st.count = 0u;  // the radix passes count the finite pixels again
+  }
 }
 
 // Threshold from median / MAD (star_detect.py:29-43, 133-137).
@@ -1370,6 +1400,10 @@ __global__ void __launch_bounds__(1024) pairwise_std_kernel(PwArgs a) {
   __shared__ int s_leaves;
   __shared__ float s_mean;
   const int nblocks = static_cast<int>((a.pixels + kPwBlock - 1) / kPwBlock);
+  bool wanted = false;
+  for (int k = threadIdx.x; k < a.count; k += blockDim.x)
+    wanted |= a.state[k].count != 0 && 1.4826 * static_cast<double>(a.state[k].mad) <= 0.0;
+  if (!__syncthreads_or(wanted)) return;
   for (int k = 0; k < a.count; ++k) {
     const StarFrameState& st = a.state[k];
     if (st.count == 0 || !(1.4826 * static_cast<double>(st.mad) <= 0.0)) continue;  // uniform branch
@@ -1505,7 +1539,6 @@ void detect_stars(gg_stack* s, const int64_t* indices, int count, const gg_star_
   std::vector<int> frames(static_cast<size_t>(count));
   for (int k = 0; k < count; ++k) frames[static_cast<size_t>(k)] = static_cast<int>(indices[k]);
   upload_params(s->stream, sc.frames, frames.data(), sizeof(int) * count, "cudaMemcpyAsync(star frames)");
-  check_cuda(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize(star frames)");
   check_cuda(cudaMemsetAsync(sc.state, 0, sizeof(StarFrameState) * count, s->stream), "cudaMemsetAsync(state)");
   const bool need_stats = !std::isfinite(p.background) || !std::isfinite(p.noise);
   SelectArgs sa{};
@@ -1523,7 +1556,8 @@ void detect_stars(gg_stack* s, const int64_t* indices, int count, const gg_star_
   if (need_stats) {
     // band buffers of the sample-bracket selection: a sixteenth of the frame
     // (the band holds ~2.5 % of a 9600 x 6422 frame's pixels)
-    const int64_t band_cap = std::min<int64_t>(s->pixels, std::max<int64_t>(65536, s->pixels / 16));
+    const int64_t band_cap =
+        (std::min<int64_t>(s->pixels, std::max<int64_t>(65536, s->pixels / 16)) + 3) / 4 * 4;
     if (sc.band_elems < band_cap * count) {
       if (sc.band) cudaFree(sc.band);
       sc.band = nullptr;
@@ -1532,52 +1566,29 @@ void detect_stars(gg_stack* s, const int64_t* indices, int count, const gg_star_
       sc.band_elems = band_cap * count;
     }
     BracketArgs ba{s->d_slots, s->d_slot_of_frame, s->stride, s->pixels, sc.frames, sc.state, sc.band, band_cap, 0};
-    ba.ghist = sc.hist;  // [count][2][kSelBins] >= 512 words per frame; the radix fallback zeroes it again
-    ba.count_frames = count;
-    // CTAs per frame for the band histograms: about eight waves of the GPU's SMs over all frames
-    const unsigned band_ctas = static_cast<unsigned>(std::max(1, std::min(64, sm_count() * 8 / std::max(count, 1))));
-    const int samples = static_cast<int>(std::min<int64_t>(kBracketSamples, s->pixels));
-    int sample_pow2 = 1;
-    while (sample_pow2 < samples) sample_pow2 <<= 1;
-    const size_t sample_smem = sizeof(unsigned) * static_cast<size_t>(sample_pow2);
-    check_cuda(cudaFuncSetAttribute(bracket_sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    static_cast<int>(sample_smem)),
-               "cudaFuncSetAttribute(bracket sample)");
+    const unsigned frames_y = static_cast<unsigned>(count);
+    const unsigned sample_ctas = static_cast<unsigned>(
+        std::max<int64_t>(1, std::min<int64_t>(kSampleCtas, (s->pixels + 4 * kSampleThreads - 1) / (4 * kSampleThreads))));
+    check_cuda(cudaMemsetAsync(sc.hist, 0, sizeof(unsigned) * count * 2 * kSelBins, s->stream),
+               "cudaMemsetAsync(hist)");
     for (int mode = 0; mode < 2; ++mode) {
       sa.mode = mode;
       ba.mode = mode;
       note_launch(3);
-      bracket_sample_kernel<<<static_cast<unsigned>(count), 1024, sample_smem, s->stream>>>(ba);
+      bracket_sample_kernel<<<dim3(sample_ctas, frames_y), kSampleThreads, 0, s->stream>>>(ba);
       if (mode == 0)
-        bracket_pass_kernel<0><<<dim3(per_frame, static_cast<unsigned>(count)), kBracketThreads, 0, s->stream>>>(ba);
+        bracket_pass_kernel<0><<<dim3(per_frame, frames_y), kBracketThreads, 0, s->stream>>>(ba);
       else
-        bracket_pass_kernel<1><<<dim3(per_frame, static_cast<unsigned>(count)), kBracketThreads, 0, s->stream>>>(ba);
+        bracket_pass_kernel<1><<<dim3(per_frame, frames_y), kBracketThreads, 0, s->stream>>>(ba);
+      bracket_band_kernel<<<dim3(kBandCtas, frames_y), kBandThreads, 0, s->stream>>>(ba);
       check_cuda(cudaGetLastError(), "bracket select launch");
-      note_launch(2);
-      bracket_band_init_kernel<<<static_cast<unsigned>(count), 32, 0, s->stream>>>(ba);
-      for (int pass = 0; pass < 4; ++pass) {
-        ba.pass = pass;
-        note_launch(2);
-        bracket_band_hist_kernel<<<dim3(band_ctas, static_cast<unsigned>(count)), 256, 0, s->stream>>>(ba);
-        bracket_band_digit_kernel<<<static_cast<unsigned>(count), 32, 0, s->stream>>>(ba);
-      }
-      bracket_band_finish_kernel<<<(count + 127) / 128, 128, 0, s->stream>>>(ba);
-      check_cuda(cudaGetLastError(), "bracket band select launch");
       // frames the bracket could not settle: three-pass radix select
-      for (int pass = 0; pass < 3; ++pass) {
-        sa.pass = pass;
-        check_cuda(cudaMemsetAsync(sc.hist, 0, sizeof(unsigned) * count * 2 * kSelBins, s->stream),
-                   "cudaMemsetAsync(hist)");
-        note_launch();
-        const dim3 hist_grid(per_frame, static_cast<unsigned>(count));
-        if (pass == 0) select_hist_kernel<0><<<hist_grid, 256, 0, s->stream>>>(sa);
-        else if (pass == 1) select_hist_kernel<1><<<hist_grid, 256, 0, s->stream>>>(sa);
-        else select_hist_kernel<2><<<hist_grid, 256, 0, s->stream>>>(sa);
-        check_cuda(cudaGetLastError(), "select_hist launch");
-        note_launch();
-        select_scan_kernel<<<static_cast<unsigned>(count), 256, 0, s->stream>>>(sa, count);
-        check_cuda(cudaGetLastError(), "select_scan launch");
-      }
+      note_launch(3);
+      const dim3 hist_grid(per_frame, frames_y);
+      select_hist_kernel<0><<<hist_grid, 256, 0, s->stream>>>(sa);
+      select_hist_kernel<1><<<hist_grid, 256, 0, s->stream>>>(sa);
+      select_hist_kernel<2><<<hist_grid, 256, 0, s->stream>>>(sa);
+      check_cuda(cudaGetLastError(), "select_hist launch");
     }
     // np.std of the finite pixels, the fallback noise when the MAD is zero
     // (star_detect.py:35-41); computed only for such frames.
