@@ -52,3 +52,63 @@ def test_gpu_order_statistics_exact(native, shape, kind):
                 assert got["mad"] == mad
     finally:
         s.close()
+
+
+FIELDS = ("x", "y", "flux", "peak", "fwhm", "eccentricity", "snr", "sharpness", "npix")
+
+
+def _compare(native, images, **params):
+    h, w = images[0].shape
+    s = native.ResidentCalibratedStack(len(images), h, w)
+    try:
+        for k, f in enumerate(images):
+            s.upload_calibrated_frame(k, f)
+        found = s.detect_stars(range(len(images)), **params)
+    finally:
+        s.close()
+    for got, image in zip(found, images):
+        exp = ostars.detect_stars(image, **params)
+        assert got.size == len(exp)
+        for i, field in enumerate(FIELDS):
+            want = np.asarray([np.nan if e[i] is None else e[i] for e in exp], dtype=np.float64)
+            np.testing.assert_allclose(got[field].astype(np.float64), want, rtol=1e-9, atol=1e-12, err_msg=field)
+    return sum(got.size for got in found)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(3, 3), (4, 4), (3, 700), (700, 3), (40, 129), (33, 511), (33, 512), (33, 513),
+                                   (31, 1025), (130, 2047)])
+def test_gpu_detection_at_chunk_edges(native, shape):
+    """Widths around the columns of one chunk, every alignment of a row's start;
+    peaks up to the border, holes beside them."""
+    h, w = shape
+    rng = np.random.default_rng(h * 4096 + w)
+    images = []
+    for _ in range(2):
+        img = 100.0 + rng.standard_normal((h, w))
+        n = max(4, h * w // 60)
+        np.add.at(img, (rng.integers(0, h, n), rng.integers(0, w, n)), rng.uniform(50.0, 5000.0, n))
+        img[rng.random((h, w)) < 0.01] = np.nan
+        images.append(img.astype(np.float32))
+    _compare(native, images, threshold_sigma=4.0, max_stars=300, window_radius=3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("min_separation_px,radius,max_stars", [(0.0, 4, 4096), (2.9, 1, 4096), (5.7, 4, 7),
+                                                                (39.3, 2, 50), (1.0e9, 3, 10)])
+def test_gpu_detection_of_crowds_and_plateaus(native, min_separation_px, radius, max_stars):
+    """More brighter neighbours than a list holds, equal fluxes (raster order
+    decides, also at the last place) and plateaus on which every pixel is a
+    candidate; whole-number pixels, so every flux is exact on both sides."""
+    rng = np.random.default_rng(5)
+    h, w = 150, 260
+    crowd = np.zeros((h, w))
+    crowd[rng.random((h, w)) < 0.08] = 1.0
+    crowd *= rng.integers(1, 900, (h, w))
+    equal = np.zeros((h, w))
+    equal[5:-5:9, 6:-6:11] = 64.0
+    plateau = np.zeros((h, w))
+    plateau[40:60, 17:150] = 5000.0
+    images = [f.astype(np.float32) for f in (crowd, equal, plateau)]
+    assert _compare(native, images, threshold_sigma=0.5, max_stars=max_stars, window_radius=radius,
+                    min_separation_px=min_separation_px, background=0.0, noise=2.0) > 0
