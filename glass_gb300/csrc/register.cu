@@ -30,9 +30,11 @@
 // GB300 mapping: FP64 is scarce on this part, so every all-pairs loop filters
 // in cheap arithmetic first (per-component descriptor bounds, float32
 // transformed coordinates) and evaluates the float64 distance only for
-// survivors.  One CTA per catalog builds descriptors in shared memory, one
-// CTA per frame pair selects matches, one warp per candidate transform fits
-// and scores it, one warp per frame pair picks the best and refits.
+// survivors.  One CTA per catalog builds descriptors in shared memory, several
+// per frame pair find the descriptor matches and one selects among them, one
+// warp per candidate transform fits it and counts its pairs in float32, the
+// candidates that can still win get their float64 rms, and one CTA per frame
+// pair picks the best and refits.
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -62,8 +64,8 @@ struct Desc {
 
 struct TriCand {
   double d0, d1, area;
-  int key;     // sorted vertex set, 7 bits per vertex
-  int packed;  // ordered vertices (7 bits each), bit 31 = kept
+  int packed;  // ordered vertices (7 bits each), bit 31 = has a descriptor
+  int pad;
 };
 
 struct RegJob {
@@ -75,8 +77,18 @@ struct Cand {
   double m[6];
   double rms;
   long long order;
+  int scored;  // rms: 0 not known, 1 the exact scorer's, 2 to rounding
+  int pad;
+};
+
+// What a candidate is ranked by: its pair count (-1: no fit, or dropped;
+// kConflictCount - c: at most c, the exact scorer's until it has run) and
+// bounds of its rms.
+constexpr int kConflictCount = -2;
+
+struct CandRank {
   int count;
-  int valid;
+  float rms_lo, rms_hi;
 };
 
 struct RegResult {
@@ -97,12 +109,15 @@ struct RegArgs {
   Desc* desc;         // [rows][kMaxDesc]
   int* ndesc;         // [rows]
   const RegJob* jobs;
+  int* match_count;      // [jobs] matches found (may exceed match_cap)
+  int* best_count;       // [jobs] most pairs of a candidate so far
   double* match_dist;    // [jobs][match_cap]
   int* match_key;        // [jobs][match_cap]
   int2* sel;             // [jobs][sel_cap]  (moving, reference) descriptor indices
   long long* sel_order;  // [jobs][sel_cap]
   int* nsel;             // [jobs]
   Cand* cands;           // [jobs][2 * sel_cap]
+  CandRank* ranks;       // [jobs][2 * sel_cap]
   RegResult* out;        // [jobs]
   short2* pairs;         // [jobs][kRegPts]
   int* overflow;
@@ -277,12 +292,16 @@ struct JobPoints {
   float mx32[kRegPts], my32[kRegPts], rx32[kRegPts], ry32[kRegPts];
   unsigned char cell_start[kGrid * kGrid + 1];
   unsigned char cell_pt[kRegPts];
+  unsigned char cell_of[kRegPts];
   float gx0, gy0, ginv;
   int gnx, gny;
   float cmax;  // max |x| + |y| of the moving stars
   float rmax;  // max |x|, |y| of the reference stars
+  int partners;  // most reference stars that can be in reach of one moving star
   int nm, nr;
 };
+
+constexpr int kNearCap = 256;
 
 struct WarpScratch {
   double tx[kRegPts], ty[kRegPts];
@@ -290,9 +309,11 @@ struct WarpScratch {
   unsigned long long key[kPairCap];  // distance bits of the pairs within tolerance
   int idx[kPairCap];                 // (moving << 8) | reference: row-major order
   int acc[kRegPts];                  // accepted entries in greedy order
+  unsigned short near[kNearCap];     // pairs of the float32 test
   double res[kRegPts];
-  unsigned used_r[3];
+  unsigned used_r[3], used_m[3];
   int count;
+  double rms;
 };
 
 // Reference stars within `r` of (x, y) in grid order; calls f(j).
@@ -341,13 +362,28 @@ __device__ double warp_pw_sum(const double* v, int n) {
   return __shfl_sync(0xffffffffu, out, 0);
 }
 
-// Exact scoring: every lane returns the greedy pair count and rms (+inf
-// without pairs); the pairs (moving, reference) go to `pairs` when not null.
-__device__ void warp_score_exact(const double (&m)[6], const JobPoints& jp, double tol, WarpScratch& w,
-                                 int& npairs, double& rms, short2* pairs, int* overflow) {
-  const int lane = threadIdx.x & 31;
-  const int nm = jp.nm;
-  for (int i = lane; i < nm; i += 32) {
+// The steps of the exact score, by a group of threads: `tid` of `threads`,
+// `sync` their barrier.
+struct WarpGroup {
+  static constexpr int kThreads = 32;
+  __device__ __forceinline__ static int tid() { return threadIdx.x & 31; }
+  __device__ __forceinline__ static void sync() { __syncwarp(); }
+  __device__ __forceinline__ static bool any(bool p) { return __any_sync(0xffffffffu, p); }
+};
+template <int THREADS>
+struct CtaGroup {
+  static constexpr int kThreads = THREADS;
+  __device__ __forceinline__ static int tid() { return threadIdx.x; }
+  __device__ __forceinline__ static void sync() { __syncthreads(); }
+  __device__ __forceinline__ static bool any(bool p) { return __syncthreads_or(p) != 0; }
+};
+
+// The moving stars at their transformed places and the list of the pairs
+// that pass the float32 test with a 0.5 px margin (w.near; the return value may
+// exceed its capacity).
+template <class G>
+__device__ int near_pairs(const double (&m)[6], const JobPoints& jp, double tol, WarpScratch& w) {
+  for (int i = G::tid(); i < jp.nm; i += G::kThreads) {
     const double x = dadd(dadd(dmul(jp.mx[i], m[0]), dmul(jp.my[i], m[1])), m[2]);
     const double y = dadd(dadd(dmul(jp.mx[i], m[3]), dmul(jp.my[i], m[4])), m[5]);
     w.tx[i] = x;
@@ -355,148 +391,332 @@ __device__ void warp_score_exact(const double (&m)[6], const JobPoints& jp, doub
     w.tx32[i] = static_cast<float>(x);
     w.ty32[i] = static_cast<float>(y);
   }
-  if (lane == 0) w.count = 0;
-  __syncwarp();
-  // pairs within tolerance (float32 prefilter with a 0.5 px margin, then the
-  // float64 distance); any order, sorted below
+  if (G::tid() == 0) w.count = 0;
+  G::sync();
   const float r = static_cast<float>(tol + 0.5);
   const float pre = r * r;
-  for (int i = lane; i < nm; i += 32) {
+  for (int i = G::tid(); i < jp.nm; i += G::kThreads) {
     const float x = w.tx32[i], y = w.ty32[i];
     grid_visit(jp, x, y, r, [&](int j) {
       const float fx = x - jp.rx32[j], fy = y - jp.ry32[j];
       if (fx * fx + fy * fy > pre) return;
-      const double d = hyp_sum(dsub(w.tx[i], jp.rx[j]), dsub(w.ty[i], jp.ry[j]));
-      if (!(d <= tol)) return;
       const int pos = atomicAdd(&w.count, 1);
-      if (pos < kPairCap) {
-        w.key[pos] = dbits_of(d);
-        w.idx[pos] = (i << 8) | j;
-      }
+      if (pos < kNearCap) w.near[pos] = static_cast<unsigned short>((i << 8) | j);
     });
   }
-  __syncwarp();
+  G::sync();
+  const int listed = w.count;
+  G::sync();
+  return listed;
+}
+
+__device__ __forceinline__ double pair_distance(const JobPoints& jp, const WarpScratch& w, int i, int j) {
+  return hyp_sum(dsub(w.tx[i], jp.rx[j]), dsub(w.ty[i], jp.ry[j]));
+}
+
+// Exact scoring: every thread of the group returns the greedy pair count and
+// rms (+inf without pairs); the pairs (moving, reference) go to `pairs` when
+// not null.
+template <class G>
+__device__ void score_exact(const double (&m)[6], const JobPoints& jp, double tol, WarpScratch& w, int& npairs,
+                            double& rms, short2* pairs, int* overflow) {
+  const int listed = near_pairs<G>(m, jp, tol, w);
+  if (G::tid() == 0) w.count = 0;
+  G::sync();
+  // the float64 distances, one pair per thread (a float64 operation costs a
+  // warp the same for one lane as for all); any order, sorted below
+  auto test = [&](int i, int j) {
+    const double d = pair_distance(jp, w, i, j);
+    if (!(d <= tol)) return;
+    const int pos = atomicAdd(&w.count, 1);
+    if (pos < kPairCap) {
+      w.key[pos] = dbits_of(d);
+      w.idx[pos] = (i << 8) | j;
+    }
+  };
+  if (listed <= kNearCap) {
+    for (int t = G::tid(); t < listed; t += G::kThreads) test(w.near[t] >> 8, w.near[t] & 255);
+  } else {
+    const float r = static_cast<float>(tol + 0.5);
+    const float pre = r * r;
+    for (int i = G::tid(); i < jp.nm; i += G::kThreads) {
+      const float x = w.tx32[i], y = w.ty32[i];
+      grid_visit(jp, x, y, r, [&](int j) {
+        const float fx = x - jp.rx32[j], fy = y - jp.ry32[j];
+        if (fx * fx + fy * fy <= pre) test(i, j);
+      });
+    }
+  }
+  G::sync();
   int L = w.count;
   if (L > kPairCap) {
-    if (lane == 0) atomicExch(overflow, 1);
+    if (G::tid() == 0) atomicExch(overflow, 1);
     L = kPairCap;
   }
-  // sort by (distance, row-major index): the stable distance sort of the
-  // row-major candidate list
-  int mlen = 1;
-  while (mlen < L) mlen <<= 1;
-  for (int t = L + lane; t < mlen; t += 32) {
-    w.key[t] = ~0ull;
-    w.idx[t] = 0x7fffffff;
+  // sort by (distance, row-major index), the stable distance sort of the
+  // row-major candidate list: two threads count the entries before one
+  constexpr int kHalf = G::kThreads / 2, kPer = kPairCap / kHalf;
+  unsigned long long key[kPer];
+  int idx[kPer], rank[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    if (u * kHalf >= L) break;
+    const int e = u * kHalf + (G::tid() >> 1);
+    key[u] = e < L ? w.key[e] : ~0ull;
+    idx[u] = e < L ? w.idx[e] : 0x7fffffff;
+    int before = 0;
+#pragma unroll 4
+    for (int q = G::tid() & 1; q < L; q += 2) {
+      const unsigned long long kq = w.key[q];
+      before += (kq < key[u] || (kq == key[u] && w.idx[q] < idx[u])) ? 1 : 0;
+    }
+    rank[u] = before + __shfl_xor_sync(0xffffffffu, before, 1);
   }
-  __syncwarp();
-  for (int size = 2; size <= mlen; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
-      for (int t = lane; t < mlen; t += 32) {
-        const int u = t ^ stride;
-        if (u > t) {
-          const bool up = (t & size) == 0;
-          const unsigned long long kt = w.key[t], ku = w.key[u];
-          const int it = w.idx[t], iu = w.idx[u];
-          const bool gt = kt > ku || (kt == ku && it > iu);
-          if (gt == up) {
-            w.key[t] = ku;
-            w.key[u] = kt;
-            w.idx[t] = iu;
-            w.idx[u] = it;
-          }
-        }
+  if (G::tid() < 3) w.used_r[G::tid()] = w.used_m[G::tid()] = 0u;
+  G::sync();
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    if (u * kHalf >= L) break;
+    if (u * kHalf + (G::tid() >> 1) < L && (G::tid() & 1) == 0) {
+      w.key[rank[u]] = key[u];
+      w.idx[rank[u]] = idx[u];
+    }
+  }
+  G::sync();
+  // greedy one-to-one pairing in distance order: every entry where no star
+  // stands in two, else one after the other
+  bool twice = false;
+  for (int t = G::tid(); t < L; t += G::kThreads) {
+    const int i = w.idx[t] >> 8, j = w.idx[t] & 255;
+    const unsigned bi = 1u << (i & 31), bj = 1u << (j & 31);
+    twice |= (atomicOr(&w.used_m[i >> 5], bi) & bi) != 0u;
+    twice |= (atomicOr(&w.used_r[j >> 5], bj) & bj) != 0u;
+    if (t < kRegPts) w.acc[t] = t;
+  }
+  int n = L;
+  if (G::any(twice)) {
+    if (G::tid() == 0) {
+      n = 0;
+      unsigned used_m[3] = {0u, 0u, 0u}, used_r[3] = {0u, 0u, 0u};
+      for (int a = 0; a < L; ++a) {
+        const int i = w.idx[a] >> 8, j = w.idx[a] & 255;
+        if ((used_m[i >> 5] >> (i & 31)) & 1u) continue;
+        if ((used_r[j >> 5] >> (j & 31)) & 1u) continue;
+        used_m[i >> 5] |= 1u << (i & 31);
+        used_r[j >> 5] |= 1u << (j & 31);
+        w.acc[n++] = a;
       }
-      __syncwarp();
+      w.count = n;
     }
+    G::sync();
+    n = w.count;
   }
-  // greedy one-to-one pairing in distance order
-  int n = 0;
-  if (lane == 0) {
-    unsigned used_m[3] = {0u, 0u, 0u}, used_r[3] = {0u, 0u, 0u};
-    for (int a = 0; a < L; ++a) {
-      const int i = w.idx[a] >> 8, j = w.idx[a] & 255;
-      if ((used_m[i >> 5] >> (i & 31)) & 1u) continue;
-      if ((used_r[j >> 5] >> (j & 31)) & 1u) continue;
-      used_m[i >> 5] |= 1u << (i & 31);
-      used_r[j >> 5] |= 1u << (j & 31);
-      w.acc[n++] = a;
-    }
-  }
-  n = __shfl_sync(0xffffffffu, n, 0);
-  __syncwarp();
-  for (int t = lane; t < n; t += 32) {
+  G::sync();
+  for (int t = G::tid(); t < n; t += G::kThreads) {
     const int a = w.acc[t];
     const double d = __longlong_as_double(static_cast<long long>(w.key[a]));
     w.res[t] = dmul(d, d);
     if (pairs) pairs[t] = make_short2(static_cast<short>(w.idx[a] >> 8), static_cast<short>(w.idx[a] & 255));
   }
-  __syncwarp();
-  const double s = warp_pw_sum(w.res, n);
+  G::sync();
+  if (G::tid() < 32) {
+    const double s = warp_pw_sum(w.res, n);
+    if (G::tid() == 0)
+      w.rms = n > 0 ? sqrt(__ddiv_rn(s, static_cast<double>(n))) : __longlong_as_double(0x7ff0000000000000ll);
+  }
+  G::sync();
   npairs = n;
-  rms = n > 0 ? sqrt(__ddiv_rn(s, static_cast<double>(n))) : __longlong_as_double(0x7ff0000000000000ll);
-  __syncwarp();
+  rms = w.rms;
+  G::sync();
 }
 
-// Fast scoring for ranking: the exact pair count when no moving or reference
-// star has two partners within tolerance (then greedy pairing keeps every
-// pair), and the sum of squared residuals in any order.  Membership is
-// decided in float32 outside a band of +-delta around the tolerance (delta
-// bounds the float32 transform error) and in float64 inside it.  `conflict`
-// reports that the exact scorer is needed.
-__device__ void warp_score_fast(const double (&m)[6], const JobPoints& jp, double tol, WarpScratch& w, int& count,
-                                double& sum_d2, bool& conflict) {
+// Count and rms of a transform in which a few stars have two partners: every
+// pair of two otherwise unpaired stars counts, and the greedy order is worked
+// out among the others alone (at most 32).  False when there are more.
+__device__ bool warp_resolve(const double (&m)[6], const JobPoints& jp, double tol, WarpScratch& w, int& npairs,
+                             double& rms) {
   const int lane = threadIdx.x & 31;
-  const float m0 = static_cast<float>(m[0]), m1 = static_cast<float>(m[1]), m2 = static_cast<float>(m[2]);
-  const float m3 = static_cast<float>(m[3]), m4 = static_cast<float>(m[4]), m5 = static_cast<float>(m[5]);
+  const int listed = near_pairs<WarpGroup>(m, jp, tol, w);
+  if (listed > kNearCap) return false;
+  int* with_m = w.acc;
+  int* with_r = reinterpret_cast<int*>(w.res);
+  for (int i = lane; i < kRegPts; i += 32) with_m[i] = with_r[i] = 0;
+  __syncwarp();
+  for (int t = lane; t < listed; t += 32) {
+    const int i = w.near[t] >> 8, j = w.near[t] & 255;
+    const double d = pair_distance(jp, w, i, j);
+    w.key[t] = d <= tol ? dbits_of(d) : ~0ull;
+    if (d <= tol) {
+      atomicAdd(&with_m[i], 1);
+      atomicAdd(&with_r[j], 1);
+    }
+  }
+  __syncwarp();
+  int n = 0, open = 0;
+  double sum = 0.0;
+  for (int t0 = 0; t0 < listed; t0 += 32) {
+    const int t = t0 + lane;
+    const unsigned long long key = t < listed ? w.key[t] : ~0ull;
+    bool alone = false;
+    if (key != ~0ull) alone = with_m[w.near[t] >> 8] == 1 && with_r[w.near[t] & 255] == 1;
+    const unsigned rest = __ballot_sync(0xffffffffu, key != ~0ull && !alone);
+    const int pos = open + __popc(rest & ((1u << lane) - 1u));
+    if (key != ~0ull && !alone && pos < 32) w.idx[pos] = t;
+    open += __popc(rest);
+    n += __popc(__ballot_sync(0xffffffffu, alone));
+    const double d = alone ? __longlong_as_double(static_cast<long long>(key)) : 0.0;
+    sum = dadd(sum, dmul(d, d));
+  }
+  if (open > 32) return false;
+  __syncwarp();
+  const bool mine = lane < open;
+  const unsigned long long key = mine ? w.key[w.idx[lane]] : ~0ull;
+  const int pair = mine ? w.near[w.idx[lane]] : 0x7fffffff;
+  int rank = 0;
+  for (int q = 0; q < open; ++q) {
+    const unsigned long long kq = __shfl_sync(0xffffffffu, key, q);
+    const int pq = __shfl_sync(0xffffffffu, pair, q);
+    rank += (kq < key || (kq == key && pq < pair)) ? 1 : 0;
+  }
+  bool free = mine, kept = false;
+  for (int s = 0; s < open; ++s) {
+    const int from = __ffs(__ballot_sync(0xffffffffu, mine && rank == s)) - 1;
+    const int taken = __shfl_sync(0xffffffffu, free ? pair : -1, from);
+    if (taken < 0) continue;
+    if (lane == from) kept = true;
+    if ((pair >> 8) == (taken >> 8) || (pair & 255) == (taken & 255)) free = false;
+  }
+  n += __popc(__ballot_sync(0xffffffffu, kept));
+  const double d = kept ? __longlong_as_double(static_cast<long long>(key)) : 0.0;
+  sum = dadd(sum, dmul(d, d));
+  for (int off = 16; off > 0; off >>= 1) sum = dadd(sum, __shfl_xor_sync(0xffffffffu, sum, off));
+  __syncwarp();
+  npairs = n;
+  rms = n > 0 ? sqrt(__ddiv_rn(sum, static_cast<double>(n))) : __longlong_as_double(0x7ff0000000000000ll);
+  return true;
+}
+
+// float32 scoring of a transform: how far it can be off.
+struct FastTransform {
+  float m[6];
+  float r;         // search radius
+  float lo2, hi2;  // squared distance certainly inside / outside the tolerance
+  float delta;     // bound of a pair distance's error
+};
+
+__device__ __forceinline__ FastTransform fast_transform(const double (&m)[6], const JobPoints& jp, double tol) {
+  FastTransform t;
+  for (int q = 0; q < 6; ++q) t.m[q] = static_cast<float>(m[q]);
   const double lin = fmax(fmax(fabs(m[0]), fabs(m[1])), fmax(fabs(m[3]), fabs(m[4])));
   const double trn = fmax(fabs(m[2]), fabs(m[5]));
   const double eps = 5.9604644775390625e-08;  // 2^-24
   const double delta = 2.0 * (1.5 * (6.0 * eps * (lin * jp.cmax + trn) + eps * jp.rmax) + 4.0 * eps * (tol + 1.0)) +
                        1.0e-6;
   const double lo = tol - delta;
-  const float lo2 = lo > 0.0 ? static_cast<float>(lo * lo) : -1.0f;
-  const float hi2 = static_cast<float>((tol + delta) * (tol + delta));
-  const float r = static_cast<float>(tol + delta);
-  if (lane < 3) w.used_r[lane] = 0u;
+  t.lo2 = lo > 0.0 ? static_cast<float>(lo * lo) : -1.0f;
+  t.hi2 = static_cast<float>((tol + delta) * (tol + delta));
+  t.r = static_cast<float>(tol + delta);
+  t.delta = static_cast<float>(delta) * 1.000001f;
+  return t;
+}
+
+// Whether candidates may be dropped unscored: the exact scorer reports more
+// pairs than it holds, and no candidate that might do so is passed over.
+__device__ __forceinline__ bool can_leave_early(const JobPoints& jp, double tol, float reach) {
+  return jp.nm * jp.partners <= kPairCap && reach <= static_cast<float>(tol + 0.5);
+}
+
+// Pairs of a transform for ranking: the exact count when no moving or
+// reference star has two partners within tolerance (then greedy pairing keeps
+// every pair), and the float32 sum of squared residuals.  Membership is
+// decided in float32 outside a band of +-delta around the tolerance (delta
+// bounds the float32 transform error) and in float64 inside it.  `conflict`
+// reports that the exact scorer is needed; the count is then the moving or the
+// reference stars with a partner, whichever are fewer: the exact count cannot
+// exceed either.
+//
+// `best`: a count that some candidate is known to reach; one that cannot reach
+// it any more is left (count -1) after any 32 stars.
+__device__ void warp_score_count(const FastTransform& t, const double* m, const JobPoints& jp, double tol, int best,
+                                 unsigned* used_r, int& count, float& sum_d2, bool& conflict) {
+  const int lane = threadIdx.x & 31;
+  if (lane < 3) used_r[lane] = 0u;
   __syncwarp();
-  int cnt = 0;
-  double acc = 0.0;
+  int cnt = 0, paired = 0;
+  float acc = 0.0f;
   bool conf = false;
-  for (int i = lane; i < jp.nm; i += 32) {
-    const float x = __fadd_rn(__fadd_rn(__fmul_rn(m0, jp.mx32[i]), __fmul_rn(m1, jp.my32[i])), m2);
-    const float y = __fadd_rn(__fadd_rn(__fmul_rn(m3, jp.mx32[i]), __fmul_rn(m4, jp.my32[i])), m5);
+  for (int i0 = 0; i0 < jp.nm; i0 += 32) {
+    const int i = min(i0 + lane, jp.nm - 1);
+    const bool real = i0 + lane < jp.nm;
+    const float x = __fadd_rn(__fadd_rn(__fmul_rn(t.m[0], jp.mx32[i]), __fmul_rn(t.m[1], jp.my32[i])), t.m[2]);
+    const float y = __fadd_rn(__fadd_rn(__fmul_rn(t.m[3], jp.mx32[i]), __fmul_rn(t.m[4], jp.my32[i])), t.m[5]);
     int hits = 0;
-    bool have64 = false;
-    double x64 = 0.0, y64 = 0.0;
-    grid_visit(jp, x, y, r, [&](int j) {
+    if (real) grid_visit(jp, x, y, t.r, [&](int j) {
       const float fx = x - jp.rx32[j], fy = y - jp.ry32[j];
       const float d2 = fx * fx + fy * fy;
-      if (d2 > hi2) return;
-      if (!have64) {
-        x64 = dadd(dadd(dmul(jp.mx[i], m[0]), dmul(jp.my[i], m[1])), m[2]);
-        y64 = dadd(dadd(dmul(jp.mx[i], m[3]), dmul(jp.my[i], m[4])), m[5]);
-        have64 = true;
+      if (d2 > t.hi2) return;
+      if (!(d2 <= t.lo2)) {
+        const double x64 = dadd(dadd(dmul(jp.mx[i], m[0]), dmul(jp.my[i], m[1])), m[2]);
+        const double y64 = dadd(dadd(dmul(jp.mx[i], m[3]), dmul(jp.my[i], m[4])), m[5]);
+        const double ex = dsub(x64, jp.rx[j]), ey = dsub(y64, jp.ry[j]);
+        if (!(sqrt(dadd(dmul(ex, ex), dmul(ey, ey))) <= tol)) return;
       }
-      const double ex = dsub(x64, jp.rx[j]), ey = dsub(y64, jp.ry[j]);
-      const double dd2 = dadd(dmul(ex, ex), dmul(ey, ey));
-      if (!(d2 <= lo2) && !(sqrt(dd2) <= tol)) return;
       ++hits;
-      acc = dadd(acc, dd2);
+      acc += d2;
       const unsigned bit = 1u << (j & 31);
-      if (atomicOr(&w.used_r[j >> 5], bit) & bit) conf = true;
+      if (atomicOr(&used_r[j >> 5], bit) & bit) conf = true;
     });
     if (hits > 1) conf = true;
     cnt += hits;
+    paired += __popc(__ballot_sync(0xffffffffu, hits > 0));
+    if (paired + max(0, jp.nm - i0 - 32) < best) {
+      count = -1;
+      sum_d2 = 0.0f;
+      conflict = false;
+      __syncwarp();
+      return;
+    }
   }
-  for (int off = 16; off > 0; off >>= 1) {
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, off);
-    acc = dadd(acc, __shfl_xor_sync(0xffffffffu, acc, off));
-  }
+  cnt = __reduce_add_sync(0xffffffffu, cnt);
+  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
   conflict = __any_sync(0xffffffffu, conf);
-  count = cnt;
+  __syncwarp();
+  count = conflict ? min(paired, __popc(used_r[0]) + __popc(used_r[1]) + __popc(used_r[2])) : cnt;
   sum_d2 = acc;
   __syncwarp();
+}
+
+// The same pairs (of a transform without conflicts) with float64 residuals:
+// the sum of their squares in any order.
+__device__ double warp_sum_d2(const double (&m)[6], const FastTransform& t, const JobPoints& jp, double tol) {
+  const int lane = threadIdx.x & 31;
+  double acc = 0.0;
+  auto residual = [&](int i, int j) {
+    const double x64 = dadd(dadd(dmul(jp.mx[i], m[0]), dmul(jp.my[i], m[1])), m[2]);
+    const double y64 = dadd(dadd(dmul(jp.mx[i], m[3]), dmul(jp.my[i], m[4])), m[5]);
+    const double ex = dsub(x64, jp.rx[j]), ey = dsub(y64, jp.ry[j]);
+    return dadd(dmul(ex, ex), dmul(ey, ey));
+  };
+  for (int i0 = 0; i0 < jp.nm; i0 += 32) {
+    const int i = i0 + lane;
+    int partner = -1;  // at most one
+    if (i < jp.nm) {
+      const float x = __fadd_rn(__fadd_rn(__fmul_rn(t.m[0], jp.mx32[i]), __fmul_rn(t.m[1], jp.my32[i])), t.m[2]);
+      const float y = __fadd_rn(__fadd_rn(__fmul_rn(t.m[3], jp.mx32[i]), __fmul_rn(t.m[4], jp.my32[i])), t.m[5]);
+      grid_visit(jp, x, y, t.r, [&](int j) {
+        const float fx = x - jp.rx32[j], fy = y - jp.ry32[j];
+        const float d2 = fx * fx + fy * fy;
+        if (d2 > t.hi2) return;
+        if (!(d2 <= t.lo2) && !(sqrt(residual(i, j)) <= tol)) return;
+        partner = j;
+      });
+    }
+    __syncwarp();  // together: a float64 operation costs the warp the same for one lane as for all
+    if (partner >= 0) acc = dadd(acc, residual(i, partner));
+  }
+  __syncwarp();
+  for (int off = 16; off > 0; off >>= 1) acc = dadd(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+  return acc;
 }
 
 // Warp-cooperative similarity fit of n <= 80 pairs: the same arithmetic as
@@ -509,13 +729,12 @@ __device__ bool warp_fit_similarity(const double* mx, const double* my, const do
   double s = 0.0;
   if (lane < 4) {
     const double* v = lane == 0 ? mx : (lane == 1 ? my : (lane == 2 ? rx : ry));
+#pragma unroll 8
     for (int i = 0; i < n; ++i) s = dadd(s, v[i]);
   }
-  const double dn = static_cast<double>(n);
-  const double mmx = __ddiv_rn(__shfl_sync(0xffffffffu, s, 0), dn);
-  const double mmy = __ddiv_rn(__shfl_sync(0xffffffffu, s, 1), dn);
-  const double mrx = __ddiv_rn(__shfl_sync(0xffffffffu, s, 2), dn);
-  const double mry = __ddiv_rn(__shfl_sync(0xffffffffu, s, 3), dn);
+  s = __ddiv_rn(s, static_cast<double>(n));  // one quotient per lane costs as much as one
+  const double mmx = __shfl_sync(0xffffffffu, s, 0), mmy = __shfl_sync(0xffffffffu, s, 1);
+  const double mrx = __shfl_sync(0xffffffffu, s, 2), mry = __shfl_sync(0xffffffffu, s, 3);
   for (int i = lane; i < n; i += 32) {
     const double cx = dsub(mx[i], mmx), cy = dsub(my[i], mmy);
     sq[2 * i] = dmul(cx, cx);
@@ -531,24 +750,34 @@ __device__ bool warp_fit_similarity(const double* mx, const double* my, const do
     variance = dadd(warp_pw_sum(sq, n2), warp_pw_sum(sq + n2, 2 * n - n2));
   }
   if (!(variance > 1.0e-12)) return false;
+  // the products by all lanes, then each sum in pair order by its own lane
+  for (int i = lane; i < n; i += 32) {
+    const double ax = dsub(mx[i], mmx), ay = dsub(my[i], mmy), bx = dsub(rx[i], mrx), by = dsub(ry[i], mry);
+    sq[i] = dmul(ax, bx);
+    sq[kRegPts + i] = dmul(ax, by);
+    sq[2 * kRegPts + i] = dmul(ay, bx);
+    sq[3 * kRegPts + i] = dmul(ay, by);
+  }
+  __syncwarp();
   double c = 0.0;
   if (lane < 4) {
-    for (int i = 0; i < n; ++i) {
-      const double a = lane < 2 ? dsub(mx[i], mmx) : dsub(my[i], mmy);
-      const double b = (lane & 1) == 0 ? dsub(rx[i], mrx) : dsub(ry[i], mry);
-      c = dadd(c, dmul(a, b));
-    }
+#pragma unroll 8
+    for (int i = 0; i < n; ++i) c = dadd(c, sq[lane * kRegPts + i]);
   }
+  __syncwarp();
   const double c00 = __shfl_sync(0xffffffffu, c, 0), c01 = __shfl_sync(0xffffffffu, c, 1);
   const double c10 = __shfl_sync(0xffffffffu, c, 2), c11 = __shfl_sync(0xffffffffu, c, 3);
-  const double e = hyp_sum(dadd(c00, c11), dsub(c01, c10));
-  const double f = hyp_sum(dsub(c00, c11), dadd(c01, c10));
-  double cs = 1.0, sn = 0.0;
-  if (e > 0.0) {
-    cs = __ddiv_rn(dadd(c00, c11), e);
-    sn = __ddiv_rn(dsub(c01, c10), e);
+  const double u = lane == 1 ? dsub(c00, c11) : dadd(c00, c11);
+  const double v = lane == 1 ? dadd(c01, c10) : dsub(c01, c10);
+  const double norm = hyp_sum(u, v);
+  const double e = __shfl_sync(0xffffffffu, norm, 0), f = __shfl_sync(0xffffffffu, norm, 1);
+  const double quot = __ddiv_rn(lane == 0 ? u : (lane == 2 ? v : fmax(e, f)), lane == 3 ? variance : e);
+  double cs = __shfl_sync(0xffffffffu, quot, 0), sn = __shfl_sync(0xffffffffu, quot, 2);
+  if (!(e > 0.0)) {
+    cs = 1.0;
+    sn = 0.0;
   }
-  const double scale = __ddiv_rn(fmax(e, f), variance);
+  const double scale = __shfl_sync(0xffffffffu, quot, 3);
   const double l00 = dmul(scale, cs), l01 = dmul(scale, -sn), l10 = dmul(scale, sn), l11 = dmul(scale, cs);
   m[0] = l00;
   m[1] = l01;
@@ -604,11 +833,19 @@ __device__ __forceinline__ double row_y(const RegArgs& a, int row, int i) {
   return a.pts[(static_cast<int64_t>(row) * kRegPts + i) * 2 + 1];
 }
 
+// Bound by latency and, where float64 compares of the all-pairs loops were,
+// by the float64 unit: those run on the order-preserving bits of the
+// (non-negative) doubles, and all threads fill the distance matrix that the
+// anchors search.  68 us for a catalog of 80 stars, 347 us before.
 __global__ void __launch_bounds__(1024) reg_desc_kernel(RegArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
   TriCand* tri = reinterpret_cast<TriCand*>(smem);
+  unsigned long long* dist = reinterpret_cast<unsigned long long*>(smem);  // [n][n], before the triangles
   __shared__ double px[kRegPts], py[kRegPts];
   __shared__ int nb[kRegPts][kMaxNeighbors];
+  __shared__ int combo[kMaxCombos][3];
+  __shared__ __align__(16) int keys[kMaxTri];  // sorted vertex set, 7 bits per vertex
+  __shared__ __align__(16) unsigned long long areas[kMaxTri];  // bits of a kept triangle's area, else 0
   __shared__ int s_kept;
   const int row = blockIdx.x;
   const int n = min(a.npts[row], a.max_stars);
@@ -616,44 +853,61 @@ __global__ void __launch_bounds__(1024) reg_desc_kernel(RegArgs a) {
     px[i] = row_x(a, row, i);
     py[i] = row_y(a, row, i);
   }
-  if (threadIdx.x == 0) s_kept = 0;
+  const int k = min(n, max(3, a.neighbors));
+  if (threadIdx.x == 0) {
+    s_kept = 0;
+    int c = 0;
+    for (int i0 = 0; i0 < k; ++i0)
+      for (int i1 = i0 + 1; i1 < k; ++i1)
+        for (int i2 = i1 + 1; i2 < k; ++i2, ++c) {
+          combo[c][0] = i0;
+          combo[c][1] = i1;
+          combo[c][2] = i2;
+        }
+  }
   __syncthreads();
   if (n < 3) {
     if (threadIdx.x == 0) a.ndesc[row] = 0;
     return;
   }
-  const int k = min(n, max(3, a.neighbors));
-  // k nearest points of each anchor (the anchor itself first), index order on ties
-  for (int an = threadIdx.x; an < n; an += blockDim.x) {
-    double bd[kMaxNeighbors];
-    int bi[kMaxNeighbors];
-    int cnt = 0;
-    for (int j = 0; j < n; ++j) {
-      const double d = hyp_sum(dsub(px[j], px[an]), dsub(py[j], py[an]));
-      if (cnt == k && !(d < bd[k - 1])) continue;
-      int pos = cnt < k ? cnt : k - 1;
-      while (pos > 0 && bd[pos - 1] > d) {
-        bd[pos] = bd[pos - 1];
-        bi[pos] = bi[pos - 1];
-        --pos;
-      }
-      bd[pos] = d;
-      bi[pos] = j;
-      if (cnt < k) ++cnt;
-    }
-    for (int q = 0; q < k; ++q) nb[an][q] = bi[q];
+  for (int q = threadIdx.x; q < n * (n / 2 + 1); q += blockDim.x) {  // symmetric: j = i .. i + n / 2
+    const int d = q / n, i = q - d * n, j = i + d < n ? i + d : i + d - n;
+    const unsigned long long b = d == 0 ? 0ull : dbits_of(hyp_sum(dsub(px[j], px[i]), dsub(py[j], py[i])));
+    dist[i * n + j] = b;
+    dist[j * n + i] = b;
   }
   __syncthreads();
-  int combo[kMaxCombos][3];
-  int ncomb = 0;
-  for (int i0 = 0; i0 < k; ++i0)
-    for (int i1 = i0 + 1; i1 < k; ++i1)
-      for (int i2 = i1 + 1; i2 < k; ++i2) {
-        combo[ncomb][0] = i0;
-        combo[ncomb][1] = i1;
-        combo[ncomb][2] = i2;
-        ++ncomb;
+  // k nearest points of each anchor (the anchor itself first), index order on ties
+  for (int an = threadIdx.x; an < n; an += blockDim.x) {
+    unsigned long long bd[kMaxNeighbors];
+    int bi[kMaxNeighbors];
+#pragma unroll
+    for (int q = 0; q < kMaxNeighbors; ++q) {
+      bd[q] = ~0ull;
+      bi[q] = 0;
+    }
+    for (int j = 0; j < n; ++j) {
+      // insertion behind every entry that is not larger
+      unsigned long long d = dist[an * n + j];
+      int at = j;
+      bool swap = false;
+#pragma unroll
+      for (int q = 0; q < kMaxNeighbors; ++q) {
+        swap = swap || d < bd[q];
+        const unsigned long long od = bd[q];
+        const int oi = bi[q];
+        bd[q] = swap ? d : od;
+        bi[q] = swap ? at : oi;
+        d = swap ? od : d;
+        at = swap ? oi : at;
       }
+    }
+#pragma unroll
+    for (int q = 0; q < kMaxNeighbors; ++q)
+      if (q < k) nb[an][q] = bi[q];
+  }
+  __syncthreads();
+  const int ncomb = k * (k - 1) * (k - 2) / 6;
   const int T = n * ncomb;
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
     const int an = t / ncomb, c = t - (t / ncomb) * ncomb;
@@ -663,7 +917,7 @@ __global__ void __launch_bounds__(1024) reg_desc_kernel(RegArgs a) {
     if (s1 > s2) { const int q = s1; s1 = s2; s2 = q; }
     if (s0 > s1) { const int q = s0; s0 = s1; s1 = q; }
     TriCand tc;
-    tc.key = (s0 << 14) | (s1 << 7) | s2;
+    keys[t] = (s0 << 14) | (s1 << 7) | s2;
     tc.packed = 0;
     tc.d0 = tc.d1 = 0.0;
     const double ex = dsub(px[r[1]], px[r[0]]), ey = dsub(py[r[1]], py[r[0]]);
@@ -698,30 +952,45 @@ __global__ void __launch_bounds__(1024) reg_desc_kernel(RegArgs a) {
       }
     }
     tri[t] = tc;
+    areas[t] = 0ull;
   }
   __syncthreads();
   // keep the first occurrence of each vertex set (whatever its validity)
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
     if (tri[t].packed >= 0) continue;
-    const int key = tri[t].key;
+    const int key = keys[t];
     bool keep = true;
-    for (int q = 0; q < t && keep; ++q)
-      if (tri[q].key == key) keep = false;
-    if (!keep) tri[t].packed &= 0x7fffffff;
+    int q = 0;
+    for (; q + 4 <= t && keep; q += 4) {
+      const int4 o = *reinterpret_cast<const int4*>(keys + q);
+      keep = o.x != key && o.y != key && o.z != key && o.w != key;
+    }
+    for (; q < t && keep; ++q) keep = keys[q] != key;
+    if (keep) areas[t] = dbits_of(tri[t].area);
   }
   __syncthreads();
   // stable area-descending rank
   for (int t = threadIdx.x; t < T; t += blockDim.x) {
-    if (tri[t].packed >= 0) continue;
-    const double ar = tri[t].area;
+    const unsigned long long ar = areas[t];
+    if (ar == 0ull) continue;
     int rank = 0;
-    for (int q = 0; q < T; ++q)
-      if (tri[q].packed < 0 && (tri[q].area > ar || (tri[q].area == ar && q < t))) ++rank;
+    int q = 0;
+    for (; q + 2 <= t; q += 2) {
+      const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(areas + q);
+      rank += (o.x >= ar ? 1 : 0) + (o.y >= ar ? 1 : 0);
+    }
+    if (q < t) rank += areas[q++] >= ar ? 1 : 0;
+    for (; (q & 1) && q < T; ++q) rank += areas[q] > ar ? 1 : 0;
+    for (; q + 2 <= T; q += 2) {
+      const ulonglong2 o = *reinterpret_cast<const ulonglong2*>(areas + q);
+      rank += (o.x > ar ? 1 : 0) + (o.y > ar ? 1 : 0);
+    }
+    if (q < T) rank += areas[q] > ar ? 1 : 0;
     if (rank < a.max_desc) {
       Desc d;
       d.d0 = tri[t].d0;
       d.d1 = tri[t].d1;
-      d.area = ar;
+      d.area = tri[t].area;
       const int p = tri[t].packed;
       d.v[0] = p & 127;
       d.v[1] = (p >> 7) & 127;
@@ -735,25 +1004,127 @@ __global__ void __launch_bounds__(1024) reg_desc_kernel(RegArgs a) {
   if (threadIdx.x == 0) a.ndesc[row] = min(s_kept, a.max_desc);
 }
 
-// ---- K2: descriptor matches, one CTA per frame pair -----------------------------------
-__device__ __forceinline__ unsigned long long dbits(double d) {
-  return static_cast<unsigned long long>(__double_as_longlong(d));
+// ---- K2: descriptor matches of a frame pair --------------------------------------------
+// Descriptor distance of a moving and a reference descriptor; false when the
+// pair is outside the radius.  `near` is the float32 bound per component
+// (conversion error <= 2^-24 relative) that most pairs fail; a list compares
+// the float32 distance itself.
+struct MatchTest {
+  double radius, bound;
+  float radf;
+  bool list_mode;
+  __device__ __forceinline__ explicit MatchTest(const RegArgs& a)
+      : radius(a.radius),
+        bound(a.radius * 1.000001 + 1.0e-300),
+        radf(static_cast<float>(a.radius) * 1.000001f + 1.0e-30f),
+        list_mode(a.mode == kDescriptorList) {}
+  __device__ __forceinline__ double list_distance(float2 rf, float2 mf) const {
+    const float e0 = __fsub_rn(rf.x, mf.x);
+    const float e1 = __fsub_rn(rf.y, mf.y);
+    return static_cast<double>(sqrtf(__fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1))));
+  }
+  __device__ __forceinline__ bool near(float2 rf, float2 mf) const {
+    if (list_mode) return list_distance(rf, mf) <= radius;
+    return !(fabsf(rf.x - mf.x) > radf + 3.0e-7f * (fabsf(rf.x) + fabsf(mf.x))) &&
+           !(fabsf(rf.y - mf.y) > radf + 3.0e-7f * (fabsf(rf.y) + fabsf(mf.y)));
+  }
+  __device__ __forceinline__ bool within(double2 r, double2 m, double& d) const {
+    if (list_mode) {
+      d = list_distance(make_float2(static_cast<float>(r.x), static_cast<float>(r.y)),
+                        make_float2(static_cast<float>(m.x), static_cast<float>(m.y)));
+      return d <= radius;
+    }
+    const double e0 = dsub(r.x, m.x);
+    if (fabs(e0) > bound) return false;
+    const double e1 = dsub(r.y, m.y);
+    if (fabs(e1) > bound) return false;
+    d = hyp_sum(e0, e1);
+    return d <= radius;
+  }
+};
+
+__device__ __forceinline__ double2 desc_f64(const Desc& d) { return make_double2(d.d0, d.d1); }
+__device__ __forceinline__ float2 desc_f32(const Desc& d) {
+  return make_float2(static_cast<float>(d.d0), static_cast<float>(d.d1));
+}
+
+// All matches of a frame pair, several CTAs per pair: a warp per moving
+// descriptor tests 32 reference descriptors at a time in float32 and collects
+// the survivors, and evaluates the float64 distance when 32 of them are
+// together: a warp pays for a float64 operation whether one lane or all need
+// it, and a few per cent of the pairs survive.  Matches come in no order.
+// Together with the selection 105 us for 32 pairs of about 500 descriptors,
+// 606 us with one CTA per pair and the distance evaluated where the test
+// passed.
+constexpr int kPairWarps = 8;
+constexpr int kPairCtas = 8;
+
+__global__ void __launch_bounds__(32 * kPairWarps) reg_pairs_kernel(RegArgs a) {
+  __shared__ float2 rdf[kMaxDesc];
+  __shared__ int s_queue[kPairWarps][64];
+  const int j = blockIdx.y;
+  const RegJob job = a.jobs[j];
+  const Desc* rd = a.desc + static_cast<int64_t>(job.ref_row) * kMaxDesc;
+  const Desc* md = a.desc + static_cast<int64_t>(job.mov_row) * kMaxDesc;
+  const int nr = a.ndesc[job.ref_row], nm = a.ndesc[job.mov_row];
+  for (int i = threadIdx.x; i < nr; i += blockDim.x) rdf[i] = desc_f32(rd[i]);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int* queue = s_queue[warp];
+  int queued = 0;  // the same in every lane
+  const MatchTest test(a);
+  double* mdist = a.match_dist + static_cast<int64_t>(j) * a.match_cap;
+  int* mkey = a.match_key + static_cast<int64_t>(j) * a.match_cap;
+  auto drain = [&](int n) {  // the first n <= 32 queued pairs
+    const int q = lane < n ? queue[lane] : 0;
+    double d = 0.0;
+    const bool in = lane < n && test.within(desc_f64(rd[q % nr]), desc_f64(md[q / nr]), d);
+    const unsigned mask = __ballot_sync(0xffffffffu, in);
+    int base = 0;
+    if (lane == 0 && mask) base = atomicAdd(a.match_count + j, __popc(mask));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    const int pos = base + __popc(mask & ((1u << lane) - 1u));
+    if (in && pos < a.match_cap) {
+      mdist[pos] = d;
+      mkey[pos] = q;
+    }
+  };
+  for (int mi = blockIdx.x * kPairWarps + warp; mi < nm; mi += gridDim.x * kPairWarps) {
+    const float2 mf = desc_f32(md[mi]);
+    for (int base = 0; base < nr; base += 32) {
+      const int ri = base + lane;
+      const bool near = ri < nr && test.near(rdf[min(ri, nr - 1)], mf);
+      const unsigned mask = __ballot_sync(0xffffffffu, near);
+      if (near) queue[queued + __popc(mask & ((1u << lane) - 1u))] = mi * nr + ri;
+      queued += __popc(mask);
+      __syncwarp();
+      if (queued >= 32) {
+        drain(32);
+        const int rest = queued > 32 + lane ? queue[32 + lane] : 0;
+        __syncwarp();
+        queue[lane] = rest;
+        queued -= 32;
+        __syncwarp();
+      }
+    }
+  }
+  if (queued) drain(queued);
 }
 
 struct SelEntry {
-  double d;
+  unsigned long long d;  // order-preserving bits of the distance
   int key;
   int pad;
 };
 
+// The max_candidates best matches in order, one CTA per frame pair.
 __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double2* rdd = reinterpret_cast<double2*>(smem);              // [kMaxDesc]
-  double2* mdd = rdd + kMaxDesc;                                // [kMaxDesc]
-  SelEntry* sel = reinterpret_cast<SelEntry*>(mdd + kMaxDesc);  // [kMaxSel]
-  float2* rdf = reinterpret_cast<float2*>(sel + kMaxSel);       // [kMaxDesc]
-  float2* mdf = rdf + kMaxDesc;                                 // [kMaxDesc]
-  __shared__ unsigned s_count;
+  double2* rdd = reinterpret_cast<double2*>(smem);         // [kMaxDesc] descriptors, for more matches than
+  double2* mdd = rdd + kMaxDesc;                           // [kMaxDesc] the list holds
+  float2* rdf = reinterpret_cast<float2*>(mdd + kMaxDesc); // [kMaxDesc]
+  float2* mdf = rdf + kMaxDesc;                            // [kMaxDesc]
+  __shared__ __align__(16) SelEntry sel[kMaxSel];
   __shared__ int s_c, s_n;
   __shared__ unsigned s_hist[256];
   __shared__ unsigned long long s_prefix;
@@ -763,63 +1134,20 @@ __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
   const Desc* rd = a.desc + static_cast<int64_t>(job.ref_row) * kMaxDesc;
   const Desc* md = a.desc + static_cast<int64_t>(job.mov_row) * kMaxDesc;
   const int nr = a.ndesc[job.ref_row], nm = a.ndesc[job.mov_row];
-  for (int i = threadIdx.x; i < nr; i += blockDim.x) {
-    rdd[i] = make_double2(rd[i].d0, rd[i].d1);
-    rdf[i] = make_float2(static_cast<float>(rd[i].d0), static_cast<float>(rd[i].d1));
-  }
-  for (int i = threadIdx.x; i < nm; i += blockDim.x) {
-    mdd[i] = make_double2(md[i].d0, md[i].d1);
-    mdf[i] = make_float2(static_cast<float>(md[i].d0), static_cast<float>(md[i].d1));
-  }
-  double* mdist = a.match_dist + static_cast<int64_t>(j) * a.match_cap;
-  int* mkey = a.match_key + static_cast<int64_t>(j) * a.match_cap;
-  if (threadIdx.x == 0) s_count = 0;
-  __syncthreads();
+  const double* mdist = a.match_dist + static_cast<int64_t>(j) * a.match_cap;
+  const int* mkey = a.match_key + static_cast<int64_t>(j) * a.match_cap;
   const int total = nm * nr;
   const double radius = a.radius;
-  const double bound = radius * 1.000001 + 1.0e-300;
-  const float radf = static_cast<float>(radius) * 1.000001f + 1.0e-30f;
-  const bool list_mode = a.mode == kDescriptorList;
-  // descriptor distance of flat index q = moving * nr + reference; false when
-  // the pair is outside the radius
+  const MatchTest test(a);
   auto match_dist = [&](int q, double& d) -> bool {
-    const int mi = q / nr, ri = q - (q / nr) * nr;
-    const float2 rf = rdf[ri], mf = mdf[mi];
-    if (list_mode) {
-      const float e0 = __fsub_rn(rf.x, mf.x);
-      const float e1 = __fsub_rn(rf.y, mf.y);
-      const float df = sqrtf(__fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1)));
-      d = static_cast<double>(df);
-      return d <= radius;
-    }
-    // float32 bounds per component (conversion error <= 2^-24 relative),
-    // then the float64 distance
-    if (fabsf(rf.x - mf.x) > radf + 3.0e-7f * (fabsf(rf.x) + fabsf(mf.x))) return false;
-    if (fabsf(rf.y - mf.y) > radf + 3.0e-7f * (fabsf(rf.y) + fabsf(mf.y))) return false;
-    const double2 r = rdd[ri], m = mdd[mi];
-    const double e0 = dsub(r.x, m.x);
-    if (fabs(e0) > bound) return false;
-    const double e1 = dsub(r.y, m.y);
-    if (fabs(e1) > bound) return false;
-    d = hyp_sum(e0, e1);
-    return d <= radius;
+    const int mi = q / nr, ri = q - mi * nr;
+    return test.near(rdf[ri], mdf[mi]) && test.within(rdd[ri], mdd[mi], d);
   };
-  for (int q = threadIdx.x; q < total; q += blockDim.x) {
-    double d;
-    if (match_dist(q, d)) {
-      const unsigned pos = atomicAdd(&s_count, 1u);
-      if (pos < static_cast<unsigned>(a.match_cap)) {
-        mdist[pos] = d;
-        mkey[pos] = q;
-      }
-    }
-  }
-  __syncthreads();
-  const int n = static_cast<int>(s_count);
+  const int n = a.match_count[j];
   const bool stored_all = n <= a.match_cap;
   int2* out = a.sel + static_cast<int64_t>(j) * a.sel_cap;
   long long* out_order = a.sel_order + static_cast<int64_t>(j) * a.sel_cap;
-  if (list_mode) {
+  if (test.list_mode) {
     // every match is a candidate; order = reference-major enumeration index
     const bool fits = stored_all && n <= a.sel_cap;
     if (fits) {
@@ -839,15 +1167,26 @@ __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
     }
     return;
   }
+  if (!stored_all) {
+    for (int i = threadIdx.x; i < nr; i += blockDim.x) {
+      rdd[i] = desc_f64(rd[i]);
+      rdf[i] = desc_f32(rd[i]);
+    }
+    for (int i = threadIdx.x; i < nm; i += blockDim.x) {
+      mdd[i] = desc_f64(md[i]);
+      mdf[i] = desc_f32(md[i]);
+    }
+    __syncthreads();
+  }
   // block-wide count of matches satisfying pred(distance bits, flat index)
   auto block_count = [&](auto pred) -> int {
     int c = 0;
     if (stored_all) {
-      for (int q = threadIdx.x; q < n; q += blockDim.x) c += pred(dbits(mdist[q]), mkey[q]) ? 1 : 0;
+      for (int q = threadIdx.x; q < n; q += blockDim.x) c += pred(dbits_of(mdist[q]), mkey[q]) ? 1 : 0;
     } else {
       for (int q = threadIdx.x; q < total; q += blockDim.x) {
         double d;
-        if (match_dist(q, d)) c += pred(dbits(d), q) ? 1 : 0;
+        if (match_dist(q, d)) c += pred(dbits_of(d), q) ? 1 : 0;
       }
     }
     __syncthreads();
@@ -862,7 +1201,7 @@ __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
   const int take = min(n, a.max_cand);
   // the take smallest (distance, index) pairs: distance threshold t, then the
   // index threshold K among the matches at exactly distance t
-  unsigned long long t = dbits(radius);
+  unsigned long long t = dbits_of(radius);
   int K = total;
   if (take == 0) {
     t = 0ull;
@@ -877,8 +1216,9 @@ __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
       for (int shift = 56; shift >= 0; shift -= 8) {
         for (int i = threadIdx.x; i < 256; i += blockDim.x) s_hist[i] = 0u;
         __syncthreads();
+#pragma unroll 4
         for (int q = threadIdx.x; q < n; q += blockDim.x) {
-          const unsigned long long k = dbits(mdist[q]);
+          const unsigned long long k = dbits_of(mdist[q]);
           if ((k & mask) == prefix) atomicAdd(&s_hist[(k >> shift) & 255u], 1u);
         }
         __syncthreads();
@@ -915,7 +1255,7 @@ __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
       need = rank + 1;  // entries at exactly distance t to keep
       equal = s_eq;     // entries at exactly distance t
     } else {
-      unsigned long long lo = 0ull, hi = dbits(radius);
+      unsigned long long lo = 0ull, hi = dbits_of(radius);
       while (lo < hi) {
         const unsigned long long mid = lo + (hi - lo) / 2;
         if (block_count([&](unsigned long long b, int) { return b <= mid; }) >= take) hi = mid;
@@ -941,17 +1281,17 @@ __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
   auto keep = [&](unsigned long long b, int q) { return b < t || (b == t && q <= K); };
   if (stored_all) {
     for (int q = threadIdx.x; q < n; q += blockDim.x) {
-      if (keep(dbits(mdist[q]), mkey[q])) {
+      if (keep(dbits_of(mdist[q]), mkey[q])) {
         const int p = atomicAdd(&s_n, 1);
-        if (p < kMaxSel) sel[p] = {mdist[q], mkey[q], 0};
+        if (p < kMaxSel) sel[p] = {dbits_of(mdist[q]), mkey[q], 0};
       }
     }
   } else {
     for (int q = threadIdx.x; q < total; q += blockDim.x) {
       double d;
-      if (match_dist(q, d) && keep(dbits(d), q)) {
+      if (match_dist(q, d) && keep(dbits_of(d), q)) {
         const int p = atomicAdd(&s_n, 1);
-        if (p < kMaxSel) sel[p] = {d, q, 0};
+        if (p < kMaxSel) sel[p] = {dbits_of(d), q, 0};
       }
     }
   }
@@ -960,7 +1300,7 @@ __global__ void __launch_bounds__(1024) reg_match_kernel(RegArgs a) {
   int m = 1;
   while (m < ns) m <<= 1;
   for (int i = ns + threadIdx.x; i < m; i += blockDim.x)
-    sel[i] = {__longlong_as_double(0x7ff0000000000000ll), 0x7fffffff, 0};
+    sel[i] = {~0ull, 0x7fffffff, 0};
   __syncthreads();
   for (int size = 2; size <= m; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -1013,71 +1353,99 @@ __device__ void load_job_points(const RegArgs& a, const RegJob& job, JobPoints& 
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    jp.nm = nm;
-    jp.nr = nr;
+  if (threadIdx.x < 32) {  // extents, by one warp
+    const int lane = threadIdx.x;
     float cmax = 0.0f, rmax = 0.0f;
-    for (int i = 0; i < nm; ++i) cmax = fmaxf(cmax, fabsf(jp.mx32[i]) + fabsf(jp.my32[i]));
+    for (int i = lane; i < nm; i += 32) cmax = fmaxf(cmax, fabsf(jp.mx32[i]) + fabsf(jp.my32[i]));
     float x0 = 3.0e38f, x1 = -3.0e38f, y0 = 3.0e38f, y1 = -3.0e38f;
-    for (int i = 0; i < nr; ++i) {
+    for (int i = lane; i < nr; i += 32) {
       x0 = fminf(x0, jp.rx32[i]);
       x1 = fmaxf(x1, jp.rx32[i]);
       y0 = fminf(y0, jp.ry32[i]);
       y1 = fmaxf(y1, jp.ry32[i]);
       rmax = fmaxf(rmax, fmaxf(fabsf(jp.rx32[i]), fabsf(jp.ry32[i])));
     }
-    jp.cmax = cmax * 1.0001f + 1.0f;
-    jp.rmax = rmax * 1.0001f + 1.0f;
-    for (int c = 0; c <= kGrid * kGrid; ++c) jp.cell_start[c] = 0;
-    if (nr == 0) {
+    for (int off = 16; off > 0; off >>= 1) {
+      cmax = fmaxf(cmax, __shfl_xor_sync(0xffffffffu, cmax, off));
+      rmax = fmaxf(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
+      x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, off));
+      x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, off));
+      y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, off));
+      y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, off));
+    }
+    if (lane == 0) {
+      jp.nm = nm;
+      jp.nr = nr;
+      jp.cmax = cmax * 1.0001f + 1.0f;
+      jp.rmax = rmax * 1.0001f + 1.0f;
+      jp.partners = 0;
       jp.gnx = jp.gny = 0;
       jp.gx0 = jp.gy0 = 0.0f;
       jp.ginv = 1.0f;
-    } else {
-      // cells at least 2 * (tol + 0.5) wide (> the widest search radius) so
-      // a search touches <= 2 x 2 cells
-      const float reach = static_cast<float>(2.0 * (tol + 0.5)) + 1.0f;
-      const float cell = fmaxf(fmaxf(x1 - x0, y1 - y0) / static_cast<float>(kGrid), reach);
-      jp.gx0 = x0;
-      jp.gy0 = y0;
-      if (cell < 1.0e30f) {
-        jp.ginv = 1.0f / cell;
-        jp.gnx = min(kGrid, static_cast<int>((x1 - x0) * jp.ginv) + 1);
-        jp.gny = min(kGrid, static_cast<int>((y1 - y0) * jp.ginv) + 1);
-      } else {  // one cell holding every star
-        jp.ginv = 0.0f;
-        jp.gnx = jp.gny = 1;
+      if (nr > 0) {
+        // cells at least 2 * (tol + 0.5) wide (> the widest search radius) so
+        // a search touches <= 2 x 2 cells
+        const float reach = static_cast<float>(2.0 * (tol + 0.5)) + 1.0f;
+        const float cell = fmaxf(fmaxf(x1 - x0, y1 - y0) / static_cast<float>(kGrid), reach);
+        jp.gx0 = x0;
+        jp.gy0 = y0;
+        if (cell < 1.0e30f) {
+          jp.ginv = 1.0f / cell;
+          jp.gnx = min(kGrid, static_cast<int>((x1 - x0) * jp.ginv) + 1);
+          jp.gny = min(kGrid, static_cast<int>((y1 - y0) * jp.ginv) + 1);
+        } else {  // one cell holding every star
+          jp.ginv = 0.0f;
+          jp.gnx = jp.gny = 1;
+        }
       }
-      unsigned char cnt[kGrid * kGrid];
-      for (int c = 0; c < kGrid * kGrid; ++c) cnt[c] = 0;
-      int cellof[kRegPts];
-      for (int i = 0; i < nr; ++i) {
-        const int cx = min(jp.gnx - 1, max(0, static_cast<int>((jp.rx32[i] - x0) * jp.ginv)));
-        const int cy = min(jp.gny - 1, max(0, static_cast<int>((jp.ry32[i] - y0) * jp.ginv)));
-        cellof[i] = cy * kGrid + cx;
-        ++cnt[cellof[i]];
-      }
-      int run = 0;
-      for (int c = 0; c < kGrid * kGrid; ++c) {
-        jp.cell_start[c] = static_cast<unsigned char>(run);
-        run += cnt[c];
-      }
-      jp.cell_start[kGrid * kGrid] = static_cast<unsigned char>(run);
-      for (int c = 0; c < kGrid * kGrid; ++c) cnt[c] = jp.cell_start[c];
-      for (int i = 0; i < nr; ++i) jp.cell_pt[cnt[cellof[i]]++] = static_cast<unsigned char>(i);
     }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nr; i += blockDim.x) {
+    const int cx = min(jp.gnx - 1, max(0, static_cast<int>((jp.rx32[i] - jp.gx0) * jp.ginv)));
+    const int cy = min(jp.gny - 1, max(0, static_cast<int>((jp.ry32[i] - jp.gy0) * jp.ginv)));
+    jp.cell_of[i] = static_cast<unsigned char>(cy * kGrid + cx);
+  }
+  __syncthreads();
+  // counting sort by cell, in index order inside a cell; stars within reach of
+  // one point are within twice the reach (tol + 0.5 at most, see
+  // can_leave_early) of each other
+  const float near = 2.0f * static_cast<float>(tol + 0.5) * 1.001f + 1.0e-6f * jp.rmax;
+  for (int i = threadIdx.x; i < nr; i += blockDim.x) {
+    const int cell = jp.cell_of[i];
+    const float x = jp.rx32[i], y = jp.ry32[i];
+    int pos = 0, close = 0;
+    for (int q = 0; q < nr; ++q) {
+      pos += (jp.cell_of[q] < cell || (jp.cell_of[q] == cell && q < i)) ? 1 : 0;
+      close += (fabsf(jp.rx32[q] - x) <= near && fabsf(jp.ry32[q] - y) <= near) ? 1 : 0;
+    }
+    jp.cell_pt[pos] = static_cast<unsigned char>(i);
+    atomicMax(&jp.partners, close);
+  }
+  for (int c = threadIdx.x; c <= kGrid * kGrid; c += blockDim.x) {
+    int start = 0;
+    for (int q = 0; q < nr; ++q) start += jp.cell_of[q] < c ? 1 : 0;
+    jp.cell_start[c] = static_cast<unsigned char>(start);
   }
 }
 
 constexpr int kScoreWarps = 4;
 
 // Cand::valid bits: 1 = fit succeeded, 2 = count and rms are exact.
+// Fits one candidate per lane, then the warp counts the pairs of one after the
+// other.  The float64 work is what a warp can do for 32 candidates at once (the
+// fit, the error bounds) and what the float32 test leaves open; residuals in
+// float64 are for the candidates that can still win (reg_rms_kernel), and a
+// candidate that falls behind the best count known is dropped.  32 pairs
+// of frames: 158 us, 114 us for the conflicts and 45 us for the residuals; 946 us
+// with exact scores on the spot, float64 residuals
+// and bounds for every candidate.
 template <int MODEL>
 __global__ void __launch_bounds__(32 * kScoreWarps) reg_score_kernel(RegArgs a) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  WarpScratch* ws = reinterpret_cast<WarpScratch*>(smem);
   __shared__ JobPoints jp;
+  __shared__ unsigned used_r[kScoreWarps][3];
   __shared__ double cm[kScoreWarps][32][6];
+  __shared__ FastTransform cf[kScoreWarps][32];
   __shared__ int cok[kScoreWarps][32];
   const int j = blockIdx.y;
   const RegJob job = a.jobs[j];
@@ -1090,6 +1458,7 @@ __global__ void __launch_bounds__(32 * kScoreWarps) reg_score_kernel(RegArgs a) 
   const int2* sel = a.sel + static_cast<int64_t>(j) * a.sel_cap;
   const long long* order = a.sel_order + static_cast<int64_t>(j) * a.sel_cap;
   Cand* cands = a.cands + static_cast<int64_t>(j) * 2 * a.sel_cap;
+  CandRank* ranks = a.ranks + static_cast<int64_t>(j) * 2 * a.sel_cap;
   for (int base = (blockIdx.x * kScoreWarps + warp) * 32; base < ncand; base += gridDim.x * kScoreWarps * 32) {
     // one 3-point fit per lane
     const int c = base + lane;
@@ -1119,92 +1488,226 @@ __global__ void __launch_bounds__(32 * kScoreWarps) reg_score_kernel(RegArgs a) 
         cd.m[q] = ok ? m[q] : 0.0;
       }
       cd.order = 2 * order[c >> 1] + (c & 1);
+      if (ok) cf[warp][lane] = fast_transform(m, jp, a.tol);
     }
     cok[warp][lane] = ok;
     __syncwarp();
     // score the chunk one candidate at a time with the whole warp
     const int nb = min(32, ncand - base);
+    int my_count = -1;  // of the lane's candidate
+    float my_sum = 0.0f;
+    int best = __shfl_sync(0xffffffffu, __ldcg(a.best_count + j), 0);  // whatever other warps have found by now
     for (int t = 0; t < nb; ++t) {
-      int count = 0, exact = 0;
-      double rms = __longlong_as_double(0x7ff0000000000000ll);
-      if (cok[warp][t]) {
-        double m[6];
-        for (int q = 0; q < 6; ++q) m[q] = cm[warp][t][q];
-        double sum_d2;
-        bool conflict;
-        warp_score_fast(m, jp, a.tol, ws[warp], count, sum_d2, conflict);
-        if (conflict) {
-          warp_score_exact(m, jp, a.tol, ws[warp], count, rms, nullptr, a.overflow);
-          exact = 1;
-        } else if (count > 0) {
-          rms = sqrt(__ddiv_rn(sum_d2, static_cast<double>(count)));
-        }
+      if (!cok[warp][t]) continue;
+      int count;
+      float sum;
+      bool conflict;
+      warp_score_count(cf[warp][t], cm[warp][t], jp, a.tol, can_leave_early(jp, a.tol, cf[warp][t].r) ? best : 0,
+                       used_r[warp], count, sum, conflict);
+      if (!conflict && count > best) {
+        best = count;
+        if (lane == 0) atomicMax(a.best_count + j, count);
       }
-      if (lane == 0) {
-        Cand& cd = cands[base + t];
-        cd.count = count;
-        cd.rms = rms;
-        cd.valid = cok[warp][t] ? (1 | (exact << 1)) : 0;
+      if (lane == t) {
+        my_count = conflict ? kConflictCount - count : count;
+        my_sum = sum;
       }
+    }
+    if (c < ncand) {
+      // bounds of the rms: every distance is known to delta, the sum to 80 roundings
+      const float rms32 = sqrtf(my_sum / static_cast<float>(max(my_count, 1)));
+      const float delta = ok ? cf[warp][lane].delta : 0.0f;
+      ranks[c] = {my_count, (rms32 - delta) * 0.99999f, (rms32 + delta) * 1.00001f};
+      cands[c].rms = __longlong_as_double(0x7ff0000000000000ll);
+      cands[c].scored = 0;
     }
     __syncwarp();
   }
 }
 
-// ---- K4: best candidate and guarded refits, one warp per frame pair --------------------
+// ---- the candidates that can win ------------------------------------------------------
+// The most pairs of any candidate and the smallest upper bound of an rms among
+// those; block-wide, the same in every thread.
+struct WinBound {
+  int count;
+  float rms;
+};
+
+__device__ WinBound win_bound(const CandRank* ranks, int ncand) {
+  __shared__ int s_count;
+  __shared__ int s_rms;  // non-negative floats compare as integers
+  if (threadIdx.x == 0) {
+    s_count = 0;
+    s_rms = 0x7f800000;
+  }
+  __syncthreads();
+  int bn = 0;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < ncand; c += blockDim.x) bn = max(bn, ranks[c].count);
+  bn = __reduce_max_sync(0xffffffffu, bn);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_count, bn);
+  __syncthreads();
+  bn = s_count;
+  int hi = 0x7f800000;
+#pragma unroll 4
+  for (int c = threadIdx.x; c < ncand; c += blockDim.x) {
+    const CandRank r = ranks[c];
+    if (r.count == bn && r.rms_hi >= 0.0f) hi = min(hi, __float_as_int(r.rms_hi));
+  }
+  hi = __reduce_min_sync(0xffffffffu, hi);
+  if ((threadIdx.x & 31) == 0) atomicMin(&s_rms, hi);
+  __syncthreads();
+  return {bn, __int_as_float(s_rms)};
+}
+
+__device__ __forceinline__ bool can_win(const CandRank& r, const WinBound& b) {
+  return b.count > 0 && r.count == b.count && !(r.rms_lo > b.rms);
+}
+
+// Counts of the candidates in which a star has two partners, where they may
+// still reach the best count.  A kernel of its own: where two stars stand close
+// together that is every good candidate of a frame pair, next to each other in
+// the order of the candidates (the two orientations of a match take turns:
+// the number of warps they are dealt to is odd).
+constexpr int kRecheckCtas = 16;
+
+__global__ void __launch_bounds__(32 * kScoreWarps) reg_exact_kernel(RegArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  WarpScratch* ws = reinterpret_cast<WarpScratch*>(smem);
+  __shared__ JobPoints jp;
+  const int j = blockIdx.y;
+  const RegJob job = a.jobs[j];
+  const int ncand = 2 * a.nsel[j];
+  CandRank* ranks = a.ranks + static_cast<int64_t>(j) * 2 * a.sel_cap;
+  Cand* cands = a.cands + static_cast<int64_t>(j) * 2 * a.sel_cap;
+  load_job_points(a, job, jp, a.tol);
+  __syncthreads();
+  const int best = a.best_count[j];
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * kScoreWarps + (threadIdx.x >> 5);
+  const int nwarps = static_cast<int>(gridDim.x * kScoreWarps - 1u) | 1;  // odd
+  if (warp >= nwarps) return;
+  for (int base = warp; base < ncand; base += 32 * nwarps) {
+    const int c = base + lane * nwarps;
+    const int count = c < ncand ? ranks[c].count : -1;
+    bool check = count <= kConflictCount;
+    if (check && kConflictCount - count < best) {
+      double m[6];
+      for (int q = 0; q < 6; ++q) m[q] = cands[c].m[q];
+      check = !can_leave_early(jp, a.tol, fast_transform(m, jp, a.tol).r);
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, check);
+    while (todo) {
+      const int t = base + (__ffs(todo) - 1) * nwarps;
+      todo &= todo - 1u;
+      double m[6];
+      for (int q = 0; q < 6; ++q) m[q] = cands[t].m[q];
+      int n;
+      double rms;
+      const bool resolved = warp_resolve(m, jp, a.tol, ws[threadIdx.x >> 5], n, rms);
+      if (!resolved) score_exact<WarpGroup>(m, jp, a.tol, ws[threadIdx.x >> 5], n, rms, nullptr, a.overflow);
+      if (lane == 0) {
+        const float rms32 = static_cast<float>(rms);
+        ranks[t] = {n, rms32 * 0.99999f, rms32 * 1.00001f};
+        cands[t].rms = rms;
+        cands[t].scored = resolved ? 2 : 1;
+      }
+    }
+  }
+}
+
+// float64 rms of the candidates that can win (a warp takes every nwarps-th
+// candidate: the likely ones stand together).
+__global__ void __launch_bounds__(32 * kScoreWarps) reg_rms_kernel(RegArgs a) {
+  __shared__ JobPoints jp;
+  __shared__ double own_m[kScoreWarps][32][6];
+  __shared__ FastTransform own_t[kScoreWarps][32];
+  const int j = blockIdx.y;
+  const RegJob job = a.jobs[j];
+  const int ncand = 2 * a.nsel[j];
+  const CandRank* ranks = a.ranks + static_cast<int64_t>(j) * 2 * a.sel_cap;
+  Cand* cands = a.cands + static_cast<int64_t>(j) * 2 * a.sel_cap;
+  load_job_points(a, job, jp, a.tol);
+  const WinBound bound = win_bound(ranks, ncand);
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * kScoreWarps + (threadIdx.x >> 5);
+  const int nwarps = gridDim.x * kScoreWarps;
+  for (int base = warp; base < ncand; base += 32 * nwarps) {
+    const int c = base + lane * nwarps;
+    unsigned todo = __ballot_sync(0xffffffffu, c < ncand && can_win(ranks[min(c, ncand - 1)], bound) &&
+                                                   cands[min(c, ncand - 1)].scored == 0);
+    double own_sum = 0.0;
+    const bool mine = (todo >> lane) & 1u;
+    if (mine) {
+      double m[6];
+      for (int q = 0; q < 6; ++q) m[q] = cands[c].m[q];
+      for (int q = 0; q < 6; ++q) own_m[threadIdx.x >> 5][lane][q] = m[q];
+      own_t[threadIdx.x >> 5][lane] = fast_transform(m, jp, a.tol);
+    }
+    __syncwarp();
+    while (todo) {
+      const int t = __ffs(todo) - 1;
+      todo &= todo - 1u;
+      double m[6];
+      for (int q = 0; q < 6; ++q) m[q] = own_m[threadIdx.x >> 5][t][q];
+      const double sum = warp_sum_d2(m, own_t[threadIdx.x >> 5][t], jp, a.tol);
+      if (lane == t) own_sum = sum;
+    }
+    if (mine) cands[c].rms = sqrt(__ddiv_rn(own_sum, static_cast<double>(bound.count)));
+    __syncwarp();
+  }
+}
+
+// ---- K4: best candidate and guarded refits, one CTA per frame pair ---------------------
 // The reference keeps the first candidate with the most pairs and, among
 // those, the smallest rms.  Counts are exact for every candidate; the fast
 // rms differs from the exact one by < 1e-13 relative, so every candidate that
 // can win lies in the window rms <= min * (1 + 1e-12) and only those are
-// re-scored exactly (usually one).
+// re-scored exactly (usually one).  Bound by the chain of scores and refits
+// (float64 sums in NumPy's order): 134 us with the whole CTA on the search and
+// the scores, 320 us by one warp.
 constexpr int kWindowCap = 1024;
+constexpr int kBestThreads = 256;
 
-__global__ void __launch_bounds__(32) reg_best_kernel(RegArgs a) {
+__global__ void __launch_bounds__(kBestThreads) reg_best_kernel(RegArgs a) {
   __shared__ JobPoints jp;
   __shared__ WarpScratch ws;
-  __shared__ double fx[kRegPts], fy[kRegPts], gx[kRegPts], gy[kRegPts], buf[2 * kRegPts];
+  __shared__ double fx[kRegPts], fy[kRegPts], gx[kRegPts], gy[kRegPts], buf[4 * kRegPts];
   __shared__ short2 prs[kRegPts], prs2[kRegPts];
   __shared__ int window[kWindowCap];
+  __shared__ unsigned long long s_min;
+  __shared__ double s_m[6];
+  __shared__ int s_nw, s_fitted;
   const int j = blockIdx.x;
   const int lane = threadIdx.x;
   const RegJob job = a.jobs[j];
   load_job_points(a, job, jp, a.tol);
-  __syncthreads();
+  const double inf = __longlong_as_double(0x7ff0000000000000ll);
+  if (threadIdx.x == 0) {
+    s_min = dbits_of(inf);
+    s_nw = 0;
+  }
   const int ncand = 2 * a.nsel[j];
   const Cand* cs = a.cands + static_cast<int64_t>(j) * 2 * a.sel_cap;
-  const double inf = __longlong_as_double(0x7ff0000000000000ll);
-  // most pairs
-  int bn = 0;
-  for (int c = lane; c < ncand; c += 32)
-    if ((cs[c].valid & 1) && cs[c].count > bn) bn = cs[c].count;
-  for (int off = 16; off > 0; off >>= 1) bn = max(bn, __shfl_xor_sync(0xffffffffu, bn, off));
-  // smallest (fast) rms among them
-  double rmin = inf;
-  if (bn > 0) {
-    for (int c = lane; c < ncand; c += 32)
-      if ((cs[c].valid & 1) && cs[c].count == bn) rmin = fmin(rmin, cs[c].rms);
-    for (int off = 16; off > 0; off >>= 1) rmin = fmin(rmin, __shfl_xor_sync(0xffffffffu, rmin, off));
-  }
+  const CandRank* ranks = a.ranks + static_cast<int64_t>(j) * 2 * a.sel_cap;
+  const WinBound bound = win_bound(ranks, ncand);
+  // smallest (fast) rms of the candidates with the most pairs
+  for (int c = threadIdx.x; c < ncand; c += kBestThreads)
+    if (can_win(ranks[c], bound) && cs[c].rms < inf) atomicMin(&s_min, dbits_of(cs[c].rms));
+  __syncthreads();
+  const double rmin = __longlong_as_double(static_cast<long long>(s_min));
   const double thr = rmin + rmin * 1.0e-12;
-  // window members in candidate order
-  int nw = 0;
-  if (bn > 0) {
-    for (int base = 0; base < ncand; base += 32) {
-      const int c = base + lane;
-      const bool in = c < ncand && (cs[c].valid & 1) && cs[c].count == bn && cs[c].rms <= thr;
-      const unsigned mask = __ballot_sync(0xffffffffu, in);
-      if (in) {
-        const int pos = nw + __popc(mask & ((1u << lane) - 1u));
-        if (pos < kWindowCap) window[pos] = c;
-      }
-      nw += __popc(mask);
+  // window members
+  for (int c = threadIdx.x; c < ncand; c += kBestThreads)
+    if (can_win(ranks[c], bound) && cs[c].rms <= thr) {
+      const int pos = atomicAdd(&s_nw, 1);
+      if (pos < kWindowCap) window[pos] = c;
     }
-  }
+  __syncthreads();
+  int nw = s_nw;
   if (nw > kWindowCap) {
-    if (lane == 0) atomicExch(a.overflow, 1);
+    if (threadIdx.x == 0) atomicExch(a.overflow, 1);
     nw = kWindowCap;
   }
-  __syncwarp();
+  using Cta = CtaGroup<kBestThreads>;
   // exact rms of the window members: smallest wins, earliest order on ties
   int bc = -1;
   double br = inf;
@@ -1212,11 +1715,11 @@ __global__ void __launch_bounds__(32) reg_best_kernel(RegArgs a) {
   for (int w = 0; w < nw; ++w) {
     const int c = window[w];
     double r = cs[c].rms;
-    if (!(cs[c].valid & 2)) {
+    if (cs[c].scored != 1 && nw > 1) {  // a single member wins as it is
       double m[6];
       for (int q = 0; q < 6; ++q) m[q] = cs[c].m[q];
       int n;
-      warp_score_exact(m, jp, a.tol, ws, n, r, nullptr, a.overflow);
+      score_exact<Cta>(m, jp, a.tol, ws, n, r, nullptr, a.overflow);
     }
     const long long o = cs[c].order;
     if (bc < 0 || r < br || (r == br && o < bo)) {
@@ -1230,35 +1733,43 @@ __global__ void __launch_bounds__(32) reg_best_kernel(RegArgs a) {
   double best_rms = inf;
   if (bc >= 0) {
     for (int q = 0; q < 6; ++q) best[q] = cs[bc].m[q];
-    warp_score_exact(best, jp, a.tol, ws, best_n, best_rms, prs, a.overflow);
+    score_exact<Cta>(best, jp, a.tol, ws, best_n, best_rms, prs, a.overflow);
   }
-  __syncwarp();
   const int iterations = a.mode == kEstimator ? 3 : 0;
   for (int it = 0; it < iterations; ++it) {
     if (best_n < 3) break;
-    for (int q = lane; q < best_n; q += 32) {
+    for (int q = threadIdx.x; q < best_n; q += kBestThreads) {
       fx[q] = jp.mx[prs[q].x];
       fy[q] = jp.my[prs[q].x];
       gx[q] = jp.rx[prs[q].y];
       gy[q] = jp.ry[prs[q].y];
     }
-    __syncwarp();
-    double m[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const bool fitted = a.model == GG_TRANSFORM_AFFINE ? warp_fit_affine(fx, fy, gx, gy, best_n, m)
-                                                       : warp_fit_similarity(fx, fy, gx, gy, best_n, buf, m);
-    if (!fitted) break;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      double m[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      const bool fitted = a.model == GG_TRANSFORM_AFFINE ? warp_fit_affine(fx, fy, gx, gy, best_n, m)
+                                                         : warp_fit_similarity(fx, fy, gx, gy, best_n, buf, m);
+      if (lane == 0) {
+        s_fitted = fitted ? 1 : 0;
+        for (int q = 0; q < 6; ++q) s_m[q] = m[q];
+      }
+    }
+    __syncthreads();
+    if (!s_fitted) break;
+    double m[6];
+    for (int q = 0; q < 6; ++q) m[q] = s_m[q];
     int n2;
     double r2;
-    warp_score_exact(m, jp, a.tol, ws, n2, r2, prs2, a.overflow);
+    score_exact<Cta>(m, jp, a.tol, ws, n2, r2, prs2, a.overflow);
     if (n2 > best_n || (n2 == best_n && r2 <= best_rms)) {
       for (int q = 0; q < 6; ++q) best[q] = m[q];
-      for (int q = lane; q < n2; q += 32) prs[q] = prs2[q];
+      for (int q = threadIdx.x; q < n2; q += kBestThreads) prs[q] = prs2[q];
       best_n = n2;
       best_rms = r2;
     }
-    __syncwarp();
+    __syncthreads();
   }
-  if (lane == 0) {
+  if (threadIdx.x == 0) {
     RegResult& r = a.out[j];
     for (int q = 0; q < 6; ++q) r.m[q] = best[q];
     r.m[6] = 0.0;
@@ -1269,7 +1780,7 @@ __global__ void __launch_bounds__(32) reg_best_kernel(RegArgs a) {
     r.inliers = best_n;
     r.status = a.mode == kEstimator ? (best_n >= a.min_inliers ? 1 : 0) : (best_n > 0 ? 1 : 0);
   }
-  for (int q = lane; q < kRegPts; q += 32)
+  for (int q = threadIdx.x; q < kRegPts; q += kBestThreads)
     a.pairs[static_cast<int64_t>(j) * kRegPts + q] = q < best_n ? prs[q] : make_short2(-1, -1);
 }
 
@@ -1291,12 +1802,14 @@ struct RegScratch {
   int* ndesc = nullptr;
   RegJob* jobs = nullptr;
   int* row_frames = nullptr;
+  int* match_count = nullptr;
   double* match_dist = nullptr;
   int* match_key = nullptr;
   int2* sel = nullptr;
   long long* sel_order = nullptr;
   int* nsel = nullptr;
   Cand* cands = nullptr;
+  CandRank* ranks = nullptr;
   RegResult* out = nullptr;
   short2* pairs = nullptr;
   int* overflow = nullptr;
@@ -1308,8 +1821,8 @@ struct RegScratch {
 };
 
 static void reg_scratch_release(RegScratch& r) {
-  void* ps[] = {r.pts, r.npts,      r.desc, r.ndesc, r.jobs, r.row_frames, r.match_dist, r.match_key,
-                r.sel, r.sel_order, r.nsel, r.cands, r.out,  r.pairs,      r.overflow};
+  void* ps[] = {r.pts, r.npts,      r.desc, r.ndesc, r.jobs,  r.row_frames, r.match_count, r.match_dist, r.match_key,
+                r.sel, r.sel_order, r.nsel, r.cands, r.ranks, r.out,        r.pairs,       r.overflow};
   for (void* p : ps)
     if (p) cudaFree(p);
   r = RegScratch{};
@@ -1319,7 +1832,7 @@ static int64_t reg_scratch_bytes(const RegScratch& r) {
   if (r.device < 0) return 0;
   const int64_t R = r.rows, J = r.jobs_cap, M = r.match_cap, S = r.sel_cap;
   return R * (16 * kRegPts + 12 + static_cast<int64_t>(sizeof(Desc)) * kMaxDesc) +
-         J * (8 + 12 * M + 16 * S + 4 + 2 * static_cast<int64_t>(sizeof(Cand)) * S +
+         J * (8 + 8 + 12 * M + 16 * S + 4 + 2 * static_cast<int64_t>(sizeof(Cand) + sizeof(CandRank)) * S +
               static_cast<int64_t>(sizeof(RegResult)) + 4 * kRegPts) +
          4;
 }
@@ -1344,12 +1857,14 @@ static void reg_scratch_ensure(RegScratch& r, int rows, int jobs, int match_cap,
   check_cuda(cudaMalloc(&r.ndesc, sizeof(int) * R), "cudaMalloc(registration descriptor counts)");
   check_cuda(cudaMalloc(&r.row_frames, sizeof(int) * R), "cudaMalloc(registration rows)");
   check_cuda(cudaMalloc(&r.jobs, sizeof(RegJob) * J), "cudaMalloc(registration jobs)");
+  check_cuda(cudaMalloc(&r.match_count, sizeof(int) * 2 * J), "cudaMalloc(registration match counts)");
   check_cuda(cudaMalloc(&r.match_dist, sizeof(double) * M * J), "cudaMalloc(registration matches)");
   check_cuda(cudaMalloc(&r.match_key, sizeof(int) * M * J), "cudaMalloc(registration match keys)");
   check_cuda(cudaMalloc(&r.sel, sizeof(int2) * S * J), "cudaMalloc(registration selection)");
   check_cuda(cudaMalloc(&r.sel_order, sizeof(long long) * S * J), "cudaMalloc(registration order)");
   check_cuda(cudaMalloc(&r.nsel, sizeof(int) * J), "cudaMalloc(registration selection counts)");
   check_cuda(cudaMalloc(&r.cands, sizeof(Cand) * 2 * S * J), "cudaMalloc(registration candidates)");
+  check_cuda(cudaMalloc(&r.ranks, sizeof(CandRank) * 2 * S * J), "cudaMalloc(registration ranks)");
   check_cuda(cudaMalloc(&r.out, sizeof(RegResult) * J), "cudaMalloc(registration results)");
   check_cuda(cudaMalloc(&r.pairs, sizeof(short2) * kRegPts * J), "cudaMalloc(registration pairs)");
   check_cuda(cudaMalloc(&r.overflow, sizeof(int)), "cudaMalloc(registration overflow)");
@@ -1378,12 +1893,15 @@ static RegArgs make_args(RegScratch& r, int mode, double tol, double radius) {
   a.desc = r.desc;
   a.ndesc = r.ndesc;
   a.jobs = r.jobs;
+  a.match_count = r.match_count;
+  a.best_count = r.match_count + r.jobs_cap;
   a.match_dist = r.match_dist;
   a.match_key = r.match_key;
   a.sel = r.sel;
   a.sel_order = r.sel_order;
   a.nsel = r.nsel;
   a.cands = r.cands;
+  a.ranks = r.ranks;
   a.out = r.out;
   a.pairs = r.pairs;
   a.overflow = r.overflow;
@@ -1421,25 +1939,35 @@ static void launch_desc(const RegArgs& a, int rows, cudaStream_t stream) {
 }
 
 static void launch_match_score_best(const RegArgs& a, int njobs, int64_t max_sel, cudaStream_t stream) {
-  const size_t smem = (sizeof(double2) + sizeof(float2)) * 2 * kMaxDesc + sizeof(SelEntry) * kMaxSel;
+  const size_t smem = (sizeof(double2) + sizeof(float2)) * 2 * kMaxDesc;
   check_cuda(cudaFuncSetAttribute(reg_match_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   static_cast<int>(smem)),
              "cudaFuncSetAttribute(reg_match)");
-  note_launch();
+  check_cuda(cudaMemsetAsync(a.match_count, 0, sizeof(int) * (a.best_count - a.match_count + njobs), stream),
+             "cudaMemsetAsync(match counts)");
+  note_launch(2);
+  reg_pairs_kernel<<<dim3(kPairCtas, static_cast<unsigned>(njobs)), 32 * kPairWarps, 0, stream>>>(a);
+  check_cuda(cudaGetLastError(), "reg_pairs launch");
   reg_match_kernel<<<njobs, 1024, smem, stream>>>(a);
   check_cuda(cudaGetLastError(), "reg_match launch");
   const int64_t per_job = (2 * max_sel + 32 * kScoreWarps - 1) / (32 * kScoreWarps);
   const unsigned gx = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(per_job, 1024)));
-  const size_t score_smem = sizeof(WarpScratch) * kScoreWarps;
   auto score = a.model == GG_TRANSFORM_AFFINE ? reg_score_kernel<GG_TRANSFORM_AFFINE>
                                               : reg_score_kernel<GG_TRANSFORM_SIMILARITY>;
-  check_cuda(cudaFuncSetAttribute(score, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(score_smem)),
-             "cudaFuncSetAttribute(reg_score)");
   note_launch();
-  score<<<dim3(gx, static_cast<unsigned>(njobs)), 32 * kScoreWarps, score_smem, stream>>>(a);
+  score<<<dim3(gx, static_cast<unsigned>(njobs)), 32 * kScoreWarps, 0, stream>>>(a);
   check_cuda(cudaGetLastError(), "reg_score launch");
-  note_launch();
-  reg_best_kernel<<<njobs, 32, 0, stream>>>(a);
+  const unsigned gr = std::min(gx, static_cast<unsigned>(kRecheckCtas));
+  const size_t exact_smem = sizeof(WarpScratch) * kScoreWarps;
+  check_cuda(cudaFuncSetAttribute(reg_exact_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  static_cast<int>(exact_smem)),
+             "cudaFuncSetAttribute(reg_exact)");
+  note_launch(3);
+  reg_exact_kernel<<<dim3(gr, static_cast<unsigned>(njobs)), 32 * kScoreWarps, exact_smem, stream>>>(a);
+  check_cuda(cudaGetLastError(), "reg_exact launch");
+  reg_rms_kernel<<<dim3(gr, static_cast<unsigned>(njobs)), 32 * kScoreWarps, 0, stream>>>(a);
+  check_cuda(cudaGetLastError(), "reg_rms launch");
+  reg_best_kernel<<<njobs, kBestThreads, 0, stream>>>(a);
   check_cuda(cudaGetLastError(), "reg_best launch");
 }
 
