@@ -303,38 +303,69 @@ __global__ void __launch_bounds__(kGnThreads, K == 8 ? 1 : 3) gn_accumulate_kern
   }
 }
 
-// Quantile q of a log2 value histogram (log-linear inside the bin).
-__device__ double histogram_quantile(const unsigned* h, int bins, double q, double log2min, double per_octave) {
-  unsigned long long total = 0;
-  for (int b = 0; b < bins; ++b) total += h[b];
-  if (total == 0) return 0.0;
-  const double want = q * static_cast<double>(total);
-  double cum = 0.0;
-  for (int b = 0; b < bins; ++b) {
-    const double c = static_cast<double>(h[b]);
-    if (cum + c >= want && c > 0.0) return exp2(log2min + (b + (want - cum) / c) / per_octave);
-    cum += c;
-  }
-  return exp2(log2min + bins / per_octave);
-}
+// Where quantile q of a histogram lies: the first bin with samples at which the
+// cumulative count reaches q * total.  The whole warp looks for it, a run of
+// bins per lane; counts are whole numbers, so the search is exact in integers
+// (a float64 sum over the bins one after the other took most of the solve).
+struct QuantileBin {
+  int bin;                 // -1: not reached (or no samples)
+  double total, cum, in;   // samples in all, below the bin, in the bin
+  double want;
+};
 
-// 1.4826 * median |r| from the job's histogram (log-linear inside the bin).
-__device__ double histogram_sigma(const unsigned* h) {
-  unsigned long long total = 0;
-  for (int b = 0; b < kGnBins; ++b) total += h[b];
-  if (total == 0) return 0.0;
-  const double half = 0.5 * static_cast<double>(total);
-  double cum = 0.0;
-  for (int b = 0; b < kGnBins; ++b) {
-    const double c = static_cast<double>(h[b]);
-    if (cum + c >= half && c > 0.0) {
-      const double f = (half - cum) / c;
-      const double l = kGnLog2Min + (b + f) / kGnBinsPerOctave;
-      return 1.4826 * exp2(l);
+__device__ QuantileBin warp_quantile_bin(const unsigned* h, int bins, double q) {
+  const int lane = threadIdx.x & 31;
+  const int per = (bins + 31) / 32;
+  const int b0 = min(bins, lane * per), b1 = min(bins, b0 + per);
+  unsigned long long mine = 0;
+#pragma unroll 8
+  for (int b = b0; b < b1; ++b) mine += h[b];
+  unsigned long long incl = mine;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, off);
+    if (lane >= off) incl += v;
+  }
+  const unsigned long long total = __shfl_sync(0xffffffffu, incl, 31);
+  QuantileBin r;
+  r.total = static_cast<double>(total);
+  r.want = q * r.total;
+  const unsigned long long need = static_cast<unsigned long long>(ceil(r.want));
+  unsigned long long cum = incl - mine;
+  int bin = -1;
+  unsigned c = 0;
+  for (int b = b0; b < b1; ++b) {
+    c = h[b];
+    if (c > 0 && cum + c >= need) {
+      bin = b;
+      break;
     }
     cum += c;
   }
-  return 1.4826 * exp2(kGnLog2Min + kGnBins / kGnBinsPerOctave);
+  const unsigned found = __ballot_sync(0xffffffffu, bin >= 0);
+  const int from = found ? __ffs(found) - 1 : 0;
+  r.bin = __shfl_sync(0xffffffffu, bin, from);
+  r.cum = static_cast<double>(__shfl_sync(0xffffffffu, cum, from));
+  r.in = static_cast<double>(__shfl_sync(0xffffffffu, c, from));
+  return r;
+}
+
+// Quantile q of a log2 value histogram (log-linear inside the bin); whole warp.
+__device__ double histogram_quantile(const unsigned* h, int bins, double q, double log2min, double per_octave) {
+  const QuantileBin r = warp_quantile_bin(h, bins, q);
+  if (r.total == 0.0) return 0.0;
+  if (r.bin < 0) return exp2(log2min + bins / per_octave);
+  return exp2(log2min + (r.bin + (r.want - r.cum) / r.in) / per_octave);
+}
+
+// 1.4826 * median |r| from the job's histogram (log-linear inside the bin); whole warp.
+__device__ double histogram_sigma(const unsigned* h) {
+  const QuantileBin r = warp_quantile_bin(h, kGnBins, 0.5);
+  if (r.total == 0.0) return 0.0;
+  if (r.bin < 0) return 1.4826 * exp2(kGnLog2Min + kGnBins / kGnBinsPerOctave);
+  const double f = (r.want - r.cum) / r.in;
+  const double l = kGnLog2Min + (r.bin + f) / kGnBinsPerOctave;
+  return 1.4826 * exp2(l);
 }
 
 // Columns of the model projection P (8 x k): the parameters the solve
@@ -374,33 +405,34 @@ __global__ void gn_solve_kernel(GnArgs a, int mode, int model, double min_sample
   if (mode != 2 && st.status != 0) return;
   for (int q = lane; q < kGnUsed; q += 32) {
     double t = 0.0;
+#pragma unroll 8
     for (int b = 0; b < a.blocks_per_job; ++b)
       t += a.partials[(static_cast<int64_t>(job) * a.blocks_per_job + b) * kGnSums + q];
     s[q] = t;
   }
   __syncwarp();
   unsigned* hist = a.hist + static_cast<int64_t>(job) * kGnHistWords;
-  double robust_sigma = 0.0;
-  if (lane == 0) robust_sigma = histogram_sigma(hist);
+  const double robust_sigma = histogram_sigma(hist);
   __syncwarp();
   for (int b = lane; b < kGnBins; b += 32) hist[b] = 0u;  // ready for the next pass
   if (mode == 3 || mode == 4) {  // photometric start
     unsigned* vh = hist + kGnBins;
-    if (lane == 0 && mode == 3) {
+    if (mode == 3) {
       const double ma = histogram_quantile(vh, kGnVBins, 0.5, kGnVLog2Min, kGnVBinsPerOctave);
       const double la = histogram_quantile(vh, kGnVBins, kGnNoiseQuantile, kGnVLog2Min, kGnVBinsPerOctave);
       const double mo = histogram_quantile(vh + kGnVBins, kGnVBins, 0.5, kGnVLog2Min, kGnVBinsPerOctave);
       const double lo = histogram_quantile(vh + kGnVBins, kGnVBins, kGnNoiseQuantile, kGnVLog2Min, kGnVBinsPerOctave);
-      st.med_ref = ma;
-      st.med_mov = mo;
-      // +inf (no ratio samples, alpha stays) when a frame has no spread
-      st.thr_ref = ma > la ? kGnBrightSigmas * (ma - la) : HUGE_VAL;
-      st.thr_mov = mo > lo ? kGnBrightSigmas * (mo - lo) : HUGE_VAL;
-    } else if (lane == 0) {
-      unsigned long long n = 0;
-      for (int b = 0; b < kGnRBins; ++b) n += vh[b];
-      if (n >= 16) {
-        const double alpha = histogram_quantile(vh, kGnRBins, 0.5, kGnRLog2Min, kGnRBinsPerOctave);
+      if (lane == 0) {
+        st.med_ref = ma;
+        st.med_mov = mo;
+        // +inf (no ratio samples, alpha stays) when a frame has no spread
+        st.thr_ref = ma > la ? kGnBrightSigmas * (ma - la) : HUGE_VAL;
+        st.thr_mov = mo > lo ? kGnBrightSigmas * (mo - lo) : HUGE_VAL;
+      }
+    } else {
+      const QuantileBin all = warp_quantile_bin(vh, kGnRBins, 0.5);
+      const double alpha = histogram_quantile(vh, kGnRBins, 0.5, kGnRLog2Min, kGnRBinsPerOctave);
+      if (lane == 0 && all.total >= 16.0) {
         st.alpha = alpha;
         st.beta = st.med_mov - alpha * st.med_ref;
       }
