@@ -1310,9 +1310,38 @@ static void validate_integrate(const gg_integrate_params_t& p) {
 
 static IntegrateArgs integrate_args(gg_stack* s, const float* d_weights, const gg_integrate_params_t& p);
 
-static void launch_integrate_args(const IntegrateArgs& a, cudaStream_t stream) {
+// Up to 32 frames and this many samples the column kernel samples the frames
+// itself: three launches, where a band takes four or five.  Measured, column
+// against band, microseconds per call: Lanczos3 8 x 128^2 37 / 59, 8 x 256^2
+// 56 / 58, 16 x 256^2 81 / 83, 32 x 256^2 130 / 130, 8 x 512^2 124 / 87,
+// 32 x 512^2 371 / 250; bilinear 8 x 256^2 38 / 52, 8 x 512^2 75 / 69,
+// 16 x 512^2 107 / 107, 32 x 512^2 169 / 198, 32 x 1024^2 699 / 511.
+constexpr int64_t kFusedColumnSamplesLanczos = int64_t(1) << 20;
+constexpr int64_t kFusedColumnSamplesBilinear = int64_t(1) << 22;
+
+// Up to 32 frames: the column kernel (the samples in registers, a thread per
+// pixel) or the tiles of integrate_px.cu, which sum in fewer operations but
+// take their samples through shared memory.  Measured, column against tiles,
+// us for 2048^2 pixels: winsorized 8 frames 210 / 193, 12 347 / 240, 16 376 /
+// 253, 20 753 / 317, 32 809 / 395; sigma clip 12 193 / 224, 16 220 / 229,
+// 20 534 / 307, 32 563 / 362; mean 16 87 / 109, 32 162 / 173.  The tiles win in
+// the same places down to 512^2 (32 frames, winsorized: 58 / 35), but stacks in
+// which the fused warp samples through the column kernel keep it, so that
+// both forms of the integration agree to the last bit.
+constexpr int64_t kColumnSamples = kFusedColumnSamplesBilinear;
+
+static bool small_stack_takes_tiles(const IntegrateArgs& a, int64_t frame_pixels) {
+  if (frame_pixels * a.frames <= kColumnSamples) return false;
+  return (a.rejection == GG_REJECT_WINSORIZED && a.frames > 8) ||
+         (a.rejection == GG_REJECT_SIGMA_CLIP && a.frames > 16);
+}
+
+// `frame_pixels`: of the whole frame, where `a` is a band of it.
+static void launch_integrate_args(const IntegrateArgs& a, int64_t frame_pixels, cudaStream_t stream) {
   const int n = a.frames;
-  if (n <= 32) {
+  if (n <= 32 && small_stack_takes_tiles(a, frame_pixels)) {
+    launch_integrate_px(a, stream);
+  } else if (n <= 32) {
     switch (a.rejection) {
       case GG_REJECT_NONE:
         n <= 8 ? launch_col<8, GG_REJECT_NONE>(a, stream)
@@ -1350,7 +1379,7 @@ static void launch_integrate_args(const IntegrateArgs& a, cudaStream_t stream) {
 }
 
 void launch_integrate(gg_stack* s, const float* d_weights, const gg_integrate_params_t& p) {
-  launch_integrate_args(integrate_args(s, d_weights, p), s->stream);
+  launch_integrate_args(integrate_args(s, d_weights, p), s->pixels, s->stream);
   s->last_count_dtype = p.count_dtype;
 }
 
@@ -1589,20 +1618,11 @@ static void launch_band_sequence(gg_stack* s, const FusedFrame* d_frames, int in
     b.high = static_cast<char*>(b.high) + p0 * count_bytes;
     if (b.dq) b.dq += p0;
     b.geometric = s->d_fused_geometric + p0;
-    launch_integrate_args(b, s->stream);
+    launch_integrate_args(b, s->pixels, s->stream);
   }
   s->last_count_dtype = p.count_dtype;
   s->has_fused_geometric = true;
 }
-
-// Up to 32 frames and this many samples the column kernel samples the frames
-// itself: three launches, where a band takes four or five.  Measured, column
-// against band, microseconds per call: Lanczos3 8 x 128^2 37 / 59, 8 x 256^2
-// 56 / 58, 16 x 256^2 81 / 83, 32 x 256^2 130 / 130, 8 x 512^2 124 / 87,
-// 32 x 512^2 371 / 250; bilinear 8 x 256^2 38 / 52, 8 x 512^2 75 / 69,
-// 16 x 512^2 107 / 107, 32 x 512^2 169 / 198, 32 x 1024^2 699 / 511.
-constexpr int64_t kFusedColumnSamplesLanczos = int64_t(1) << 20;
-constexpr int64_t kFusedColumnSamplesBilinear = int64_t(1) << 22;
 
 // The device part of the fused warp-integration: every argument already on
 // the device, nothing but kernel launches on the stack's stream (so it can

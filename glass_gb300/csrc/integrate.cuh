@@ -143,7 +143,7 @@ __device__ __forceinline__ int count_below(const float* S, int T, int cnt, float
   return lo;
 }
 
-// Integration of 33 to 256 resident frames, one thread per pixel
+// Integration of up to 256 resident frames, one thread per pixel
 // (integrate_px.cu): mean, sigma clip and winsorized sigma clip.
 void launch_integrate_px(const IntegrateArgs& args, cudaStream_t stream);
 
