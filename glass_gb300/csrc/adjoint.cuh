@@ -193,7 +193,7 @@ __device__ __forceinline__ void lanczos3_weights_grad_poly(float t, float (&w)[6
 // weights cancel (|D| <= 1e-12).
 // UNROLL = true issues all 36 tap loads of the window at once (more loads in
 // flight, more registers); false walks it row by row.
-template <bool UNROLL = false>
+template <bool UNROLL = false, bool PROBE = false>
 __device__ __forceinline__ bool lanczos3_value_grad(const float* src, int W, int x0, int y0, float tx, float ty,
                                                     float& O, float& Ox, float& Oy) {
   float wx[6], wy[6], dwx[6], dwy[6];
@@ -216,13 +216,20 @@ __device__ __forceinline__ bool lanczos3_value_grad(const float* src, int W, int
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       const float v = __ldg(row + i);
-      finite = finite && isfinite(v);
+      if constexpr (!PROBE) finite = finite && isfinite(v);
       r = __fmaf_rn(wx[i], v, r);
       rx = __fmaf_rn(dwx[i], v, rx);
     }
     N = __fmaf_rn(wy[j], r, N);
     Nx = __fmaf_rn(wy[j], rx, Nx);
     Ny = __fmaf_rn(dwy[j], r, Ny);
+  }
+  // a tap that is not finite leaves N infinite or NaN whatever its weight
+  // (0 * inf is NaN); with PROBE the taps are looked at only where finite ones
+  // may have overflowed
+  if (PROBE && !isfinite(N)) {
+#pragma unroll 1
+    for (int q = 0; q < 36; ++q) finite = finite && isfinite(__ldg(src + static_cast<int64_t>(y0 - 2 + q / 6) * W + (x0 - 2 + q % 6)));
   }
   // all taps finite: D = (sum wx)(sum wy), D_x = (sum wx')(sum wy), D_y = (sum wx)(sum wy')
   const float D = sx * sy;

@@ -176,7 +176,7 @@ __device__ __forceinline__ void gn_sample(const GnArgs& a, const AffineCoef& coe
   if constexpr (INTERP == GG_INTERP_BILINEAR)
     ok = bilinear_value_grad(mov, W, H, x0, y0, tx, ty, O, Ox, Oy);
   else
-    ok = lanczos3_value_grad<UNROLL>(mov, W, x0, y0, tx, ty, O, Ox, Oy);
+    ok = lanczos3_value_grad<UNROLL, K == 0>(mov, W, x0, y0, tx, ty, O, Ox, Oy);
   if (!ok) return;
   if constexpr (K == 0) {
     if (a.phase == 1) {
@@ -233,11 +233,13 @@ __device__ __forceinline__ void gn_sample(const GnArgs& a, const AffineCoef& coe
   }
 }
 
-// Three CTAs per SM for the statistics and projected passes (at most a few
-// bytes of spills); the 46 accumulators of the full pass keep the compiler's
-// register count.
+// Three CTAs per SM for the projected passes (at most a few bytes of spills),
+// four for the statistics pass (three accumulators; 31 jobs x 262,144 samples:
+// 277 us at three, 229 us at four and with the probe instead of a test per tap,
+// which in the projected passes costs registers and 4 % instead); the 46
+// accumulators of the full pass keep the compiler's register count.
 template <int INTERP, int K, bool UNROLL>
-__global__ void __launch_bounds__(kGnThreads, K == 8 ? 1 : 3) gn_accumulate_kernel(GnArgs a) {
+__global__ void __launch_bounds__(kGnThreads, K == 8 ? 1 : K == 0 ? 4 : 3) gn_accumulate_kernel(GnArgs a) {
   using L = GnLayout<K>;
   __shared__ AffineCoef s_coef;
   __shared__ float s_phot[3];
