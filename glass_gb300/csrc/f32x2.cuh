@@ -80,4 +80,29 @@ struct FF2 {
   }
 };
 
+// Float-float sums of two sequences and of their squares: FF::add and
+// FF::add_prod in packed instructions, each rounded alike.  Zeros change
+// nothing.
+struct F2Moments {
+  FF2 first;
+  F2 hi, lo;  // of the squares
+  __device__ __forceinline__ void add(F2 x) {
+    first.add(x);
+    const F2 np = f2_mul(x, f2_mul(x, f2(-1.0f)));  // -(x * x)
+    const F2 pe = f2_fma(x, x, np);                 // its rounding error
+    const F2 s = f2_sub(hi, np);
+    const F2 b = f2_sub(s, hi);
+    const F2 e = f2_sub(f2_sub(hi, f2_sub(s, b)), f2_add(np, b));
+    hi = s;
+    lo = f2_add(f2_add(lo, e), pe);
+  }
+  // (sum, sum of squares) of the two sequences
+  __device__ __forceinline__ void split(FF& s1, FF& s2, FF& t1, FF& t2) const {
+    f2_split(first.hi, s1.hi, t1.hi);
+    f2_split(first.lo, s1.lo, t1.lo);
+    f2_split(hi, s2.hi, t2.hi);
+    f2_split(lo, s2.lo, t2.lo);
+  }
+};
+
 }  // namespace gg

@@ -49,25 +49,6 @@ struct LnArgs {
   double eps;
 };
 
-// Sums of a source and a reference pixel (the two lanes) and of their squares,
-// float-float: FF::add and FF::add_prod in packed instructions, each rounded
-// alike; a pair that does not count adds zeros.
-struct LnSums {
-  FF2 first;
-  F2 hi, lo;  // of the squares
-  __device__ __forceinline__ void add(F2 x) {
-    first.add(x);
-    const F2 minus = f2_mul(x, f2(-1.0f));
-    const F2 np = f2_mul(x, minus);        // -(x * x)
-    const F2 pe = f2_fma(x, x, np);        // its rounding error
-    const F2 s = f2_sub(hi, np);
-    const F2 b = f2_sub(s, hi);
-    const F2 e = f2_sub(f2_sub(hi, f2_sub(s, b)), f2_add(np, b));
-    hi = s;
-    lo = f2_add(f2_add(lo, e), pe);
-  }
-};
-
 // Bound by the packed arithmetic (17 instructions per pixel pair), then memory:
 // 31 pairs of 2048^2 in 324 us, 452 us in scalar instructions with a division
 // and a remainder per pixel.
@@ -82,7 +63,7 @@ __global__ void __launch_bounds__(kLnThreads) ln_pair_stats_kernel(LnArgs a) {
   const int w = min(a.tile_w, a.width - x0), h = min(a.tile_h, a.height - y0);
   const float* src = a.slots + static_cast<int64_t>(a.slot_of_frame[a.frames[pair]]) * a.stride;
   const float* ref = a.slots + static_cast<int64_t>(a.slot_of_frame[a.ref_frame]) * a.stride;
-  LnSums sums;
+  F2Moments sums;  // lanes: source, reference; a pair that does not count adds zeros
   unsigned n = 0;
   const int npx = w * h;
   // pixels threadIdx.x, + kLnThreads, ...: the position follows by addition
@@ -113,10 +94,7 @@ __global__ void __launch_bounds__(kLnThreads) ln_pair_stats_kernel(LnArgs a) {
     }
   }
   FF s1, s2, r1, r2;
-  f2_split(sums.first.hi, s1.hi, r1.hi);
-  f2_split(sums.first.lo, s1.lo, r1.lo);
-  f2_split(sums.hi, s2.hi, r2.hi);
-  f2_split(sums.lo, s2.lo, r2.lo);
+  sums.split(s1, s2, r1, r2);
   double v[4] = {static_cast<double>(s1.hi) + static_cast<double>(s1.lo),
                  static_cast<double>(s2.hi) + static_cast<double>(s2.lo),
                  static_cast<double>(r1.hi) + static_cast<double>(r1.lo),
