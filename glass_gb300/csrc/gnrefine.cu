@@ -233,13 +233,14 @@ __device__ __forceinline__ void gn_sample(const GnArgs& a, const AffineCoef& coe
   }
 }
 
-// Three CTAs per SM for the projected passes (at most a few bytes of spills),
-// four for the statistics pass (three accumulators; 31 jobs x 262,144 samples:
-// 277 us at three, 229 us at four and with the probe instead of a test per tap,
-// which in the projected passes costs registers and 4 % instead); the 46
-// accumulators of the full pass keep the compiler's register count.
+// Four CTAs per SM: the statistics pass fits in 64 registers, the projected
+// passes spill up to 300 bytes and still gain (31 jobs of 30 CTAs are 1.5 waves
+// instead of 2.04: similarity columns over 31 x 2^20 samples 645 -> 530 us,
+// statistics 277 -> 228 us with the probe instead of a test per tap, which in
+// the projected passes costs more registers than it saves).  The 46 accumulators
+// of the full pass keep the compiler's register count.
 template <int INTERP, int K, bool UNROLL>
-__global__ void __launch_bounds__(kGnThreads, K == 8 ? 1 : K == 0 ? 4 : 3) gn_accumulate_kernel(GnArgs a) {
+__global__ void __launch_bounds__(kGnThreads, K == 8 ? 1 : 4) gn_accumulate_kernel(GnArgs a) {
   using L = GnLayout<K>;
   __shared__ AffineCoef s_coef;
   __shared__ float s_phot[3];
