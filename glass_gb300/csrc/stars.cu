@@ -741,7 +741,7 @@ struct DetectArgs {
 // are appended in column order with one atomic and noted in the chunk table,
 // so the raster order of the whole frame is a prefix sum over the table
 // (star_order_kernel) and needs no sort.  Bound by issue slots (69 %), then
-// the loads: 8 frames of 4096^2 in 134 us, 194 us with scalar loads.  MESH: per-pixel threshold from the
+// the loads: 8 frames of 4096^2 in 121 us, 194 us with scalar loads.  MESH: per-pixel threshold from the
 // background mesh (float64), else the frame's float32 threshold.
 constexpr int kChunk = 512;
 
@@ -756,9 +756,15 @@ __global__ void __launch_bounds__(256) star_detect_kernel(DetectArgs a) {
   const int lane = threadIdx.x & 31;
   const unsigned warps = gridDim.x * (blockDim.x >> 5);
   float4 next[4];
-  auto load = [&](unsigned e) {
-    const int64_t row_at = static_cast<int64_t>(1 + e / a.chunks_per_row) * W;
-    const int x0 = static_cast<int>(e % a.chunks_per_row) * kChunk - static_cast<int>(row_at & 3) + 4 * lane;
+  // row and chunk of the row of the vectors in `next`, advanced without a division
+  unsigned e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  int next_y = 1 + static_cast<int>(e / a.chunks_per_row);
+  unsigned next_c = e % a.chunks_per_row;
+  const int step_y = static_cast<int>(warps / a.chunks_per_row);
+  const unsigned step_c = warps % a.chunks_per_row;
+  auto load = [&]() {
+    const int64_t row_at = static_cast<int64_t>(next_y) * W;
+    const int x0 = static_cast<int>(next_c) * kChunk - static_cast<int>(row_at & 3) + 4 * lane;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       // rows 1 .. H - 2: a vector that starts before the row or ends behind it stays inside the frame
@@ -767,16 +773,20 @@ __global__ void __launch_bounds__(256) star_detect_kernel(DetectArgs a) {
           x <= W - 2 ? __ldg(reinterpret_cast<const float4*>(img + row_at + x)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   };
-  unsigned e = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (e < a.chunk_count) load(e);
+  if (e < a.chunk_count) load();
   for (; e < a.chunk_count; e += warps) {
-    const int y = 1 + static_cast<int>(e / a.chunks_per_row);
+    const int y = next_y;
     const int64_t row_at = static_cast<int64_t>(y) * W;
     const float* row = img + row_at;
-    const int x0 =
-        static_cast<int>(e % a.chunks_per_row) * kChunk - static_cast<int>(row_at & 3) + 4 * lane;  // lane's first column
+    const int x0 = static_cast<int>(next_c) * kChunk - static_cast<int>(row_at & 3) + 4 * lane;  // lane's first column
     const float4 q[4] = {next[0], next[1], next[2], next[3]};
-    if (e + warps < a.chunk_count) load(e + warps);  // in flight while this chunk's candidates are tested
+    next_y += step_y;
+    next_c += step_c;
+    if (next_c >= a.chunks_per_row) {
+      next_c -= a.chunks_per_row;
+      ++next_y;
+    }
+    if (e + warps < a.chunk_count) load();  // in flight while this chunk's candidates are tested
     // threshold first: most chunks hold no candidate
     if constexpr (!MESH) {
       float top = -CUDART_INF_F;  // NaN drops out
