@@ -210,7 +210,7 @@ int gg_stack_compute_weights(gg_stack* s, int mode, const float* host_prior, flo
   // eight CTAs per SM over all frames (two per SM and frame, 9728 CTAs for
   // 32 x 2048^2, spent as long on their reductions and tickets as on the 13
   // vectors of a thread), at least two vectors per thread
-  const int64_t fill = (int64_t{8} * sm_count() + count - 1) / count;
+  const int64_t fill = int64_t{8} * sm_count() / count;  // rounded down: no CTAs in a wave of their own
   const int blocks = static_cast<int>(std::max<int64_t>(
       1, std::min<int64_t>(std::min<int64_t>(fill, sm_count() * 2), (s->pixels + 2047) / 2048)));
   const size_t partial_doubles = static_cast<size_t>(count) * blocks * 3;
