@@ -134,7 +134,7 @@ __device__ __forceinline__ void add_theta(float (&acc)[6], float gsx, float gsy,
 // takes the place of 36 per output pixel.  Any other step writes all six rows.
 // Bound: latency at 12 warps per SM (168 registers), then issue (706
 // instructions per pixel: 166 for the weights and their derivatives, 126 for the
-// taps, 80 for the cells).  4096^2: 619 us, 1102 us with an atomic per tap.
+// taps, 80 for the cells).  4096^2: 658 us, 1102 us with an atomic per tap.
 constexpr int kScatterThreads = 128;
 
 // Adds the cells of source row R, columns C .. C + 5 of every lane.
@@ -270,12 +270,16 @@ __global__ void __launch_bounds__(kScatterThreads) lanczos3_scatter_kernel(Adjoi
       // the other lanes read the image's first window (a live lane proves that
       // the image holds one)
       const float* at = a.src + (live ? static_cast<int64_t>(y0 - 2) * W + (x0 - 2) : 0);
+      // taps relative to the middle one: the derivatives are the same, (Nx - O
+      // dsx swy) / D for taps v + c equals that for v, without the rounding
+      // that a background of many times its noise leaves in Nx
+      const float middle = __ldg(at + 2 * static_cast<int64_t>(W) + 2);
 #pragma unroll
       for (int j = 0; j < 6; ++j, at += W) {
         float rv = 0.0f, rd = 0.0f;
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
-          const float v = __ldg(at + i);
+          const float v = __fsub_rn(__ldg(at + i), middle);
           rv = __fmaf_rn(wx[i], v, rv);
           rd = __fmaf_rn(dwx[i], v, rd);
         }

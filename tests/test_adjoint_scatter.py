@@ -59,3 +59,24 @@ def test_image_and_parameter_gradients(native, name, h, w):
     # times the incoming gradient and the coordinate
     limit = 1e-4 * np.abs(grad).sum() * np.array([w, h, 1, w, h, 1])
     assert np.all(np.abs((got_t - want_t).numpy()) <= limit)
+
+
+def test_parameter_gradient_over_a_background(native):
+    """A background of 3000 times its noise adds nothing to the derivatives; the
+    terms of the sum keep their own rounding (a few 2^-24 each of up to twice the
+    noise) and the sum of 6000 of them cancels to some tenth of its root."""
+    from glass_gb300.adjoint import warp_affine
+
+    h, w = 64, 96
+    rng = np.random.default_rng(17)
+    image = (30000.0 + 10.0 * rng.standard_normal((h, w))).astype(np.float32)
+    grad = rng.standard_normal((h, w)).astype(np.float32)
+    theta = np.array(_maps(h, w)["small"], dtype=np.float64)
+    src = torch.from_numpy(image).cuda().requires_grad_()  # both gradients: the scatter kernel's sums
+    t = torch.from_numpy(theta).requires_grad_()
+    out = warp_affine(src, t, "lanczos3", 0.0)
+    _, got = torch.autograd.grad(out, (src, t), torch.from_numpy(grad).cuda())
+    t64 = torch.from_numpy(theta).requires_grad_()
+    out64 = warp_affine_reference(torch.from_numpy(image.astype(np.float64)), t64, "lanczos3", 0.0)
+    (want,) = torch.autograd.grad(out64, (t64,), torch.from_numpy(grad.astype(np.float64)))
+    assert ((got - want).norm() / want.norm()).item() <= 1e-5
