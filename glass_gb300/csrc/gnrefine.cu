@@ -235,7 +235,7 @@ __device__ __forceinline__ void gn_sample(const GnArgs& a, const AffineCoef& coe
 
 // Four CTAs per SM: the statistics pass fits in 64 registers, the projected
 // passes spill up to 300 bytes and still gain (31 jobs of 30 CTAs are 1.5 waves
-// instead of 2.04: similarity columns over 31 x 2^20 samples 645 -> 530 us,
+// instead of 2.04: similarity columns over 31 x 2^20 samples 646 -> 490 us,
 // statistics 277 -> 228 us with the probe instead of a test per tap, which in
 // the projected passes costs more registers than it saves).  The 46 accumulators
 // of the full pass keep the compiler's register count.
