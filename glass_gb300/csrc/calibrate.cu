@@ -225,19 +225,25 @@ static CalibArgs make_args(gg_stack* s, const gg_calib_params_t& p) {
   return a;
 }
 
+// A launch deals the last pixels of its frames to threads in no order and
+// publishes one non-finite count per frame, so its frames are distinct: a frame
+// that comes again starts another launch, and its last entry wins.
 void launch_calibrate(gg_stack* s, const CalibLaunch& job, const gg_calib_params_t& p) {
   CalibArgs a = make_args(s, p);
-  a.raw = job.raw;
   a.light_f32 = job.light_f32;
   a.big_endian_bzero = job.big_endian_bzero;
-  a.nframes = job.nframes;
-  for (int i = 0; i < job.nframes; ++i) a.frame[i] = job.frame[i];
-  note_launch();
-  if (job.raw != nullptr)
-    calibrate_u16_kernel<<<grid_for(static_cast<size_t>((s->pixels + 7) / 8), 256, 8), 256, 0, s->stream>>>(a);
-  else
-    calibrate_f32_kernel<<<grid_for(static_cast<size_t>(s->pixels), 256, 8), 256, 0, s->stream>>>(a);
-  check_cuda(cudaGetLastError(), "calibrate kernel launch");
+  for (int k = 0; k < job.nframes;) {
+    if (job.raw != nullptr) a.raw = job.raw + static_cast<int64_t>(k) * s->pixels;
+    a.nframes = 0;
+    while (k < job.nframes && std::find(a.frame, a.frame + a.nframes, job.frame[k]) == a.frame + a.nframes)
+      a.frame[a.nframes++] = job.frame[k++];
+    note_launch();
+    if (job.raw != nullptr)
+      calibrate_u16_kernel<<<grid_for(static_cast<size_t>((s->pixels + 7) / 8), 256, 8), 256, 0, s->stream>>>(a);
+    else
+      calibrate_f32_kernel<<<grid_for(static_cast<size_t>(s->pixels), 256, 8), 256, 0, s->stream>>>(a);
+    check_cuda(cudaGetLastError(), "calibrate kernel launch");
+  }
 }
 
 void launch_count_nonfinite(gg_stack* s, int64_t frame) {
@@ -379,12 +385,7 @@ int gg_stack_calibrate_u16_device(gg_stack* s, const int64_t* indices, int64_t c
     CalibLaunch job{};
     job.raw = raw + static_cast<size_t>(k0) * static_cast<size_t>(s->pixels);
     job.big_endian_bzero = big_endian_bzero;
-    // a frame that comes again starts another launch
-    auto repeated = [&](int64_t k) {
-      return std::find(job.frame, job.frame + job.nframes, static_cast<int>(indices[k])) != job.frame + job.nframes;
-    };
-    while (k0 < count && job.nframes < GG_MAX_BATCH_FRAMES && !repeated(k0))
-      job.frame[job.nframes++] = static_cast<int>(indices[k0++]);
+    while (k0 < count && job.nframes < GG_MAX_BATCH_FRAMES) job.frame[job.nframes++] = static_cast<int>(indices[k0++]);
     launch_calibrate(s, job, *params);
   }
   for (int64_t k = 0; k < count; ++k) stack_mark_loaded(s, indices[k]);
