@@ -45,7 +45,8 @@ struct PxTable {
   float4 w[NB * L / 2];        // weights of a row pair: high parts, low parts
   const float* base[NB * L];   // frames with a valid weight, in order
   float total[2];              // sum of the weights
-  float unit;                  // rounds a weight to its high part
+  float unit;                  // rounds a weight to its high part (0: no split)
+  int narrow;                  // the parts' sums are exact (narrow_weights)
   int active;
   int allvalid;
 };
@@ -71,6 +72,19 @@ __device__ __forceinline__ Split split_range(float least, float most, float m) {
   r.round = __int_as_float(__float_as_int(range) & 0x7f800000) * 98304.0f;
   r.ok = least > most || (range <= low && (least > 0.0f) == (most > 0.0f));
   return r;
+}
+
+// Weights are split in two parts as well: w = wh + wl, wh a multiple of q with
+// |wh| <= 2^9 q, |wl| <= q / 2.  A thread's sums over `pairs` row pairs of wh
+// and of wh dh (2^17 units each) are exact in float32; those of wl are where the
+// least weight's last place is at least pairs x q / 2^25.  Then the weight of a
+// pixel is the frames' total minus the weights that do not count, exactly,
+// whatever little is left of it.  Weights further apart (a ratio of 8 for 256
+// frames, of 32 for 64), or at the ends of the float32 range, are not split: the
+// weights that do count are added up in float-float.
+__device__ __forceinline__ bool narrow_weights(float least, float most, int pairs) {
+  const int low = max(__float_as_int(least) >> 23, 1), high = __float_as_int(most) >> 23;  // biased exponents
+  return high >= 32 && high <= 127 + 110 && high - low <= 10 && (pairs << (high - low)) <= 1024;
 }
 
 __device__ __forceinline__ void split(F2 d, F2 round, F2& dh, F2& dl) {
@@ -247,7 +261,7 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
   if (warp == 0) {
     int rows = 0;
     unsigned bad = 0, invalid = 0;
-    float most = 0.0f;
+    float least = kInf, most = 0.0f;
     FF total;
     for (int f0 = 0; f0 < a.frames; f0 += 32) {
       const int f = f0 + lane;
@@ -258,6 +272,7 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
         invalid |= ok ? 0u : 1u;
       }
       if (ok) {
+        least = fminf(least, w);
         most = fmaxf(most, w);
         total.add(w);
       }
@@ -270,6 +285,7 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
     invalid = __reduce_or_sync(0xffffffffu, invalid);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
+      least = fminf(least, __shfl_xor_sync(0xffffffffu, least, off));
       most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, off));
       FF o;
       o.hi = __shfl_xor_sync(0xffffffffu, total.hi, off);
@@ -279,7 +295,8 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
     if (lane == 0) {
       tab.total[0] = total.hi;
       tab.total[1] = total.lo;
-      tab.unit = split_range(0.0f, most, 0.0f).round;
+      tab.narrow = narrow_weights(least, most, (rows + 1) / 2) ? 1 : 0;
+      tab.unit = tab.narrow ? 0.5f * split_range(0.0f, most, 0.0f).round : 0.0f;
       tab.active = rows;
       tab.allvalid = (bad == 0u && invalid == 0u) ? 1 : 0;
     }
@@ -310,7 +327,7 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
     }
   }
   __syncthreads();
-  const bool allvalid = tab.allvalid != 0;
+  const bool allvalid = tab.allvalid != 0, narrow = tab.narrow != 0;
   const int pairs = L == 2 ? na : (na + 1) / 2;
   const int64_t P = a.pixels;
   const int64_t tiles = (P + 31) / 32;
@@ -474,12 +491,14 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
       kept_split = split_range(fmaxf(least, lt), fminf(most, ht), pivot);
     }
     // weighted sum over the kept samples, two rows at a time: pivot plus
-    // split deviations by split weights where the kept samples allow it
-    const bool plain = __all_sync(0xffffffffu, kept_split.ok);
+    // split deviations by split weights where the kept samples and the weights
+    // allow it
+    const bool plain = narrow && __all_sync(0xffffffffu, kept_split.ok);
     const F2 m = f2(pivot), round = f2(kept_split.round);
     FF2 ws;
     F2 hh, hl, lh;
-    F2 gone_h, gone_l;  // weights of the samples that do not count
+    F2 gone_h, gone_l;  // weights of the samples that do not count (narrow)
+    FF2 counted;        // weights of those that do (else)
     int n2 = 0;
     const int64_t next = t + stride;
     for (int c = 0; c < kChunks; ++c) {
@@ -489,25 +508,34 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
       __syncwarp();
       const float* col = tile + lane + c * kPxChunk * (L == 2 ? 32 : 64);
       const float4* tw = tab.w + c * kPxChunk;
-      auto row_pair = [&](int k, F2& v, F2& wh, F2& wl) {
+      auto row_pair = [&](int k, F2& v, F2& wh, F2& wl, F2& drop) {
         const float x = col[(L == 2 ? k : 2 * k) * 32], y = col[(L == 2 ? NB + k : 2 * k + 1) * 32];
         const float4 w = tw[k];
         const bool kx = x >= lt && x <= ht, ky = y >= lt && y <= ht;
         v = f2(kx ? x : pivot, ky ? y : pivot);
         wh = f2(w.x, w.y);
         wl = f2(w.z, w.w);
-        const F2 drop = f2(kx ? 0.0f : 1.0f, ky ? 0.0f : 1.0f);
+        drop = f2(kx ? 0.0f : 1.0f, ky ? 0.0f : 1.0f);
         gone_h = f2_fma(drop, wh, gone_h);
         gone_l = f2_fma(drop, wl, gone_l);
         if (a.rejection == GG_REJECT_NONE) n2 += (kx ? 1 : 0) + (ky ? 1 : 0);
       };
       auto add_split = [&](int k) {
-        F2 v, wh, wl, dh, dl;
-        row_pair(k, v, wh, wl);
+        F2 v, wh, wl, drop, dh, dl;
+        row_pair(k, v, wh, wl, drop);
         split(f2_sub(v, m), round, dh, dl);
         hh = f2_fma(wh, dh, hh);
         hl = f2_fma(wh, dl, hl);
         lh = f2_fma(wl, dh, f2_fma(wl, dl, lh));
+      };
+      auto add_rounded = [&](int k, F2& w, F2& drop) {
+        F2 v, wh, wl, d, e;
+        row_pair(k, v, wh, wl, drop);
+        f2_two_sum(v, f2(-pivot), d, e);
+        w = f2_add(wh, wl);
+        const F2 prod = f2_mul(d, w);
+        ws.lo = f2_add(ws.lo, f2_fma(w, e, f2_fma(d, w, f2_sub(F2(), prod))));
+        ws.add(prod);
       };
       const int in_chunk = min(kPxChunk, pairs - c * kPxChunk);
       if (plain && in_chunk == kPxChunk) {
@@ -516,16 +544,18 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
       } else if (plain) {
 #pragma unroll 1
         for (int k = 0; k < in_chunk; ++k) add_split(k);
-      } else {
+      } else if (narrow) {
 #pragma unroll 2
         for (int k = 0; k < in_chunk; ++k) {
-          F2 v, wh, wl, d, e;
-          row_pair(k, v, wh, wl);
-          f2_two_sum(v, f2(-pivot), d, e);
-          const F2 w = f2_add(wh, wl);
-          const F2 prod = f2_mul(d, w);
-          ws.lo = f2_add(ws.lo, f2_fma(w, e, f2_fma(d, w, f2_sub(F2(), prod))));
-          ws.add(prod);
+          F2 w, drop;
+          add_rounded(k, w, drop);
+        }
+      } else {
+#pragma unroll 1
+        for (int k = 0; k < in_chunk; ++k) {
+          F2 w, drop;
+          add_rounded(k, w, drop);
+          counted.add(f2_fma(drop, f2_mul(w, f2(-1.0f)), w));
         }
       }
       __syncwarp();
@@ -542,11 +572,19 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
     } else {
       s = ws.merged();
     }
-    w.hi = tab.total[0];
-    w.lo = tab.total[1];
-    FF gone;
-    two_sum(-f2_sum(gone_h), -f2_sum(gone_l), gone.hi, gone.lo);
-    ff_merge2(w, gone);
+    if (narrow) {
+      w.hi = tab.total[0];
+      w.lo = tab.total[1];
+      float x, y, low, e;
+      f2_split(gone_l, x, y);
+      two_sum(x, y, low, e);
+      FF gone;
+      two_sum(-f2_sum(gone_h), -low, gone.hi, gone.lo);
+      gone.lo = __fsub_rn(gone.lo, e);
+      ff_merge2(w, gone);
+    } else {
+      w = counted.merged();
+    }
     float master = 0.0f, weight = 0.0f;
     if (kept > 0 && w.hi > 0.0f) {
       // pivot + s / w
