@@ -376,15 +376,19 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
         float v[NB];
 #pragma unroll
         for (int k = 0; k < NB; ++k) v[k] = col[k * 32];
-        // 0 * x is NaN for the samples that are not finite
+        // 0 * x is NaN for the samples that are not finite: of the n rows only, the
+        // others hold +inf
         F2 probe;
 #pragma unroll
-        for (int k = 0; k + 8 < NB; k += 2) probe = f2_fma(f2(v[k], v[k + 1]), F2(), probe);
+        for (int k = 0; k < NB; k += 8)
+          if (k + 8 <= n) {
+#pragma unroll
+            for (int q = k; q < k + 8; q += 2) probe = f2_fma(f2(v[q], v[q + 1]), F2(), probe);
+          }
         float p0, p1;
         f2_split(probe, p0, p1);
-#pragma unroll
-        for (int k = NB - 8; k < NB; ++k)
-          if (k < n) p0 = __fmaf_rn(v[k], 0.0f, p0);
+#pragma unroll 1
+        for (int k = n & ~7; k < n; ++k) p0 = __fmaf_rn(col[k * 32], 0.0f, p0);
         int valid = n;
         if (!__all_sync(0xffffffffu, p0 + p1 == 0.0f)) {
           valid = 0;
