@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
     // weighted sum over the kept samples, two rows at a time: pivot plus
     // split deviations by split weights where the kept samples and the weights
     // allow it
-    const bool plain = narrow && __all_sync(0xffffffffu, kept_split.ok);
+    const bool plain = __all_sync(0xffffffffu, narrow && kept_split.ok);
     const F2 m = f2(pivot), round = f2(kept_split.round);
     FF2 ws;
     F2 hh, hl, lh;
@@ -603,17 +603,25 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
   }
 }
 
-// Warps per CTA that keep the most warps on an SM.
+// Warps per CTA.  A CTA's warps take turns on the SM's four schedulers, so the
+// busiest one has ceil(w / 4) of each resident CTA; all warps have as many tiles,
+// and that scheduler's run last.  A warp slows down by about one over the
+// warps beside it, hence warps on the SM over 1 + warps on the busiest
+// scheduler.  (The most warps alone picked two CTAs of five for 160 frames: 4.4
+// ps per sample, 3.5 with one CTA of eight; 112 frames 4.0 and 3.3 with two of
+// seven and three of four.)
 template <int NB, int L>
 static int px_best_warps() {
   constexpr size_t kWarpBytes = size_t(NB) * L * 128;
   auto kern = integrate_px_kernel<NB, L>;
-  int most = 0, pick = 1;
+  double most = 0.0;
+  int pick = 1;
   for (int w = kPxMaxWarps; w >= 2; --w) {
     if (kWarpBytes * w + sizeof(PxTable<NB, L>) > 227 * 1024) continue;
     const int per_sm = kernel_ctas_per_sm(kern, 32 * w, kWarpBytes * w, "launch shape (integrate_px)");
-    if (per_sm * w > most) {
-      most = per_sm * w;
+    const double score = static_cast<double>(per_sm * w) / (1 + per_sm * ((w + 3) / 4));
+    if (score > most) {
+      most = score;
       pick = w;
     }
   }
@@ -636,23 +644,21 @@ static void launch_px(const IntegrateArgs& args, cudaStream_t stream) {
   check_cuda(cudaGetLastError(), "integrate_px launch");
 }
 
-// List lengths in steps of 8 to 16: a pixel sorts at most a few rows of
-// padding, and each length is one more unrolled network to compile.
+// One list up to 64 frames, two of half the frames above; list lengths in steps
+// of 8, so that a list sorts at most seven rows of padding (two lists: of a
+// frame more or less) whatever the count.  Each length is one more unrolled
+// network to compile.
+template <int L, int NB, int LAST>
+static void launch_px_list(const IntegrateArgs& a, cudaStream_t stream) {
+  if constexpr (NB < LAST) {
+    if (a.frames > NB * L) return launch_px_list<L, NB + 8, LAST>(a, stream);
+  }
+  launch_px<NB, L>(a, stream);
+}
+
 void launch_integrate_px(const IntegrateArgs& a, cudaStream_t stream) {
-  const int n = a.frames;
-  if (n <= 16) launch_px<16, 1>(a, stream);
-  else if (n <= 24) launch_px<24, 1>(a, stream);
-  else if (n <= 32) launch_px<32, 1>(a, stream);
-  else if (n <= 40) launch_px<40, 1>(a, stream);
-  else if (n <= 48) launch_px<48, 1>(a, stream);
-  else if (n <= 64) launch_px<64, 1>(a, stream);
-  else if (n <= 80) launch_px<40, 2>(a, stream);
-  else if (n <= 96) launch_px<48, 2>(a, stream);
-  else if (n <= 128) launch_px<64, 2>(a, stream);
-  else if (n <= 160) launch_px<80, 2>(a, stream);
-  else if (n <= 192) launch_px<96, 2>(a, stream);
-  else if (n <= 208) launch_px<104, 2>(a, stream);
-  else launch_px<128, 2>(a, stream);
+  if (a.frames <= 64) launch_px_list<1, 16, 64>(a, stream);
+  else launch_px_list<2, 40, 128>(a, stream);
 }
 
 }  // namespace gg
