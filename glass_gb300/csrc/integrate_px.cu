@@ -70,7 +70,7 @@ __device__ __forceinline__ Split split_range(float least, float most, float m) {
   Split r;
   // 1.5 * 2^23 q with q = 2^(exponent of the range - 7): the range is below 2^8 q
   r.round = __int_as_float(__float_as_int(range) & 0x7f800000) * 98304.0f;
-  r.ok = least > most || (range <= low && (least > 0.0f) == (most > 0.0f));
+  r.ok = least > most || (range <= low && (least > 0.0f) == (most > 0.0f) && r.round < kInf);
   return r;
 }
 
@@ -492,6 +492,9 @@ __global__ void __launch_bounds__(32 * kPxMaxWarps, NB <= 64 ? 2 : 1) integrate_
       // nothing rejected: every finite sample is kept, whatever the thresholds
       lt = nl + nh > 0 ? fmaxf(lt, -FLT_MAX) : -FLT_MAX;
       ht = nl + nh > 0 ? fminf(ht, FLT_MAX) : FLT_MAX;
+      // samples that span the float32 range have no finite difference from a
+      // median, nor always a median
+      if (!(fabsf(pivot) < kInf && __fsub_rn(most, least) < kInf)) pivot = 0.0f;
       kept_split = split_range(fmaxf(least, lt), fminf(most, ht), pivot);
     }
     // weighted sum over the kept samples, two rows at a time: pivot plus

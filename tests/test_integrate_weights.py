@@ -32,6 +32,7 @@ def _check(native, frames, weights, repeat=1, rejections=("winsorized_sigma", "s
         np.testing.assert_array_equal(cov, ec, err_msg=rej)
         np.testing.assert_array_equal(low, el, err_msg=rej)
         np.testing.assert_array_equal(high, eh, err_msg=rej)
+        assert np.isfinite(em).all() and np.isfinite(master).all() and np.isfinite(weight).all()
         assert_within_ulp(weight, ew, 1, rej + " weight")
         assert_within_ulp(master, em, 1, rej + " master")
     s.close()
