@@ -417,13 +417,6 @@ __device__ __forceinline__ unsigned count_nonfinite(F2 probe, const float* out, 
   return bad;
 }
 
-// __fdividef for a divisor that needs no scaling (near 1).
-__device__ __forceinline__ float quotient_near_one(float a, float b) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-  return __fmul_rn(a, r);
-}
-
 // Sums of both columns' 6 x 6 windows at na, nb.
 template <bool STAGED>
 __device__ __forceinline__ F2 window_sum(const Window<STAGED>& win, typename Window<STAGED>::Index na,
@@ -506,7 +499,7 @@ __device__ __forceinline__ unsigned lanczos3_rows(const TileGrid& grid, const Wi
       f2_split(acc[q], sa, sb);
       f2_split(wsum[q], da, db);
       // all taps count: the weights sum to 1 within a few per cent
-      const float va = quotient_near_one(sa, da), vb = quotient_near_one(sb, db);
+      const float va = __fdividef(sa, da), vb = __fdividef(sb, db);
       if constexpr (MASK) {
         // the walk has moved on by two rows
         const long long k = 2 - q;
