@@ -1784,18 +1784,12 @@ extern "C" int gg_stack_graph_capture_step(gg_stack* s, const void* dev_raw, con
 }
 
 // ---- several stacks in one graph ------------------------------------------------
-namespace gg {
-void* warp_items_device(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd);
-void launch_warp_items_device(gg_stack* s, void* d_items, int64_t count, int interp, float fill, float clamp);
-}  // namespace gg
-
 struct gg_stacks_graph {
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   cudaStream_t stream = nullptr;
   int device = 0;
-  std::vector<void*> items;       // per step: device warp descriptors (or null)
-  std::vector<int64_t> warped;    // per step: descriptor count
+  std::vector<gg::WarpBatch> warps;  // per step: the frames to warp (none: items is null)
   int kernels = 0;
 };
 
@@ -1805,15 +1799,15 @@ static void stacks_graph_free(gg_stacks_graph* g) {
   if (!g) return;
   if (g->exec) cudaGraphExecDestroy(g->exec);
   if (g->graph) cudaGraphDestroy(g->graph);
-  for (void* p : g->items)
-    if (p) cudaFree(p);
+  for (const WarpBatch& w : g->warps)
+    if (w.items) cudaFree(w.items);
   delete g;
 }
 
 // One stack's step on its (current) stream: decode + calibration of every
 // frame, frame weights, the warp of every frame whose matrix is not the
 // identity, rejection + integration with the device weights.
-static void run_stack_step(const gg_stack_step_t& st, void* d_items, int64_t warped) {
+static void run_stack_step(const gg_stack_step_t& st, const WarpBatch& warp) {
   gg_stack* s = st.stack;
   std::vector<int64_t> idx(static_cast<size_t>(s->frames));
   for (int64_t k = 0; k < s->frames; ++k) idx[static_cast<size_t>(k)] = k;
@@ -1821,7 +1815,7 @@ static void run_stack_step(const gg_stack_step_t& st, void* d_items, int64_t war
   if (rc != GG_OK) fail(rc, "stacks graph: calibration failed");
   rc = gg_stack_compute_weights(s, st.weighting, nullptr, 1.0e-6f, nullptr);
   if (rc != GG_OK) fail(rc, "stacks graph: frame weighting failed");
-  if (warped > 0) launch_warp_items_device(s, d_items, warped, st.interpolation, NAN, st.clamping_threshold);
+  if (warp.count > 0) launch_warp_batch(s, warp, NAN);
   launch_integrate(s, s->d_weights, st.integrate);
 }
 
@@ -1880,18 +1874,18 @@ extern "C" int gg_stacks_graph_capture(const gg_stack_step_t* steps, int32_t cou
     for (int64_t f = 0; f < st.stack->frames; ++f) all[static_cast<size_t>(f)] = f;
     const int rc = gg_stack_calibrate_u16_device(st.stack, all.data(), st.stack->frames, st.dev_raw, 0, &st.calib);
     if (rc != GG_OK) fail(rc, "stacks graph: calibration failed");
-    g->items.push_back(idx.empty() ? nullptr : warp_items_device(st.stack, idx.data(), static_cast<int64_t>(idx.size()),
-                                                                  mats.data()));
-    g->warped.push_back(static_cast<int64_t>(idx.size()));
+    g->warps.push_back(idx.empty() ? WarpBatch{} : warp_batch_device(st.stack, idx.data(),
+                                                                      static_cast<int64_t>(idx.size()), mats.data(),
+                                                                      st.interpolation, st.clamping_threshold));
   }
   // one eager pass sizes every lazily allocated buffer and settles the
   // autotuner, so the capture records launches and stream-ordered copies only
-  for (int k = 0; k < count; ++k) run_stack_step(steps[k], g->items[k], g->warped[k]);
+  for (int k = 0; k < count; ++k) run_stack_step(steps[k], g->warps[k]);
   check_cuda(cudaStreamSynchronize(g->stream), "cudaStreamSynchronize(stacks graph warm-up)");
   const int64_t before = gg::launch_count();
   check_cuda(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture");
   try {
-    for (int k = 0; k < count; ++k) run_stack_step(steps[k], g->items[k], g->warped[k]);
+    for (int k = 0; k < count; ++k) run_stack_step(steps[k], g->warps[k]);
   } catch (...) {
     cudaGraph_t broken = nullptr;
     cudaStreamEndCapture(g->stream, &broken);

@@ -52,7 +52,8 @@ namespace gg {
 
 constexpr int kTileW = 64;
 constexpr int kTileH = 64;       // rows of a tile
-constexpr int kSmallTileH = 16;  // where a launch has few tiles
+constexpr int kMidTileH = 48;    // where a footprint of 64 rows does not fit the box
+constexpr int kSmallTileH = 16;  // where one of 48 does not, or a launch has few tiles
 constexpr int kWarpThreads = 128;
 constexpr int kRowClasses = 4;  // rows y, y + 4, y + 8, ... of a tile share a chain of coordinates
 // Affine source coordinates are stepped by 4 output rows in float-float and
@@ -69,6 +70,7 @@ struct WarpItem {
   unsigned src_nonfinite;
   int affine;
   int int_shift;  // inverse is an exact integer translation
+  int form;       // WarpForm
   float* dst;     // first row of the output rows (filled on the device)
   float m[9][2];  // inverse matrix, float-float (hi, lo), row-major
   double inv[6];  // its first two rows
@@ -95,6 +97,25 @@ struct WarpArgs {
   int counted;      // whole tiles (counts_whole) are in it already
   int* error;
 };
+
+// How a launch takes its frames: staged boxes of tiles of 64, 48 or 16 rows, or
+// windows straight from global memory, by straight-line rows or by the general
+// path alone.
+//
+// Two boxes in each of four CTAs leave next to no L1, and a tile whose footprint
+// misses its box reads its windows through it.  So the launch's form goes by the
+// maps: the tallest tiles whose footprints fit (a shorter tile pays more for its
+// plan and its box), else no boxes, and then the general path without the
+// registers of the straight-line rows.  8 frames of 2048^2, us, boxes of 64 rows
+// whatever the map -> by form:
+//                        Lanczos3       Lanczos3, clamp  bilinear     nearest
+//   turned by  7 degrees  376 -> 290       704 -> 502     98 -> 100   218 -> 218
+//             20          986 -> 375      1026 -> 544    210 -> 163   329 -> 252
+//             45         2123 -> 380      1259 -> 524    307 -> 161   313 -> 252
+//   scaled by  1.15       421 -> 392       981 -> 621    182 -> 190   349 -> 276
+//              2          415 -> 385       797 -> 487    188 -> 184   309 -> 223
+// Without boxes at all (2048 x 2046): clamp 840 -> 660, nearest 308 -> 273.
+enum WarpForm { kStaged64, kStaged48, kStaged16, kDirectRows, kDirectGeneral, kWarpForms };
 
 // Register copy of one item's inverse matrix (loaded once per work item so
 // that output stores cannot force re-reads of the descriptor).
@@ -653,9 +674,10 @@ __device__ __forceinline__ bool counts_whole(const WarpArgs& a, const TilePlan& 
 // computed.
 constexpr size_t kWarpTileBytes = size_t(2) * kBoxH * kBoxW * sizeof(float);
 
-template <int INTERP, bool USE_TMA, int TH>
-__global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __grid_constant__ CUtensorMap tmap,
-                                                                  WarpArgs a) {
+// GENERAL: the general path alone.
+template <int INTERP, bool USE_TMA, int TH, bool GENERAL = false>
+__global__ void __launch_bounds__(kWarpThreads, GENERAL ? 6 : 4)
+    warp_tiles_kernel(const __grid_constant__ CUtensorMap tmap, WarpArgs a) {
   extern __shared__ __align__(128) float warp_boxes[];  // USE_TMA: [2][kBoxH * kBoxW]
   __shared__ alignas(8) uint64_t bar[2];
   __shared__ TilePlan s_plan[2];
@@ -683,7 +705,7 @@ __global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __gri
     TilePlan p = plan_tile_warp<TH>(co, tile_x0, tile_y0, kLanczos ? 3 : 1, vlo, static_cast<float>(a.width) - off,
                                 static_cast<float>(a.height) - off);
     if (!USE_TMA) p.fits = 0;
-    if (INTERP != GG_INTERP_NEAREST && p.grid)
+    if (INTERP != GG_INTERP_NEAREST && !GENERAL && p.grid)
       tile_grid_warp(ip->inv, tile_x0, tile_y0, p.fits != 0, p.bx, p.by, s_grid[buf]);
     if (tid != 0) return;
     s_plan[buf] = p;
@@ -726,7 +748,7 @@ __global__ void __launch_bounds__(kWarpThreads, 4) warp_tiles_kernel(const __gri
     }
     const bool whole = counts_whole<INTERP, TH>(a, p, finite, tile_x0, tile_y0);
     unsigned bad = 0;
-    if (INTERP != GG_INTERP_NEAREST && p.grid && (!kLanczos || a.clamp < 0.0f) &&
+    if (INTERP != GG_INTERP_NEAREST && !GENERAL && p.grid && (!kLanczos || a.clamp < 0.0f) &&
         (p.fits || !kLanczos || (a.width >= 6 && a.height >= 6))) {
       const int lx = tid & 31, ly = (tid >> 5) * (TH / 4);
       const TileGrid& grid = s_grid[buf];
@@ -1024,13 +1046,13 @@ static void launch_warp_geometry(gg_stack* s, const WarpArgs& a) {
   check_cuda(cudaGetLastError(), "warp_geometry launch");
 }
 
-template <int INTERP, int TH>
+template <int INTERP, int TH, bool STAGED, bool GENERAL = false>
 static void launch_warp_tiles(gg_stack* s, WarpArgs args) {
-  const bool use_tma = s->has_slot_tmap;
   args.tiles_y = (args.row1 - args.row0 + TH - 1) / TH;
-  if (args.counted) launch_warp_geometry<INTERP, TH>(s, args);
-  auto kern = use_tma ? warp_tiles_kernel<INTERP, true, TH> : warp_tiles_kernel<INTERP, false, TH>;
-  const size_t smem = use_tma ? kWarpTileBytes : 0;
+  if constexpr (INTERP != GG_INTERP_NEAREST && TH != kMidTileH && !GENERAL)  // the bands' forms
+    if (args.counted) launch_warp_geometry<INTERP, TH>(s, args);
+  auto kern = warp_tiles_kernel<INTERP, STAGED, TH, GENERAL>;
+  const size_t smem = STAGED ? kWarpTileBytes : 0;
   const int per_sm = kernel_ctas_per_sm(kern, kWarpThreads, smem, "warp launch shape");
   const int64_t items = static_cast<int64_t>(args.item_count) * args.tiles_x * args.tiles_y;
   unsigned grid =
@@ -1061,23 +1083,68 @@ static WarpArgs warp_args(gg_stack* s, WarpItem* d_items, int count, int row0, i
   return a;
 }
 
-static void launch_warp_rows(gg_stack* s, const WarpArgs& a, int interp) {
+template <int INTERP>
+static void launch_warp_form(gg_stack* s, const WarpArgs& a, WarpForm form) {
   // With less than two 64-row tiles per SM the launch takes as long as a tile
   // does: 16-row tiles spread it over four times as many CTAs.
   const int64_t tiles = static_cast<int64_t>(a.item_count) * a.tiles_x * ((a.row1 - a.row0 + kTileH - 1) / kTileH);
-  const bool small = tiles < 2 * sm_count();
-  if (interp == GG_INTERP_NEAREST)
-    launch_warp_tiles<GG_INTERP_NEAREST, kTileH>(s, a);
-  else if (interp == GG_INTERP_BILINEAR)
-    small ? launch_warp_tiles<GG_INTERP_BILINEAR, kSmallTileH>(s, a)
-          : launch_warp_tiles<GG_INTERP_BILINEAR, kTileH>(s, a);
+  const bool small = tiles < 2 * sm_count() && INTERP != GG_INTERP_NEAREST;
+  if constexpr (INTERP != GG_INTERP_NEAREST) {
+    if (form == kDirectRows) {
+      small ? launch_warp_tiles<INTERP, kSmallTileH, false>(s, a) : launch_warp_tiles<INTERP, kTileH, false>(s, a);
+      return;
+    }
+  }
+  if (form == kDirectGeneral)
+    small ? launch_warp_tiles<INTERP, kSmallTileH, false, true>(s, a)
+          : launch_warp_tiles<INTERP, kMidTileH, false, true>(s, a);
+  else if (form == kStaged16 || small)
+    launch_warp_tiles<INTERP, kSmallTileH, true>(s, a);
+  else if (form == kStaged48)
+    launch_warp_tiles<INTERP, kMidTileH, true>(s, a);
   else
-    small ? launch_warp_tiles<GG_INTERP_LANCZOS3, kSmallTileH>(s, a)
-          : launch_warp_tiles<GG_INTERP_LANCZOS3, kTileH>(s, a);
+    launch_warp_tiles<INTERP, kTileH, true>(s, a);
 }
 
-// Host descriptors of a warp batch (validated; inverse coefficients).
-static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd) {
+static void launch_warp_rows(gg_stack* s, const WarpArgs& a, int interp, WarpForm form) {
+  if (interp == GG_INTERP_NEAREST)
+    launch_warp_form<GG_INTERP_NEAREST>(s, a, form);
+  else if (interp == GG_INTERP_BILINEAR)
+    launch_warp_form<GG_INTERP_BILINEAR>(s, a, form);
+  else
+    launch_warp_form<GG_INTERP_LANCZOS3>(s, a, form);
+}
+
+// The form of a frame's warp.  Boxes where every tile's footprint fits one: an
+// affine map takes a tile to source columns and rows that span |a| 63 + |b| (rows
+// - 1) and |d| 63 + |e| (rows - 1), and a box holds the taps, the pixel of margin
+// and the columns before its 16-byte boundary besides (plan_of_range).
+static WarpForm warp_form(const gg_stack* s, const WarpItem& it, int interp, float clamp) {
+  const bool lanczos = interp == GG_INTERP_LANCZOS3;
+  const int radius = lanczos ? 3 : 1;
+  if (s->has_slot_tmap) {
+    auto fits = [&](int rows) {
+      const double x = std::fabs(it.inv[0]) * (kTileW - 1) + std::fabs(it.inv[1]) * (rows - 1);
+      const double y = std::fabs(it.inv[3]) * (kTileW - 1) + std::fabs(it.inv[4]) * (rows - 1);
+      return x <= kBoxW - 5 - 2 * radius && y <= kBoxH - 2 - 2 * radius;
+    };
+    // a projective map's tiles are looked at one by one
+    if (!it.affine || fits(kTileH)) return kStaged64;
+    if (fits(kMidTileH)) return kStaged48;
+    if (fits(kSmallTileH)) return kStaged16;
+  }
+  const bool straight = it.affine && interp != GG_INTERP_NEAREST && (!lanczos || clamp < 0.0f);
+  return straight ? kDirectRows : kDirectGeneral;
+}
+
+// How many descriptors of a batch take each form (they stand in that order).
+struct WarpForms {
+  int64_t count[kWarpForms] = {};
+};
+
+// Host descriptors of a warp batch (validated; inverse coefficients), by form.
+static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd,
+                                             int interp, float clamp, WarpForms& forms) {
   std::vector<WarpItem> items(static_cast<size_t>(count));
   for (int64_t k = 0; k < count; ++k) {
     stack_require_loaded(s, indices[k], "warp");
@@ -1099,18 +1166,23 @@ static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices
                     std::fabs(m[5]) < 1.0e7)
                        ? 1
                        : 0;
+    it.form = warp_form(s, it, interp, clamp);
+    ++forms.count[it.form];
   }
+  std::stable_sort(items.begin(), items.end(), [](const WarpItem& a, const WarpItem& b) { return a.form < b.form; });
   return items;
 }
 
 // The kernels of a warp batch whose descriptors are already in device
-// memory (d_items, `count` of them): per group of at most `spares` frames,
-// resolve slots (unless that is done: `prepared`), warp into the spare slots,
-// swap the slot table.  Only launches on the stack's stream (safe inside a stream
-// capture).
-static void launch_warp_items(gg_stack* s, WarpItem* d_items, int64_t count, int interp, float fill, float clamp,
-                              bool track_coverage, bool prepared = false) {
+// memory (d_items, `count` of them in the order of `forms`): per group of at most
+// `spares` frames, resolve slots (unless that is done: `prepared`), warp into the
+// spare slots, swap the slot table; a launch per form.  Only launches on the
+// stack's stream (safe inside a stream capture).
+static void launch_warp_items(gg_stack* s, WarpItem* d_items, int64_t count, const WarpForms& forms, int interp,
+                              float fill, float clamp, bool track_coverage, bool prepared = false) {
   stack_slots_moved(s);
+  int form = 0;
+  int64_t form_end = forms.count[0];
   for (int64_t k0 = 0; k0 < count; k0 += s->spares) {
     const int nb = static_cast<int>(std::min<int64_t>(s->spares, count - k0));
     if (!prepared) {
@@ -1120,21 +1192,27 @@ static void launch_warp_items(gg_stack* s, WarpItem* d_items, int64_t count, int
                                                                    s->stride);
       check_cuda(cudaGetLastError(), "warp_prepare launch");
     }
-    WarpArgs a = warp_args(s, d_items + k0, nb, 0, static_cast<int>(s->height));
-    a.nonfinite = s->d_frame_nonfinite;
-    a.fill = fill;
-    a.clamp = clamp;
-    a.coverage = track_coverage ? s->d_warp_coverage : nullptr;
-    a.slot_of_frame = s->d_slot_of_frame;
-    a.spare = s->d_spare_slot;
-    a.ticket = s->d_tickets + s->frames;
-    launch_warp_rows(s, a, interp);
+    for (int64_t k = k0; k < k0 + nb;) {
+      while (k >= form_end) form_end += forms.count[++form];
+      const int run = static_cast<int>(std::min<int64_t>(form_end, k0 + nb) - k);
+      WarpArgs a = warp_args(s, d_items + k, run, 0, static_cast<int>(s->height));
+      a.nonfinite = s->d_frame_nonfinite;
+      a.fill = fill;
+      a.clamp = clamp;
+      a.coverage = track_coverage ? s->d_warp_coverage : nullptr;
+      a.slot_of_frame = s->d_slot_of_frame;
+      a.spare = s->d_spare_slot + (k - k0);
+      a.ticket = s->d_tickets + s->frames;
+      launch_warp_rows(s, a, interp, static_cast<WarpForm>(form));
+      k += run;
+    }
   }
 }
 
 void warp_frames(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd, int interp, float fill,
                  float clamp, bool track_coverage) {
-  const std::vector<WarpItem> items = warp_items_host(s, indices, count, fwd);
+  WarpForms forms;
+  const std::vector<WarpItem> items = warp_items_host(s, indices, count, fwd, interp, clamp, forms);
   ensure_warp_items(s, std::max<int64_t>(count, s->spares));
   if (track_coverage) ensure_warp_coverage(s);
   auto* d_items = static_cast<WarpItem*>(s->d_warp_items);
@@ -1144,7 +1222,7 @@ void warp_frames(gg_stack* s, const int64_t* indices, int64_t count, const doubl
   if (count <= std::min<int64_t>(s->spares, kLargeBlock)) {
     if (count <= kSmallBlock) launch_prepare_block<kSmallBlock>(s, d_items, items);
     else launch_prepare_block<kLargeBlock>(s, d_items, items);
-    launch_warp_items(s, d_items, count, interp, fill, clamp, track_coverage, true);
+    launch_warp_items(s, d_items, count, forms, interp, fill, clamp, track_coverage, true);
     if (track_coverage) s->warp_coverage_frames += count;
     return;
   }
@@ -1154,23 +1232,27 @@ void warp_frames(gg_stack* s, const int64_t* indices, int64_t count, const doubl
   upload_params(s->stream, s->d_warp_items, s->h_warp_items, sizeof(WarpItem) * items.size(),
                 "cudaMemcpyAsync(warp items)");
   check_cuda(cudaEventRecord(s->warp_items_free, s->stream), "cudaEventRecord(warp items)");
-  launch_warp_items(s, d_items, count, interp, fill, clamp, track_coverage);
+  launch_warp_items(s, d_items, count, forms, interp, fill, clamp, track_coverage);
   if (track_coverage) s->warp_coverage_frames += count;
 }
 
-// Warp descriptors in a caller-owned device buffer (for captured graphs):
-// returns the device pointer (cudaMalloc, the caller frees it with cudaFree)
-// and their count through `count_out`.
-void* warp_items_device(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd) {
-  const std::vector<WarpItem> items = warp_items_host(s, indices, count, fwd);
-  void* d = nullptr;
-  check_cuda(cudaMalloc(&d, sizeof(WarpItem) * items.size()), "cudaMalloc(graph warp items)");
-  const cudaError_t err = cudaMemcpy(d, items.data(), sizeof(WarpItem) * items.size(), cudaMemcpyHostToDevice);
+// Warp descriptors in a caller-owned device buffer (for captured graphs).
+WarpBatch warp_batch_device(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd, int interp,
+                            float clamp) {
+  WarpForms forms;
+  const std::vector<WarpItem> items = warp_items_host(s, indices, count, fwd, interp, clamp, forms);
+  WarpBatch batch;
+  batch.count = count;
+  batch.interp = interp;
+  batch.clamp = clamp;
+  batch.forms.assign(forms.count, forms.count + kWarpForms);
+  check_cuda(cudaMalloc(&batch.items, sizeof(WarpItem) * items.size()), "cudaMalloc(graph warp items)");
+  const cudaError_t err = cudaMemcpy(batch.items, items.data(), sizeof(WarpItem) * items.size(), cudaMemcpyHostToDevice);
   if (err != cudaSuccess) {
-    cudaFree(d);
+    cudaFree(batch.items);
     check_cuda(err, "cudaMemcpy(graph warp items)");
   }
-  return d;
+  return batch;
 }
 
 // ---- warp of every frame into a band of rows (fused warp + integration) --------
@@ -1276,7 +1358,7 @@ void launch_warp_band(gg_stack* s, void* d_items, int interp, float clamp, int r
   a.clamp = clamp;
   a.coverage = geometric;
   a.counted = 1;
-  launch_warp_rows(s, a, interp);
+  launch_warp_rows(s, a, interp, s->has_slot_tmap ? kStaged64 : kDirectRows);
 }
 
 void launch_warp_band_prepare(gg_stack* s, void* d_items, const FusedFrame* d_frames, int interp, float clamp,
@@ -1302,8 +1384,10 @@ void launch_warp_band_prepare(gg_stack* s, void* d_items, const FusedFrame* d_fr
   check_cuda(cudaGetLastError(), "warp_nonfinite launch");
 }
 
-void launch_warp_items_device(gg_stack* s, void* d_items, int64_t count, int interp, float fill, float clamp) {
-  launch_warp_items(s, static_cast<WarpItem*>(d_items), count, interp, fill, clamp, false);
+void launch_warp_batch(gg_stack* s, const WarpBatch& batch, float fill) {
+  WarpForms forms;
+  std::copy(batch.forms.begin(), batch.forms.end(), forms.count);
+  launch_warp_items(s, static_cast<WarpItem*>(batch.items), batch.count, forms, batch.interp, fill, batch.clamp, false);
 }
 
 }  // namespace gg

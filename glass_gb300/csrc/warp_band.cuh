@@ -1,10 +1,26 @@
-// Interface of the warp (warp.cu) to the fused warp + integration (integrate.cu)
-// and to the differentiable warp (adjoint.cu).
+// Interface of the warp (warp.cu) to the integration and the graphs
+// (integrate.cu) and to the differentiable warp (adjoint.cu).
 #pragma once
+
+#include <vector>
 
 #include "stack.cuh"
 
 namespace gg {
+
+// An in-place warp of some frames whose descriptors stay on the device, for
+// captured graphs.  `items` is the caller's to free with cudaFree.
+struct WarpBatch {
+  void* items = nullptr;
+  int64_t count = 0;
+  std::vector<int64_t> forms;  // descriptors per launch form, in order
+  int interp = 0;
+  float clamp = -1.0f;
+};
+WarpBatch warp_batch_device(gg_stack* s, const int64_t* indices, int64_t count, const double* fwd, int interp,
+                            float clamp);
+// Only launches on the stack's stream (safe inside a stream capture).
+void launch_warp_batch(gg_stack* s, const WarpBatch& batch, float fill);
 
 // Fused warp (integrate_matrix_warped_*): a frame's samples come from its
 // source pixels through the inverse of its matrix instead of from the stack.
