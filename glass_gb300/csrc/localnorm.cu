@@ -161,17 +161,19 @@ __global__ void ln_coeff_kernel(LnArgs a, int pairs) {
 }
 
 // In place v * scale + offset for every pixel of each listed frame; frames
-// whose pair had no finite pixel (totals == 0) are left as they are.  Blocks
-// take rows, threads the row's 16-byte vectors (the first and last may reach
-// into the neighbouring rows: those go sample by sample).  Bound by memory:
-// 31 frames of 2048^2 in 236 us, 483 us with a 64-bit division per sample.
-__global__ void __launch_bounds__(256) ln_apply_kernel(LnArgs a, int check_totals) {
+// whose pair had no finite pixel (totals == 0) are left as they are.  Groups of
+// `lanes` threads take rows, threads the row's 16-byte vectors (the first and last
+// may reach into the neighbouring rows: those go sample by sample).  Bound by
+// memory: 31 frames of 2048^2 in 236 us, 483 us with a 64-bit division per
+// sample; rows of less than 1024 columns share a CTA.
+__global__ void __launch_bounds__(256) ln_apply_kernel(LnArgs a, int check_totals, int lanes) {
   const int pair = blockIdx.y;
   if (check_totals && a.totals[pair] == 0) return;
   float* img = const_cast<float*>(a.slots) + static_cast<int64_t>(a.slot_of_frame[a.frames[pair]]) * a.stride;
   const int W = a.width;
   const unsigned tile_w = static_cast<unsigned>(a.tile_w);
-  for (int y = blockIdx.x; y < a.height; y += gridDim.x) {
+  const int rows = 256 / lanes, lane = static_cast<int>(threadIdx.x) % lanes;
+  for (int y = blockIdx.x * rows + static_cast<int>(threadIdx.x) / lanes; y < a.height; y += gridDim.x * rows) {
     const int64_t at = static_cast<int64_t>(y) * W;
     const int64_t row_tile = (static_cast<int64_t>(pair) * a.rows + min(y / a.tile_h, a.rows - 1)) * a.cols;
     const float* sc = a.scales + row_tile;
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(256) ln_apply_kernel(LnArgs a, int check_total
     float* row = img + at;
     auto tile = [&](int x) { return min(static_cast<int>(static_cast<unsigned>(x) / tile_w), a.cols - 1); };
     auto apply = [&](float v, int t) { return __fadd_rn(__fmul_rn(v, __ldg(sc + t)), __ldg(of + t)); };
-    for (int x = 4 * static_cast<int>(threadIdx.x) - static_cast<int>(at & 3); x < W; x += 4 * 256) {
+    for (int x = 4 * lane - static_cast<int>(at & 3); x < W; x += 4 * lanes) {
       if (x >= 0 && x + 3 < W) {
         float4 v = *reinterpret_cast<const float4*>(row + x);
         const int t0 = tile(x), t3 = tile(x + 3);
@@ -281,9 +283,15 @@ static void upload_frames(gg_stack* s, LnScratch& g, const int64_t* idx, int64_t
   upload_params(s->stream, g.frames, g.h_frames, sizeof(int) * count, "cudaMemcpyAsync(local norm frames)");
 }
 
-static unsigned apply_grid_x(gg_stack* s, int pairs) {
+static void launch_ln_apply(gg_stack* s, const LnArgs& a, int pairs, int check_totals) {
+  int lanes = 8;  // of a row: its vectors, one more where it starts off a 16-byte boundary
+  while (lanes < 256 && 4 * lanes < s->width + 3) lanes *= 2;
+  const int64_t ctas = (s->height + 256 / lanes - 1) / (256 / lanes);
   const int64_t want = static_cast<int64_t>(sm_count()) * 8 / std::max(pairs, 1) + 1;
-  return static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(s->height, want)));
+  note_launch();
+  ln_apply_kernel<<<dim3(static_cast<unsigned>(std::min(ctas, want)), static_cast<unsigned>(pairs)), 256, 0,
+                    s->stream>>>(a, check_totals, lanes);
+  check_cuda(cudaGetLastError(), "ln_apply launch");
 }
 
 // statistics + coefficients (+ apply) for `count` source frames
@@ -305,11 +313,7 @@ static void ln_run(gg_stack* s, int64_t ref, const int64_t* sources, int64_t cou
   note_launch();
   ln_coeff_kernel<<<static_cast<unsigned>((tiles + 255) / 256), 256, 0, s->stream>>>(a, pairs);
   check_cuda(cudaGetLastError(), "ln_coeff launch");
-  if (apply) {
-    note_launch();
-    ln_apply_kernel<<<dim3(apply_grid_x(s, pairs), static_cast<unsigned>(pairs)), 256, 0, s->stream>>>(a, 1);
-    check_cuda(cudaGetLastError(), "ln_apply launch");
-  }
+  if (apply) launch_ln_apply(s, a, pairs, 1);
   if (update_weights) {
     note_launch();
     ln_zero_weights_kernel<<<(pairs + 127) / 128, 128, 0, s->stream>>>(g.totals, g.frames, pairs, s->d_weights);
@@ -377,10 +381,7 @@ int gg_stack_apply_grid_normalization(gg_stack* s, const int64_t* indices, int64
   upload_params(s->stream, g.offsets, host_offsets, sizeof(float) * tiles * count,
                 "cudaMemcpyAsync(local norm offsets)");
   LnArgs a = ln_args(s, tile_h, tile_w, grid_rows, grid_cols, 0, g);
-  note_launch();
-  ln_apply_kernel<<<dim3(apply_grid_x(s, static_cast<int>(count)), static_cast<unsigned>(count)), 256, 0,
-                    s->stream>>>(a, 0);
-  check_cuda(cudaGetLastError(), "ln_apply launch");
+  launch_ln_apply(s, a, static_cast<int>(count), 0);
   check_cuda(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize(local norm apply)");
   GG_API_END
 }
@@ -424,9 +425,7 @@ int gg_stack_apply_global_normalization(gg_stack* s, int64_t index, float scale,
   upload_params(s->stream, g.scales, &scale, sizeof(float), "cudaMemcpyAsync(global scale)");
   upload_params(s->stream, g.offsets, &offset, sizeof(float), "cudaMemcpyAsync(global offset)");
   LnArgs a = ln_args(s, static_cast<int>(s->height), static_cast<int>(s->width), 1, 1, 0, g);
-  note_launch();
-  ln_apply_kernel<<<dim3(apply_grid_x(s, 1), 1), 256, 0, s->stream>>>(a, 0);
-  check_cuda(cudaGetLastError(), "ln_apply launch");
+  launch_ln_apply(s, a, 1, 0);
   check_cuda(cudaStreamSynchronize(s->stream), "cudaStreamSynchronize(global normalization)");
   GG_API_END
 }
