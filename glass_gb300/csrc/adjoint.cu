@@ -208,17 +208,23 @@ __global__ void __launch_bounds__(kScatterThreads) lanczos3_scatter_kernel(Adjoi
     for (int r = 0; r < rows; ++r) {
       const int y = ybase + r;
       int x0, y0;
-      float tx, ty;
+      CentredOffset tx, ty;
       if constexpr (FIXED) {
-        auto fraction = [](long long v) {
-          const float high = __uint2float_rn(static_cast<unsigned>(v >> 30) & 0xffffffu);
-          const float low = __uint2float_rn(static_cast<unsigned>(v >> 6) & 0xffffffu);
-          return __fmul_rn(__fmaf_rn(low, 5.9604644775390625e-08f, high), 5.9604644775390625e-08f);
+        // distance from the nearer tap: two exact halves of 24 bits, rounded once
+        auto offset = [](long long v) {
+          constexpr long long kMask = (1ll << 54) - 1;
+          CentredOffset o;
+          o.lower = ((v >> 53) & 1) == 0;
+          const long long d = (o.lower ? v : -v) & kMask;
+          const float high = __uint2float_rn(static_cast<unsigned>(d >> 30));
+          const float low = __uint2float_rn(static_cast<unsigned>(d >> 6) & 0xffffffu);
+          o.s = __fmul_rn(__fmaf_rn(low, 5.9604644775390625e-08f, high), 5.9604644775390625e-08f);
+          return o;
         };
         x0 = ox + static_cast<int>(fx >> 54);
         y0 = oy + static_cast<int>(fy >> 54);
-        tx = fraction(fx);
-        ty = fraction(fy);
+        tx = offset(fx);
+        ty = offset(fy);
         fx += step_x;
         fy += step_y;
       } else {
@@ -226,8 +232,16 @@ __global__ void __launch_bounds__(kScatterThreads) lanczos3_scatter_kernel(Adjoi
         source_coord(a.coef, static_cast<float>(x), static_cast<float>(y), sx, sy);
         // far outside: any position without a valid sample
         const bool near = fabsf(sx.hi) < 1.0e9f && fabsf(sy.hi) < 1.0e9f;
-        ff_floor_frac(near ? sx : FFv{-100.0f, 0.0f}, x0, tx);
-        ff_floor_frac(near ? sy : FFv{-100.0f, 0.0f}, y0, ty);
+        auto offset = [](FFv v, int& whole) {
+          float t;
+          ff_floor_frac(v, whole, t);
+          CentredOffset o;
+          o.lower = t <= 0.5f;
+          o.s = o.lower ? t : __fsub_rn(__fsub_rn(static_cast<float>(whole) + 1.0f, v.hi), v.lo);
+          return o;
+        };
+        tx = offset(near ? sx : FFv{-100.0f, 0.0f}, x0);
+        ty = offset(near ? sy : FFv{-100.0f, 0.0f}, y0);
       }
       // 2 <= s < size - 3 of the coordinate is that of its whole part
       const bool valid = x < W && x0 >= 2 && x0 < W - 3 && y0 >= 2 && y0 < a.height - 3;
@@ -255,24 +269,14 @@ __global__ void __launch_bounds__(kScatterThreads) lanczos3_scatter_kernel(Adjoi
       if (!isfinite(g)) g = 0.0f;
       const bool live = g != 0.0f;
       if (!__any_sync(0xffffffffu, live)) continue;
-      float wx[6], wy[6], dwx[6], dwy[6];
-      lanczos3_weights_grad_poly(tx, wx, dwx);
-      lanczos3_weights_grad_poly(ty, wy, dwy);
-      float swx = 0.0f, swy = 0.0f, dsx = 0.0f, dsy = 0.0f;
-#pragma unroll
-      for (int i = 0; i < 6; ++i) {
-        swx += wx[i];
-        swy += wy[i];
-        dsx += dwx[i];
-        dsy += dwy[i];
-      }
+      const LanczosAxis ax = lanczos3_axis_centred(tx), ay = lanczos3_axis_centred(ty);
       float N = 0.0f, Nx = 0.0f, Ny = 0.0f;
       // the other lanes read the image's first window (a live lane proves that
       // the image holds one)
       const float* at = a.src + (live ? static_cast<int64_t>(y0 - 2) * W + (x0 - 2) : 0);
       // taps relative to the middle one: the derivatives are the same, (Nx - O
-      // dsx swy) / D for taps v + c equals that for v, without the rounding
-      // that a background of many times its noise leaves in Nx
+      // Dx) / D for taps v + c equals that for v, without the rounding that a
+      // background of many times its noise leaves in Nx
       const float middle = __ldg(at + 2 * static_cast<int64_t>(W) + 2);
 #pragma unroll
       for (int j = 0; j < 6; ++j, at += W) {
@@ -280,24 +284,24 @@ __global__ void __launch_bounds__(kScatterThreads) lanczos3_scatter_kernel(Adjoi
 #pragma unroll
         for (int i = 0; i < 6; ++i) {
           const float v = __fsub_rn(__ldg(at + i), middle);
-          rv = __fmaf_rn(wx[i], v, rv);
-          rd = __fmaf_rn(dwx[i], v, rd);
+          rv = __fmaf_rn(ax.w[i], v, rv);
+          rd = __fmaf_rn(ax.dw[i], v, rd);
         }
-        N = __fmaf_rn(wy[j], rv, N);
-        Nx = __fmaf_rn(wy[j], rd, Nx);
-        Ny = __fmaf_rn(dwy[j], rv, Ny);
+        N = __fmaf_rn(ay.w[j], rv, N);
+        Nx = __fmaf_rn(ay.w[j], rd, Nx);
+        Ny = __fmaf_rn(ay.dw[j], rv, Ny);
       }
       float gd = 0.0f;
       if (live) {
         float gsx = 0.0f, gsy = 0.0f;
         if (isfinite(N) && isfinite(Nx) && isfinite(Ny)) {
           // a window of finite taps: its weights sum to 1 within a few per cent
-          const float iD = __frcp_rn(swx * swy);
+          const float iD = __frcp_rn(ax.sum * ay.sum);
           const float O = N * iD;
           gd = g * iD;
-          gsx = gd * (Nx - O * (dsx * swy));
-          gsy = gd * (Ny - O * (swx * dsy));
-        } else if (!lanczos3_adjoint_taps(a.src, a.grad_src, W, x0, y0, tx, ty, g, gsx, gsy)) {
+          gsx = gd * (Nx - O * (ax.dsum * ay.sum));
+          gsy = gd * (Ny - O * (ax.sum * ay.dsum));
+        } else if (!lanczos3_adjoint_taps(a.src, a.grad_src, W, x0, y0, tx.t(), ty.t(), g, gsx, gsy)) {
           gsx = gsy = 0.0f;
         }
         const float rf = static_cast<float>(r);
@@ -308,9 +312,9 @@ __global__ void __launch_bounds__(kScatterThreads) lanczos3_scatter_kernel(Adjoi
       }
 #pragma unroll
       for (int j = 0; j < 6; ++j) {
-        const float gy = gd * wy[j];
+        const float gy = gd * ay.w[j];
 #pragma unroll
-        for (int i = 0; i < 6; ++i) cell[j][i] = __fmaf_rn(gy, wx[i], cell[j][i]);
+        for (int i = 0; i < 6; ++i) cell[j][i] = __fmaf_rn(gy, ax.w[i], cell[j][i]);
       }
     }
     if (rows > 0) {

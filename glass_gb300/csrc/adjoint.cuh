@@ -187,6 +187,92 @@ __device__ __forceinline__ void lanczos3_weights_grad_poly(float t, float (&w)[6
   dw[5] = __fsub_rn(dec, doc);
 }
 
+// Polynomials about the nearer tap (printed by glass_gb300/lanczos_poly.py
+// --centred, lowest power first): with s its distance and x = s^2 the weights are
+// 1 + x p(x), x q_k(x) +- s r_k(x) of the taps k - s and k + s away, and x s(s) of
+// the one 3 - s away.
+static __device__ constexpr float kCentred_p[6] = {
+    -1.827704549e+00f, 1.122409225e+00f, -3.558606505e-01f, 6.957933307e-02f, -9.242961183e-03f, 8.455788484e-04f};
+static __device__ constexpr float kCentred_s[8] = {
+    1.111111119e-01f, 7.407423854e-02f, -1.660469323e-01f, -1.188418269e-01f, 6.327397376e-02f, 5.818251893e-02f, -1.446728036e-02f, -7.642415352e-03f};
+static __device__ constexpr float kCentred_q1[6] = {
+    1.153986692e+00f, -9.057731032e-01f, 3.043932617e-01f, -5.974025652e-02f, 7.811781019e-03f, -6.994246505e-04f};
+static __device__ constexpr float kCentred_r1[6] = {
+    8.269933462e-01f, -3.328193426e-01f, -2.008740790e-02f, 3.335780278e-02f, -8.541316725e-03f, 1.143358182e-03f};
+static __device__ constexpr float kCentred_q2[6] = {
+    -3.317483366e-01f, 4.847887456e-01f, -1.847165525e-01f, 3.562755883e-02f, -4.283661488e-03f, 3.411271609e-04f};
+static __device__ constexpr float kCentred_r2[6] = {
+    -2.067483366e-01f, 1.733886003e-01f, 7.678152621e-02f, -5.502928793e-02f, 1.328185573e-02f, -1.744203619e-03f};
+
+// Value and derivative of a polynomial.
+template <int N>
+__device__ __forceinline__ void horner_grad(const float (&c)[N], float x, float& p, float& dp) {
+  p = c[N - 1];
+  dp = static_cast<float>(N - 1) * c[N - 1];
+#pragma unroll
+  for (int j = N - 2; j >= 0; --j) {
+    p = __fmaf_rn(p, x, c[j]);
+    if (j > 0) dp = __fmaf_rn(dp, x, static_cast<float>(j) * c[j]);
+  }
+}
+
+// A sample's offset by its distance `s` from the nearer tap: that of k = 0
+// (t = s), else that of k = 1 (t = 1 - s).
+struct CentredOffset {
+  float s;
+  bool lower;
+  __device__ __forceinline__ float t() const { return lower ? s : __fsub_rn(1.0f, s); }
+};
+
+// Weights w(t - k) and derivatives, k = -2..3, and their sums.
+struct LanczosAxis {
+  float w[6], dw[6];
+  float sum, dsum;
+};
+
+// Each weight to relative accuracy (about 2e-7): the ones that vanish at a whole
+// offset do so with it.  The image gradient is made of the weights themselves, and next
+// to a whole offset the others' absolute rounding (lanczos3_weights_grad_poly)
+// and that of their sum were most of its error.  The sums follow from the even
+// parts alone, the odd ones cancel.
+__device__ __forceinline__ LanczosAxis lanczos3_axis_centred(const CentredOffset& o) {
+  const float s = o.s;
+  const float x = __fmul_rn(s, s), s2 = __fadd_rn(s, s), x2 = __fadd_rn(x, x);
+  float v[6], d[6];  // in order of k for the lower half, mirrored for the upper
+  float p, dp, p3, dp3;
+  horner_grad(kCentred_p, x, p, dp);
+  v[2] = __fmaf_rn(x, p, 1.0f);
+  d[2] = __fmul_rn(s2, __fmaf_rn(x, dp, p));
+  float even = 0.0f, deven = 0.0f;  // of the pairs
+  auto pair = [&](const float (&qc)[6], const float (&rc)[6], int near, int far) {
+    float q, dq, r, dr;
+    horner_grad(qc, x, q, dq);
+    horner_grad(rc, x, r, dr);
+    const float e = __fmul_rn(x, q), de = __fmul_rn(s2, __fmaf_rn(x, dq, q)), odd = __fmaf_rn(x2, dr, r);
+    v[near] = __fmaf_rn(s, r, e);
+    v[far] = __fmaf_rn(-s, r, e);
+    d[near] = __fadd_rn(de, odd);
+    d[far] = __fsub_rn(de, odd);
+    even = __fadd_rn(even, q);
+    deven = __fadd_rn(deven, de);
+  };
+  pair(kCentred_q1, kCentred_r1, 3, 1);
+  pair(kCentred_q2, kCentred_r2, 4, 0);
+  horner_grad(kCentred_s, s, p3, dp3);
+  v[5] = __fmul_rn(x, p3);
+  d[5] = __fmaf_rn(x, dp3, __fmul_rn(s2, p3));
+  LanczosAxis a;
+  a.sum = __fmaf_rn(x, __fmaf_rn(2.0f, even, __fadd_rn(p, p3)), 1.0f);
+  const float dsum = __fmaf_rn(2.0f, deven, __fadd_rn(d[2], d[5]));
+  a.dsum = o.lower ? dsum : -dsum;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) {
+    a.w[i] = o.lower ? v[i] : v[5 - i];
+    a.dw[i] = o.lower ? d[i] : -d[5 - i];
+  }
+  return a;
+}
+
 // Lanczos3 value and its derivatives with respect to the sample position
 // over a window whose 36 taps are all finite (the warp's polynomial weights
 // and their exact derivatives); false when a tap is not finite or the

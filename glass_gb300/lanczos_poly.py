@@ -12,7 +12,17 @@ error is below 3e-10, far under float32 rounding.  It also prints the
 derivatives d/dx of those float32 polynomials (coefficients j * c_j, degree
 4), pasted into csrc/adjoint.cuh: the Gauss-Newton refinement differentiates
 exactly the weights the warp samples with.
-Run: python -m glass_gb300.lanczos_poly
+
+Those weights are accurate in absolute terms: near a whole offset, where all
+but one tap vanish, the vanishing ones are what rounding leaves of E +- O.  The
+image gradient of the warp adjoint spreads each pixel by its weights, so it takes
+them from polynomials about the nearer tap instead (fit_centred): with s in
+[0, 1/2] the distance to it and x = s^2, L(s) = 1 + x P(x), the pairs L(k - s)
+and L(k + s), k = 1 and 2, are x Q(x) +- s R(x), and L(3 - s) = x S(s), so each
+vanishes with s to full relative accuracy.  Fitted in float64 at Chebyshev points
+(above s = 0.003, below which the quotients lose digits); the fit error is below
+3e-11, for S 1e-9.
+Run: python -m glass_gb300.lanczos_poly [--derivatives | --centred]
 """
 
 from __future__ import annotations
@@ -40,6 +50,26 @@ def fit(center: float, samples: int = 20001):
     return e, o, err
 
 
+CENTRED_DEGREE = {"p": 5, "q1": 5, "r1": 5, "q2": 5, "r2": 5, "s": 7}
+
+
+def fit_centred(samples: int = 4000) -> dict[str, tuple[np.ndarray, float]]:
+    """Coefficients (lowest power first) and fit error of each polynomial."""
+    s = 0.25 * (1.0 - np.cos(np.pi * (np.arange(samples) + 0.5) / samples))
+    s = s[s > 0.003]
+    x = s * s
+    values = {"p": ((lanczos3(s) - 1.0) / x, x), "s": (lanczos3(3.0 - s) / x, s)}
+    for k in (1, 2):
+        values[f"q{k}"] = (0.5 * (lanczos3(k - s) + lanczos3(k + s)) / x, x)
+        values[f"r{k}"] = (0.5 * (lanczos3(k - s) - lanczos3(k + s)) / s, x)
+    out = {}
+    for name, (y, v) in values.items():
+        basis = np.vander(v, CENTRED_DEGREE[name] + 1, increasing=True)
+        c, *_ = np.linalg.lstsq(basis, y, rcond=None)
+        out[name] = (c, float(np.abs(basis @ c - y).max()))
+    return out
+
+
 def horner_source(name: str, coefs) -> str:
     c = [f"{float(v):.9e}f" for v in coefs]
     body = f"  float p = {c[5]};\n"
@@ -60,6 +90,14 @@ def derivative_source(name: str, coefs32) -> str:
     return f"__device__ __forceinline__ float l3_{name}_dx(float x) {{\n{body}}}"
 
 
+def centred_source() -> str:
+    lines = []
+    for name, (c, _) in fit_centred().items():
+        body = ", ".join(f"{float(np.float32(v)):.9e}f" for v in c)
+        lines.append(f"constexpr float kCentred_{name}[{len(c)}] = {{{body}}};")
+    return "\n".join(lines)
+
+
 def main(derivatives: bool = False) -> None:
     for name, center in (("a", 0.5), ("b", 1.5), ("c", 2.5)):
         e, o, err = fit(center)
@@ -75,4 +113,7 @@ def main(derivatives: bool = False) -> None:
 if __name__ == "__main__":
     import sys
 
-    main(derivatives="--derivatives" in sys.argv[1:])
+    if "--centred" in sys.argv[1:]:
+        print(centred_source())
+    else:
+        main(derivatives="--derivatives" in sys.argv[1:])
