@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(256) affine_backward_kernel(AdjointArgs a) {
         atomicAdd(a.grad_src + static_cast<int64_t>(y1) * W + x0, g * ox * ty);
         atomicAdd(a.grad_src + static_cast<int64_t>(y1) * W + x1, g * tx * ty);
       }
-    } else if (float Os, Osx, Osy; lanczos3_value_grad<true>(a.src, W, x0, y0, tx, ty, Os, Osx, Osy)) {
+    } else if (float Os, Osx, Osy; lanczos3_value_grad<true, false, true>(a.src, W, x0, y0, tx, ty, Os, Osx, Osy)) {
       // a window of finite taps: the separable sums with the warp's polynomial
       // weights and their exact derivatives
       gsx = g * Osx;

@@ -279,7 +279,10 @@ __device__ __forceinline__ LanczosAxis lanczos3_axis_centred(const CentredOffset
 // weights cancel (|D| <= 1e-12).
 // UNROLL = true issues all 36 tap loads of the window at once (more loads in
 // flight, more registers); false walks it row by row.
-template <bool UNROLL = false, bool PROBE = false>
+// RELATIVE = true takes the taps relative to the middle one: the derivatives are
+// the same without the rounding that a background of many times its noise
+// leaves in them, and O is the value less that tap.
+template <bool UNROLL = false, bool PROBE = false, bool RELATIVE = false>
 __device__ __forceinline__ bool lanczos3_value_grad(const float* src, int W, int x0, int y0, float tx, float ty,
                                                     float& O, float& Ox, float& Oy) {
   float wx[6], wy[6], dwx[6], dwy[6];
@@ -295,13 +298,16 @@ __device__ __forceinline__ bool lanczos3_value_grad(const float* src, int W, int
   }
   float N = 0.0f, Nx = 0.0f, Ny = 0.0f;
   bool finite = true;
+  float middle = 0.0f;
+  if constexpr (RELATIVE) middle = __ldg(src + static_cast<int64_t>(y0) * W + x0);
 #pragma unroll(UNROLL ? 6 : 1)
   for (int j = 0; j < 6; ++j) {
     const float* row = src + static_cast<int64_t>(y0 - 2 + j) * W + (x0 - 2);
     float r = 0.0f, rx = 0.0f;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      const float v = __ldg(row + i);
+      float v = __ldg(row + i);
+      if constexpr (RELATIVE) v = __fsub_rn(v, middle);
       if constexpr (!PROBE) finite = finite && isfinite(v);
       r = __fmaf_rn(wx[i], v, r);
       rx = __fmaf_rn(dwx[i], v, rx);
