@@ -19,9 +19,10 @@
 //   - each CTA takes 64x64 output tiles; a tile's source footprint (an 80x80
 //     box for the small rotations registration produces) is copied to shared
 //     memory by one cp.async.bulk.tensor (TMA) load while the SM's other CTAs
-//     compute.  Footprints that do not fit the box (large rotation/scale) and
-//     image widths that TMA cannot describe (W % 4 != 0) read the taps straight
-//     from global memory instead;
+//     compute.  Larger rotations take shorter tiles, whose footprints fit the box
+//     again; where none does (scale), and at image widths that TMA cannot describe
+//     (W % 4 != 0), a launch without boxes reads the taps straight from global
+//     memory (WarpForm);
 //   - output goes to a spare slot; the launch's last CTA swaps the frame->slot
 //     table, so nothing is copied back (8 B/pixel instead of 16 B);
 //   - Lanczos3 weights are paired even/odd polynomials in (t - 1/2)^2
@@ -142,9 +143,6 @@ struct TilePlan {
   int grid;  // affine, and small enough for the fixed-point coordinates
 };
 
-// interior: an affine map sends the whole tile at least one pixel inside the
-// valid source range (valid_lo <= s <= valid_hi on both axes), so no pixel
-// of the tile needs its own validity test.
 // Source range of a tile: bounding box of its corners' source points; !ok: a
 // corner has none.
 struct TileRange {
@@ -152,6 +150,9 @@ struct TileRange {
   bool ok;
 };
 
+// interior: an affine map sends the whole tile at least one pixel inside the
+// valid source range (valid_lo <= s <= valid_hi on both axes), so no pixel
+// of the tile needs its own validity test.
 __device__ __forceinline__ TilePlan plan_of_range(const TileRange& s, bool affine, int radius, float valid_lo,
                                                   float valid_hi_x, float valid_hi_y) {
   TilePlan p{0, 0, 0, 0, 0};
@@ -1169,7 +1170,8 @@ static std::vector<WarpItem> warp_items_host(gg_stack* s, const int64_t* indices
     it.form = warp_form(s, it, interp, clamp);
     ++forms.count[it.form];
   }
-  std::stable_sort(items.begin(), items.end(), [](const WarpItem& a, const WarpItem& b) { return a.form < b.form; });
+  if (forms.count[items[0].form] != count)
+    std::stable_sort(items.begin(), items.end(), [](const WarpItem& a, const WarpItem& b) { return a.form < b.form; });
   return items;
 }
 
