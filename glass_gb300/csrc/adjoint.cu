@@ -132,9 +132,8 @@ __device__ __forceinline__ void add_theta(float (&acc)[6], float gsx, float gsy,
 // column: its six cells are summed with the neighbouring lanes' over shuffles,
 // and one atomic per source pixel and strip (and a few along the strip's edge)
 // takes the place of 36 per output pixel.  Any other step writes all six rows.
-// Bound: latency at 12 warps per SM (168 registers), then issue (706
-// instructions per pixel: 166 for the weights and their derivatives, 126 for the
-// taps, 80 for the cells).  4096^2: 658 us, 1102 us with an atomic per tap.
+// Bound: latency at 12 warps per SM (168 registers), then issue (789
+// instructions per pixel).  4096^2: 660 us, 1102 us with an atomic per tap.
 constexpr int kScatterThreads = 128;
 
 // Adds the cells of source row R, columns C .. C + 5 of every lane.

@@ -1431,7 +1431,6 @@ __device__ void load_job_points(const RegArgs& a, const RegJob& job, JobPoints& 
 
 constexpr int kScoreWarps = 4;
 
-// Cand::valid bits: 1 = fit succeeded, 2 = count and rms are exact.
 // Fits one candidate per lane, then the warp counts the pairs of one after the
 // other.  The float64 work is what a warp can do for 32 candidates at once (the
 // fit, the error bounds) and what the float32 test leaves open; residuals in

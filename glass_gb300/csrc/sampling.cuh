@@ -47,7 +47,7 @@ constexpr float kPiF = 3.14159265358979323846f;
 // E_c even and O_c odd, evaluated as degree-5 polynomials in u^2 (fit error
 // below 3e-10, coefficients from glass_gb300/lanczos_poly.py), so the six
 // weights cost 36 FMAs and no transcendental or division.  Each weight is
-// within 1.3e-7 of the exact value (float24 rounding included); callers
+// within 1.3e-7 of the exact value (float32 rounding included); callers
 // that need the exact weights 0, 0, 1, 0, 0, 0 of an integer coordinate
 // (exact integer translations) take the source sample directly.
 // pair A (c = 0.5): max fit error 7.3e-11
