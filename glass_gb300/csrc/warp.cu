@@ -637,9 +637,12 @@ __device__ __forceinline__ unsigned bilinear_rows(const TileGrid& grid, const Wi
     const int xa = RowWalk::whole(at.xa), xb = RowWalk::whole(at.xb);
     const int ya = RowWalk::whole(at.ya), yb = RowWalk::whole(at.yb);
     const auto na = win.template at<MASK>(xa, ya), nb = win.template at<MASK>(xb, yb);
-    // the last column's and row's right and lower neighbours are themselves
-    const int ra = !MASK || xa < win.x1 ? 1 : 0, rb = !MASK || xb < win.x1 ? 1 : 0;
-    const int da = !MASK || ya < win.y1 ? pitch : 0, db = !MASK || yb < win.y1 ? pitch : 0;
+    // the last column's and row's right and lower neighbours are themselves, and so
+    // are those of a position outside (its clamped place may be the last one: a
+    // frame of one row or column has no other)
+    auto step = [](int at_, int first, int last, int by) { return !MASK || (at_ >= first && at_ < last) ? by : 0; };
+    const int ra = step(xa, win.x0, win.x1, 1), rb = step(xb, win.x0, win.x1, 1);
+    const int da = step(ya, win.y0, win.y1, pitch), db = step(yb, win.y0, win.y1, pitch);
     const F2 v00 = f2(win.load(na), win.load(nb)), v01 = f2(win.load(na + ra), win.load(nb + rb));
     const F2 v10 = f2(win.load(na + da), win.load(nb + db));
     const F2 v11 = f2(win.load(na + da + ra), win.load(nb + db + rb));
