@@ -805,7 +805,7 @@ __global__ void __launch_bounds__(T) integrate_smem_kernel(IntegrateArgs a) {
 }
 
 // ---- kernel W: 256 < N <= 512, one warp per pixel ------------------------------
-// (integrate_px.cu has up to 256.)
+// (integrate_px.cuh has up to 256.)
 // A CTA stages a tile of kWarpTilePx consecutive pixels of every frame in
 // shared memory ([frame][pixel], rows padded to kWarpTilePx + 1 floats so a
 // warp reading one pixel's column is bank-conflict free; every frame row is
@@ -1320,7 +1320,7 @@ constexpr int64_t kFusedColumnSamplesLanczos = int64_t(1) << 20;
 constexpr int64_t kFusedColumnSamplesBilinear = int64_t(1) << 22;
 
 // Up to 32 frames: the column kernel (the samples in registers, a thread per
-// pixel) or the tiles of integrate_px.cu, which sum in fewer operations but
+// pixel) or the tiles of integrate_px.cuh, which sum in fewer operations but
 // take their samples through shared memory.  Measured, column against tiles,
 // us for 2048^2 pixels: winsorized 8 frames 210 / 193, 12 347 / 249, 16 376 /
 // 275, 20 753 / 348, 32 809 / 393; sigma clip 12 193 / 224, 16 220 / 229,

@@ -1,4 +1,4 @@
-// Shared pieces of the integration kernels (integrate.cu, integrate_px.cu):
+// Shared pieces of the integration kernels (integrate.cu, integrate_px.cuh):
 // the launch arguments, the sorting network, the output writer and small
 // per-pixel helpers.
 #pragma once
@@ -144,7 +144,7 @@ __device__ __forceinline__ int count_below(const float* S, int T, int cnt, float
 }
 
 // Integration of up to 256 resident frames, one thread per pixel
-// (integrate_px.cu): mean, sigma clip and winsorized sigma clip.
+// (integrate_px.cuh): mean, sigma clip and winsorized sigma clip.
 void launch_integrate_px(const IntegrateArgs& args, cudaStream_t stream);
 
 }  // namespace gg
