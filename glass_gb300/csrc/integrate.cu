@@ -1322,9 +1322,9 @@ constexpr int64_t kFusedColumnSamplesBilinear = int64_t(1) << 22;
 // Up to 32 frames: the column kernel (the samples in registers, a thread per
 // pixel) or the tiles of integrate_px.cuh, which sum in fewer operations but
 // take their samples through shared memory.  Measured, column against tiles,
-// us for 2048^2 pixels: winsorized 8 frames 210 / 193, 12 347 / 249, 16 376 /
-// 275, 20 753 / 348, 32 809 / 393; sigma clip 12 193 / 224, 16 220 / 229,
-// 20 534 / 307, 32 563 / 362; mean 16 87 / 109, 32 162 / 173.  The tiles win in
+// us for 2048^2 pixels: winsorized 8 frames 210 / 193, 12 347 / 226, 16 376 /
+// 247, 20 753 / 297, 32 809 / 371; sigma clip 12 193 / 224, 16 220 / 229,
+// 20 534 / 281, 32 563 / 367; mean 16 87 / 109, 32 162 / 173.  The tiles win in
 // the same places down to 512^2 (32 frames, winsorized: 58 / 35), but stacks in
 // which the fused warp samples through the column kernel keep it, so that
 // both forms of the integration agree to the last bit.
@@ -1587,7 +1587,7 @@ static void ensure_fused_buffers(gg_stack* s) {
 // band buffer (the tiled warp of warp.cu), then the resident integrator runs
 // over the band.  The tiled warp samples from shared memory and plans whole
 // tiles, which the column kernel's per-pixel sampling through L1 cannot: for
-// 32 x 2048 x 2048, Lanczos3, winsorized, 1.3 ms (warp 0.87, integration 0.43)
+// 32 x 2048 x 2048, Lanczos3, winsorized, 1.3 ms (warp 0.87, integration 0.39)
 // against 6.5 ms (a 1.0 ms pass that counted the invalid samples, 5.5 ms).
 static void launch_band_sequence(gg_stack* s, const FusedFrame* d_frames, int interp, float clamp,
                                  const float* d_weights, const gg_integrate_params_t& p) {

@@ -23,12 +23,12 @@
 //
 // Bound: latency at two warps per scheduler (a warp's tile takes 128 B x frames
 // of shared memory), then the min / max pipe (64 lanes per clock and SM; the
-// sort takes 22 per sample of the 63 instructions in all): half of the issue
+// sort takes 22 per sample of the 60 instructions in all): half of the issue
 // slots and of that pipe.  200 frames of 2400 x 1605, winsorized: 7.51 ms with a
-// half-warp per pixel, 2.80 ms here (3.6 ps per sample); 40 frames of 3000 x
-// 2000, sigma clip: 4.36 ms, 0.84 ms; 32 frames of 2048^2, winsorized: 0.81 ms with
-// the column kernel, 0.41 ms here.  Samples around zero take the sums that round:
-// 4.3 ps per sample for 200 frames; weights over three decades 4.2.
+// half-warp per pixel, 2.70 ms here (3.5 ps per sample); 40 frames of 3000 x
+// 2000, sigma clip: 4.36 ms, 0.82 ms; 32 frames of 2048^2, winsorized: 0.81 ms with
+// the column kernel, 0.39 ms here.  Samples around zero take the sums that round:
+// 4.2 ps per sample for 200 frames; weights over three decades 4.0.
 #pragma once
 
 #include <algorithm>
@@ -618,7 +618,7 @@ __global__ void __launch_bounds__(32 * px_max_warps(NB), NB <= 32 ? 5 : NB <= 80
 // and that scheduler's run last.  A warp slows down by about one over the
 // warps beside it, hence warps on the SM over 1 + warps on the busiest
 // scheduler.  (The most warps alone picked two CTAs of five for 160 frames: 4.4
-// ps per sample, 3.5 with one CTA of eight; 112 frames 4.0 and 3.3 with two of
+// ps per sample, 3.4 with one CTA of eight; 112 frames 4.0 and 3.2 with two of
 // seven and three of four.)
 template <int NB, int L, int MODE>
 static int px_best_warps() {
